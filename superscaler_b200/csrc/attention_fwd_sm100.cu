@@ -1,0 +1,527 @@
+// Flash-attention forward for sm_100a: two query tiles per CTA in ping-pong, probabilities kept in tensor memory.
+//
+// Replaces four reference ops and three CUDA extensions at once: ParallelAttentionScoreOp (baddbmm),
+// ParallelSoftmaxFusionOp (scaled [causal|masked] softmax), ParallelSoftmaxDropoutOp and ParallelContextOp (bmm) --
+// runtime/megatron/model/flex_ops.py:711-1015 -- without ever writing the [b, np, sq, sk] score matrix to memory.
+//
+// A work item is 256 queries of one (batch, head): two tiles of 128.  Every tile has its own four softmax warps, one
+// thread per query row, so row maxima and sums need no exchange at all.  Per key block of 128 and tile:
+//   S   = Q . K_j^T       fp32 accumulator in TMEM columns [128 t, 128 t + 128)
+//   softmax warps: S -> registers, running maximum, P = exp2(..) as bf16 -> TMEM columns [128 t + 64, 128 t + 128)
+//   O  += P . V_j         P is the A operand straight from TMEM; accumulator in columns [256 + 128 t, .. + HD)
+// While the tensor core runs O += P V and the next S of one tile, the softmax warps of the other tile work: both units
+// stay busy and P never passes through shared memory.
+// The accumulator O stays in TMEM in the frame of a reference maximum m that may lag behind the true running maximum by
+// up to 8 in the log2 domain (probabilities up to 256, exact in the same relative precision); only when a row exceeds
+// that are O and the row sum rescaled, by the softmax warps themselves.  P, the sums and O are what they were before:
+// bf16 operand, fp32 sums of the unrounded probabilities, fp32 accumulation.
+//
+// The kernel is persistent (one CTA per SM): the loads and the first product of the next item run under the epilogue
+// of the previous one.  Under the causal mask items are numbered heavy (late) query blocks first over all heads and
+// dealt out in snake order: the busiest SM gets 1.01 to 1.09 of the mean for 64 to 256 heads of 2048 tokens, without a
+// counter in memory (grouping heads for the L2 instead left 1.15 to 1.33; K and V at 3 TB/s do not bound the kernel).
+// Without the mask all items cost the same and neighbours share a head.
+//
+// Measured against the one-tile kernel it replaces (128 queries a CTA, P through shared memory, four threads a row): causal,
+// 16 x 16 heads of 2048 x 128: 588 -> 343 us (801 TFLOP/s), with dropout 807 -> 434 us, unmasked 921 -> 529 us (1039 TFLOP/s);
+// one sequence of 16 heads 58 -> 43 us.  What bounds it now is the chain S -> softmax -> P.V of a tile (tensor pipe a third
+// busy, issue slots 43 %); with dropout the integer work of the mask.
+//
+// Warps: 0 = TMA producer, 1 = TMEM allocator + MMA issuer, 2 and 3 idle, 4..7 = softmax of tile 0, 8..11 = of tile 1.
+#include "attention_device.cuh"
+
+namespace ssb {
+
+int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
+                     uint32_t box_rows, uint32_t box_cols);
+
+namespace {
+
+using namespace attn;
+
+constexpr int kFwdThreads = 384;   // three warpgroups: {TMA, MMA, 2 idle}, softmax of tile 0, softmax of tile 1
+// Register split: 384 threads are launched with 168 registers each (64512 in all); the first warpgroup keeps 120 and the
+// two softmax warpgroups take 192: 128 * 120 + 256 * 192 = 64512.
+constexpr int kFwdRegsOther = 120, kFwdRegsSoftmax = 192;
+constexpr float kLazyLog2 = 8.0f;  // how far (log2) the reference maximum may lag before O is rescaled
+
+template <int HD>
+struct FwdCfg {
+  static constexpr int kCh = HD / 64;
+  static constexpr int kTile = 128 * HD * 2;               // Q / K / V tile of 128 rows
+  static constexpr int kStages = HD == 128 ? 4 : 6;        // K and V tiles in flight, in the order K0 V0 K1 V1 ...
+  static constexpr int kOutBytes = 8 * 32 * 128;           // per softmax warp: 32 rows x 64 output columns
+  static constexpr int kBarBytes = 256;
+  static constexpr int kSmem = 2 * kTile + kStages * kTile + kOutBytes + kBarBytes + 1024;
+  static constexpr int kTmemCols = 512;                    // S/P 0, S/P 1, O 0, O 1: 128 columns each
+};
+
+struct FwdItems {
+  int total, n_qb, heads;  // work items, 256-query blocks per head, B * NH
+};
+
+struct FwdItem {
+  int head, b, q0, kv_len, n[2];
+};
+
+__device__ __forceinline__ FwdItem fwd_item(int idx, const FwdItems& it, const AttnParams& p) {
+  FwdItem w;
+  const int outer = idx / (p.causal ? it.heads : it.n_qb), inner = idx - outer * (p.causal ? it.heads : it.n_qb);
+  const int qb = p.causal ? it.n_qb - 1 - outer : inner;
+  const int hh = p.causal ? inner : outer;
+  w.b = hh / p.NH;
+  w.head = hh - w.b * p.NH;
+  w.q0 = qb * 256;
+  w.kv_len = p.kv_lens ? max(0, min(p.kv_lens[w.b], p.SK)) : p.SK;
+  const int n_kv = (w.kv_len + 127) >> 7;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    const int qt = w.q0 + t * 128;
+    w.n[t] = qt >= p.SQ ? 0 : (p.causal ? min(n_kv, (qt >> 7) + 1) : n_kv);
+  }
+  return w;
+}
+
+// Index of this CTA's k-th item, or -1 past the end (odd rounds run backwards through the CTAs).
+__device__ __forceinline__ int fwd_item_index(int k, int total) {
+  const int base = k * static_cast<int>(gridDim.x);
+  if (base >= total) return -1;
+  return base + ((k & 1) ? static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
+}
+
+// Bytes of four keys for this lane's query: lane `sub` of a query quad holds the hash of key `sub` (byte i decides query
+// i); a 4 x 4 byte transpose inside the quad leaves byte e = the byte of key e for this lane's query.
+__device__ __forceinline__ uint32_t quad_transpose(uint32_t h, uint32_t sel1, uint32_t sel2) {
+  const uint32_t r1 = __shfl_xor_sync(0xffffffffu, h, 1);
+  const uint32_t x = __byte_perm(h, r1, sel1);
+  const uint32_t r2 = __shfl_xor_sync(0xffffffffu, x, 2);
+  return __byte_perm(x, r2, sel2);
+}
+
+template <int HD, bool DROPOUT, bool BIAS>
+__global__ void __launch_bounds__(kFwdThreads, 1)
+attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const FwdItems items) {
+  using Cfg = FwdCfg<HD>;
+  constexpr int CH = Cfg::kCh, NS = Cfg::kStages;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sQ = smem;                          // 2 tiles
+  uint8_t* sKV = sQ + 2 * Cfg::kTile;          // NS stages
+  uint8_t* sOut = sKV + NS * Cfg::kTile;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes);
+  uint64_t* q_full = bars;             // 2
+  uint64_t* q_empty = bars + 2;        // 2: the last S of the tile retired
+  uint64_t* s_full = bars + 4;         // 2: S of a block complete (and with it P.V of the block before)
+  uint64_t* p_full = bars + 6;         // 2 (one arrival per softmax warp): P written, O rescaled if need be
+  uint64_t* o_full = bars + 8;         // 2: last P.V of the item complete
+  uint64_t* kv_full = bars + 10;       // NS
+  uint64_t* kv_empty = bars + 10 + NS; // NS
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10 + 2 * NS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int t = 0; t < 2; ++t) {
+      mbar_init(&q_full[t], 1);
+      mbar_init(&q_empty[t], 1);
+      mbar_init(&s_full[t], 1);
+      mbar_init(&p_full[t], 4);
+      mbar_init(&o_full[t], 1);
+    }
+    for (int s = 0; s < NS; ++s) {
+      mbar_init(&kv_full[s], 1);
+      mbar_init(&kv_empty[s], 1);
+    }
+    *abort_flag = 0;
+    fence_mbar_init();
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, Cfg::kTmemCols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < 4) {
+    reg_dealloc<kFwdRegsOther>();  // one instruction for the whole warpgroup
+    // ------------------------------------------ TMA producer ------------------------------------------
+    if (warp == 0 && elect_one()) {
+      Pipe pp;
+      uint32_t qn[2] = {0, 0};  // items loaded per tile
+      bool ok = true;
+      auto load_kv = [&](const CUtensorMap* tm, int col0, int row) {
+        if (!mbar_wait(&kv_empty[pp.stage], pp.phase ^ 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&kv_full[pp.stage], Cfg::kTile);
+#pragma unroll
+        for (int c = 0; c < CH; ++c)
+          tma_load_2d(sKV + pp.stage * Cfg::kTile + c * 16384, tm, &kv_full[pp.stage], col0 + c * 64, row);
+        pp.advance(NS);
+        return true;
+      };
+      for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
+        if (idx >= items.total) continue;
+        const FwdItem w = fwd_item(idx, items, p);
+        const int n = max(w.n[0], w.n[1]);
+        const int kcol = p.k_col0 + w.head * HD, vcol = p.v_col0 + w.head * HD;
+        for (int t = 0; t < 2 && ok && n > 0; ++t) {
+          if (w.n[t] > 0) {
+            if (!mbar_wait(&q_empty[t], (qn[t] & 1) ^ 1, abort_flag)) { ok = false; break; }
+            mbar_arrive_expect_tx(&q_full[t], Cfg::kTile);
+#pragma unroll
+            for (int c = 0; c < CH; ++c)
+              tma_load_2d(sQ + t * Cfg::kTile + c * 16384, &tm_q, &q_full[t], p.q_col0 + w.head * HD + c * 64,
+                          w.b * p.SQ + w.q0 + t * 128);
+            ++qn[t];
+          }
+          if (t == 0) ok = load_kv(&tm_k, kcol, w.b * p.SK);
+        }
+        for (int j = 0; j < n && ok; ++j) {
+          ok = load_kv(&tm_v, vcol, w.b * p.SK + j * 128);
+          if (ok && j + 1 < n) ok = load_kv(&tm_k, kcol, w.b * p.SK + (j + 1) * 128);
+        }
+      }
+      if (!ok) {  // let the copies in flight land before the CTA leaves
+        for (int t = 0; t < 2; ++t)
+          for (uint32_t it = 0; qn[t] > 0 && it < (1u << 20); ++it)
+            if (mbar_try_wait(&q_full[t], (qn[t] - 1) & 1)) break;
+        for (int s = 0; s < NS; ++s) {
+          const uint32_t armed = (s < pp.stage) ? pp.phase : (pp.phase ^ 1);
+          for (uint32_t it = 0; it < (1u << 20); ++it)
+            if (mbar_try_wait(&kv_full[s], armed)) break;
+        }
+      }
+    }
+    // ------------------------------------------ MMA issuer --------------------------------------------
+    if (warp == 1 && elect_one()) {
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);
+      constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, false, true);
+      Pipe pp;                               // next K / V stage to consume
+      uint32_t qn[2] = {0, 0}, pn[2] = {0, 0};
+      bool ok = true;
+      auto issue_s = [&](int t, int stage) {
+        const uint32_t a = smem_u32(sQ + t * Cfg::kTile), bb = smem_u32(sKV + stage * Cfg::kTile);
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk) {
+          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
+          umma_f16_ss(tmem_base + t * 128, umma_desc_sw128(a + off, 16, 1024), umma_desc_sw128(bb + off, 16, 1024),
+                      idesc_s, kk != 0);
+        }
+        umma_commit(&s_full[t]);
+      };
+      for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
+        if (idx >= items.total) continue;
+        const FwdItem w = fwd_item(idx, items, p);
+        const int n = max(w.n[0], w.n[1]);
+        if (n == 0) continue;
+        int sk = pp.stage;
+        if (!mbar_wait(&kv_full[sk], pp.phase, abort_flag)) break;
+        for (int t = 0; t < 2 && ok; ++t) {
+          if (w.n[t] == 0) continue;
+          if (!mbar_wait(&q_full[t], qn[t] & 1, abort_flag)) { ok = false; break; }
+          ++qn[t];
+          tc_fence_after_sync();
+          issue_s(t, sk);
+          if (w.n[t] == 1) umma_commit(&q_empty[t]);
+        }
+        if (!ok) break;
+        umma_commit(&kv_empty[sk]);
+        pp.advance(NS);
+        for (int j = 0; j < n && ok; ++j) {
+          const int sv = pp.stage;
+          const uint32_t phv = pp.phase;
+          pp.advance(NS);
+          sk = pp.stage;
+          bool have_v = false, have_k = false;
+          for (int t = 0; t < 2; ++t) {
+            if (j >= w.n[t]) continue;
+            if (!have_v && !mbar_wait(&kv_full[sv], phv, abort_flag)) { ok = false; break; }
+            have_v = true;
+            if (!mbar_wait(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
+            ++pn[t];
+            tc_fence_after_sync();
+            const uint32_t bb = smem_u32(sKV + sv * Cfg::kTile);
+#pragma unroll
+            for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16 (8 TMEM columns of packed bf16 pairs)
+              umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + 64 + kk * 8,
+                          umma_desc_sw128(bb + kk * 2048, 16384, 1024), idesc_o, (j | kk) != 0);
+            if (j + 1 == w.n[t]) {
+              umma_commit(&o_full[t]);
+            } else {
+              if (!have_k && !mbar_wait(&kv_full[sk], pp.phase, abort_flag)) { ok = false; break; }
+              have_k = true;
+              tc_fence_after_sync();
+              issue_s(t, sk);  // overwrites S / P of the tile: products retire in issue order
+              if (j + 2 == w.n[t]) umma_commit(&q_empty[t]);
+            }
+          }
+          if (!ok) break;
+          umma_commit(&kv_empty[sv]);
+          if (j + 1 < n) {
+            umma_commit(&kv_empty[sk]);
+            pp.advance(NS);
+          }
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------ softmax warps -----------------------------------------
+    reg_alloc<kFwdRegsSoftmax>();
+    const int quarter = warp & 3;
+    const int t = (warp - 4) >> 2;
+    const int r = quarter * 32 + lane;
+    const uint32_t tm_s = tmem_base + t * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t tm_o = tm_s + 256;
+    uint8_t* stage = sOut + (warp - 4) * 4096;
+    const float c = p.scale * kLog2e;
+    // With a bias the logits are brought into the log2 domain first (x c + bias log2 e) and everything below works on
+    // them with a factor of one; without it the raw accumulator is used and the factor is c.
+    const float cc = BIAS ? 1.0f : c;
+    const float lazy_c = fabsf(cc);
+    const uint32_t keep8 = dropout_keep8(p.dropout_p);
+    const float inv_keep = DROPOUT ? 256.0f / static_cast<float>(keep8) : 1.0f;  // applied once, to O
+    const uint32_t qquads = (p.SQ + 3) >> 2;
+    const int sub = lane & 3;
+    const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u, sel2 = (lane & 2) ? 0x3276u : 0x5410u;
+    const uint32_t drop_c = (256u - keep8) * 0x01010101u;  // byte + drop_c carries out <=> byte >= keep8
+    uint32_t sn = 0, on = 0;  // blocks and items of this tile so far
+    bool ok = true;
+    for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
+      if (idx >= items.total) continue;
+      const FwdItem w = fwd_item(idx, items, p);
+      const int qt = w.q0 + t * 128, q = qt + r;
+      if (qt >= p.SQ) continue;
+      const int nt = w.n[t];
+      uint32_t hash_base = 0, hash_step = 0;
+      if constexpr (DROPOUT) {
+        // attn_col_hash mixes (key qquads + quad) * 0x9E3779B1 + seed: linear in the key, so a step of four keys is an add
+        const uint32_t bh_seed = static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(w.b) * p.NH + w.head));
+        hash_base = (static_cast<uint32_t>(sub) * qquads + (static_cast<uint32_t>(q) >> 2)) * 0x9E3779B1u + bh_seed;
+        hash_step = 4u * qquads * 0x9E3779B1u;
+      }
+      const float* bias_row = BIAS ? p.bias_table + static_cast<size_t>(w.head) * (p.SQ + p.SK - 1) + (p.SQ - 1) - min(q, p.SQ - 1)
+                                   : nullptr;
+      float m = -INFINITY, l = 0.f;
+      for (int j = 0; j < nt; ++j) {
+        const int kv0 = j * 128;
+        if (!mbar_wait_warp(&s_full[t], sn & 1, abort_flag)) { ok = false; break; }
+        ++sn;
+        tc_fence_after_sync();
+        // A row does not fit the registers next to everything else: the first half is read for the maximum and again for the exponentials, the second half
+        // stays.  P goes over the columns of the second half, so the first half is intact when it is read again.
+        const bool masked = (p.causal && kv0 + 127 > qt) || kv0 + 128 > w.kv_len;  // diagonal block or ragged end
+        const int lim = min(w.kv_len - 1, p.causal ? q : w.kv_len) - kv0;          // last visible key of this row
+        auto prepare = [&](uint32_t (&x)[32], int k0) {
+          if constexpr (BIAS) {
+            const float* br = bias_row + kv0 + k0;
+            if (kv0 + 128 <= p.SK) {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                x[i] = __float_as_uint(fmaf(__uint_as_float(x[i]), c, __ldg(br + i) * kLog2e));
+            } else {
+#pragma unroll
+              for (int i = 0; i < 32; ++i)
+                x[i] = __float_as_uint(fmaf(__uint_as_float(x[i]), c, __ldg(bias_row + min(kv0 + k0 + i, p.SK - 1)) * kLog2e));
+            }
+          }
+          if (masked) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+              if (k0 + i > lim) x[i] = 0xff800000u;  // -inf
+          }
+        };
+        auto row_max = [&](const uint32_t (&x)[32], const uint32_t (&y)[32], float start) {  // four independent chains
+          float mm[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            mm[e] = fmaxf(__uint_as_float(x[e]), __uint_as_float(y[e]));
+#pragma unroll
+            for (int i = 4; i < 32; i += 4) mm[e] = fmaxf(mm[e], fmaxf(__uint_as_float(x[e + i]), __uint_as_float(y[e + i])));
+          }
+          return fmaxf(fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])), start);
+        };
+        float mx;
+        uint32_t x0[32], x1[32], x2[32], x3[32];
+        tmem_ld_32x32(tm_s, x0);
+        tmem_ld_32x32(tm_s + 32, x1);
+        tmem_ld_wait();
+        prepare(x0, 0);
+        prepare(x1, 32);
+        mx = row_max(x0, x1, -INFINITY);
+        tmem_ld_32x32(tm_s + 64, x2);
+        tmem_ld_32x32(tm_s + 96, x3);
+        tmem_ld_wait();
+        prepare(x2, 64);
+        prepare(x3, 96);
+        mx = row_max(x2, x3, mx);
+        if (j == 0) {
+          m = mx;
+        } else {
+          // m = -inf: no visible key so far; the row takes the new maximum (its O and l are zero)
+          const bool lag = mx > m && ((mx - m) * lazy_c > kLazyLog2 || m == -INFINITY);
+          if (__any_sync(0xffffffffu, lag)) {
+            const float mn = fmaxf(m, mx);
+            const float alpha = mn == -INFINITY ? 1.f : ex2((m - mn) * cc);
+            l *= alpha;
+            m = mn;
+            // P.V of the block before completed with s_full (products retire in issue order)
+#pragma unroll
+            for (int ch = 0; ch < HD / 32; ++ch) {
+              uint32_t oo[32];
+              tmem_ld_32x32(tm_o + ch * 32, oo);
+              tmem_ld_wait();
+#pragma unroll
+              for (int i = 0; i < 32; ++i) oo[i] = __float_as_uint(__uint_as_float(oo[i]) * alpha);
+              tmem_st_32x32(tm_o + ch * 32, oo);
+            }
+          }
+        }
+        const float mc = (m == -INFINITY) ? 0.f : m * cc;  // no visible key: keep the exponents finite
+        float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        const float2 c2 = make_float2(cc, cc), nm2 = make_float2(-mc, -mc);
+        auto exponentials = [&](const uint32_t (&x)[32], int ch) {
+          uint32_t pw[16];
+          uint32_t hash = hash_base + static_cast<uint32_t>(ch * 8) * hash_step;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            float2 a = fma_f32x2(make_float2(__uint_as_float(x[i]), __uint_as_float(x[i + 1])), c2, nm2);
+            float2 b2 = fma_f32x2(make_float2(__uint_as_float(x[i + 2]), __uint_as_float(x[i + 3])), c2, nm2);
+            a.x = ex2(a.x);  // masked entries: ex2(-inf) = 0
+            a.y = ex2(a.y);
+            b2.x = ex2(b2.x);
+            b2.y = ex2(b2.y);
+            rs[0] = add_f32x2(rs[0], a);
+            rs[1] = add_f32x2(rs[1], b2);
+            uint32_t w0 = pack_bf16x2(a.x, a.y), w1 = pack_bf16x2(b2.x, b2.y);
+            if constexpr (DROPOUT) {
+              const uint32_t xb = quad_transpose(fmix32(hash), sel1, sel2);
+              hash += hash_step;
+              const uint32_t cs = (xb & 0x7f7f7f7fu) + (drop_c & 0x7f7f7f7fu);
+              const uint32_t d = (xb & drop_c) | ((xb | drop_c) & cs);  // bit 7 of byte e: carry out of that byte
+              w0 &= ~spread_sign_bytes(d, 0x9988);                        // sign bits of bytes 0, 1 spread over a half each
+              w1 &= ~spread_sign_bytes(d, 0xBBAA);
+            }
+            pw[i >> 1] = w0;
+            pw[(i >> 1) + 1] = w1;
+          }
+          tmem_st_32x16(tm_s + 64 + ch * 16, pw);
+        };
+        exponentials(x2, 2);
+        tmem_ld_32x32(tm_s, x0);
+        exponentials(x3, 3);
+        tmem_ld_wait();
+        tmem_ld_32x32(tm_s + 32, x1);
+        prepare(x0, 0);
+        exponentials(x0, 0);
+        tmem_ld_wait();
+        prepare(x1, 32);
+        exponentials(x1, 1);
+        hash_base += 32u * hash_step;
+        tmem_st_wait();
+        tc_fence_before_sync();
+        warp_arrive(&p_full[t], lane);
+        l += (rs[0].x + rs[0].y) + (rs[1].x + rs[1].y);
+      }
+      if (!ok) break;
+      if (nt > 0) {
+        if (!mbar_wait_warp(&o_full[t], on & 1, abort_flag)) { ok = false; break; }
+        ++on;
+        tc_fence_after_sync();
+      }
+      const float inv_l = l > 0.f ? inv_keep / l : 0.f;
+      __nv_bfloat16* obase = reinterpret_cast<__nv_bfloat16*>(p.O) + (static_cast<size_t>(w.b) * p.SQ + qt + quarter * 32) * p.ldo +
+                             p.o_col0 + w.head * HD + (lane & 7) * 8;
+      const int rows_left = p.SQ - qt - quarter * 32;
+#pragma unroll
+      for (int ch = 0; ch < CH; ++ch) {  // 64 columns at a time through shared memory: 128-byte row segments to memory
+        uint32_t oo[64];
+        if (nt > 0) {
+          tmem_ld_32x32(tm_o + ch * 64, *reinterpret_cast<uint32_t(*)[32]>(&oo[0]));
+          tmem_ld_32x32(tm_o + ch * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&oo[32]));
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) oo[i] = 0u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint4 v;
+          v.x = pack_bf16x2(__uint_as_float(oo[8 * i + 0]) * inv_l, __uint_as_float(oo[8 * i + 1]) * inv_l);
+          v.y = pack_bf16x2(__uint_as_float(oo[8 * i + 2]) * inv_l, __uint_as_float(oo[8 * i + 3]) * inv_l);
+          v.z = pack_bf16x2(__uint_as_float(oo[8 * i + 4]) * inv_l, __uint_as_float(oo[8 * i + 5]) * inv_l);
+          v.w = pack_bf16x2(__uint_as_float(oo[8 * i + 6]) * inv_l, __uint_as_float(oo[8 * i + 7]) * inv_l);
+          *reinterpret_cast<uint4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = v;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int row = i * 4 + (lane >> 3);
+          const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+          if (row < rows_left) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row) * p.ldo + ch * 64) = v;
+        }
+        __syncwarp();
+      }
+      // rows with no visible key get +inf so that the backward probabilities exp(s - lse) vanish
+      if (q < p.SQ)
+        p.LSE[(static_cast<size_t>(w.b) * p.NH + w.head) * p.SQ + q] =
+            l > 0.f ? m * (BIAS ? 1.0f / kLog2e : p.scale) + logf(l) : INFINITY;
+      // the reads of O are ordered before the next item's P.V by the p_full arrival of its first block
+      tc_fence_before_sync();
+    }
+  }
+
+  tc_fence_before_sync();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag && p.status != nullptr) atomicMax(p.status, static_cast<int>(kStatusMbarTimeout));
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_base, Cfg::kTmemCols);
+  }
+}
+
+template <int HD, bool DROPOUT, bool BIAS>
+int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, int num_sms,
+               cudaStream_t stream) {
+  const int rc = static_cast<int>(cudaFuncSetAttribute(attn_fwd_kernel<HD, DROPOUT, BIAS>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<HD>::kSmem));
+  if (rc) return rc;
+  FwdItems it;
+  it.n_qb = (p.SQ + 255) / 256;
+  it.heads = p.B * p.NH;
+  it.total = it.n_qb * it.heads;
+  const int grid = it.total < num_sms ? it.total : num_sms;
+  attn_fwd_kernel<HD, DROPOUT, BIAS><<<grid, kFwdThreads, FwdCfg<HD>::kSmem, stream>>>(tq, tk, tv, p, it);
+  return static_cast<int>(cudaGetLastError());
+}
+
+}  // namespace
+
+// q/k/v: base pointers of the 2-D matrices that hold the heads (see AttnParams); ld in elements.
+int attn_fwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const AttnParams& p,
+                    int num_sms, cudaStream_t stream) {
+  if (p.HD != 64 && p.HD != 128) return -2;
+  if (p.causal && p.SQ != p.SK) return -2;
+  if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (p.ldo % 8) || (p.q_col0 % 8) || (p.k_col0 % 8) || (p.v_col0 % 8) ||
+      (p.o_col0 % 8))
+    return -3;
+  CUtensorMap tq, tk, tv;
+  int rc;
+  if ((rc = make_tma_2d_bf16(&tq, q, static_cast<uint64_t>(p.B) * p.SQ, ldq, ldq, 128, 64))) return rc;
+  if ((rc = make_tma_2d_bf16(&tk, k, static_cast<uint64_t>(p.B) * p.SK, ldk, ldk, 128, 64))) return rc;
+  if ((rc = make_tma_2d_bf16(&tv, v, static_cast<uint64_t>(p.B) * p.SK, ldv, ldv, 128, 64))) return rc;
+  const bool drop = p.dropout_p > 0.f, bias = p.bias_table != nullptr;
+#define SSB_FWD(HD, D, BI) launch_fwd<HD, D, BI>(tq, tk, tv, p, num_sms, stream)
+  if (p.HD == 128)
+    return drop ? (bias ? SSB_FWD(128, true, true) : SSB_FWD(128, true, false))
+                : (bias ? SSB_FWD(128, false, true) : SSB_FWD(128, false, false));
+  return drop ? (bias ? SSB_FWD(64, true, true) : SSB_FWD(64, true, false))
+              : (bias ? SSB_FWD(64, false, true) : SSB_FWD(64, false, false));
+#undef SSB_FWD
+}
+
+}  // namespace ssb

@@ -56,7 +56,7 @@ int ce_finalize_launch(void* logits, int ld, const long long* targets, const flo
                        const float* gtgt, const float* loss_mask, float* loss, long long rows, int V, long long v0,
                        float grad_scale, int write_grad, cudaStream_t stream);
 int attn_fwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const AttnParams& p,
-                    cudaStream_t stream);
+                    int num_sms, cudaStream_t stream);
 int attn_bwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const void* dout,
                     int lddo, const AttnParams& p, float* delta_scratch, cudaStream_t stream);
 long long attn_bwd_fused_scratch_floats(int B, int NH, int SQ, int HD);
@@ -452,7 +452,7 @@ std::vector<Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, 
     p.bias_table = bias_table->data_ptr<float>();
   }
   check_launch(ssb::attn_fwd_launch(q.data_ptr(), static_cast<int>(q.stride(0)), k.data_ptr(), static_cast<int>(k.stride(0)),
-                                    v.data_ptr(), static_cast<int>(v.stride(0)), p, cur_stream()),
+                                    v.data_ptr(), static_cast<int>(v.stride(0)), p, num_sms(), cur_stream()),
                "attn_fwd");
   return {o, lse};
 }
