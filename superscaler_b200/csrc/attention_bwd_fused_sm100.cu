@@ -6,87 +6,96 @@
 // (runtime/megatron/model/flex_ops.py:711-1015) together with the softmax backward kernels of the reference
 // (runtime/megatron/fused_kernels/scaled_masked_softmax.h:329-423).
 //
-// A CTA owns 128 keys of one (batch, head) and walks over the query blocks (64 queries each) that see them:
-//   S^T  = K . Q_i^T          [128 keys x 64 queries]     TMEM columns [0, 64)
-//   dP^T = V . dO_i^T         [128 keys x 64 queries]     TMEM columns [64, 128)
-//   math : P^T = exp2(S^T c - lse2) (x dropout mask), dS^T = P^T (dP^T mask - delta), written to shared memory as bf16
-//          tiles; the softmax scale is applied once, to dK and dQ, at the end
-//   dV  += P^T  . dO_i        [128 keys x HD]             TMEM columns [256, 256 + HD)
-//   dK  += dS^T . Q_i         [128 keys x HD]             TMEM columns [384, 384 + HD)
-//   dQ   = dS . K             [128 queries x HD]          TMEM columns [128, 128 + HD), once per PAIR of query blocks
-// The dS^T tiles of two consecutive query blocks sit side by side in shared memory as the two 64-column chunks of
-// one [128 keys][128 queries] tile; read MN-major, that tile is the A operand dS of the dQ product with M = 128, so
-// the dQ product runs at the full tile width.  Its result is one key block's share of dQ.  Four drain warps (one per
-// TMEM lane quarter) copy it to shared memory and add it to an fp32 accumulator [batch, head, 128-query tile][128][HD]
-// in global memory with bulk tensor reductions (cp.reduce.async.bulk.tensor ... add): the additions run in the L2 and
-// leave the load/store units of the SM to the math warps.  A small kernel scales the accumulator and writes the bf16
-// dQ matrix afterwards.  The order in which the key blocks add their shares is not fixed, so dQ can differ in the
-// last bit from run to run; the two-kernel backward stays available for bitwise-reproducible runs.
+// A CTA owns 128 keys of one (batch, head) and walks over the query blocks (128 queries each) that see them:
+//   S^T  = K . Q_i^T          [128 keys x 128 queries]    TMEM columns [0, 128)
+//   P^T  = exp2(S^T c - lse2) (x dropout mask)            bf16, over the columns of S^T the same warpgroup has read
+//   dP^T = V . dO_i^T         [128 keys x 128 queries]    TMEM columns [128, 256)
+//   dV  += P^T  . dO_i        [128 keys x HD]             A operand straight from TMEM
+//   dS^T = P^T (dP^T mask - delta)                        bf16, shared memory
+//   dQ   = dS . K             [128 queries x HD]          same tile read MN-major; over dP^T (HD 128), own columns (HD 64)
+//   dK  += dS^T . Q_i         [128 keys x HD]
+// The softmax scale is applied once, to dK and dQ, and the dropout scale of P once, to dV, at the end.
 //
-// Order of the tensor-core work (one issuing thread; products retire in issue order).  While the math warps work on
-// block i, the issuing thread queues: dV of block i - 1 (frees the single P^T buffer early), then S^T / dP^T of block
-// i + 1 (the math warps have copied block i into registers and released the TMEM buffers: sdp_free), then dQ of the
-// pair that block i - 1 completed and dK of block i - 1.  So the next block's scores are never queued behind more
-// than four small products, and everything the math warps wait for was issued a whole block earlier.
+// dQ is one key block's share: four drain warps read it from TMEM and add it to an fp32 accumulator in global memory
+// with 16-byte vector reductions.  The accumulator is laid out [tile][lane quarter][HD / 4][32 lanes][4], so that one
+// instruction of a warp covers 512 contiguous bytes, and nothing passes through shared memory, whose bandwidth bounds
+// this kernel (a 128 x 128 x 16 product with both operands in shared memory alone needs 128 bytes per clock, all there
+// is).  A small kernel scales the accumulator and writes the bf16 dQ matrix afterwards.  The order in which the key
+// blocks add their shares is not fixed, so dQ can differ in the last bit from run to run; the two-kernel backward stays
+// available for bitwise-reproducible runs.
+//
+// Order of the tensor-core work (one issuing thread; products retire in issue order), step i:
+//   dV_i (needs P_i) | S_{i+1} | dQ_i, dK_i (need dS_i) | dP_{i+1} (needs dQ_i drained at HD 128)
+// The math warps turn S_{i+1} into P_{i+1} while dQ_i, dK_i and dP_{i+1} run, and dP_{i+1} into dS_{i+1} while dV_{i+1}
+// and S_{i+2} run.
+//
+// Threads: warpgroup 0 = {TMA warp, MMA warp, two idle}, 1 .. 4 = math (warpgroup 1 + g: queries [32 g, 32 g + 32) of a block,
+// one key row per thread), 5 = drain.  The math of a step is a chain of waits and dependent arithmetic: with two warpgroups
+// of twice the columns (two warps per SM sub-partition) it, and not the tensor core, set the pace.
+//
+// Measured against the kernel it replaces (query blocks of 64, dQ through shared memory and bulk reductions), 16 x 16 heads of
+// 2048 x 128, whole backward: causal with dropout 1458 -> 1127 us (1181 with eight math warps), without 1377 -> 1065,
+// unmasked 2234 -> 1698; 32 x 16 heads of 512 x 64 with bias and dropout 613 -> 363 (490 with the diagonal sums as one
+// dependent chain of shuffles).  What bounds it at head size 128: the 64 KB of dQ a step that leave the SM (a copy of the
+// kernel without the reductions takes 1364 us unmasked, with plain stores in their place 1670).
 #include "attention_device.cuh"
 
 namespace ssb {
 
 int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                      uint32_t box_rows, uint32_t box_cols);
-int make_tma_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows);
 
 namespace {
 
 using namespace attn;
 
-constexpr int kDrainWarps = 4;  // one per TMEM lane quarter
-constexpr int kFusedThreads = kAttnThreads + 32 * kDrainWarps;
+constexpr int kFusedThreads = 768;
+constexpr int kFusedMathWarps = 16;
+// Register split of the 768 x 80 registers the block is launched with: 128 (56 + 4 * 80 + 104) = 61440.
+constexpr int kFusedRegsIssue = 56, kFusedRegsMath = 80, kFusedRegsDrain = 104;
 
 template <int HD>
 struct FusedCfg {
   static constexpr int kCh = HD / 64;
-  static constexpr int kKvTile = 128 * HD * 2;   // K_j / V_j, resident
-  static constexpr int kQStages = 3;
-  static constexpr int kQTile = 64 * HD * 2;     // Q_i / dO_i, kQStages stages each
-  static constexpr int kPBytes = 128 * 64 * 2;   // P^T (one buffer), dS^T (two chunks = one pair tile)
-  static constexpr int kStageBytes = 32 * 128;   // per drain warp: 32 rows x 32 floats, swizzled like a TMA tile
-  static constexpr int kSmem = 2 * kKvTile + 2 * kQStages * kQTile + 3 * kPBytes + kDrainWarps * kStageBytes + 1024 + 256;
+  static constexpr int kTile = 128 * HD * 2;      // K_j / V_j (resident), Q_i / dO_i (two stages each)
+  static constexpr int kDsBytes = 128 * 128 * 2;  // dS^T: two chunks of 64 queries
+  static constexpr int kStatBytes = 2 * 128 * 4;  // -lse2 and -delta of a query block, per Q stage
+  static constexpr int kBarBytes = 256;
+  static constexpr int kSmem = 6 * kTile + kDsBytes + 2 * kStatBytes + kBarBytes;
   static constexpr int kTmemCols = 512;
-  static constexpr int kColS = 0, kColDP = 64, kColDQ = 128, kColDV = 256, kColDK = 384;
+  static constexpr int kColS = 0, kColDP = 128, kColDV = 256;
+  static constexpr int kColDK = HD == 128 ? 384 : 320, kColDQ = HD == 128 ? kColDP : 384;
 };
 
 template <int HD, bool DROPOUT, bool BIAS>
 __global__ void __launch_bounds__(kFusedThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                      const __grid_constant__ CUtensorMap tm_acc, const AttnParams p) {
+                      float* __restrict__ dq_acc, const AttnParams p) {
   using Cfg = FusedCfg<HD>;
   constexpr int CH = Cfg::kCh;
-  constexpr int QS = Cfg::kQStages;
-  constexpr int OC = HD / 4;  // accumulator columns per math group
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
-  uint8_t* sV = sK + Cfg::kKvTile;
-  uint8_t* sQ = sV + Cfg::kKvTile;       // QS stages
-  uint8_t* sdO = sQ + QS * Cfg::kQTile;  // QS stages
-  uint8_t* sPt = sdO + QS * Cfg::kQTile;
-  uint8_t* sdSt = sPt + Cfg::kPBytes;    // two chunks: query block parity
-  uint8_t* sStage = sdSt + 2 * Cfg::kPBytes;  // kDrainWarps x 4 KB
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + kDrainWarps * Cfg::kStageBytes);
-  uint64_t* kv_full = bars;          // 1
-  uint64_t* qdo_full = bars + 1;     // 3
-  uint64_t* qdo_empty = bars + 4;    // 3: dK of that stage's block retired (the last reader of Q_i, dO_i)
-  uint64_t* s_full = bars + 7;       // 1
-  uint64_t* sdp_free = bars + 8;     // 1 (one arrival per math warp): S^T / dP^T copied to registers
-  uint64_t* p_full = bars + 9;       // 1 (one arrival per math warp)
-  uint64_t* pv_done = bars + 10;     // 1: dV of a block retired (P^T free)
-  uint64_t* dk_done = bars + 11;     // 2 (block parity): dK of a block retired (that dS^T chunk free of dK)
-  uint64_t* dq_done = bars + 13;     // 1: dQ of a pair retired (both dS^T chunks free of dQ; accumulator ready)
-  uint64_t* dq_empty = bars + 14;    // 1 (one arrival per drain warp): dQ accumulator copied out
-  uint64_t* acc_full = bars + 15;    // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+  uint8_t* sV = sK + Cfg::kTile;
+  uint8_t* sQ = sV + Cfg::kTile;        // 2 stages
+  uint8_t* sdO = sQ + 2 * Cfg::kTile;   // 2 stages
+  uint8_t* sdS = sdO + 2 * Cfg::kTile;
+  float* sStat = reinterpret_cast<float*>(sdS + Cfg::kDsBytes);  // [2 stages][nlse2: 128, nd: 128]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(sStat) + 2 * Cfg::kStatBytes);
+  uint64_t* k_full = bars;           // 1
+  uint64_t* v_full = bars + 1;       // 1
+  uint64_t* q_full = bars + 2;       // 2 (with the statistics of the block)
+  uint64_t* q_empty = bars + 4;      // 2: dK of the block retired, which follows every other reader of the stage
+  uint64_t* do_full = bars + 6;      // 2
+  uint64_t* do_empty = bars + 8;     // 2: dV of the block retired
+  uint64_t* s_full = bars + 10;      // 1
+  uint64_t* p_full = bars + 11;      // 1 (one arrival per math warp): P^T in TMEM
+  uint64_t* dp_full = bars + 12;     // 1 (also: dQ and dK of the block before retired, dS^T free)
+  uint64_t* ds_full = bars + 13;     // 1 (one arrival per math warp): dS^T in shared memory, dP^T read
+  uint64_t* dq_full = bars + 14;     // 1
+  uint64_t* dq_empty = bars + 15;    // 1 (one arrival per drain warp): dQ read from TMEM
+  uint64_t* acc_full = bars + 16;    // 1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -94,25 +103,26 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   const int head = blockIdx.y, b = blockIdx.z;
   const int kv0 = jb * 128;
   const int kv_len = p.kv_lens ? min(p.kv_lens[b], p.SK) : p.SK;
-  const int nq = (p.SQ + 63) / 64;
-  const int i0 = p.causal ? (kv0 / 64) : 0;  // even: kv0 is a multiple of 128
-  const int n_it = (kv0 < kv_len && nq > i0) ? nq - i0 : 0;
   const int n_tiles = (p.SQ + 127) / 128;
+  const int i0 = p.causal ? jb : 0;
+  const int n_it = (kv0 < kv_len && n_tiles > i0) ? n_tiles - i0 : 0;
+  const size_t tile0 = (static_cast<size_t>(b) * p.NH + head) * n_tiles + i0;  // first query block of the walk
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int s = 0; s < QS; ++s) {
-      mbar_init(&qdo_full[s], 1);
-      mbar_init(&qdo_empty[s], 1);
+    mbar_init(k_full, 1);
+    mbar_init(v_full, 1);
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&q_full[s], 1);
+      mbar_init(&q_empty[s], 1);
+      mbar_init(&do_full[s], 1);
+      mbar_init(&do_empty[s], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(sdp_free, kMathWarps);
-    mbar_init(p_full, kMathWarps);
-    mbar_init(pv_done, 1);
-    mbar_init(&dk_done[0], 1);
-    mbar_init(&dk_done[1], 1);
-    mbar_init(dq_done, 1);
-    mbar_init(dq_empty, kDrainWarps);
+    mbar_init(p_full, kFusedMathWarps);
+    mbar_init(dp_full, 1);
+    mbar_init(ds_full, kFusedMathWarps);
+    mbar_init(dq_full, 1);
+    mbar_init(dq_empty, 4);
     mbar_init(acc_full, 1);
     *abort_flag = 0;
     fence_mbar_init();
@@ -120,7 +130,6 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
     tma_prefetch_desc(&tm_do);
-    tma_prefetch_desc(&tm_acc);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, Cfg::kTmemCols);
@@ -130,323 +139,349 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_dq = tmem_base + Cfg::kColDQ, tmem_dv = tmem_base + Cfg::kColDV, tmem_dk = tmem_base + Cfg::kColDK;
+  const uint32_t tmem_s = tmem_base + Cfg::kColS, tmem_dp = tmem_base + Cfg::kColDP, tmem_dq = tmem_base + Cfg::kColDQ;
+  const uint32_t tmem_dv = tmem_base + Cfg::kColDV, tmem_dk = tmem_base + Cfg::kColDK;
 
-  if (warp == 0) {
-    // ------------------------------------------ TMA producer ------------------------------------------
-    if (elect_one() && n_it > 0) {
-      mbar_arrive_expect_tx(kv_full, 2 * Cfg::kKvTile);
+  if (warp < 4) {
+    reg_dealloc<kFusedRegsIssue>();
+    if (warp == 0 && elect_one() && n_it > 0) {
+      // ---------------------------------------- TMA producer ----------------------------------------
+      const int qrow0 = b * p.SQ + i0 * 128;
+      auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
 #pragma unroll
-      for (int c = 0; c < CH; ++c) {
-        tma_load_2d(sK + c * 16384, &tm_k, kv_full, p.k_col0 + head * HD + c * 64, b * p.SK + kv0);
-        tma_load_2d(sV + c * 16384, &tm_v, kv_full, p.v_col0 + head * HD + c * 64, b * p.SK + kv0);
-      }
-      Pipe pp;
-      bool ok = true;
-      for (int it = 0; it < n_it && ok; ++it) {
-        if (!mbar_wait(&qdo_empty[pp.stage], pp.phase ^ 1, abort_flag)) { ok = false; break; }
-        mbar_arrive_expect_tx(&qdo_full[pp.stage], 2 * Cfg::kQTile);
-        const int row = b * p.SQ + (i0 + it) * 64;
-#pragma unroll
-        for (int c = 0; c < CH; ++c) {
-          tma_load_2d(sQ + pp.stage * Cfg::kQTile + c * 8192, &tm_q, &qdo_full[pp.stage],
-                      p.q_col0 + head * HD + c * 64, row);
-          tma_load_2d(sdO + pp.stage * Cfg::kQTile + c * 8192, &tm_do, &qdo_full[pp.stage],
-                      p.o_col0 + head * HD + c * 64, row);
-        }
-        pp.advance(QS);
+        for (int c = 0; c < CH; ++c) tma_load_2d(dst + c * 16384, tm, bar, col + c * 64, row);
+      };
+      auto load_q = [&](int i) {
+        const int st = i & 1;
+        if (!mbar_wait(&q_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&q_full[st], Cfg::kTile + Cfg::kStatBytes);
+        load_tile(sQ + st * Cfg::kTile, &tm_q, &q_full[st], p.q_col0 + head * HD, qrow0 + i * 128);
+        bulk_load(sStat + st * 256, p.LSE + (tile0 + i) * 128, 512, &q_full[st]);
+        bulk_load(sStat + st * 256 + 128, p.delta + (tile0 + i) * 128, 512, &q_full[st]);
+        return true;
+      };
+      auto load_do = [&](int i) {
+        const int st = i & 1;
+        if (!mbar_wait(&do_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) return false;
+        mbar_arrive_expect_tx(&do_full[st], Cfg::kTile);
+        load_tile(sdO + st * Cfg::kTile, &tm_do, &do_full[st], p.o_col0 + head * HD, qrow0 + i * 128);
+        return true;
+      };
+      mbar_arrive_expect_tx(k_full, Cfg::kTile);
+      load_tile(sK, &tm_k, k_full, p.k_col0 + head * HD, b * p.SK + kv0);
+      int nq = 0, ndo = 0;  // loads issued
+      bool ok = load_q(0);
+      nq += ok;
+      mbar_arrive_expect_tx(v_full, Cfg::kTile);
+      load_tile(sV, &tm_v, v_full, p.v_col0 + head * HD, b * p.SK + kv0);
+      if (ok) ok = load_do(0);
+      ndo += ok;
+      for (int i = 1; i < n_it && ok; ++i) {
+        ok = load_q(i);
+        nq += ok;
+        if (ok) ok = load_do(i);
+        ndo += ok;
       }
       if (!ok) {  // let the copies in flight land before the CTA leaves
-        for (uint32_t it = 0; it < (1u << 20); ++it)
-          if (mbar_try_wait(kv_full, 0)) break;
-        for (int s = 0; s < QS; ++s) {
-          const uint32_t armed = (s < pp.stage) ? pp.phase : (pp.phase ^ 1);
+        auto settle = [&](uint64_t* bar, uint32_t parity) {
           for (uint32_t it = 0; it < (1u << 20); ++it)
-            if (mbar_try_wait(&qdo_full[s], armed)) break;
-        }
+            if (mbar_try_wait(bar, parity)) break;
+        };
+        settle(k_full, 0);
+        settle(v_full, 0);
+        for (int i = max(nq - 2, 0); i < nq; ++i) settle(&q_full[i & 1], (i >> 1) & 1);
+        for (int i = max(ndo - 2, 0); i < ndo; ++i) settle(&do_full[i & 1], (i >> 1) & 1);
       }
     }
-  } else if (warp == 1) {
-    // ------------------------------------------ MMA issuer --------------------------------------------
-    if (elect_one() && n_it > 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64, false, false);   // [keys x queries], reduce over HD
+    if (warp == 1 && elect_one() && n_it > 0) {
+      // ---------------------------------------- MMA issuer ------------------------------------------
+      constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);  // [keys x queries], reduce over HD
       constexpr uint32_t idesc_acc = umma_idesc_bf16(128, HD, false, true);  // [keys x HD], reduce over queries
       constexpr uint32_t idesc_dq = umma_idesc_bf16(128, HD, true, true);    // [queries x HD], reduce over keys
-      bool ok = mbar_wait(kv_full, 0, abort_flag);
-      const uint32_t k = smem_u32(sK), v = smem_u32(sV);
-      const uint32_t pt = smem_u32(sPt), dst = smem_u32(sdSt);
-      auto issue_sdp = [&](int it) {
-        const int qs = it % QS;
-        const uint32_t qq = smem_u32(sQ + qs * Cfg::kQTile), dd = smem_u32(sdO + qs * Cfg::kQTile);
+      // One descriptor per operand and orientation; a step along the operand is an addition to its address field.
+      const uint64_t k_k = umma_desc_sw128(smem_u32(sK), 16, 1024), k_mn = umma_desc_sw128(smem_u32(sK), 16384, 1024);
+      const uint64_t v_k = umma_desc_sw128(smem_u32(sV), 16, 1024);
+      const uint64_t ds_k = umma_desc_sw128(smem_u32(sdS), 16, 1024), ds_mn = umma_desc_sw128(smem_u32(sdS), 16384, 1024);
+      const uint64_t q_k = umma_desc_sw128(smem_u32(sQ), 16, 1024), q_mn = umma_desc_sw128(smem_u32(sQ), 16384, 1024);
+      const uint64_t do_k = umma_desc_sw128(smem_u32(sdO), 16, 1024), do_mn = umma_desc_sw128(smem_u32(sdO), 16384, 1024);
+      constexpr uint64_t kStage = Cfg::kTile >> 4;  // descriptor distance of the two Q / dO stages
+      auto product = [&](uint32_t d, uint64_t a, uint64_t bb) {  // [128 x 128] = A . B^T over HD, both K-major
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;
-          const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;
-          umma_f16_ss(tmem_base + Cfg::kColS, umma_desc_sw128(k + offa, 16, 1024), umma_desc_sw128(qq + offb, 16, 1024),
-                      idesc_s, kk != 0);
+          const uint64_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+          umma_f16_ss(d, a + off, bb + off, idesc_s, kk != 0);
         }
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t offa = (kk >> 2) * 16384 + (kk & 3) * 32;
-          const uint32_t offb = (kk >> 2) * 8192 + (kk & 3) * 32;
-          umma_f16_ss(tmem_base + Cfg::kColDP, umma_desc_sw128(v + offa, 16, 1024),
-                      umma_desc_sw128(dd + offb, 16, 1024), idesc_s, kk != 0);
-        }
-        umma_commit(s_full);
       };
-      if (ok) ok = mbar_wait(&qdo_full[0], 0, abort_flag);
+      bool ok = mbar_wait(k_full, 0, abort_flag) && mbar_wait(&q_full[0], 0, abort_flag);
       if (ok) {
         tc_fence_after_sync();
-        issue_sdp(0);
+        product(tmem_s, k_k, q_k);
+        umma_commit(s_full);
+        ok = mbar_wait(v_full, 0, abort_flag) && mbar_wait(&do_full[0], 0, abort_flag);
       }
-      // step `it` queues the work that can run while the math warps are busy with block it
-      for (int it = 0; it <= n_it && ok; ++it) {
-        const int j = it - 1;  // the block whose P^T / dS^T the math warps have just delivered
-        const int jq = j % QS, jc = j & 1, jt = j >> 1;
-        if (j >= 0) {
-          if (!mbar_wait(p_full, j & 1, abort_flag)) { ok = false; break; }
+      if (ok) {
+        tc_fence_after_sync();
+        product(tmem_dp, v_k, do_k);
+        umma_commit(dp_full);
+      }
+      for (int i = 0; i < n_it && ok; ++i) {
+        const int st = i & 1, nx = st ^ 1;
+        const uint32_t ph = i & 1, phn = ((i + 1) >> 1) & 1;
+        if (!mbar_wait(p_full, ph, abort_flag)) break;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)  // 128 queries = 8 steps of 16; the warpgroups' shares of P^T start 32 columns apart
+          umma_f16_ts(tmem_dv, tmem_s + (kk >> 1) * 32 + (kk & 1) * 8, do_mn + st * kStage + (kk * 2048 >> 4), idesc_acc,
+                      (i | kk) != 0);
+        umma_commit(&do_empty[st]);
+        if (i + 1 < n_it) {
+          if (!mbar_wait(&q_full[nx], phn, abort_flag)) break;
           tc_fence_after_sync();
-          const uint32_t dd = smem_u32(sdO + jq * Cfg::kQTile);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)  // 64 queries = 4 steps of 16
-            umma_f16_ss(tmem_dv, umma_desc_sw128(pt + kk * 32, 16, 1024), umma_desc_sw128(dd + kk * 2048, 8192, 1024),
-                        idesc_acc, (j | kk) != 0);
-          umma_commit(pv_done);
+          product(tmem_s, k_k, q_k + nx * kStage);
+          umma_commit(s_full);
         }
-        if (it + 1 < n_it) {
-          if (!mbar_wait(&qdo_full[(it + 1) % QS], ((it + 1) / QS) & 1, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(sdp_free, it & 1, abort_flag)) { ok = false; break; }  // block `it` sits in registers
+        if (!mbar_wait(ds_full, ph, abort_flag)) break;
+        if (HD == 64 && i >= 1 && !mbar_wait(dq_empty, (i - 1) & 1, abort_flag)) break;
+        tc_fence_after_sync();
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16
+          umma_f16_ss(tmem_dq, ds_mn + (kk * 2048 >> 4), k_mn + (kk * 2048 >> 4), idesc_dq, kk != 0);
+        umma_commit(dq_full);
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)
+          umma_f16_ss(tmem_dk, ds_k + (((kk >> 2) * 16384 + (kk & 3) * 32) >> 4), q_mn + st * kStage + (kk * 2048 >> 4),
+                      idesc_acc, (i | kk) != 0);
+        umma_commit(&q_empty[st]);
+        if (i + 1 < n_it) {
+          if (!mbar_wait(&do_full[nx], phn, abort_flag)) break;
+          if (HD == 128 && !mbar_wait(dq_empty, ph, abort_flag)) break;  // dP^T takes the columns of dQ
           tc_fence_after_sync();
-          issue_sdp(it + 1);
-        }
-        if (j >= 0) {
-          if (jc == 1 || j == n_it - 1) {
-            // dQ of the pair: A = dS^T pair tile read MN-major (M = 128 queries in two 64-query chunks), B = K
-            if (jt >= 1 && !mbar_wait(dq_empty, (jt - 1) & 1, abort_flag)) { ok = false; break; }
-            tc_fence_after_sync();
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16
-              umma_f16_ss(tmem_dq, umma_desc_sw128(dst + kk * 2048, 16384, 1024),
-                          umma_desc_sw128(k + kk * 2048, 16384, 1024), idesc_dq, kk != 0);
-            umma_commit(dq_done);
-          }
-          const uint32_t qq = smem_u32(sQ + jq * Cfg::kQTile);
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk)
-            umma_f16_ss(tmem_dk, umma_desc_sw128(dst + jc * 16384 + kk * 32, 16, 1024),
-                        umma_desc_sw128(qq + kk * 2048, 8192, 1024), idesc_acc, (j | kk) != 0);
-          umma_commit(&qdo_empty[jq]);
-          umma_commit(&dk_done[jc]);
+          product(tmem_dp, v_k, do_k + nx * kStage);
+          umma_commit(dp_full);
+        } else {
+          umma_commit(acc_full);
         }
       }
-      if (ok) umma_commit(acc_full);
     }
-  } else if (warp >= 2 + kMathWarps) {
-    // ------------- drain warps: dQ tile of every finished pair -> fp32 accumulator in global memory -------------
+  } else if (warp >= 20) {
+    // -------------- drain warps: dQ of every step -> fp32 accumulator in global memory --------------
+    reg_alloc<kFusedRegsDrain>();
     const int quarter = warp & 3;
-    const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
-    uint8_t* stage = sStage + (warp - 2 - kMathWarps) * Cfg::kStageBytes;
-    const int n_pairs = (n_it + 1) >> 1;
-    const int row0 = ((b * p.NH + head) * n_tiles) * 128 + quarter * 32;
-    bool ok = true;
-    for (int tt = 0; tt < n_pairs && ok; ++tt) {
-      if (!mbar_wait_warp(dq_done, tt & 1, abort_flag)) { ok = false; break; }
+    const uint32_t src = tmem_dq + (static_cast<uint32_t>(quarter * 32) << 16);
+    float* dst = dq_acc + tile0 * (128 * HD) + quarter * (32 * HD) + lane * 4;
+    for (int i = 0; i < n_it; ++i) {
+      if (!mbar_wait_warp(dq_full, i & 1, abort_flag)) break;
       tc_fence_after_sync();
-      const int tile = (i0 >> 1) + tt;
+      // Registers hold 64 columns; the columns are free for dP^T of the next block once the second half is in registers,
+      // and the reductions leave at 32 bytes a clock.
 #pragma unroll
-      for (int ch = 0; ch < HD / 32; ++ch) {
-        uint32_t rq[32];
-        tmem_ld_32x32(tmem_dq + lane_addr + ch * 32, rq);
+      for (int half = 0; half < HD / 64; ++half) {
+        uint32_t a[2][32];
+        tmem_ld_32x32(src + half * 64, a[0]);
+        tmem_ld_32x32(src + half * 64 + 32, a[1]);
         tmem_ld_wait();
-        if (lane == 0) tma_store_wait_read<0>();  // the previous reduction has read this warp's staging tile
-        __syncwarp();
-        uint8_t* row = stage + lane * 128;
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          *reinterpret_cast<uint4*>(row + ((i ^ (lane & 7)) << 4)) =
-              make_uint4(rq[4 * i], rq[4 * i + 1], rq[4 * i + 2], rq[4 * i + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          tma_reduce_add_2d(&tm_acc, stage, ch * 32, row0 + tile * 128);
-          tma_store_commit();
+        if (half == HD / 64 - 1) {
+          tc_fence_before_sync();
+          warp_arrive(dq_empty, lane);
         }
+#pragma unroll
+        for (int e = 0; e < 16; ++e)
+          red_add_v4(dst + (half * 16 + e) * 128, a[e >> 3][4 * (e & 7)], a[e >> 3][4 * (e & 7) + 1], a[e >> 3][4 * (e & 7) + 2],
+                     a[e >> 3][4 * (e & 7) + 3]);
       }
-      tc_fence_before_sync();
-      warp_arrive(dq_empty, lane);  // the dQ product of the next pair may overwrite the accumulator
+      dst += 128 * HD;
     }
-    if (lane == 0) tma_store_wait<0>();  // reductions complete before the CTA's shared memory goes away
   } else {
     // ------------------------------------------ math warps --------------------------------------------
+    // (the math warpgroups keep the registers they were launched with)
     const int quarter = warp & 3;
-    const int g = (warp - 2) >> 2;      // column group: 16 of the 64 queries of a block, HD/4 output columns
+    const int g = (warp - 4) >> 2;      // queries [32 g, 32 g + 32) of a block; columns [g HD/4, ..) of dK and dV
     const int r = quarter * 32 + lane;  // key row inside the tile
     const int kv = kv0 + r;
     const uint32_t lane_addr = static_cast<uint32_t>(quarter * 32) << 16;
+    const uint32_t my_s = tmem_s + lane_addr + g * 32, my_dp = tmem_dp + lane_addr + g * 32;
     const float c = p.scale * kLog2e;
     const uint32_t keep8 = dropout_keep8(p.dropout_p);
     const float inv_keep = DROPOUT ? 256.0f / static_cast<float>(keep8) : 1.0f;
+    const uint32_t drop_c = (256u - keep8) * 0x01010101u;  // byte + drop_c carries out <=> byte >= keep8
     const uint32_t bh_seed = static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(b) * p.NH + head));
-    const uint32_t qquads = (p.SQ + 3) >> 2;
-    // per (batch, head) statistics prepared by attn_bwd_prep_kernel: lse2 = LSE log2(e), nd = -rowsum(dO O)
-    const float* lse_row = p.LSE + (static_cast<size_t>(b) * p.NH + head) * p.SQ;
-    const float* nd_row = p.delta + (static_cast<size_t>(b) * p.NH + head) * p.SQ;
+    // attn_col_hash mixes (key quads + quad) * 0x9E3779B1 + seed: linear in the quad
+    const uint32_t hash0 = (static_cast<uint32_t>(kv) * ((p.SQ + 3) >> 2) + static_cast<uint32_t>(i0 * 32 + g * 8)) * 0x9E3779B1u + bh_seed;
     const bool kv_ok = kv < kv_len;
-    const bool stats_vec = (p.SQ & 3) == 0;
-    // shared-memory offsets of this thread's two 16-byte pieces of a [128][128 B] swizzled tile row: fixed for the
-    // whole kernel (row r, pieces 2 g and 2 g + 1)
-    // score bias: bias2[q] = bias_table[head][kv - q + SQ - 1] log2(e); its gradient is dS summed along the diagonals
+    // score bias: bias_table[head][kv - q + SQ - 1] log2(e); its gradient is dS summed along the diagonals
     const int n_dist = p.SQ + p.SK - 1;
     const float* bias_head = BIAS ? p.bias_table + static_cast<size_t>(head) * n_dist : nullptr;
     float* dbias_head = BIAS ? p.dbias_table + static_cast<size_t>(head) * n_dist : nullptr;
-    const uint32_t piece_a = static_cast<uint32_t>(r * 128 + (((2 * g) ^ (r & 7)) << 4));
-    const uint32_t piece_b = static_cast<uint32_t>(r * 128 + (((2 * g + 1) ^ (r & 7)) << 4));
+    uint8_t* ds_row = sdS + (g >> 1) * 16384 + r * 128;
 
     bool ok = true;
-    for (int it = 0; it < n_it && ok; ++it) {
-      const int cpar = it & 1;
-      const int qbase = (i0 + it) * 64 + g * 16;
-      // statistics of this thread's 16 queries, requested before the accumulators are ready
-      float lse2[16], nd[16];
-      if (stats_vec && qbase + 16 <= p.SQ) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float4 a = __ldg(reinterpret_cast<const float4*>(lse_row + qbase) + i);
-          const float4 d = __ldg(reinterpret_cast<const float4*>(nd_row + qbase) + i);
-          lse2[4 * i] = a.x; lse2[4 * i + 1] = a.y; lse2[4 * i + 2] = a.z; lse2[4 * i + 3] = a.w;
-          nd[4 * i] = d.x; nd[4 * i + 1] = d.y; nd[4 * i + 2] = d.z; nd[4 * i + 3] = d.w;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          const bool in = qbase + i < p.SQ;
-          lse2[i] = in ? __ldg(lse_row + qbase + i) : INFINITY;
-          nd[i] = in ? __ldg(nd_row + qbase + i) : 0.f;
-        }
-      }
-      // dropout: this key's hashes of the four query quads of the step (byte e of hash j decides query 4 j + e)
-      uint32_t hq[4];
+    for (int i = 0; i < n_it && ok; ++i) {
+      const int qblk0 = (i0 + i) * 128, qbase = qblk0 + g * 32;
+      const float* nlse2 = sStat + (i & 1) * 256 + g * 32;
+      const float* nd = nlse2 + 128;
+      const bool need_mask = (p.causal && kv0 + 127 > qblk0) || qblk0 + 128 > p.SQ || kv0 + 128 > kv_len;
+      // queries lo .. hi - 1 of this thread's 32 see its key
+      const int lo = p.causal ? kv - qbase : 0, hi = kv_ok ? p.SQ - qbase : 0;
+      uint32_t drop = 0u;  // bit 7 - n of byte e: query 4 n + e dropped for this key; hashed before the scores are there
       if constexpr (DROPOUT) {
+        uint32_t h = hash0 + static_cast<uint32_t>(i) * (32u * 0x9E3779B1u);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) hq[j] = attn_col_hash(bh_seed, kv, qquads, (qbase >> 2) + j);
+        for (int n = 0; n < 8; ++n) {
+          const uint32_t x = fmix32(h);
+          h += 0x9E3779B1u;
+          const uint32_t cs = (x & 0x7f7f7f7fu) + (drop_c & 0x7f7f7f7fu);
+          drop |= (((x & drop_c) | ((x | drop_c) & cs)) & 0x80808080u) >> n;
+        }
       }
-      const int qblk0 = (i0 + it) * 64;
-      const bool need_mask = (p.causal && kv0 + 127 > qblk0) || qblk0 + 64 > p.SQ || kv0 + 128 > kv_len;
-      if (!mbar_wait_warp(s_full, it & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(&q_full[i & 1], (i >> 1) & 1, abort_flag)) { ok = false; break; }  // the statistics
+      if (!mbar_wait_warp(s_full, i & 1, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
-      uint32_t rs[16], rp[16];
-      tmem_ld_32x16(tmem_base + lane_addr + Cfg::kColS + g * 16, rs);
-      tmem_ld_32x16(tmem_base + lane_addr + Cfg::kColDP + g * 16, rp);
-      tmem_ld_wait();
-      tc_fence_before_sync();
-      warp_arrive(sdp_free, lane);  // the products of the next query block may overwrite S^T / dP^T now
-      uint32_t wp[8], wd[8];
-      float dsv[BIAS ? 16 : 1];
+      float pr[32];
+      {
+        uint32_t rs[32], w[16];
+        tmem_ld_32x32(my_s, rs);
+        tmem_ld_wait();
+        const float2 c2 = make_float2(c, c);
 #pragma unroll
-      for (int i = 0; i < 16; i += 2) {
-        float pv[2], dv[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          float shift = -lse2[i + e];
+        for (int e = 0; e < 32; e += 4) {
+          float4 nl = *reinterpret_cast<const float4*>(nlse2 + e);
           if constexpr (BIAS) {
-            const int d = min(max(kv - (qbase + i + e) + p.SQ - 1, 0), n_dist - 1);
-            shift = fmaf(__ldg(bias_head + d), kLog2e, shift);
+            const int d = kv - (qbase + e) + p.SQ - 1;  // entries run down as the query runs up
+            nl.x = fmaf(__ldg(bias_head + min(max(d, 0), n_dist - 1)), kLog2e, nl.x);
+            nl.y = fmaf(__ldg(bias_head + min(max(d - 1, 0), n_dist - 1)), kLog2e, nl.y);
+            nl.z = fmaf(__ldg(bias_head + min(max(d - 2, 0), n_dist - 1)), kLog2e, nl.z);
+            nl.w = fmaf(__ldg(bias_head + min(max(d - 3, 0), n_dist - 1)), kLog2e, nl.w);
           }
-          const float pr = ex2(fmaf(__uint_as_float(rs[i + e]), c, shift));
-          const float dp = __uint_as_float(rp[i + e]);
-          if constexpr (DROPOUT) {
-            const float mk = keep_byte(hq[(i + e) >> 2], (i + e) & 3, keep8) ? inv_keep : 0.f;
-            pv[e] = pr * mk;
-            dv[e] = pr * fmaf(dp, mk, nd[i + e]);
-          } else {
-            pv[e] = pr;
-            dv[e] = pr * (dp + nd[i + e]);
-          }
+          const float2 a = fma_f32x2(make_float2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), c2, make_float2(nl.x, nl.y));
+          const float2 b2 = fma_f32x2(make_float2(__uint_as_float(rs[e + 2]), __uint_as_float(rs[e + 3])), c2, make_float2(nl.z, nl.w));
+          pr[e] = ex2(a.x);
+          pr[e + 1] = ex2(a.y);
+          pr[e + 2] = ex2(b2.x);
+          pr[e + 3] = ex2(b2.y);
         }
         if (need_mask) {  // uniform branch: only blocks on the diagonal or at the ragged ends pay for the tests
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const int q = qbase + i + e;
-            if (!(kv_ok && q < p.SQ && !(p.causal && kv > q))) pv[e] = dv[e] = 0.f;
-          }
+          for (int e = 0; e < 32; ++e)
+            if (e < lo || e >= hi) pr[e] = 0.f;
         }
-        wp[i >> 1] = pack_bf16x2(pv[0], pv[1]);
-        wd[i >> 1] = pack_bf16x2(dv[0], dv[1]);
-        if constexpr (BIAS) {
-          dsv[i] = dv[0];
-          dsv[i + 1] = dv[1];
-        }
-      }
-      if constexpr (BIAS) {
-        // Gradient of the bias table: dS (before the softmax scale) summed along the diagonals key - query.  Lane l
-        // holds key kv and queries qbase .. qbase + 15; the diagonal through (l, i) continues at (l + 1, i + 1), so a
-        // running sum handed from lane l + 1 to lane l while i walks down collects a warp's share of every diagonal:
-        // at the end lane l holds the diagonal through (l, 0), and the diagonals that leave the warp at lane 0 are
-        // flushed as they complete.  47 reductions per warp and step instead of 512.
-        float run = 0.f;
 #pragma unroll
-        for (int i = 15; i >= 0; --i) {
-          run = dsv[i] + __shfl_down_sync(0xffffffffu, run, 1) * (lane < 31 ? 1.f : 0.f);
-          if (i > 0 && lane == 0) {
-            const int d = kv - (qbase + i) + p.SQ - 1;
-            if (d >= 0 && d < n_dist) atomicAdd(dbias_head + d, run);
+        for (int e = 0; e < 16; ++e) {
+          w[e] = pack_bf16x2(pr[2 * e], pr[2 * e + 1]);
+          if constexpr (DROPOUT) w[e] &= ~spread_sign_bytes(drop << (e >> 1), (e & 1) ? 0xBBAA : 0x9988);
+        }
+        tmem_st_32x16(my_s, w);
+      }
+      tmem_st_wait();
+      tc_fence_before_sync();
+      warp_arrive(p_full, lane);
+      if (!mbar_wait_warp(dp_full, i & 1, abort_flag)) { ok = false; break; }
+      tc_fence_after_sync();
+      float diag = 0.f, wrap = 0.f;  // BIAS: sums along the diagonals through (lane, 0) and, wrapped, 32 distances below
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        uint32_t rp[16], w[8];
+        tmem_ld_32x16(my_dp + ch * 16, rp);
+        tmem_ld_wait();
+        const float2 k2 = make_float2(inv_keep, inv_keep);
+#pragma unroll
+        for (int e = 0; e < 16; e += 4) {
+          const int q = ch * 16 + e;
+          const float4 n4 = *reinterpret_cast<const float4*>(nd + q);
+          if constexpr (DROPOUT) {
+            const uint32_t d = drop << (q >> 2);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) rp[e + u] &= ~spread_sign_bytes(d, 0x8888 + 0x1111 * u);
+          }
+          float2 a = make_float2(__uint_as_float(rp[e]), __uint_as_float(rp[e + 1]));
+          float2 b2 = make_float2(__uint_as_float(rp[e + 2]), __uint_as_float(rp[e + 3]));
+          if constexpr (DROPOUT) {
+            a = fma_f32x2(a, k2, make_float2(n4.x, n4.y));
+            b2 = fma_f32x2(b2, k2, make_float2(n4.z, n4.w));
+          } else {
+            a = add_f32x2(a, make_float2(n4.x, n4.y));
+            b2 = add_f32x2(b2, make_float2(n4.z, n4.w));
+          }
+          a = mul_f32x2(make_float2(pr[q], pr[q + 1]), a);
+          b2 = mul_f32x2(make_float2(pr[q + 2], pr[q + 3]), b2);
+          if (need_mask) {  // rows and keys outside hold another sample's data, or nothing: not even 0 x NaN may enter
+            if (q < lo || q >= hi) a.x = 0.f;
+            if (q + 1 < lo || q + 1 >= hi) a.y = 0.f;
+            if (q + 2 < lo || q + 2 >= hi) b2.x = 0.f;
+            if (q + 3 < lo || q + 3 >= hi) b2.y = 0.f;
+          }
+          w[e >> 1] = pack_bf16x2(a.x, a.y);
+          w[(e >> 1) + 1] = pack_bf16x2(b2.x, b2.y);
+          if constexpr (BIAS) {
+            // Gradient of the bias table: dS (before the softmax scale) summed along the diagonals key - query.  Lane l
+            // takes entry (l + q, q) from lane l + q: all on its own diagonal, or 32 distances below it where the
+            // lane index wraps.  Independent shuffles, two coalesced reductions per warp and step.
+            const float v4[4] = {a.x, a.y, b2.x, b2.y};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const float y = __shfl_sync(0xffffffffu, v4[u], (lane + q + u) & 31);
+              if (lane + q + u < 32) diag += y;
+              else wrap += y;
+            }
           }
         }
-        const int d = kv - qbase + p.SQ - 1;
-        if (d >= 0 && d < n_dist) atomicAdd(dbias_head + d, run);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + ch * 2 + e) ^ (r & 7)) << 4)) =
+              make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
       }
-      // P^T: read by dV of the previous block (queued at the start of this block).  This parity's dS^T chunk: read by
-      // dK of block it - 2 and by dQ of the previous pair, which reads both chunks and was queued during this block
-      // when `it` is even, one block earlier when it is odd (then this thread saw it retire at block it - 1).
-      if (it >= 1 && !mbar_wait_warp(pv_done, (it - 1) & 1, abort_flag)) { ok = false; break; }
-      if (it >= 2) {
-        if (!mbar_wait_warp(&dk_done[cpar], ((it >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-        if (cpar == 0 && !mbar_wait_warp(dq_done, ((it >> 1) - 1) & 1, abort_flag)) { ok = false; break; }
-      }
-      *reinterpret_cast<uint4*>(sPt + piece_a) = make_uint4(wp[0], wp[1], wp[2], wp[3]);
-      *reinterpret_cast<uint4*>(sPt + piece_b) = make_uint4(wp[4], wp[5], wp[6], wp[7]);
-      uint8_t* ds_chunk = sdSt + cpar * Cfg::kPBytes;
-      *reinterpret_cast<uint4*>(ds_chunk + piece_a) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-      *reinterpret_cast<uint4*>(ds_chunk + piece_b) = make_uint4(wd[4], wd[5], wd[6], wd[7]);
       tc_fence_before_sync();
       fence_proxy_async_smem();
-      warp_arrive(p_full, lane);
+      warp_arrive(ds_full, lane);
+      if constexpr (BIAS) {
+        const int d = kv - qbase + p.SQ - 1;
+        if (d >= 0 && d < n_dist) atomicAdd(dbias_head + d, diag);
+        if (lane > 0 && d - 32 >= 0 && d - 32 < n_dist) atomicAdd(dbias_head + d - 32, wrap);
+      }
     }
     if (ok && n_it > 0) ok = mbar_wait(acc_full, 0, abort_flag);
     // tcgen05.ld is warp-collective: the whole warp runs the loads, only the stores are predicated
     ok = __all_sync(0xffffffffu, ok);
-    const bool store_row = kv < p.SK;
     if (ok) {
+      // 32 keys x HD / 4 columns per warp and matrix, through shared memory (every load and product of the walk is
+      // complete, the operand stages are free) so that memory sees whole 64- or 32-byte row segments
       tc_fence_after_sync();
-      __nv_bfloat16* dvrow = reinterpret_cast<__nv_bfloat16*>(p.dV) +
-                             (static_cast<size_t>(b) * p.SK + kv) * p.lddv + p.dv_col0 + head * HD + g * OC;
-      __nv_bfloat16* dkrow = reinterpret_cast<__nv_bfloat16*>(p.dK) +
-                             (static_cast<size_t>(b) * p.SK + kv) * p.lddk + p.dk_col0 + head * HD + g * OC;
-      uint32_t rv[OC], rk[OC];
-      if (n_it > 0) {
-        tmem_ld_cols<OC>(tmem_dv + lane_addr + g * OC, rv);
-        tmem_ld_cols<OC>(tmem_dk + lane_addr + g * OC, rk);
-        tmem_ld_wait();
-      } else {
+      constexpr int OC = HD / 4, PIECES = OC / 8, RPI = 32 / PIECES;  // columns, 16-byte pieces, rows per store
+      uint8_t* stage = sQ + (warp - 4) * 2048;
+      auto cell = [&](int row, int piece) { return stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4); };
 #pragma unroll
-        for (int i = 0; i < OC; ++i) rv[i] = rk[i] = 0u;
-      }
-      const float sc = p.scale;
+      for (int which = 0; which < 2; ++which) {
+        const float sc = which ? p.scale : inv_keep;
+        const uint32_t src = (which ? tmem_dk : tmem_dv) + lane_addr + g * OC;
+        uint32_t a[OC];
+        if (n_it > 0) {
+          tmem_ld_cols<OC>(src, a);
+          tmem_ld_wait();
+        } else {
 #pragma unroll
-      for (int i = 0; i < OC / 8; ++i) {
-        uint4 wv, wk;
-        wv.x = pack_bf16x2(__uint_as_float(rv[8 * i + 0]), __uint_as_float(rv[8 * i + 1]));
-        wv.y = pack_bf16x2(__uint_as_float(rv[8 * i + 2]), __uint_as_float(rv[8 * i + 3]));
-        wv.z = pack_bf16x2(__uint_as_float(rv[8 * i + 4]), __uint_as_float(rv[8 * i + 5]));
-        wv.w = pack_bf16x2(__uint_as_float(rv[8 * i + 6]), __uint_as_float(rv[8 * i + 7]));
-        wk.x = pack_bf16x2(__uint_as_float(rk[8 * i + 0]) * sc, __uint_as_float(rk[8 * i + 1]) * sc);
-        wk.y = pack_bf16x2(__uint_as_float(rk[8 * i + 2]) * sc, __uint_as_float(rk[8 * i + 3]) * sc);
-        wk.z = pack_bf16x2(__uint_as_float(rk[8 * i + 4]) * sc, __uint_as_float(rk[8 * i + 5]) * sc);
-        wk.w = pack_bf16x2(__uint_as_float(rk[8 * i + 6]) * sc, __uint_as_float(rk[8 * i + 7]) * sc);
-        if (store_row) {
-          reinterpret_cast<uint4*>(dvrow)[i] = wv;
-          reinterpret_cast<uint4*>(dkrow)[i] = wk;
+          for (int e = 0; e < OC; ++e) a[e] = 0u;
         }
+#pragma unroll
+        for (int e = 0; e < PIECES; ++e) {
+          uint4 v;
+          v.x = pack_bf16x2(__uint_as_float(a[8 * e + 0]) * sc, __uint_as_float(a[8 * e + 1]) * sc);
+          v.y = pack_bf16x2(__uint_as_float(a[8 * e + 2]) * sc, __uint_as_float(a[8 * e + 3]) * sc);
+          v.z = pack_bf16x2(__uint_as_float(a[8 * e + 4]) * sc, __uint_as_float(a[8 * e + 5]) * sc);
+          v.w = pack_bf16x2(__uint_as_float(a[8 * e + 6]) * sc, __uint_as_float(a[8 * e + 7]) * sc);
+          *reinterpret_cast<uint4*>(cell(lane, e)) = v;
+        }
+        __syncwarp();
+        const int ld = which ? p.lddk : p.lddv;
+        const int piece = lane % PIECES;
+        __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(which ? p.dK : p.dV) +
+                             (static_cast<size_t>(b) * p.SK + kv0 + quarter * 32) * ld + (which ? p.dk_col0 : p.dv_col0) +
+                             head * HD + g * OC + piece * 8;
+#pragma unroll
+        for (int e = 0; e < 32 / RPI; ++e) {
+          const int row = e * RPI + lane / PIECES;
+          const uint4 v = *reinterpret_cast<const uint4*>(cell(row, piece));
+          if (kv0 + quarter * 32 + row < p.SK) *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * ld) = v;
+        }
+        __syncwarp();
       }
     }
   }
@@ -460,36 +495,51 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
 }
 
-// dQ[b, q, head, :] (bf16) = scale * the fp32 accumulator [b, head, tile][128][HD]; one thread per 8 columns.
+// dQ[b, q, head, :] (bf16) = scale * the fp32 accumulator [b, head, tile][quarter][HD / 4][32][4].  A warp turns 32 queries x
+// 64 columns: 512-byte reads, a transpose through shared memory, 128-byte row segments out.
 template <int HD>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 attn_dq_convert_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq, int lddq, int dq_col0, int NH,
                        int SQ, int n_tiles, float scale) {
-  constexpr int OCT = HD / 8;
+  __shared__ __align__(16) uint8_t tile_smem[4][4096];
   const int head = blockIdx.y, b = blockIdx.z;
-  const int idx = blockIdx.x * 256 + threadIdx.x;
-  const int q = idx / OCT, j = idx % OCT;
-  if (q >= SQ) return;
-  const float* src = acc + ((static_cast<size_t>(b) * NH + head) * n_tiles * 128 + q) * HD + j * 8;
-  const float4 lo = *reinterpret_cast<const float4*>(src);
-  const float4 hi = *reinterpret_cast<const float4*>(src + 4);
-  uint4 w;
-  w.x = pack_bf16x2(lo.x * scale, lo.y * scale);
-  w.y = pack_bf16x2(lo.z * scale, lo.w * scale);
-  w.z = pack_bf16x2(hi.x * scale, hi.y * scale);
-  w.w = pack_bf16x2(hi.z * scale, hi.w * scale);
-  *reinterpret_cast<uint4*>(dq + (static_cast<size_t>(b) * SQ + q) * lddq + dq_col0 + head * HD + j * 8) = w;
+  const int tile = blockIdx.x / (HD / 64), c0 = (blockIdx.x % (HD / 64)) * 64;
+  const int quarter = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int q0 = tile * 128 + quarter * 32;
+  if (q0 >= SQ) return;
+  const float* src = acc + (((static_cast<size_t>(b) * NH + head) * n_tiles + tile) * 4 + quarter) * (32 * HD) + c0 * 32 + lane * 4;
+  float4 v[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) v[e] = *reinterpret_cast<const float4*>(src + e * 128);
+  uint8_t* stage = tile_smem[quarter];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    uint4 w;
+    w.x = pack_bf16x2(v[2 * e].x * scale, v[2 * e].y * scale);
+    w.y = pack_bf16x2(v[2 * e].z * scale, v[2 * e].w * scale);
+    w.z = pack_bf16x2(v[2 * e + 1].x * scale, v[2 * e + 1].y * scale);
+    w.w = pack_bf16x2(v[2 * e + 1].z * scale, v[2 * e + 1].w * scale);
+    *reinterpret_cast<uint4*>(stage + lane * 128 + ((e ^ (lane & 7)) << 4)) = w;
+  }
+  __syncwarp();
+  __nv_bfloat16* out = dq + (static_cast<size_t>(b) * SQ + q0) * lddq + dq_col0 + head * HD + c0 + (lane & 7) * 8;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int row = e * 4 + (lane >> 3);
+    const uint4 w = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
+    if (q0 + row < SQ) *reinterpret_cast<uint4*>(out + static_cast<size_t>(row) * lddq) = w;
+  }
 }
 
-// Row statistics in the form the fused kernel consumes: nd[b, h, q] = -sum_d dO O and lse2[b, h, q] = LSE log2(e).
-// A warp takes one head and 32 consecutive queries of one sequence.  LPR = HD / 8 lanes read one (token, head) row
+// Row statistics in the form the fused kernel consumes: nd[b, h, q] = -sum_d dO O and nlse2[b, h, q] = -LSE log2(e), rows
+// padded to whole query blocks (the padding is read but never used).  A warp takes one head and 32 consecutive queries of one sequence.  LPR = HD / 8 lanes read one (token, head) row
 // with 16-byte loads, so one load instruction of the warp covers 32 / LPR tokens; after the butterfly sum inside the
 // lane group every lane of the group holds the row's result, and lane L keeps token (L % LPR) * (32 / LPR) + L / LPR.
 template <int HD>
 __global__ void __launch_bounds__(128)
 attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, int ldo, int o_col0, const __nv_bfloat16* __restrict__ dout,
-                     int lddo, const float* __restrict__ lse, float* __restrict__ nd, float* __restrict__ lse2, int B,
-                     int NH, int SQ) {
+                     int lddo, const float* __restrict__ lse, float* __restrict__ nd, float* __restrict__ nlse2, int B,
+                     int NH, int SQ, int SQp) {
   constexpr int LPR = HD / 8, TPI = 32 / LPR;
   const int lane = threadIdx.x & 31;
   const int qblocks = (SQ + 31) / 32;
@@ -521,9 +571,9 @@ attn_bwd_prep_kernel(const __nv_bfloat16* __restrict__ o, int ldo, int o_col0, c
   }
   const int q = qb * 32 + sub * TPI + grp;
   if (q < SQ) {
-    const size_t idx = (static_cast<size_t>(b) * NH + head) * SQ + q;
-    nd[idx] = -mine;
-    lse2[idx] = lse[idx] * kLog2e;
+    const size_t bh = static_cast<size_t>(b) * NH + head;
+    nd[bh * SQp + q] = -mine;
+    nlse2[bh * SQp + q] = -lse[bh * SQ + q] * kLog2e;
   }
 }
 
@@ -534,27 +584,23 @@ int set_smem(K kernel, int bytes) {
 
 template <int HD, bool DROPOUT, bool BIAS>
 int launch_fused(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                 const CUtensorMap& tacc, const AttnParams& p, const float* dq_acc, cudaStream_t stream) {
-  static bool done = false;
+                 const AttnParams& p, float* dq_acc, cudaStream_t stream) {
   int rc;
-  if (!done) {
-    if ((rc = set_smem(attn_bwd_fused_kernel<HD, DROPOUT, BIAS>, FusedCfg<HD>::kSmem))) return rc;
-    done = true;
-  }
+  if ((rc = set_smem(attn_bwd_fused_kernel<HD, DROPOUT, BIAS>, FusedCfg<HD>::kSmem))) return rc;
   const int n_tiles = (p.SQ + 127) / 128;
   dim3 grid_kv((p.SK + 127) / 128, p.NH, p.B);
-  attn_bwd_fused_kernel<HD, DROPOUT, BIAS><<<grid_kv, kFusedThreads, FusedCfg<HD>::kSmem, stream>>>(tq, tk, tv, tdo, tacc, p);
-  dim3 grid_cv((p.SQ * (HD / 8) + 255) / 256, p.NH, p.B);
-  attn_dq_convert_kernel<HD><<<grid_cv, 256, 0, stream>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(p.dQ), p.lddq,
+  attn_bwd_fused_kernel<HD, DROPOUT, BIAS><<<grid_kv, kFusedThreads, FusedCfg<HD>::kSmem, stream>>>(tq, tk, tv, tdo, dq_acc, p);
+  dim3 grid_cv(n_tiles * (HD / 64), p.NH, p.B);
+  attn_dq_convert_kernel<HD><<<grid_cv, 128, 0, stream>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(p.dQ), p.lddq,
                                                           p.dq_col0, p.NH, p.SQ, n_tiles, p.scale);
   return static_cast<int>(cudaGetLastError());
 }
 
 }  // namespace
 
-// Floats of fp32 scratch the fused backward needs: the dQ accumulator, then the two row-statistic arrays.
+// Floats of fp32 scratch the fused backward needs: the dQ accumulator, then the two row-statistic arrays (padded rows).
 long long attn_bwd_fused_scratch_floats(int B, int NH, int SQ, int HD) {
-  return static_cast<long long>(B) * NH * ((SQ + 127) / 128) * 128 * HD + 2LL * B * NH * SQ;
+  return static_cast<long long>(B) * NH * ((SQ + 127) / 128) * 128 * (HD + 2);
 }
 
 // dout shares the layout of O (p.ldo / p.o_col0 describe both).  `scratch` holds attn_bwd_fused_scratch_floats()
@@ -563,8 +609,8 @@ int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const 
                           int lddo, const AttnParams& p, float* scratch, cudaStream_t stream) {
   if (p.HD != 64 && p.HD != 128) return -2;
   if (p.causal && p.SQ != p.SK) return -2;
-  // 16-byte granularity everywhere: TMA x coordinates (column offsets of Q / K / V / dO), the 16-byte stores of dK /
-  // dV and the bulk reductions of dQ; a misaligned offset would fault on the device instead of failing here
+  // 16-byte granularity everywhere: TMA x coordinates (column offsets of Q / K / V / dO), the 16-byte stores of
+  // dQ, dK and dV; a misaligned offset would fault on the device instead of failing here
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (p.lddq % 8) || (p.lddk % 8) || (p.lddv % 8) ||
       (p.dq_col0 % 8) || (p.dk_col0 % 8) || (p.dv_col0 % 8) || (p.q_col0 % 8) || (p.k_col0 % 8) || (p.v_col0 % 8))
     return -3;
@@ -572,10 +618,9 @@ int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const 
   const int n_tiles = (p.SQ + 127) / 128;
   const long long acc_rows = static_cast<long long>(p.B) * p.NH * n_tiles * 128;
   const long long acc_floats = acc_rows * p.HD;
-  const long long stat_floats = static_cast<long long>(p.B) * p.NH * p.SQ;
   float* dq_acc = scratch;
   float* nd = scratch + acc_floats;
-  float* lse2 = nd + stat_floats;
+  float* nlse2 = nd + acc_rows;
   {
     if ((p.ldo % 8) || (p.o_col0 % 8)) return -3;
     const long long warps = static_cast<long long>(p.B) * p.NH * ((p.SQ + 31) / 32);
@@ -583,35 +628,34 @@ int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const 
     const auto* db = reinterpret_cast<const __nv_bfloat16*>(dout);
     const unsigned blocks = static_cast<unsigned>((warps + 3) / 4);
     if (p.HD == 128)
-      attn_bwd_prep_kernel<128><<<blocks, 128, 0, stream>>>(ob, p.ldo, p.o_col0, db, lddo, p.LSE, nd, lse2, p.B, p.NH, p.SQ);
+      attn_bwd_prep_kernel<128><<<blocks, 128, 0, stream>>>(ob, p.ldo, p.o_col0, db, lddo, p.LSE, nd, nlse2, p.B, p.NH, p.SQ, n_tiles * 128);
     else
-      attn_bwd_prep_kernel<64><<<blocks, 128, 0, stream>>>(ob, p.ldo, p.o_col0, db, lddo, p.LSE, nd, lse2, p.B, p.NH, p.SQ);
+      attn_bwd_prep_kernel<64><<<blocks, 128, 0, stream>>>(ob, p.ldo, p.o_col0, db, lddo, p.LSE, nd, nlse2, p.B, p.NH, p.SQ, n_tiles * 128);
   }
   if ((rc = static_cast<int>(cudaMemsetAsync(dq_acc, 0, sizeof(float) * acc_floats, stream)))) return rc;
   AttnParams pp = p;
   pp.delta = nd;
-  pp.LSE = lse2;
-  CUtensorMap tq64, tk128, tv128, tdo64, tacc;
+  pp.LSE = nlse2;
+  CUtensorMap tq, tk, tv, tdo;
   const uint64_t rq = static_cast<uint64_t>(p.B) * p.SQ, rk = static_cast<uint64_t>(p.B) * p.SK;
-  if ((rc = make_tma_2d_bf16(&tq64, q, rq, ldq, ldq, 64, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tdo64, dout, rq, lddo, lddo, 64, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tk128, k, rk, ldk, ldk, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tv128, v, rk, ldv, ldv, 128, 64))) return rc;
-  if ((rc = make_tma_2d_f32(&tacc, dq_acc, static_cast<uint64_t>(acc_rows), static_cast<uint64_t>(p.HD), 32))) return rc;
+  if ((rc = make_tma_2d_bf16(&tq, q, rq, ldq, ldq, 128, 64))) return rc;
+  if ((rc = make_tma_2d_bf16(&tdo, dout, rq, lddo, lddo, 128, 64))) return rc;
+  if ((rc = make_tma_2d_bf16(&tk, k, rk, ldk, ldk, 128, 64))) return rc;
+  if ((rc = make_tma_2d_bf16(&tv, v, rk, ldv, ldv, 128, 64))) return rc;
   const bool drop = p.dropout_p > 0.f;
   if (p.bias_table != nullptr) {
     if (p.dbias_table == nullptr) return -2;
     if (p.HD == 128)
-      return drop ? launch_fused<128, true, true>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream)
-                  : launch_fused<128, false, true>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream);
-    return drop ? launch_fused<64, true, true>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream)
-                : launch_fused<64, false, true>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream);
+      return drop ? launch_fused<128, true, true>(tq, tk, tv, tdo, pp, dq_acc, stream)
+                  : launch_fused<128, false, true>(tq, tk, tv, tdo, pp, dq_acc, stream);
+    return drop ? launch_fused<64, true, true>(tq, tk, tv, tdo, pp, dq_acc, stream)
+                : launch_fused<64, false, true>(tq, tk, tv, tdo, pp, dq_acc, stream);
   }
   if (p.HD == 128)
-    return drop ? launch_fused<128, true, false>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream)
-                : launch_fused<128, false, false>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream);
-  return drop ? launch_fused<64, true, false>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream)
-              : launch_fused<64, false, false>(tq64, tk128, tv128, tdo64, tacc, pp, dq_acc, stream);
+    return drop ? launch_fused<128, true, false>(tq, tk, tv, tdo, pp, dq_acc, stream)
+                : launch_fused<128, false, false>(tq, tk, tv, tdo, pp, dq_acc, stream);
+  return drop ? launch_fused<64, true, false>(tq, tk, tv, tdo, pp, dq_acc, stream)
+              : launch_fused<64, false, false>(tq, tk, tv, tdo, pp, dq_acc, stream);
 }
 
 }  // namespace ssb

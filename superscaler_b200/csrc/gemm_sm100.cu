@@ -288,26 +288,6 @@ int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
-// fp32 row-major matrix [rows][cols] (contiguous rows): box = box_rows x 32 columns (128 bytes), 128-byte swizzle.
-// Used as the destination of bulk tensor reductions (shared memory tile added to global memory).
-int make_tma_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  EncodeTiledFn fn = get_encode_fn();
-  if (fn == nullptr) return -1;
-  static thread_local bool ctx_bound = false;
-  if (!ctx_bound) {
-    cudaFree(nullptr);
-    ctx_bound = true;
-  }
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {cols * 4};
-  cuuint32_t box[2] = {32, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
-}
-
 namespace {
 
 // D[m][n] (+)= sum over the slices, in slice order, of ws[slice][m][n] (N a multiple of 4).
