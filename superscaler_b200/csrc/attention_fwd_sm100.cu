@@ -4,10 +4,11 @@
 // ParallelSoftmaxFusionOp (scaled [causal|masked] softmax), ParallelSoftmaxDropoutOp and ParallelContextOp (bmm) --
 // runtime/megatron/model/flex_ops.py:711-1015 -- without ever writing the [b, np, sq, sk] score matrix to memory.
 //
-// A work item is 256 queries of one (batch, head): two tiles of 128.  Every tile has its own four softmax warps, one
-// thread per query row, so row maxima and sums need no exchange at all.  Per key block of 128 and tile:
+// A work item is 256 queries of one (batch, head): two tiles of 128.  Every tile has eight softmax warps; two threads share a
+// query row (64 keys of a block each) and exchange one maximum per block through shared memory.
+// Per key block of 128 and tile:
 //   S   = Q . K_j^T       fp32 accumulator in TMEM columns [128 t, 128 t + 128)
-//   softmax warps: S -> registers, running maximum, P = exp2(..) as bf16 -> TMEM columns [128 t + 64, 128 t + 128)
+//   softmax warps: S -> registers, running maximum, P = exp2(..) as bf16 -> TMEM, each half over its own columns of S
 //   O  += P . V_j         P is the A operand straight from TMEM; accumulator in columns [256 + 128 t, .. + HD)
 // While the tensor core runs O += P V and the next S of one tile, the softmax warps of the other tile work: both units
 // stay busy and P never passes through shared memory.
@@ -23,11 +24,13 @@
 // Without the mask all items cost the same and neighbours share a head.
 //
 // Measured against the one-tile kernel it replaces (128 queries a CTA, P through shared memory, four threads a row): causal,
-// 16 x 16 heads of 2048 x 128: 588 -> 343 us (801 TFLOP/s), with dropout 807 -> 434 us, unmasked 921 -> 529 us (1039 TFLOP/s);
-// one sequence of 16 heads 58 -> 43 us.  What bounds it now is the chain S -> softmax -> P.V of a tile (tensor pipe a third
-// busy, issue slots 43 %); with dropout the integer work of the mask.
+// 16 x 16 heads of 2048 x 128: 588 -> 346 us (794 TFLOP/s), with dropout 807 -> 405 us, unmasked 921 -> 488 us (1126 TFLOP/s);
+// one sequence of 16 heads 58.9 -> 41.0 us.  With one thread per row and four warps per tile the dropout form took 434 to
+// 449 us and T5's (bias, dropout, head size 64) 160 instead of 137: two warps per SM sub-partition could not cover the chain
+// S -> maximum -> exponentials -> P.  Tried on top, no gain: starting P.V on three quarters of the keys; slower: a separate
+// warpgroup for the masks (664 us, its hashes take longer than a step).
 //
-// Warps: 0 = TMA producer, 1 = TMEM allocator + MMA issuer, 2 and 3 idle, 4..7 = softmax of tile 0, 8..11 = of tile 1.
+// Warps: 0 = TMA producer, 1 = TMEM allocator + MMA issuer, 2 and 3 idle, then per tile 8 softmax warps (4 per half row).
 #include "attention_device.cuh"
 
 namespace ssb {
@@ -39,10 +42,10 @@ namespace {
 
 using namespace attn;
 
-constexpr int kFwdThreads = 384;   // three warpgroups: {TMA, MMA, 2 idle}, softmax of tile 0, softmax of tile 1
-// Register split: 384 threads are launched with 168 registers each (64512 in all); the first warpgroup keeps 120 and the
-// two softmax warpgroups take 192: 128 * 120 + 256 * 192 = 64512.
-constexpr int kFwdRegsOther = 120, kFwdRegsSoftmax = 192;
+constexpr int kFwdThreads = 640;   // five warpgroups: {TMA, MMA, 2 idle}, then two (column halves) per tile
+// Register split: 640 threads are launched with 96 registers each (61440 in all); the first warpgroup keeps 64 and the four
+// softmax warpgroups take 104: 128 * 64 + 512 * 104 = 61440.
+constexpr int kFwdRegsOther = 64, kFwdRegsSoftmax = 104;
 constexpr float kLazyLog2 = 8.0f;  // how far (log2) the reference maximum may lag before O is rescaled
 
 template <int HD>
@@ -50,9 +53,10 @@ struct FwdCfg {
   static constexpr int kCh = HD / 64;
   static constexpr int kTile = 128 * HD * 2;               // Q / K / V tile of 128 rows
   static constexpr int kStages = HD == 128 ? 4 : 6;        // K and V tiles in flight, in the order K0 V0 K1 V1 ...
-  static constexpr int kOutBytes = 8 * 32 * 128;           // per softmax warp: 32 rows x 64 output columns
+  static constexpr int kOutBytes = 16 * 32 * 64;           // per softmax warp: 32 rows x 32 output columns
+  static constexpr int kXchBytes = 2 * 2 * 128 * 4;        // row maxima: [tile][half][row]
   static constexpr int kBarBytes = 256;
-  static constexpr int kSmem = 2 * kTile + kStages * kTile + kOutBytes + kBarBytes + 1024;
+  static constexpr int kSmem = 2 * kTile + kStages * kTile + kOutBytes + kXchBytes + kBarBytes;
   static constexpr int kTmemCols = 512;                    // S/P 0, S/P 1, O 0, O 1: 128 columns each
 };
 
@@ -104,12 +108,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const FwdItems items) {
   using Cfg = FwdCfg<HD>;
   constexpr int CH = Cfg::kCh, NS = Cfg::kStages;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sQ = smem;                          // 2 tiles
   uint8_t* sKV = sQ + 2 * Cfg::kTile;          // NS stages
   uint8_t* sOut = sKV + NS * Cfg::kTile;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes);
+  float* sXch = reinterpret_cast<float*>(sOut + Cfg::kOutBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sOut + Cfg::kOutBytes + Cfg::kXchBytes);
   uint64_t* q_full = bars;             // 2
   uint64_t* q_empty = bars + 2;        // 2: the last S of the tile retired
   uint64_t* s_full = bars + 4;         // 2: S of a block complete (and with it P.V of the block before)
@@ -126,7 +130,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_init(&q_full[t], 1);
       mbar_init(&q_empty[t], 1);
       mbar_init(&s_full[t], 1);
-      mbar_init(&p_full[t], 4);
+      mbar_init(&p_full[t], 8);
       mbar_init(&o_full[t], 1);
     }
     for (int s = 0; s < NS; ++s) {
@@ -201,16 +205,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (warp == 1 && elect_one()) {
       constexpr uint32_t idesc_s = umma_idesc_bf16(128, 128, false, false);
       constexpr uint32_t idesc_o = umma_idesc_bf16(128, HD, false, true);
+      // one descriptor per operand; a step along it is an addition to the address field
+      const uint64_t q_k = umma_desc_sw128(smem_u32(sQ), 16, 1024), kv_k = umma_desc_sw128(smem_u32(sKV), 16, 1024);
+      const uint64_t kv_mn = umma_desc_sw128(smem_u32(sKV), 16384, 1024);
+      constexpr uint64_t kStep = Cfg::kTile >> 4;
       Pipe pp;                               // next K / V stage to consume
       uint32_t qn[2] = {0, 0}, pn[2] = {0, 0};
       bool ok = true;
       auto issue_s = [&](int t, int stage) {
-        const uint32_t a = smem_u32(sQ + t * Cfg::kTile), bb = smem_u32(sKV + stage * Cfg::kTile);
+        const uint64_t a = q_k + t * kStep, bb = kv_k + stage * kStep;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
-          const uint32_t off = (kk >> 2) * 16384 + (kk & 3) * 32;
-          umma_f16_ss(tmem_base + t * 128, umma_desc_sw128(a + off, 16, 1024), umma_desc_sw128(bb + off, 16, 1024),
-                      idesc_s, kk != 0);
+          const uint64_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
+          umma_f16_ss(tmem_base + t * 128, a + off, bb + off, idesc_s, kk != 0);
         }
         umma_commit(&s_full[t]);
       };
@@ -245,11 +252,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (!mbar_wait(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
             ++pn[t];
             tc_fence_after_sync();
-            const uint32_t bb = smem_u32(sKV + sv * Cfg::kTile);
+            const uint64_t bb = kv_mn + sv * kStep;
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16 (8 TMEM columns of packed bf16 pairs)
-              umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + 64 + kk * 8,
-                          umma_desc_sw128(bb + kk * 2048, 16384, 1024), idesc_o, (j | kk) != 0);
+              umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + (kk >> 2) * 64 + (kk & 3) * 8,
+                          bb + (kk * 2048 >> 4), idesc_o, (j | kk) != 0);
             if (j + 1 == w.n[t]) {
               umma_commit(&o_full[t]);
             } else {
@@ -273,11 +280,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     // ------------------------------------------ softmax warps -----------------------------------------
     reg_alloc<kFwdRegsSoftmax>();
     const int quarter = warp & 3;
-    const int t = (warp - 4) >> 2;
+    const int t = (warp - 4) >> 3, half = ((warp - 4) >> 2) & 1;  // tile; keys [64 half, 64 half + 64) of a block
     const int r = quarter * 32 + lane;
-    const uint32_t tm_s = tmem_base + t * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t tm_o = tm_s + 256;
-    uint8_t* stage = sOut + (warp - 4) * 4096;
+    const uint32_t tm_row = tmem_base + t * 128 + (static_cast<uint32_t>(quarter * 32) << 16);
+    const uint32_t tm_s = tm_row + half * 64, tm_o = tm_row + 256 + half * (HD / 2);
+    uint8_t* stage = sOut + (warp - 4) * 2048;
+    float* xch = sXch + t * 256 + r;   // + half * 128
+    auto pair_sync = [&]() {  // the two warps that share these 32 rows
+      asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory");
+    };
     const float c = p.scale * kLog2e;
     // With a bias the logits are brought into the log2 domain first (x c + bias log2 e) and everything below works on
     // them with a factor of one; without it the raw accumulator is used and the factor is c.
@@ -301,25 +312,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       if constexpr (DROPOUT) {
         // attn_col_hash mixes (key qquads + quad) * 0x9E3779B1 + seed: linear in the key, so a step of four keys is an add
         const uint32_t bh_seed = static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(w.b) * p.NH + w.head));
-        hash_base = (static_cast<uint32_t>(sub) * qquads + (static_cast<uint32_t>(q) >> 2)) * 0x9E3779B1u + bh_seed;
+        hash_base = (static_cast<uint32_t>(half * 64 + sub) * qquads + (static_cast<uint32_t>(q) >> 2)) * 0x9E3779B1u + bh_seed;
         hash_step = 4u * qquads * 0x9E3779B1u;
       }
       const float* bias_row = BIAS ? p.bias_table + static_cast<size_t>(w.head) * (p.SQ + p.SK - 1) + (p.SQ - 1) - min(q, p.SQ - 1)
                                    : nullptr;
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < nt; ++j) {
-        const int kv0 = j * 128;
+        const int kv0 = j * 128 + half * 64;
         if (!mbar_wait_warp(&s_full[t], sn & 1, abort_flag)) { ok = false; break; }
         ++sn;
         tc_fence_after_sync();
-        // A row does not fit the registers next to everything else: the first half is read for the maximum and again for the exponentials, the second half
-        // stays.  P goes over the columns of the second half, so the first half is intact when it is read again.
-        const bool masked = (p.causal && kv0 + 127 > qt) || kv0 + 128 > w.kv_len;  // diagonal block or ragged end
-        const int lim = min(w.kv_len - 1, p.causal ? q : w.kv_len) - kv0;          // last visible key of this row
+        const bool masked = (p.causal && kv0 + 63 > qt) || kv0 + 64 > w.kv_len;  // diagonal block or ragged end
+        const int lim = min(w.kv_len - 1, p.causal ? q : w.kv_len) - kv0;        // last visible key of this row
         auto prepare = [&](uint32_t (&x)[32], int k0) {
           if constexpr (BIAS) {
             const float* br = bias_row + kv0 + k0;
-            if (kv0 + 128 <= p.SK) {
+            if (kv0 + 64 <= p.SK) {
 #pragma unroll
               for (int i = 0; i < 32; ++i)
                 x[i] = __float_as_uint(fmaf(__uint_as_float(x[i]), c, __ldg(br + i) * kLog2e));
@@ -345,20 +354,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           }
           return fmaxf(fmaxf(fmaxf(mm[0], mm[1]), fmaxf(mm[2], mm[3])), start);
         };
-        float mx;
-        uint32_t x0[32], x1[32], x2[32], x3[32];
+        uint32_t x0[32], x1[32];
         tmem_ld_32x32(tm_s, x0);
         tmem_ld_32x32(tm_s + 32, x1);
         tmem_ld_wait();
         prepare(x0, 0);
         prepare(x1, 32);
-        mx = row_max(x0, x1, -INFINITY);
-        tmem_ld_32x32(tm_s + 64, x2);
-        tmem_ld_32x32(tm_s + 96, x3);
-        tmem_ld_wait();
-        prepare(x2, 64);
-        prepare(x3, 96);
-        mx = row_max(x2, x3, mx);
+        float mx = row_max(x0, x1, -INFINITY);
+        // The other half of the row: its maximum.  The slot is free again for the next block: its scores (s_full) follow
+        // this block's P of both halves, hence both reads.
+        xch[half * 128] = mx;
+        pair_sync();
+        mx = fmaxf(mx, xch[(half ^ 1) * 128]);
         if (j == 0) {
           m = mx;
         } else {
@@ -371,13 +378,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             m = mn;
             // P.V of the block before completed with s_full (products retire in issue order)
 #pragma unroll
-            for (int ch = 0; ch < HD / 32; ++ch) {
-              uint32_t oo[32];
-              tmem_ld_32x32(tm_o + ch * 32, oo);
+            for (int ch = 0; ch < HD / 32; ++ch) {  // this half's columns of O
+              uint32_t oo[16];
+              tmem_ld_32x16(tm_o + ch * 16, oo);
               tmem_ld_wait();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) oo[i] = __float_as_uint(__uint_as_float(oo[i]) * alpha);
-              tmem_st_32x32(tm_o + ch * 32, oo);
+              for (int i = 0; i < 16; ++i) oo[i] = __float_as_uint(__uint_as_float(oo[i]) * alpha);
+              tmem_st_32x16(tm_o + ch * 16, oo);
             }
           }
         }
@@ -385,7 +392,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         float2 rs[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         const float2 c2 = make_float2(cc, cc), nm2 = make_float2(-mc, -mc);
         auto exponentials = [&](const uint32_t (&x)[32], int ch) {
-          uint32_t pw[16];
+          uint32_t pw[8];
           uint32_t hash = hash_base + static_cast<uint32_t>(ch * 8) * hash_step;
 #pragma unroll
           for (int i = 0; i < 32; i += 4) {
@@ -406,20 +413,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
               w0 &= ~spread_sign_bytes(d, 0x9988);                        // sign bits of bytes 0, 1 spread over a half each
               w1 &= ~spread_sign_bytes(d, 0xBBAA);
             }
-            pw[i >> 1] = w0;
-            pw[(i >> 1) + 1] = w1;
+            pw[(i >> 1) & 7] = w0;
+            pw[((i >> 1) + 1) & 7] = w1;
+            if ((i & 15) == 12) tmem_st_32x8(tm_s + ch * 16 + (i >> 4) * 8, pw);
           }
-          tmem_st_32x16(tm_s + 64 + ch * 16, pw);
         };
-        exponentials(x2, 2);
-        tmem_ld_32x32(tm_s, x0);
-        exponentials(x3, 3);
-        tmem_ld_wait();
-        tmem_ld_32x32(tm_s + 32, x1);
-        prepare(x0, 0);
         exponentials(x0, 0);
-        tmem_ld_wait();
-        prepare(x1, 32);
         exponentials(x1, 1);
         hash_base += 32u * hash_step;
         tmem_st_wait();
@@ -433,41 +432,51 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         ++on;
         tc_fence_after_sync();
       }
+      {  // row sum: the two halves, added in one order by both (in the staging tiles, which are free here)
+        float* mine = reinterpret_cast<float*>(stage) + lane;
+        const float* other = reinterpret_cast<const float*>(sOut + (warp - 4 + (half ? -4 : 4)) * 2048) + lane;
+        *mine = l;
+        pair_sync();
+        const float lo = *other;
+        l = half ? lo + l : l + lo;
+        pair_sync();
+      }
       const float inv_l = l > 0.f ? inv_keep / l : 0.f;
+      // 32 columns at a time through shared memory: 64-byte row segments to memory
+      auto cell = [&](int row, int piece) { return stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4); };
       __nv_bfloat16* obase = reinterpret_cast<__nv_bfloat16*>(p.O) + (static_cast<size_t>(w.b) * p.SQ + qt + quarter * 32) * p.ldo +
-                             p.o_col0 + w.head * HD + (lane & 7) * 8;
+                             p.o_col0 + w.head * HD + half * (HD / 2) + (lane & 3) * 8;
       const int rows_left = p.SQ - qt - quarter * 32;
 #pragma unroll
-      for (int ch = 0; ch < CH; ++ch) {  // 64 columns at a time through shared memory: 128-byte row segments to memory
-        uint32_t oo[64];
+      for (int ch = 0; ch < HD / 64; ++ch) {
+        uint32_t oo[32];
         if (nt > 0) {
-          tmem_ld_32x32(tm_o + ch * 64, *reinterpret_cast<uint32_t(*)[32]>(&oo[0]));
-          tmem_ld_32x32(tm_o + ch * 64 + 32, *reinterpret_cast<uint32_t(*)[32]>(&oo[32]));
+          tmem_ld_32x32(tm_o + ch * 32, oo);
           tmem_ld_wait();
         } else {
 #pragma unroll
-          for (int i = 0; i < 64; ++i) oo[i] = 0u;
+          for (int i = 0; i < 32; ++i) oo[i] = 0u;
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
           uint4 v;
           v.x = pack_bf16x2(__uint_as_float(oo[8 * i + 0]) * inv_l, __uint_as_float(oo[8 * i + 1]) * inv_l);
           v.y = pack_bf16x2(__uint_as_float(oo[8 * i + 2]) * inv_l, __uint_as_float(oo[8 * i + 3]) * inv_l);
           v.z = pack_bf16x2(__uint_as_float(oo[8 * i + 4]) * inv_l, __uint_as_float(oo[8 * i + 5]) * inv_l);
           v.w = pack_bf16x2(__uint_as_float(oo[8 * i + 6]) * inv_l, __uint_as_float(oo[8 * i + 7]) * inv_l);
-          *reinterpret_cast<uint4*>(stage + lane * 128 + ((i ^ (lane & 7)) << 4)) = v;
+          *reinterpret_cast<uint4*>(cell(lane, i)) = v;
         }
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int row = i * 4 + (lane >> 3);
-          const uint4 v = *reinterpret_cast<const uint4*>(stage + row * 128 + (((lane & 7) ^ (row & 7)) << 4));
-          if (row < rows_left) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row) * p.ldo + ch * 64) = v;
+        for (int i = 0; i < 4; ++i) {
+          const int row = i * 8 + (lane >> 2);
+          const uint4 v = *reinterpret_cast<const uint4*>(cell(row, lane & 3));
+          if (row < rows_left) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row) * p.ldo + ch * 32) = v;
         }
         __syncwarp();
       }
       // rows with no visible key get +inf so that the backward probabilities exp(s - lse) vanish
-      if (q < p.SQ)
+      if (half == 0 && q < p.SQ)
         p.LSE[(static_cast<size_t>(w.b) * p.NH + w.head) * p.SQ + q] =
             l > 0.f ? m * (BIAS ? 1.0f / kLog2e : p.scale) + logf(l) : INFINITY;
       // the reads of O are ordered before the next item's P.V by the p_full arrival of its first block
