@@ -72,6 +72,13 @@ int reduce_scatter_scale_sumsq_f32_launch(void* const* peer_ptrs, void* mc_ptr, 
 int allgather_b16_launch(void* const* peer_ptrs, void* mc_ptr, void* const* flag_ptrs, int rank, int world,
                          long long n, unsigned epoch, int* status, cudaStream_t stream);
 void comm_slice_of(long long n_units, int world, int rank, long long* lo, long long* hi);
+bool conv_implicit_ok(long long M, int N, int C, int KH, int KW, int stride, int pad, bool columns_are_patches, int num_sms);
+int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, int ldw, int KH, int KW, int stride, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream);
+int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void* w, int ldw, int C, int KH, int KW, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream);
+int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int W, int C, int KH, int KW, int stride, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream);
 int bn_slices(long long rows);
 int im2col_launch(const void* x, void* cols, int N, int H, int W, int C, int KH, int KW, int stride, int pad, int Kpad,
                   int num_sms, cudaStream_t stream);
@@ -505,6 +512,80 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
 }
 
 // ------------------------------ convolution / batch-norm / pooling ------------------------------
+// k x k convolutions without a patch matrix.  conv_plan: which of {forward, input gradient, filter gradient} of this layer
+// the implicit kernels take (bits 0, 1, 2); the others go through im2col / col2im.
+int64_t conv_plan(int64_t N, int64_t H, int64_t W, int64_t C, int64_t Kout, int64_t KH, int64_t KW, int64_t stride, int64_t pad) {
+  const int64_t Ho = (H + 2 * pad - KH) / stride + 1, Wo = (W + 2 * pad - KW) / stride + 1;
+  auto ok = [&](int64_t M, int64_t n, int64_t c, bool patches) {
+    return M > 0 && M < (1LL << 31) && n < (1LL << 31) &&
+           ssb::conv_implicit_ok(M, static_cast<int>(n), static_cast<int>(c), static_cast<int>(KH), static_cast<int>(KW),
+                                 static_cast<int>(stride), static_cast<int>(pad), patches, num_sms());
+  };
+  if (C % 8 || Kout % 8 || H + 2 * pad < KH || W + 2 * pad < KW) return 0;
+  return (ok(N * Ho * Wo, Kout, C, false) ? 1 : 0) | (stride == 1 && ok(N * H * W, C, Kout, false) ? 2 : 0) |
+         (ok(Kout, KH * KW * C, C, true) ? 4 : 0);
+}
+
+void check_conv(const Tensor& x, const Tensor& w, int64_t C, int64_t KH, int64_t KW) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 4);
+  TORCH_CHECK((reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0, "convolution: 16-byte aligned activations");
+  check_bf16_2d(w, "filter");
+  TORCH_CHECK(w.size(1) == KH * KW * C && w.stride(0) % 8 == 0 && (reinterpret_cast<uintptr_t>(w.data_ptr()) & 15) == 0,
+              "convolution: filter [Cout, KH * KW * C]");
+}
+
+Tensor conv_fprop(const Tensor& x, const Tensor& w, int64_t KH, int64_t KW, int64_t stride, int64_t pad) {
+  const int64_t N = x.size(0), H = x.size(1), W = x.size(2), C = x.size(3), K = w.size(0);
+  check_conv(x, w, C, KH, KW);
+  TORCH_CHECK(conv_plan(N, H, W, C, K, KH, KW, stride, pad) & 1, "convolution: not a shape of the implicit kernel");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t Ho = (H + 2 * pad - KH) / stride + 1, Wo = (W + 2 * pad - KW) / stride + 1;
+  Tensor y = torch::empty({N, Ho, Wo, K}, x.options());
+  ssb::GemmParams p{};
+  p.M = static_cast<int>(N * Ho * Wo); p.N = static_cast<int>(K); p.K = static_cast<int>(KH * KW * C);
+  p.D = y.data_ptr(); p.ldd = static_cast<int>(K); p.alpha = 1.0f; p.status = status_tensor().data_ptr<int>();
+  check_launch(ssb::conv_fprop_launch(x.data_ptr(), N, H, W, C, w.data_ptr(), static_cast<int>(w.stride(0)), KH, KW, stride, pad, p,
+                                      num_sms(), cur_stream()), "conv_fprop");
+  return y;
+}
+
+Tensor conv_dgrad(const Tensor& dy, const Tensor& w, int64_t H, int64_t W, int64_t C, int64_t KH, int64_t KW, int64_t pad) {
+  const int64_t N = dy.size(0), K = dy.size(3);
+  check_conv(dy, w, C, KH, KW);
+  TORCH_CHECK(w.size(0) == K && dy.size(1) == H + 2 * pad - KH + 1 && dy.size(2) == W + 2 * pad - KW + 1, "convolution: dy shape");
+  TORCH_CHECK(conv_plan(N, H, W, C, K, KH, KW, 1, pad) & 2, "convolution: not a shape of the implicit kernel");
+  c10::cuda::CUDAGuard guard(dy.device());
+  Tensor dx = torch::empty({N, H, W, C}, dy.options());
+  ssb::GemmParams p{};
+  p.M = static_cast<int>(N * H * W); p.N = static_cast<int>(C); p.K = static_cast<int>(KH * KW * K);
+  p.D = dx.data_ptr(); p.ldd = static_cast<int>(C); p.alpha = 1.0f; p.status = status_tensor().data_ptr<int>();
+  check_launch(ssb::conv_dgrad_launch(dy.data_ptr(), N, H, W, K, w.data_ptr(), static_cast<int>(w.stride(0)), C, KH, KW, pad, p,
+                                      num_sms(), cur_stream()), "conv_dgrad");
+  return dx;
+}
+
+// dw fp32 [K, KH * KW * C] (+)= the filter gradient
+void conv_wgrad(const Tensor& dy, const Tensor& x, Tensor& dw, int64_t KH, int64_t KW, int64_t stride, int64_t pad, bool accumulate) {
+  const int64_t N = x.size(0), H = x.size(1), W = x.size(2), C = x.size(3), K = dy.size(1);
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 4);
+  check_bf16_2d(dy, "dy");
+  const int64_t Ho = (H + 2 * pad - KH) / stride + 1, Wo = (W + 2 * pad - KW) / stride + 1;
+  TORCH_CHECK(dy.size(0) == N * Ho * Wo, "convolution: dy rows");
+  TORCH_CHECK(dw.is_cuda() && dw.scalar_type() == torch::kFloat32 && dw.is_contiguous() && dw.size(0) == K &&
+              dw.size(1) == KH * KW * C, "convolution: dw must be fp32 [Cout, KH * KW * C]");
+  const uintptr_t low = reinterpret_cast<uintptr_t>(dy.data_ptr()) | reinterpret_cast<uintptr_t>(x.data_ptr()) |
+                        reinterpret_cast<uintptr_t>(dw.data_ptr());
+  TORCH_CHECK((low & 15) == 0 && dy.stride(0) % 8 == 0, "convolution: 16-byte aligned operands");
+  TORCH_CHECK(conv_plan(N, H, W, C, K, KH, KW, stride, pad) & 4, "convolution: not a shape of the implicit kernel");
+  c10::cuda::CUDAGuard guard(x.device());
+  ssb::GemmParams p{};
+  p.M = static_cast<int>(K); p.N = static_cast<int>(KH * KW * C); p.K = static_cast<int>(N * Ho * Wo);
+  p.D = dw.data_ptr(); p.ldd = static_cast<int>(dw.stride(0)); p.out_fp32 = 1; p.accumulate = accumulate; p.alpha = 1.0f;
+  p.status = status_tensor().data_ptr<int>();
+  check_launch(ssb::conv_wgrad_launch(dy.data_ptr(), static_cast<int>(dy.stride(0)), x.data_ptr(), N, H, W, C, KH, KW, stride, pad, p,
+                                      num_sms(), cur_stream()), "conv_wgrad");
+}
+
 // x: NHWC bf16 [N, H, W, C] contiguous -> patch matrix [N*Ho*Wo, Kpad]
 Tensor im2col(const Tensor& x, int64_t KH, int64_t KW, int64_t stride, int64_t pad, int64_t Kpad) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == torch::kBFloat16 && x.is_contiguous() && x.dim() == 4);
@@ -810,6 +891,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attn_bwd", &attn_bwd);
   m.def("set_attn_bwd_deterministic", [](bool on) { g_attn_bwd_deterministic = on; });
   m.def("attn_bwd_deterministic", []() { return g_attn_bwd_deterministic; });
+  m.def("conv_plan", &conv_plan);
+  m.def("conv_fprop", &conv_fprop);
+  m.def("conv_dgrad", &conv_dgrad);
+  m.def("conv_wgrad", &conv_wgrad);
   m.def("im2col", &im2col);
   m.def("col2im", &col2im);
   m.def("subsample", &subsample);

@@ -3,7 +3,7 @@
 // Convolutions run as GEMMs on the tcgen05 kernel of gemm_sm100.cu:
 //   1x1 stride 1 : the NHWC activation IS the [N*H*W, C] GEMM operand (no copy);
 //   1x1 stride s : `subsample` gathers the strided pixels first;
-//   k x k        : `im2col` writes the patch matrix [N*Ho*Wo, k*k*C] (tap-major, channel-minor), the
+//   k x k        : large layers gather their patches inside the GEMM (gemm2_sm100.cu); for the others `im2col` writes the patch matrix [N*Ho*Wo, k*k*C] (tap-major, channel-minor), the
 //                  filter is stored [Cout, k*k*C]; dgrad is a GEMM followed by `col2im` (gather form,
 //                  no atomics), wgrad is the MN-major GEMM of the output gradient with the patch matrix.
 // They replace cuDNN behind torch.nn.Conv2d / BatchNorm2d / MaxPool2d / AdaptiveAvgPool2d in the

@@ -30,6 +30,8 @@ namespace ssb {
 
 int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                      uint32_t box_rows, uint32_t box_cols);
+int make_tma_im2col_bf16(CUtensorMap* map, const void* base, int N, int H, int W, int C, int lower_h, int lower_w,
+                         int upper_h, int upper_w, int stride, int pixels);
 
 namespace {
 
@@ -44,6 +46,7 @@ constexpr int kEpiWarps = 16;
 constexpr int kThreads2 = 64 + kEpiWarps * 32;
 constexpr int kThreadsGather = kThreads2 + 32;    // + pusher warp
 constexpr int kGroupM2 = 8;
+constexpr int kConvNone = 0, kConvA = 1, kConvB = 2;
 constexpr int kABytes2 = BM2 * BK2 * 2;
 constexpr int kBBytes2 = BNH * BK2 * 2;
 constexpr int kStageBytes2 = kABytes2 + kBBytes2;
@@ -76,6 +79,16 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
       "[%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(smem_dst)),
       "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      : "memory");
+}
+// The same for an im2col map over an NHWC tensor: pixels from (w, h, n) on, 64 channels from c, filter tap (ow, oh).
+__device__ __forceinline__ void tma_load_im2col_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+                                                     int c, int w, int h, int n, int ow, int oh) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.im2col.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};" ::"r"(smem_u32(smem_dst)),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c), "r"(w), "r"(h), "r"(n),
+      "h"(static_cast<uint16_t>(ow)), "h"(static_cast<uint16_t>(oh))
       : "memory");
 }
 __device__ __forceinline__ void umma_f16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
@@ -150,10 +163,19 @@ __device__ __forceinline__ TileCoord2 tile_coord2(int tile, int num_m, int num_n
 // gemm_ag_sm100.cu for the protocol): tma_a addresses this rank's own rows, tma_a2 the local gather buffer, output
 // tiles are ordered own rows first, the producer waits for the "arrived" flag of a 128-row block before loading it,
 // and warp 18 pushes this rank's rows to every peer.
-template <bool A_MN, bool B_MN, bool GATHER>
+//
+// CONV: one operand is the patch matrix of a k x k convolution that never exists in memory: its tiles are fetched by TMA
+// im2col loads straight from the NHWC activation.  Writing the patch matrix (k * k times the activation), reading it
+// back and scattering its gradient were a third to a half of a 3 x 3 layer: 640 channels, 16 x 28 x 28, forward and backward
+// with BatchNorm 439 -> 317 us; 61 x 7 x 7 of 1280 channels 364 -> 311, stride 2 (64 x 28 x 28 of 640) 462 -> 410.
+//   kConvA: A's rows are pixels, the reduction runs over (tap, 64-channel block); forward (B = filter, K-major) and
+//           input gradient (A = output gradient, taps flipped, B = filter read MN-major).  A channel block that reaches past C
+//           is zero-filled, so what the filter's block holds there (the next tap) does not matter.
+//   kConvB: filter gradient; the reduction runs over the pixels, B's columns are (tap, channel), C a multiple of 64.
+template <bool A_MN, bool B_MN, bool GATHER, int CONV>
 __global__ void __launch_bounds__(GATHER ? kThreadsGather : kThreads2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a2,
-                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm) {
+                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv) {
   constexpr int kStages2 = GATHER ? kStagesGather : kStagesPlain;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -180,7 +202,8 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const int num_m = (p.M + 2 * BM2 - 1) / (2 * BM2);
   const int num_n = (p.N + BN2 - 1) / BN2;
   const int num_tiles = num_m * num_n;
-  const int num_kb = (p.K + BK2 - 1) / BK2;
+  const int conv_cblk = CONV == kConvA ? (cv.C + BK2 - 1) / BK2 : 1;  // channel blocks per tap
+  const int num_kb = CONV == kConvA ? cv.KH * cv.KW * conv_cblk : (p.K + BK2 - 1) / BK2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages2; ++s) {
@@ -233,6 +256,26 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             ta = &tma_a2;
           }
         }
+        // base position (w, h, n) of output pixel `pix`
+        auto pixel = [&](int pix, int& w, int& h, int& n) {
+          const int row = pix / cv.Wo;
+          n = row / cv.Ho;
+          h = (row - n * cv.Ho) * cv.stride + cv.lower_h;
+          w = (pix - row * cv.Wo) * cv.stride + cv.lower_w;
+        };
+        int pw = 0, ph = 0, pn = 0;       // kConvA: base position of this CTA's first row
+        int tap_r = 0, tap_s = 0, cb = 0;  // kConvA: filter tap and channel block of the K block
+        int bc[2] = {0, 0}, br[2] = {0, 0}, bs[2] = {0, 0};  // kConvB: channel and tap of the two column chunks
+        if (CONV == kConvA) pixel(min(m0, (p.M - 1) & ~(BM2 - 1)), pw, ph, pn);  // a CTA past the last row repeats it
+        if (CONV == kConvB) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int col = min(n0 + c * 64, p.N - 64), tap = col / cv.C;  // past the last column: repeated, not stored
+            bc[c] = col - tap * cv.C;
+            br[c] = tap / cv.KW;
+            bs[c] = tap - br[c] * cv.KW;
+          }
+        }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
             ok = false;
@@ -242,17 +285,42 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           const uint32_t bar = mapa_smem(smem_u32(&full_bar[stage]), 0);
           uint8_t* sa = smem_a + stage * kABytes2;
           uint8_t* sb = smem_b + stage * kBBytes2;
-          if (!A_MN) {
+          if (CONV == kConvA) {
+            const int tap = tap_r * cv.KW + tap_s;
+            const int ow = cv.flip ? cv.KW - 1 - tap_s : tap_s, oh = cv.flip ? cv.KH - 1 - tap_r : tap_r;
+            tma_load_im2col_pair(sa, ta, bar, cb * BK2, pw, ph, pn, ow, oh);
+            if (!B_MN) {
+              tma_load_2d_pair(sb, &tma_b, bar, tap * cv.tap_cols + cb * BK2, n0);
+            } else {
+#pragma unroll
+              for (int c = 0; c < BNH / 64; ++c)
+                tma_load_2d_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, tap * cv.tap_cols + n0 + c * 64, cb * BK2);
+            }
+            if (++cb == conv_cblk) {
+              cb = 0;
+              if (++tap_s == cv.KW) {
+                tap_s = 0;
+                ++tap_r;
+              }
+            }
+          } else if (!A_MN) {
             tma_load_2d_pair(sa, ta, bar, kb * BK2, m0);
           } else {
 #pragma unroll
             for (int c = 0; c < BM2 / 64; ++c) tma_load_2d_pair(sa + c * (64 * BK2 * 2), ta, bar, m0 + c * 64, kb * BK2);
           }
-          if (!B_MN) {
-            tma_load_2d_pair(sb, &tma_b, bar, kb * BK2, n0);
-          } else {
+          if (CONV == kConvB) {
+            pixel(kb * BK2, pw, ph, pn);
 #pragma unroll
-            for (int c = 0; c < BNH / 64; ++c) tma_load_2d_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, n0 + c * 64, kb * BK2);
+            for (int c = 0; c < BNH / 64; ++c)
+              tma_load_im2col_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, bc[c], pw, ph, pn, bs[c], br[c]);
+          } else if (CONV == kConvNone) {
+            if (!B_MN) {
+              tma_load_2d_pair(sb, &tma_b, bar, kb * BK2, n0);
+            } else {
+#pragma unroll
+              for (int c = 0; c < BNH / 64; ++c) tma_load_2d_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, n0 + c * 64, kb * BK2);
+            }
           }
           if (++stage == kStages2) {
             stage = 0;
@@ -489,23 +557,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   }
 }
 
-template <bool A_MN, bool B_MN, bool GATHER>
-int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams& p, const GemmAgComm& cm, int num_sms,
-                cudaStream_t stream) {
-  CUtensorMap ta, ta2, tb;
-  int rc;
-  if (GATHER) {  // A = this rank's rows [M / tp][K]; the gather buffer holds all M rows
-    rc = make_tma_2d_bf16(&ta, A, p.M / cm.tp, p.K, lda, BM2, BK2);
-    if (rc != 0) return rc;
-    rc = make_tma_2d_bf16(&ta2, cm.gather_ptrs_host_local, p.M, p.K, p.K, BM2, BK2);
-  } else {
-    rc = !A_MN ? make_tma_2d_bf16(&ta, A, p.M, p.K, lda, BM2, BK2) : make_tma_2d_bf16(&ta, A, p.K, p.M, lda, BK2, 64);
-    ta2 = ta;
-  }
-  if (rc != 0) return rc;
-  rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, BNH, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
-  if (rc != 0) return rc;
-  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER>;
+template <bool A_MN, bool B_MN, bool GATHER, int CONV>
+int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap& tb, const GemmParams& p,
+                const GemmAgComm& cm, const ConvLoad& cv, int num_sms, cudaStream_t stream) {
+  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV>;
   constexpr int threads = GATHER ? kThreadsGather : kThreads2;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -541,7 +596,26 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, ta2, tb, p, cm));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, ta2, tb, p, cm, cv));
+}
+
+template <bool A_MN, bool B_MN, bool GATHER>
+int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams& p, const GemmAgComm& cm, int num_sms,
+                cudaStream_t stream) {
+  CUtensorMap ta, ta2, tb;
+  int rc;
+  if (GATHER) {  // A = this rank's rows [M / tp][K]; the gather buffer holds all M rows
+    rc = make_tma_2d_bf16(&ta, A, p.M / cm.tp, p.K, lda, BM2, BK2);
+    if (rc != 0) return rc;
+    rc = make_tma_2d_bf16(&ta2, cm.gather_ptrs_host_local, p.M, p.K, p.K, BM2, BK2);
+  } else {
+    rc = !A_MN ? make_tma_2d_bf16(&ta, A, p.M, p.K, lda, BM2, BK2) : make_tma_2d_bf16(&ta, A, p.K, p.M, lda, BK2, 64);
+    ta2 = ta;
+  }
+  if (rc != 0) return rc;
+  rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, BNH, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
+  if (rc != 0) return rc;
+  return launch_maps<A_MN, B_MN, GATHER, kConvNone>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
 }
 
 }  // namespace
@@ -562,6 +636,51 @@ int gemm2_ag_launch(const void* W, int ldw, const GemmParams& p, const GemmAgCom
   const int rows_local = p.M / cm.tp;
   if (rows_local % (2 * BM2) || p.N < BN2 || (static_cast<size_t>(BM2) * p.K * 2) % kPushChunk2) return -100;
   return launch_pair<false, false, true>(cm.x_local, p.K, W, ldw, p, cm, num_sms, stream);
+}
+
+// Whether the implicit convolution takes this GEMM view of a k x k convolution: the two-SM tile must be worth it (the rule of
+// gemm_bf16_launch), channel blocks of 64 may waste at most a fifth of the reduction (kConvA), and the limits of an
+// im2col map hold (offsets below 256, corners within a signed byte).
+bool conv_implicit_ok(long long M, int N, int C, int KH, int KW, int stride, int pad, bool columns_are_patches, int num_sms) {
+  if (C % 8 || KH > 16 || KW > 16 || stride > 8 || pad < 0 || pad >= KH || pad >= KW || M > 0x7fffff00LL) return false;
+  if (columns_are_patches ? C % 64 != 0 : (C % 64 != 0 && C < 256)) return false;
+  const long long tiles = ((M + 255) / 256) * ((N + 255) / 256);
+  return M >= 256 && N >= 256 && tiles >= num_sms / 4;
+}
+
+// y[N, Ho, Wo, K] = conv(x[N, H, W, C], w[K, KH * KW * C]); p describes the GEMM [N Ho Wo, K] with K = KH * KW * C.
+int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, int ldw, int KH, int KW, int stride, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream) {
+  CUtensorMap ta, tb;
+  int rc;
+  if ((rc = make_tma_im2col_bf16(&ta, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BM2))) return rc;
+  if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, BNH, BK2))) return rc;
+  ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
+  return launch_maps<false, false, false, kConvA>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+}
+
+// dx[N, H, W, C] of a stride-1 convolution from dy[N, Ho, Wo, K]; p describes the GEMM [N H W, C] with K = KH * KW * K.
+int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void* w, int ldw, int C, int KH, int KW, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream) {
+  CUtensorMap ta, tb;
+  int rc;
+  const int Ho = H + 2 * pad - KH + 1, Wo = W + 2 * pad - KW + 1;
+  const int lh = pad - (KH - 1), lw = pad - (KW - 1);
+  if ((rc = make_tma_im2col_bf16(&ta, dy, N, Ho, Wo, Kout, lh, lw, -pad, -pad, 1, BM2))) return rc;
+  if ((rc = make_tma_2d_bf16(&tb, w, Kout, static_cast<uint64_t>(KH) * KW * C, ldw, BK2, 64))) return rc;
+  ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
+  return launch_maps<false, true, false, kConvA>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+}
+
+// dw[K, KH * KW * C] from dy[N Ho Wo, K] and x; p describes the GEMM [K, KH * KW * C] with K = N Ho Wo.
+int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int W, int C, int KH, int KW, int stride, int pad,
+                      const GemmParams& p, int num_sms, cudaStream_t stream) {
+  CUtensorMap ta, tb;
+  int rc;
+  if ((rc = make_tma_2d_bf16(&ta, dy, p.K, p.M, lddy, BK2, 64))) return rc;
+  if ((rc = make_tma_im2col_bf16(&tb, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BK2))) return rc;
+  ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
+  return launch_maps<true, true, false, kConvB>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
 }
 
 }  // namespace ssb

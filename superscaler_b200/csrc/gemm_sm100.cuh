@@ -51,6 +51,18 @@ struct GemmParams {
   float* split_ws;
 };
 
+// How a convolution addresses its pixels as rows of a GEMM operand (implicit patch matrix, k x k filters over NHWC): the
+// TMA im2col loads of gemm2_sm100.cu walk the output pixels in row order and add the filter tap as an offset.
+struct ConvLoad {
+  int C;                 // channels of the gathered tensor
+  int KH, KW;
+  int stride;            // between base positions of neighbouring pixels
+  int lower_h, lower_w;  // base position of pixel (0, 0): -pad, or pad - (k - 1) for the input gradient
+  int Ho, Wo;            // pixels per image
+  int flip;              // input gradient: tap (r, s) of the filter meets offset (KH - 1 - r, KW - 1 - s)
+  int tap_cols;          // columns of the filter matrix per tap
+};
+
 // Number of reduction slices gemm_bf16_launch would like for this problem (1 = none): small outputs with a long
 // reduction (weight gradients of narrow layers over many tokens or pixels) otherwise leave most SMs idle.
 int gemm_splitk_splits(int M, int N, int K, int num_sms);

@@ -1,8 +1,9 @@
 """Differentiable convolution / BatchNorm / pooling ops for NHWC bf16 activations.
 
-A convolution is a GEMM on the tcgen05 kernel: directly on the activation for 1x1 filters, on the patch matrix
-written by the im2col kernel for k x k filters (weights are stored [Cout, kh*kw*Cin], tap-major).  CPU tensors take
-plain PyTorch restatements (used by the oracles and the gloo tests).
+A convolution is a GEMM on the tcgen05 kernel (weights are stored [Cout, kh*kw*Cin], tap-major): directly on the
+activation for 1x1 filters; for k x k filters its tiles are gathered from the activation by the loads of the GEMM itself
+where the layer is large enough for the two-SM tile (`conv_plan`), else from the patch matrix written by the im2col
+kernel.  CPU tensors take plain PyTorch restatements (used by the oracles and the gloo tests).
 Reference counterparts: ParallelConvOp, ParallelBatchNormOp, ParallelMaxPoolOp, ParallelAdapAvgPoolOp
 (runtime/megatron/model/flex_ops.py:1423-1719).
 """
@@ -17,6 +18,27 @@ from .functional import _vec_grad, _wgrad, gemm
 
 def _pad8(n: int) -> int:
     return (n + 7) // 8 * 8
+
+
+FPROP, DGRAD, WGRAD = 1, 2, 4      # bits of `conv_plan`
+
+
+def _implicit_plan(ext, x, w, kh, kw, stride, pad) -> int:
+    """Which passes of a k x k convolution gather their patches inside the GEMM (bits FPROP, DGRAD, WGRAD)."""
+    N, H, W, C = x.shape
+    if w.shape[1] != kh * kw * C or not w.is_contiguous() or (x.data_ptr() | w.data_ptr()) % 16:
+        return 0
+    return ext.conv_plan(N, H, W, C, w.shape[0], kh, kw, stride, pad)
+
+
+def _conv_wgrad(w, g, x, kh, kw, stride, pad):
+    """As `functional._wgrad`, on the activation instead of its patch matrix."""
+    mg = getattr(w, "main_grad", None)
+    out = mg.view(w.shape[0], -1) if mg is not None else torch.empty(w.shape, dtype=torch.float32, device=w.device)
+    if out.data_ptr() % 16 or not out.is_contiguous() or g.data_ptr() % 16:
+        return _wgrad(w, g, native.ext().im2col(x, kh, kw, stride, pad, w.shape[1]))
+    native.ext().conv_wgrad(g, x, out, kh, kw, stride, pad, mg is not None)
+    return None if mg is not None else out.to(w.dtype)
 
 
 class Conv2dFn(torch.autograd.Function):
@@ -37,7 +59,20 @@ class Conv2dFn(torch.autograd.Function):
             xs = x if stride == 1 else ext.subsample(x.contiguous(), H, W, stride, False)
             a = xs.reshape(-1, C)
         else:
-            a = ext.im2col(x.contiguous(), kh, kw, stride, pad, w.shape[1])
+            a = x.contiguous()
+            plan = ctx.plan = _implicit_plan(ext, a, w, kh, kw, stride, pad)
+            if plan & FPROP:
+                y = ext.conv_fprop(a, w, kh, kw, stride, pad)
+                ctx.save_for_backward(a, w)
+                return y
+            if not plan & WGRAD:
+                # the patch matrix serves the forward and the filter gradient
+                a = ext.im2col(a, kh, kw, stride, pad, w.shape[1])
+                y = gemm(a, w)
+            else:
+                y = gemm(ext.im2col(a, kh, kw, stride, pad, w.shape[1]), w)
+            ctx.save_for_backward(a, w)
+            return y.view(N, Ho, Wo, -1)
         y = gemm(a, w)
         ctx.save_for_backward(a, w)
         return y.view(N, Ho, Wo, -1)
@@ -57,9 +92,17 @@ class Conv2dFn(torch.autograd.Function):
             return gx.to(x.dtype), _vec_grad(w, gw), None, None, None, None
         ext = native.ext()
         g = dy.reshape(-1, dy.shape[-1]).contiguous()
-        dw = _wgrad(w, g, a) if ctx.needs_input_grad[1] else None
-        dx = None
+        dw = dx = None
+        if ctx.needs_input_grad[1]:
+            if kh == 1 and kw == 1 or not ctx.plan & (FPROP | WGRAD):
+                dw = _wgrad(w, g, a)
+            elif ctx.plan & WGRAD:
+                dw = _conv_wgrad(w, g, a, kh, kw, stride, pad)
+            else:           # the forward kept the activation only
+                dw = _wgrad(w, g, ext.im2col(a, kh, kw, stride, pad, w.shape[1]))
         if ctx.needs_input_grad[0]:
+            if not (kh == 1 and kw == 1) and ctx.plan & DGRAD:
+                return ext.conv_dgrad(g.view(N, Ho, Wo, -1), w, H, W, C, kh, kw, pad), dw, None, None, None, None
             da = gemm(g, w, b_mn=True)                      # [N*Ho*Wo, Kpad]
             if kh == 1 and kw == 1:
                 da = da.view(N, Ho, Wo, C)
