@@ -79,6 +79,9 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
                       const GemmParams& p, int num_sms, cudaStream_t stream);
 int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int W, int C, int KH, int KW, int stride, int pad,
                       const GemmParams& p, int num_sms, cudaStream_t stream);
+bool ce_fused_ok(int V);
+int ce_fused_launch(void* logits, int ld, const long long* targets, const float* loss_mask, float* loss, long long rows, int V,
+                    long long v0, float grad_scale, cudaStream_t stream);
 int bn_slices(long long rows);
 int im2col_launch(const void* x, void* cols, int N, int H, int W, int C, int KH, int KW, int stride, int pad, int Kpad,
                   int num_sms, cudaStream_t stream);
@@ -418,6 +421,24 @@ Tensor ce_finalize(Tensor& logits, const Tensor& targets, const Tensor& stats, c
                                        logits.size(0), static_cast<int>(logits.size(1)), v0,
                                        static_cast<float>(grad_scale), write_grad, cur_stream()),
                "ce_finalize");
+  return loss;
+}
+
+// Per-row loss of logits held by this rank alone; overwrites them with d loss_sum / d logits * grad_scale.
+Tensor ce_loss_grad(Tensor& logits, const Tensor& targets, const OptTensor& loss_mask, int64_t v0, double grad_scale) {
+  check_bf16_2d(logits, "logits");
+  if (!ssb::ce_fused_ok(static_cast<int>(logits.size(1))))
+    return ce_finalize(logits, targets, ce_stats(logits, targets, v0), loss_mask, v0, grad_scale, true);
+  TORCH_CHECK(targets.scalar_type() == torch::kInt64 && targets.is_contiguous() && targets.numel() == logits.size(0));
+  c10::cuda::CUDAGuard guard(logits.device());
+  Tensor loss = torch::empty({logits.size(0)}, torch::dtype(torch::kFloat32).device(logits.device()));
+  if (loss_mask.has_value()) TORCH_CHECK(loss_mask->scalar_type() == torch::kFloat32 && loss_mask->is_contiguous());
+  check_launch(ssb::ce_fused_launch(logits.data_ptr(), static_cast<int>(logits.stride(0)),
+                                    reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()),
+                                    loss_mask.has_value() ? loss_mask->data_ptr<float>() : nullptr, loss.data_ptr<float>(),
+                                    logits.size(0), static_cast<int>(logits.size(1)), v0, static_cast<float>(grad_scale),
+                                    cur_stream()),
+               "ce_loss_grad");
   return loss;
 }
 
@@ -885,6 +906,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);
   m.def("embedding_bwd_sorted", &embedding_bwd_sorted);
+  m.def("ce_loss_grad", &ce_loss_grad);
   m.def("ce_stats", &ce_stats);
   m.def("ce_finalize", &ce_finalize);
   m.def("attn_fwd", &attn_fwd);

@@ -220,7 +220,91 @@ ce_finalize_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* 
   }
 }
 
+// Loss and gradient of whole rows in one pass over memory, for logits that no other rank shares.  The row is read once, into
+// shared memory; every thread keeps a running maximum and the sum of exponentials relative to it on the way, so that the
+// special-function unit works under the loads, and only the gradient is left for a second pass.  Same quantities as
+// ce_stats + ce_finalize, which read the row three times.  Two CTAs per SM: one loads while the other writes.  Head and loss
+// of 4096 rows x 51200, forward and backward: 2571 -> 2532 us; the kernel itself 232 us (3.6 TB/s, two exponentials an element).
+constexpr int kCeThreads = 512;
+constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per SM
+
+__global__ void __launch_bounds__(kCeThreads, 2)
+ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __restrict__ targets,
+                const float* __restrict__ loss_mask, float* __restrict__ loss, int V, long long v0, float grad_scale) {
+  extern __shared__ uint4 row_smem[];
+  __shared__ float sm[32];
+  const long long row = blockIdx.x;
+  __nv_bfloat16* x = logits + row * ld;
+  uint4* xv = reinterpret_cast<uint4*>(x);
+  const int nvec = V / 8;
+  const int k0 = nvec * 8 + threadIdx.x;           // at most seven columns behind the last whole vector
+  const float tail = k0 < V ? __bfloat162float(x[k0]) : -INFINITY;
+  const long long t = targets[row] - v0;
+  const float tgt = (t >= 0 && t < V) ? __bfloat162float(x[t]) : 0.f;
+  __syncthreads();                                 // the target is read before any thread overwrites the row
+  float tmax = tail, tsum = tail != -INFINITY ? __expf(tail - tail) : 0.f;  // this thread's maximum and sum exp(x - maximum)
+  for (int v = threadIdx.x; v < nvec; v += 4 * kCeThreads) {
+    uint4 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (v + u * kCeThreads < nvec) q[u] = __ldcs(xv + v + u * kCeThreads);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (v + u * kCeThreads < nvec) {
+        row_smem[v + u * kCeThreads] = q[u];       // each thread reads back what it wrote: no barrier needed
+        const float2 a = unpack_bf16x2(q[u].x), b = unpack_bf16x2(q[u].y), c = unpack_bf16x2(q[u].z), d = unpack_bf16x2(q[u].w);
+        const float m8 = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y)), fmaxf(fmaxf(c.x, c.y), fmaxf(d.x, d.y)));
+        if (m8 > tmax) {
+          tsum *= __expf(tmax - m8);               // tmax = -inf: 0
+          tmax = m8;
+        }
+        const float off = tmax == -INFINITY ? 0.f : tmax;
+        tsum += ((__expf(a.x - off) + __expf(a.y - off)) + (__expf(b.x - off) + __expf(b.y - off))) +
+                ((__expf(c.x - off) + __expf(c.y - off)) + (__expf(d.x - off) + __expf(d.y - off)));
+      }
+    }
+  }
+  const float mx = block_reduce(tmax, true, sm);
+  const float s = block_reduce(tmax == -INFINITY ? tsum : tsum * __expf(tmax - mx), false, sm);
+  const float w = loss_mask ? loss_mask[row] : 1.0f;
+  if (threadIdx.x == 0) loss[row] = (logf(s) + mx - tgt) * w;
+  const float inv = 1.0f / s, gs = grad_scale * w;
+  for (int v = threadIdx.x; v < nvec; v += kCeThreads) {
+    const uint4 q = row_smem[v];
+    const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
+    float f[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float pr = __expf(f[j] - mx) * inv;
+      if (static_cast<long long>(v) * 8 + j == t) pr -= 1.0f;
+      f[j] = pr * gs;
+    }
+    uint4 o;
+    o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
+    o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
+    xv[v] = o;
+  }
+  if (k0 < V) {
+    float pr = __expf(tail - mx) * inv;
+    if (k0 == t) pr -= 1.0f;
+    x[k0] = __float2bfloat16(pr * gs);
+  }
+}
+
 }  // namespace
+
+bool ce_fused_ok(int V) { return V <= kCeMaxCols; }
+
+int ce_fused_launch(void* logits, int ld, const long long* targets, const float* loss_mask, float* loss, long long rows, int V,
+                    long long v0, float grad_scale, cudaStream_t stream) {
+  if (ld % 8) return -3;
+  const int smem = (V / 8) * 16;
+  const int rc = static_cast<int>(cudaFuncSetAttribute(ce_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeMaxCols * 2));
+  if (rc) return rc;
+  ce_fused_kernel<<<static_cast<unsigned>(rows), kCeThreads, smem, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets,
+                                                                             loss_mask, loss, V, v0, grad_scale);
+  return static_cast<int>(cudaGetLastError());
+}
 
 int embedding_fwd_launch(const long long* ids, const long long* pos, const void* W, const void* P, void* out,
                          long long tokens, int H, long long v0, long long v1, float dropout_p,

@@ -775,14 +775,16 @@ class LMHeadCrossEntropyFn(torch.autograd.Function):
         logits = gemm(x, W)
         tflat = targets.contiguous().view(-1)
         if x.is_cuda:
-            st = native.ext().ce_stats(logits, tflat, v0)
             if group is not None and torch.distributed.get_world_size(group) > 1:
+                st = native.ext().ce_stats(logits, tflat, v0)
                 gmax = st[0].clone()
                 torch.distributed.all_reduce(gmax, op=torch.distributed.ReduceOp.MAX, group=group)
                 st[1].mul_(torch.exp(st[0] - gmax))
                 st[0].copy_(gmax)
                 torch.distributed.all_reduce(st[1:], group=group)
-            losses = native.ext().ce_finalize(logits, tflat, st, loss_mask, v0, loss_scale, True)
+                losses = native.ext().ce_finalize(logits, tflat, st, loss_mask, v0, loss_scale, True)
+            else:
+                losses = native.ext().ce_loss_grad(logits, tflat, loss_mask, v0, loss_scale)
             loss = losses.sum() * loss_scale
             dlogits = logits
         else:
@@ -829,8 +831,7 @@ class CrossEntropyFn(torch.autograd.Function):
         tflat = targets.contiguous().view(-1)
         if logits.is_cuda:
             work = logits.contiguous().clone()
-            st = native.ext().ce_stats(work, tflat, 0)
-            losses = native.ext().ce_finalize(work, tflat, st, None, 0, loss_scale, True)
+            losses = native.ext().ce_loss_grad(work, tflat, None, 0, loss_scale)
             ctx.save_for_backward(work)
             return losses.sum() * loss_scale
         lf = logits.float()

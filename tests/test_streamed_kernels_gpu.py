@@ -14,6 +14,30 @@ def _rel(a, e):
     return float((a.double() - e).norm() / e.norm().clamp_min(1e-30))
 
 
+@pytest.mark.parametrize("V,ld", [(8, 8), (1000, 1000), (1003, 1008), (51200, 51200), (57344, 57344), (57352, 57352)])
+def test_cross_entropy_rows(V, ld):
+    rows = 5
+    g = torch.Generator(device="cuda").manual_seed(V)
+    buf = (torch.randn(rows, ld, generator=g, device="cuda") * 4).bfloat16()
+    buf[1, : V // 2] = float("-inf")                      # half a row masked out
+    t = torch.randint(V // 2, V, (rows,), generator=g, device="cuda")
+    t[2] = V + 3                                          # another rank's target: no entry of this row
+    w = torch.rand(rows, generator=g, device="cuda")
+    x = buf[:, :V].double()
+    work = buf.clone()
+    loss = native.ext().ce_loss_grad(work[:, :V], t, w, 0, 0.5)
+    lse = torch.logsumexp(x, -1)
+    own = t < V
+    hit = torch.zeros(rows, dtype=torch.float64, device="cuda")
+    hit[own] = x[own, t[own]]
+    assert torch.allclose(loss.double(), (lse - hit) * w.double(), rtol=1e-5, atol=1e-5)
+    grad = torch.softmax(x, -1)
+    grad[own, t[own]] -= 1.0
+    grad = grad * w.double()[:, None] * 0.5
+    assert _rel(work[:, :V], grad) < 2.0 ** -8
+    assert torch.equal(work[:, V:], buf[:, V:])
+
+
 @pytest.mark.parametrize("n,start", [(1, 0), (5, 0), (4096, 0), (4099, 0), (300001, 0), (4096, 1), (4096, 2)])
 def test_adam_vector_and_scalar_parts(n, start):
     g = torch.Generator(device="cuda").manual_seed(n)
