@@ -47,7 +47,9 @@ int embedding_fwd_launch(const long long* ids, const long long* pos, const void*
 int embedding_bwd_launch(const long long* ids, const long long* pos, const void* g, float* dW, float* dP,
                          long long tokens, int H, long long v0, long long v1, float dropout_p,
                          unsigned long long seed, int num_sms, cudaStream_t stream);
-int embedding_bwd_sorted_launch(const long long* keys, const long long* order, const void* g, float* dst,
+int embedding_keys_launch(const long long* ids, void* keys, int key_bytes, long long tokens, long long k0, long long n,
+                          cudaStream_t stream);
+int embedding_bwd_sorted_launch(const void* keys, int key_bytes, const long long* order, const void* g, float* dst,
                                 long long tokens, int H, long long k0, long long k1, float dropout_p,
                                 unsigned long long seed, cudaStream_t stream);
 int ce_stats_launch(const void* logits, int ld, const long long* targets, float* row_max, float* row_sum,
@@ -375,14 +377,27 @@ void embedding_bwd(const Tensor& ids, const OptTensor& pos, const Tensor& g, con
 }
 
 // dst[key - k0] += sum of the (dropout-masked) rows of g whose key equals `key`; keys ascending, order[p] = token of keys[p]
+// Keys for the sort in front of embedding_bwd_sorted: rows of a table of n rows that starts at id k0, in the narrowest type
+// that holds them (ids outside become n, which that call skips with k0 = 0).
+Tensor embedding_keys(const Tensor& ids, int64_t k0, int64_t n) {
+  TORCH_CHECK(ids.is_cuda() && ids.scalar_type() == torch::kInt64 && ids.is_contiguous() && n >= 0 && n < 0x7fffffffLL);
+  c10::cuda::CUDAGuard guard(ids.device());
+  Tensor keys = torch::empty({ids.numel()}, ids.options().dtype(n < 0x7fff ? torch::kInt16 : torch::kInt32));
+  check_launch(ssb::embedding_keys_launch(reinterpret_cast<const long long*>(ids.data_ptr<int64_t>()), keys.data_ptr(),
+                                          static_cast<int>(keys.element_size()), ids.numel(), k0, n, cur_stream()),
+               "embedding_keys");
+  return keys;
+}
+
 void embedding_bwd_sorted(const Tensor& keys, const Tensor& order, const Tensor& g, const Tensor& dst, int64_t k0,
                           double dropout_p, int64_t seed) {
   TORCH_CHECK(g.scalar_type() == torch::kBFloat16 && g.is_contiguous() && g.is_cuda());
-  TORCH_CHECK(keys.scalar_type() == torch::kInt64 && order.scalar_type() == torch::kInt64 && keys.is_contiguous() &&
-              order.is_contiguous() && keys.numel() == order.numel() && keys.numel() * g.size(-1) == g.numel());
+  const auto kt = keys.scalar_type();
+  TORCH_CHECK((kt == torch::kInt64 || kt == torch::kInt32 || kt == torch::kInt16) && keys.is_cuda() &&
+              order.scalar_type() == torch::kInt64 && keys.is_contiguous() && order.is_contiguous() && keys.numel() == order.numel() && keys.numel() * g.size(-1) == g.numel());
   TORCH_CHECK(dst.scalar_type() == torch::kFloat32 && dst.is_contiguous() && dst.size(-1) == g.size(-1));
   c10::cuda::CUDAGuard guard(g.device());
-  check_launch(ssb::embedding_bwd_sorted_launch(reinterpret_cast<const long long*>(keys.data_ptr<int64_t>()),
+  check_launch(ssb::embedding_bwd_sorted_launch(keys.data_ptr(), static_cast<int>(keys.element_size()),
                                                 reinterpret_cast<const long long*>(order.data_ptr<int64_t>()),
                                                 g.data_ptr(), dst.data_ptr<float>(), keys.numel(),
                                                 static_cast<int>(g.size(-1)), k0, k0 + dst.size(0),
@@ -905,6 +920,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sgd_step", &sgd_step);
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);
+  m.def("embedding_keys", &embedding_keys);
   m.def("embedding_bwd_sorted", &embedding_bwd_sorted);
   m.def("ce_loss_grad", &ce_loss_grad);
   m.def("ce_stats", &ce_stats);

@@ -97,8 +97,9 @@ embedding_bwd_kernel(const long long* __restrict__ ids, const long long* __restr
 // ascending order and `order[p]` is the token that holds keys[p].  Block p works only if it is the first of its
 // run of equal keys; it then sums the run's rows in the order given and adds the total to row keys[p] - k0 of dst
 // with plain stores (no other block touches that row), so repeated runs give bitwise equal results.
+template <typename Key>
 __global__ void __launch_bounds__(256)
-embedding_bwd_sorted_kernel(const long long* __restrict__ keys, const long long* __restrict__ order,
+embedding_bwd_sorted_kernel(const Key* __restrict__ keys, const long long* __restrict__ order,
                             const __nv_bfloat16* __restrict__ g, float* __restrict__ dst, long long tokens, int H,
                             long long k0, long long k1, float dropout_p, unsigned long long seed) {
   const long long p = blockIdx.x;
@@ -133,6 +134,17 @@ embedding_bwd_sorted_kernel(const long long* __restrict__ keys, const long long*
     hi.x += acc[4]; hi.y += acc[5]; hi.z += acc[6]; hi.w += acc[7];
     out[0] = lo;
     out[1] = hi;
+  }
+}
+
+// Sort keys of the rows a table holds: ids of [k0, k0 + n) as 0 .. n - 1, every other id as n.  In 16 or 32 bits the radix sort
+// makes two or four passes over the tokens instead of the eight that 64-bit ids take (9 us each for 16384 tokens).
+template <typename Key>
+__global__ void __launch_bounds__(256)
+embedding_keys_kernel(const long long* __restrict__ ids, Key* __restrict__ keys, long long tokens, long long k0, long long n) {
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < tokens; i += gridDim.x * 256LL) {
+    const long long id = ids[i];
+    keys[i] = static_cast<Key>(id >= k0 && id - k0 < n ? id - k0 : n);
   }
 }
 
@@ -330,13 +342,34 @@ int embedding_bwd_launch(const long long* ids, const long long* pos, const void*
   return static_cast<int>(cudaGetLastError());
 }
 
-int embedding_bwd_sorted_launch(const long long* keys, const long long* order, const void* g, float* dst,
+// key_bytes: 2, 4 or 8 (short, int, long long)
+int embedding_keys_launch(const long long* ids, void* keys, int key_bytes, long long tokens, long long k0, long long n,
+                          cudaStream_t stream) {
+  if (tokens < 1) return -4;
+  const long long want = (tokens + 255) / 256;
+  const unsigned blocks = static_cast<unsigned>(want < 1184 ? want : 1184);
+  if (key_bytes == 2)
+    embedding_keys_kernel<<<blocks, 256, 0, stream>>>(ids, reinterpret_cast<short*>(keys), tokens, k0, n);
+  else if (key_bytes == 4)
+    embedding_keys_kernel<<<blocks, 256, 0, stream>>>(ids, reinterpret_cast<int*>(keys), tokens, k0, n);
+  else
+    return -2;
+  return static_cast<int>(cudaGetLastError());
+}
+
+int embedding_bwd_sorted_launch(const void* keys, int key_bytes, const long long* order, const void* g, float* dst,
                                 long long tokens, int H, long long k0, long long k1, float dropout_p,
                                 unsigned long long seed, cudaStream_t stream) {
   if (H % 8) return -3;
   if (tokens < 1 || tokens > 0x7fffffffLL) return -4;
-  embedding_bwd_sorted_kernel<<<static_cast<unsigned>(tokens), 256, 0, stream>>>(
-      keys, order, reinterpret_cast<const __nv_bfloat16*>(g), dst, tokens, H, k0, k1, dropout_p, seed);
+  const auto* gb = reinterpret_cast<const __nv_bfloat16*>(g);
+  const unsigned blocks = static_cast<unsigned>(tokens);
+  if (key_bytes == 2)
+    embedding_bwd_sorted_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const short*>(keys), order, gb, dst, tokens, H, k0, k1, dropout_p, seed);
+  else if (key_bytes == 4)
+    embedding_bwd_sorted_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const int*>(keys), order, gb, dst, tokens, H, k0, k1, dropout_p, seed);
+  else
+    embedding_bwd_sorted_kernel<<<blocks, 256, 0, stream>>>(reinterpret_cast<const long long*>(keys), order, gb, dst, tokens, H, k0, k1, dropout_p, seed);
   return static_cast<int>(cudaGetLastError());
 }
 

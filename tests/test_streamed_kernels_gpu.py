@@ -57,3 +57,23 @@ def test_adam_vector_and_scalar_parts(n, start):
     pd = pd - 1e-2 * ((md / (1 - 0.9 ** 7)) / ((vd / (1 - 0.999 ** 7)).sqrt() + 1e-8) + decay * pd)
     assert _rel(m, md) < 1e-6 and _rel(v, vd) < 1e-6 and _rel(p, pd) < 1e-5
     assert torch.equal(p16, p.bfloat16()) and not grad.any()
+
+
+@pytest.mark.parametrize("n", [300, 4096])                # below and at the token count that takes them
+@pytest.mark.parametrize("V", [3, 32766, 32767, 40000])   # 16-bit keys up to 32766 rows, 32-bit beyond
+def test_embedding_gradient_keys(V, n):
+    H, v0 = 64, 5
+    g = torch.Generator(device="cuda").manual_seed(V)
+    ids = torch.randint(v0, v0 + V, (2, n), generator=g, device="cuda")
+    ids[0, :4] = torch.tensor([0, v0 - 1, v0 + V, 2 ** 40], device="cuda")    # outside the table, one past 32 bits
+    ids[1, 10:60] = v0 + V - 1                                               # a long run
+    W = torch.nn.Parameter(torch.randn(V, H, generator=g, device="cuda").bfloat16())
+    W.main_grad = torch.zeros(V, H, device="cuda")
+    y = F.embedding(ids, None, W, None, v0)
+    dy = torch.randn(2 * n, H, generator=g, device="cuda").bfloat16()
+    y.backward(dy)
+    want = torch.zeros(V, H, dtype=torch.float64, device="cuda")
+    flat = ids.view(-1) - v0
+    ok = (flat >= 0) & (flat < V)
+    want.index_add_(0, flat[ok], dy.double()[ok])
+    assert _rel(W.main_grad, want) < 1e-6
