@@ -23,7 +23,7 @@ int ln_bwd_slices(int rows);
 int ln_bwd_part_rows(int rows, int H, int num_sms);
 int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                          const void* dres, void* dx, float* dgamma, float* dbeta, float* part_g, float* part_b,
-                         int accumulate_wgrad, int rows, int H, int num_sms, cudaStream_t stream);
+                         int accumulate_wgrad, int rows, int H, int* status, int num_sms, cudaStream_t stream);
 int colsum_tickets();
 int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N,
                   cudaStream_t stream);
@@ -236,7 +236,7 @@ Tensor layernorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& gamma, con
   check_launch(ssb::layernorm_bwd_launch(dy.data_ptr(), x.data_ptr(), gamma.data_ptr<float>(), mean.data_ptr<float>(),
                                          rstd.data_ptr<float>(), opt_ptr(dres), dx.data_ptr(), dgamma.data_ptr<float>(),
                                          dbeta.data_ptr<float>(), part[0].data_ptr<float>(), part[1].data_ptr<float>(),
-                                         accumulate, rows, H, num_sms(), cur_stream()),
+                                         accumulate, rows, H, status_tensor().data_ptr<int>(), num_sms(), cur_stream()),
                "layernorm_bwd");
   return dx;
 }

@@ -5,8 +5,9 @@
 // backward produces dx and per-column partial sums for dgamma / dbeta that a
 // second small kernel folds (deterministic, no atomics).
 //
-// HBM-bound: every kernel moves 16 bytes per lane per access and keeps the row in
-// registers between the statistics pass and the normalisation pass.
+// HBM-bound.  The one-pass backward streams rows through a ring of shared-memory stages filled by bulk asynchronous
+// copies, so that the bytes in flight (about 100 KB per SM) do not depend on how many registers a warp can spare; the
+// other kernels move 16 bytes per lane per access.
 #include "common.cuh"
 
 namespace ssb {
@@ -201,129 +202,189 @@ ln_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
   }
 }
 
-// One pass over dy and x for H = VPL * 256 * WPR: dx, and in the same sweep every lane keeps running sums of
-// dy * xhat and dy for its 8 * VPL columns over all rows its warp visits.  WPR warps share a row (each owns a
-// contiguous part of the columns, so that the running sums fit in registers) and exchange their two row sums through
-// shared memory.  The warps of a block fold their column sums through shared memory in a fixed order and the block
-// writes ONE row of partials (part_g[block][h], part_b[block][h]); fold_partials_kernel adds the blocks.  dy and x
-// are read once instead of twice, and the result does not depend on the order of execution.
-template <int VPL, int WPR>
-__global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
-ln_bwd_onepass_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                      const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
-                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                      float* __restrict__ part_g, float* __restrict__ part_b, int rows, int H) {
-  constexpr int RPB = kLnWarpsPerBlock / WPR;        // rows a block works on at a time
-  __shared__ float fold_g[VPL * 256 * WPR], fold_b[VPL * 256 * WPR];
+constexpr int kLnWarps = 8;        // warps that compute; one more issues the copies
+constexpr int kLnStages = 3;
+
+// Ring of stages filled by one thread; `chunk` c of this block sits in stage c % kLnStages.
+struct LnRing {
+  uint64_t* full;
+  uint64_t* empty;
+  volatile int* abort_flag;
+  __device__ __forceinline__ bool wait_full(int c) const {
+    return mbar_wait_one(&full[c % kLnStages], (c / kLnStages) & 1);
+  }
+  __device__ __forceinline__ bool wait_empty(int c) const {
+    return mbar_wait_one(&empty[c % kLnStages], ((c / kLnStages) & 1) ^ 1);
+  }
+  __device__ __forceinline__ bool mbar_wait_one(uint64_t* bar, uint32_t parity) const {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+  }
+  __device__ __forceinline__ void release(int c, int lane) const {  // one arrival per computing warp
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&empty[c % kLnStages]);
+  }
+};
+
+__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
+  const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+
+// One pass over dy, x and dres for any H <= 512 * WPR: dx, and in the same sweep every lane keeps running sums of
+// dy * xhat and dy for its 16 columns over all rows its warp visits (their gamma stays in registers).  A chunk is
+// 8 / WPR consecutive rows of the three matrices; WPR warps share a row (each owns 512 columns) and exchange their two
+// row sums through shared memory.  The warps of a block fold their column sums through shared memory in a fixed order
+// and the block writes ONE row of partials (part_g[block][h], part_b[block][h]); fold_partials2_kernel adds the blocks.
+// The result does not depend on the order of execution.  32768 x 2048 with residual gradient, this kernel and the fold:
+// 119 -> 106 us (register-staged form, H 1024 and 2048 only; other H took two kernels that read dy and x twice).  The
+// same ring under the forward changed nothing (68 us: bound by its arithmetic), so that stays as it was.
+template <int WPR>
+__global__ void __launch_bounds__((kLnWarps + 1) * 32, 2)
+ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                     const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
+                     const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                     float* __restrict__ part_g, float* __restrict__ part_b, int rows, int H, int* __restrict__ status) {
+  constexpr int VPL = 2, RPB = kLnWarps / WPR;       // vectors per lane, rows of a chunk
+  extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ float xch[2][RPB][WPR][2];
+  __shared__ uint64_t bars[2 * kLnStages];
+  __shared__ int aborted;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int rslot = warp / WPR, part = warp % WPR;
-  const int v0 = part * VPL * 32;                    // first 16-byte vector of this warp's columns
+  const int row_bytes = H * 2, part_bytes = RPB * row_bytes, stage_bytes = 3 * part_bytes, nvec = H / 8;
+  const int chunks = (rows + RPB - 1) / RPB;
+  float* fold_g = reinterpret_cast<float*>(ring_smem + kLnStages * stage_bytes);  // [512 WPR] each
+  float* fold_b = fold_g + 512 * WPR;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < kLnStages; ++i) {
+      mbar_init(&bars[i], 1);
+      mbar_init(&bars[kLnStages + i], kLnWarps);
+    }
+    aborted = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  const LnRing ring{bars, bars + kLnStages, &aborted};
   float ag[VPL][8], ab[VPL][8];
-#pragma unroll
-  for (int i = 0; i < VPL; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ag[i][j] = ab[i][j] = 0.f;
-  int it = 0;
-  // every warp of a row slot runs the same number of iterations: the named barrier below is reached by all of them
-  for (int row = blockIdx.x * RPB + rslot; row < rows; row += gridDim.x * RPB, ++it) {
-    const uint4* dyr = reinterpret_cast<const uint4*>(dy + static_cast<size_t>(row) * H);
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
-    const float mu = mean[row], rs = rstd[row];
-    uint4 qd[VPL], qx[VPL];
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      qd[i] = dyr[v0 + i * 32 + lane];
-      qx[i] = xr[v0 + i * 32 + lane];
-    }
-    float s1 = 0.f, s2 = 0.f;
-#pragma unroll
-    for (int i = 0; i < VPL; ++i) {
-      const int v = v0 + i * 32 + lane;
-      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * v);
-      const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * v + 1);
-      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-      const float2 d0 = unpack_bf16x2(qd[i].x), d1 = unpack_bf16x2(qd[i].y), d2 = unpack_bf16x2(qd[i].z), d3 = unpack_bf16x2(qd[i].w);
-      const float2 x0 = unpack_bf16x2(qx[i].x), x1 = unpack_bf16x2(qx[i].y), x2 = unpack_bf16x2(qx[i].z), x3 = unpack_bf16x2(qx[i].w);
-      const float d[8] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y};
-      const float xv[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float xhat = (xv[j] - mu) * rs;
-        const float dg = d[j] * g[j];
-        s1 += dg;
-        s2 += dg * xhat;
-        ag[i][j] += d[j] * xhat;
-        ab[i][j] += d[j];
-      }
-    }
-    s1 = warp_sum(s1);
-    s2 = warp_sum(s2);
-    if constexpr (WPR > 1) {
-      float* slot = &xch[it & 1][rslot][0][0];
+  const int rslot = warp / WPR, part = warp % WPR;
+  if (warp == kLnWarps) {
+    int c = 0;
+    for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
+      if (!ring.wait_empty(c)) break;
       if (lane == 0) {
-        slot[part * 2] = s1;
-        slot[part * 2 + 1] = s2;
+        const int st = c % kLnStages, bytes = min(RPB, rows - ch * RPB) * row_bytes;
+        const size_t at = static_cast<size_t>(ch) * RPB * H;
+        uint8_t* dst = ring_smem + st * stage_bytes;
+        mbar_arrive_expect_tx(&bars[st], bytes * (dres ? 3 : 2));
+        bulk_load(dst, dy + at, bytes, &bars[st]);
+        bulk_load(dst + part_bytes, x + at, bytes, &bars[st]);
+        if (dres) bulk_load(dst + 2 * part_bytes, dres + at, bytes, &bars[st]);
       }
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + rslot), "r"(32 * WPR) : "memory");
-      s1 = 0.f;
-      s2 = 0.f;
-#pragma unroll
-      for (int w = 0; w < WPR; ++w) {
-        s1 += slot[w * 2];
-        s2 += slot[w * 2 + 1];
-      }
+      __syncwarp();
     }
-    s1 /= static_cast<float>(H);
-    s2 /= static_cast<float>(H);
-    uint4* dxr = reinterpret_cast<uint4*>(dx + static_cast<size_t>(row) * H);
-    const uint4* drr = dres ? reinterpret_cast<const uint4*>(dres + static_cast<size_t>(row) * H) : nullptr;
+  } else {
+    const float inv_h = 1.0f / static_cast<float>(H);
+    float g[VPL][8];
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
-      const int v = v0 + i * 32 + lane;
-      const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * v);
-      const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma) + 2 * v + 1);
-      const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-      const float2 d0 = unpack_bf16x2(qd[i].x), d1 = unpack_bf16x2(qd[i].y), d2 = unpack_bf16x2(qd[i].z), d3 = unpack_bf16x2(qd[i].w);
-      const float2 x0 = unpack_bf16x2(qx[i].x), x1 = unpack_bf16x2(qx[i].y), x2 = unpack_bf16x2(qx[i].z), x3 = unpack_bf16x2(qx[i].w);
-      const float d[8] = {d0.x, d0.y, d1.x, d1.y, d2.x, d2.y, d3.x, d3.y};
-      const float xv[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
-      float o[8];
+      const int v = (part * VPL + i) * 32 + lane;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float xhat = (xv[j] - mu) * rs;
-        o[j] = rs * (d[j] * g[j] - s1 - xhat * s2);
+        g[i][j] = v < nvec ? __ldg(gamma + v * 8 + j) : 0.f;  // once: any alignment
+        ag[i][j] = ab[i][j] = 0.f;
       }
-      if (drr) {
-        const uint4 qr = drr[v];
-        const float2 r0 = unpack_bf16x2(qr.x), r1 = unpack_bf16x2(qr.y), r2 = unpack_bf16x2(qr.z), r3 = unpack_bf16x2(qr.w);
-        o[0] += r0.x; o[1] += r0.y; o[2] += r1.x; o[3] += r1.y; o[4] += r2.x; o[5] += r2.y; o[6] += r3.x; o[7] += r3.y;
+    }
+    int c = 0;
+    for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
+      const int row = ch * RPB + rslot;
+      const bool have = row < rows;                  // the same for all warps of a row slot
+      const float mu = have ? __ldg(mean + row) : 0.f, rs = have ? __ldg(rstd + row) : 0.f;
+      if (!ring.wait_full(c)) break;
+      if (have) {
+        const uint8_t* base = ring_smem + (c % kLnStages) * stage_bytes + rslot * row_bytes;
+        const uint4* pd = reinterpret_cast<const uint4*>(base);
+        const uint4* px = reinterpret_cast<const uint4*>(base + part_bytes);
+        const uint4* pr = reinterpret_cast<const uint4*>(base + 2 * part_bytes);
+        float d[VPL][8], xh[VPL][8], s1 = 0.f, s2 = 0.f;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+          const int v = (part * VPL + i) * 32 + lane;
+          const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+          float xv[8];
+          unpack8(v < nvec ? pd[v] : zero, d[i]);
+          unpack8(v < nvec ? px[v] : zero, xv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            xh[i][j] = (xv[j] - mu) * rs;
+            const float dg = d[i][j] * g[i][j];
+            s1 += dg;
+            s2 += dg * xh[i][j];
+            ag[i][j] += d[i][j] * xh[i][j];
+            ab[i][j] += d[i][j];
+          }
+        }
+        s1 = warp_sum(s1);
+        s2 = warp_sum(s2);
+        if constexpr (WPR > 1) {
+          float* slot = &xch[c & 1][rslot][0][0];
+          if (lane == 0) {
+            slot[part * 2] = s1;
+            slot[part * 2 + 1] = s2;
+          }
+          asm volatile("bar.sync %0, %1;" ::"r"(1 + rslot), "r"(32 * WPR) : "memory");
+          s1 = 0.f;
+          s2 = 0.f;
+#pragma unroll
+          for (int w = 0; w < WPR; ++w) {
+            s1 += slot[w * 2];
+            s2 += slot[w * 2 + 1];
+          }
+        }
+        s1 *= inv_h;
+        s2 *= inv_h;
+        uint4* dxr = reinterpret_cast<uint4*>(dx) + static_cast<size_t>(row) * nvec;
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) {
+          const int v = (part * VPL + i) * 32 + lane;
+          if (v >= nvec) break;
+          float o[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = rs * (d[i][j] * g[i][j] - s1 - xh[i][j] * s2);
+          if (dres) {
+            float r[8];
+            unpack8(pr[v], r);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += r[j];
+          }
+          uint4 w;
+          w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]);
+          w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
+          dxr[v] = w;
+        }
       }
-      uint4 w;
-      w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]);
-      w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
-      dxr[v] = w;
+      ring.release(c, lane);
     }
   }
+  __syncthreads();
   // fold the row slots of the block in the order 0, 1, ...: slot s adds its warps' sums to the columns they own
   for (int sl = 0; sl < RPB; ++sl) {
-    if (rslot == sl) {
+    if (warp < kLnWarps && rslot == sl) {
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
-        const int c = (v0 + i * 32 + lane) * 8;
+        const int col = ((part * VPL + i) * 32 + lane) * 8;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          fold_g[c + j] = (sl == 0 ? 0.f : fold_g[c + j]) + ag[i][j];
-          fold_b[c + j] = (sl == 0 ? 0.f : fold_b[c + j]) + ab[i][j];
+          fold_g[col + j] = (sl == 0 ? 0.f : fold_g[col + j]) + ag[i][j];
+          fold_b[col + j] = (sl == 0 ? 0.f : fold_b[col + j]) + ab[i][j];
         }
       }
     }
     __syncthreads();
   }
-  for (int c = threadIdx.x; c < H; c += blockDim.x) {
-    part_g[static_cast<size_t>(blockIdx.x) * H + c] = fold_g[c];
-    part_b[static_cast<size_t>(blockIdx.x) * H + c] = fold_b[c];
+  for (int col = threadIdx.x; col < H; col += blockDim.x) {
+    part_g[static_cast<size_t>(blockIdx.x) * H + col] = fold_g[col];
+    part_b[static_cast<size_t>(blockIdx.x) * H + col] = fold_b[col];
   }
+  if (threadIdx.x == 0 && aborted && status != nullptr) atomicMax(status, static_cast<int>(kStatusMbarTimeout));
 }
 
 // Partial column sums over a slice of rows: part_g[slice][h] = sum dy*xhat, part_b[slice][h] = sum dy.
@@ -377,24 +438,25 @@ __global__ void fold_partials_kernel(const float* __restrict__ part, float* __re
   out[h] = accumulate ? out[h] + s : s;
 }
 
-// Both LayerNorm weight gradients in one launch: block (x, which) folds 64 columns of part_g (which = 0) or part_b
-// (which = 1); its 256 threads are 64 columns x 4 groups of slices, added in a fixed order.
-__global__ void __launch_bounds__(256)
+// Both LayerNorm weight gradients in one launch: block (x, which) folds 32 columns of part_g (which = 0) or part_b
+// (which = 1); its 1024 threads are 32 columns x 32 groups of slices, added in a fixed order (four groups per column took
+// 11 us for 296 slices: a chain of 74 loads).
+__global__ void __launch_bounds__(1024)
 fold_partials2_kernel(const float* __restrict__ part_g, const float* __restrict__ part_b, float* __restrict__ dgamma,
                       float* __restrict__ dbeta, int slices, int H, int accumulate) {
-  __shared__ float sm[4][64];
+  __shared__ float sm[32][33];
   const float* part = blockIdx.y == 0 ? part_g : part_b;
   float* out = blockIdx.y == 0 ? dgamma : dbeta;
-  const int c = threadIdx.x & 63, sg = threadIdx.x >> 6, h = blockIdx.x * 64 + c;
+  const int c = threadIdx.x & 31, sg = threadIdx.x >> 5, h = blockIdx.x * 32 + c;
   float s = 0.f;
   if (h < H)
-    for (int k = sg; k < slices; k += 4) s += part[static_cast<size_t>(k) * H + h];
+    for (int k = sg; k < slices; k += 32) s += part[static_cast<size_t>(k) * H + h];
   sm[sg][c] = s;
   __syncthreads();
-  if (sg == 0 && h < H) {
-    const float t = (sm[0][c] + sm[1][c]) + (sm[2][c] + sm[3][c]);
-    out[h] = accumulate ? out[h] + t : t;
-  }
+  // warp w adds column w's 32 groups by a butterfly: the same order every time
+  const float t = warp_sum(sm[c][sg]);
+  const int hw = blockIdx.x * 32 + sg;
+  if (c == 0 && hw < H) out[hw] = accumulate ? out[hw] + t : t;
 }
 
 // Column sum of a bf16 matrix [rows, N] (bias gradients) in ONE launch, for 16-byte aligned rows (N, lda multiples
@@ -497,6 +559,8 @@ colsum_partial_kernel(const __nv_bfloat16* __restrict__ a, int lda, float* __res
 
 }  // namespace
 
+constexpr int kLnStreamMaxH = 512 * kLnWarps;
+
 int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
                          void* sum_out, float* mean, float* rstd, int rows, int H, float eps, int num_sms,
                          cudaStream_t stream) {
@@ -509,7 +573,9 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
   auto* sb = reinterpret_cast<__nv_bfloat16*>(sum_out);
 #define SSB_LN_CASE(V)                                                                                       \
   ln_fwd_kernel<V><<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
-  switch (H) {
+  // 16-byte loads of gamma and beta; parameters that start elsewhere take the generic kernel
+  const bool wide = ((reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0;
+  switch (wide ? H : 0) {
     case 512: SSB_LN_CASE(2); break;
     case 1024: SSB_LN_CASE(4); break;
     case 2048: SSB_LN_CASE(8); break;
@@ -526,47 +592,58 @@ int ln_bwd_slices(int rows) {
   return s < 1 ? 1 : (s > 128 ? 128 : s);
 }
 
+static int ln_bwd_warps_per_row(int H) { return H <= 512 ? 1 : H <= 1024 ? 2 : H <= 2048 ? 4 : 8; }
+
 // Rows of partial sums the backward needs in each of part_g / part_b (then H floats per row).
 int ln_bwd_part_rows(int rows, int H, int num_sms) {
-  if (H == 1024 || H == 2048) {  // one-pass kernel: one row of partials per block
-    const int rpb = H == 1024 ? kLnWarpsPerBlock : kLnWarpsPerBlock / 2;   // rows a block works on at a time
+  if (H <= kLnStreamMaxH) {  // one-pass kernel: one row of partials per block, two resident blocks per SM
+    const int rpb = kLnWarps / ln_bwd_warps_per_row(H);
     const int want = (rows + rpb - 1) / rpb;
-    const int cap = num_sms * (H == 1024 ? 2 : 3);   // resident blocks per SM at the kernels' register counts
-    return want < cap ? want : cap;
+    return want < num_sms * 2 ? want : num_sms * 2;
   }
   return ln_bwd_slices(rows);
 }
 
 int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                          const void* dres, void* dx, float* dgamma, float* dbeta, float* part_g, float* part_b,
-                         int accumulate_wgrad, int rows, int H, int num_sms, cudaStream_t stream) {
+                         int accumulate_wgrad, int rows, int H, int* status, int num_sms, cudaStream_t stream) {
   if (H % 8) return -3;
   const auto* dyb = reinterpret_cast<const __nv_bfloat16*>(dy);
   const auto* xb = reinterpret_cast<const __nv_bfloat16*>(x);
   const auto* drb = reinterpret_cast<const __nv_bfloat16*>(dres);
   auto* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
-  if (H == 1024 || H == 2048) {
+  // 16-byte copies of the three matrices; the partial rows that ln_bwd_part_rows promised also hold the two-kernel form's
+  const bool wide = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dres)) & 15) == 0;
+  if (H <= kLnStreamMaxH && wide) {
     // dy and x are read once: dx and the per-column sums come out of the same sweep
-    const int nb = ln_bwd_part_rows(rows, H, num_sms);
-    const dim3 g(nb), b(kLnWarpsPerBlock * 32);
-    if (H == 1024)
-      ln_bwd_onepass_kernel<4, 1><<<g, b, 0, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, part_g, part_b, rows, H);
-    else
-      ln_bwd_onepass_kernel<4, 2><<<g, b, 0, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, part_g, part_b, rows, H);
-    fold_partials2_kernel<<<dim3((H + 63) / 64, 2), 256, 0, stream>>>(part_g, part_b, dgamma, dbeta, nb, H,
+    const int nb = ln_bwd_part_rows(rows, H, num_sms), wpr = ln_bwd_warps_per_row(H);
+    const int smem = kLnStages * 3 * (kLnWarps / wpr) * H * 2 + 2 * 512 * wpr * 4;
+    int rc = 0;
+#define SSB_LN_BWD(W)                                                                                                        \
+  rc = static_cast<int>(cudaFuncSetAttribute(ln_bwd_stream_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));    \
+  if (rc) return rc;                                                                                                         \
+  ln_bwd_stream_kernel<W><<<nb, (kLnWarps + 1) * 32, smem, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, part_g, part_b, rows, H, status)
+    switch (wpr) {
+      case 1: SSB_LN_BWD(1); break;
+      case 2: SSB_LN_BWD(2); break;
+      case 4: SSB_LN_BWD(4); break;
+      default: SSB_LN_BWD(8); break;
+    }
+#undef SSB_LN_BWD
+    fold_partials2_kernel<<<dim3((H + 31) / 32, 2), 1024, 0, stream>>>(part_g, part_b, dgamma, dbeta, nb, H,
                                                                       accumulate_wgrad);
     return static_cast<int>(cudaGetLastError());
   }
   const int blocks = min((rows + kLnWarpsPerBlock - 1) / kLnWarpsPerBlock, num_sms * 16);
   const dim3 g(blocks), b(kLnWarpsPerBlock * 32);
   ln_bwd_dx_kernel<<<g, b, 0, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, rows, H);
-  const int slices = ln_bwd_slices(rows);
+  const int slices = min(ln_bwd_slices(rows), ln_bwd_part_rows(rows, H, num_sms));
   const int rps = (rows + slices - 1) / slices;
   dim3 grid((H / 2 + 31) / 32, slices);
   ln_bwd_gb_partial_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(dy),
                                                      reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd, part_g,
                                                      part_b, rows, H, rps);
-  fold_partials2_kernel<<<dim3((H + 63) / 64, 2), 256, 0, stream>>>(part_g, part_b, dgamma, dbeta, slices, H,
+  fold_partials2_kernel<<<dim3((H + 31) / 32, 2), 1024, 0, stream>>>(part_g, part_b, dgamma, dbeta, slices, H,
                                                                     accumulate_wgrad);
   return static_cast<int>(cudaGetLastError());
 }

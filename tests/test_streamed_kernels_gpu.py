@@ -14,6 +14,28 @@ def _rel(a, e):
     return float((a.double() - e).norm() / e.norm().clamp_min(1e-30))
 
 
+@pytest.mark.parametrize("rows", [1, 7, 301])
+@pytest.mark.parametrize("H", [8, 64, 504, 520, 1096, 2048, 2056, 4096, 4104])
+@pytest.mark.parametrize("shift", [0, 1])        # 1: gamma / beta start 4 bytes off a 16-byte boundary
+def test_layernorm_rows(rows, H, shift):
+    g = torch.Generator(device="cuda").manual_seed(H + rows)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, dy, dres = (r(rows, H).bfloat16() for _ in range(3))
+    x.requires_grad_(True)
+    par = [torch.nn.Parameter((r(H + 4) + 1.0)[shift:shift + H]) for _ in range(2)]
+    for p in par:
+        p.main_grad = torch.zeros(H, device="cuda")
+    y, keep = F.layernorm_keep_input(x, *par, 1e-5)
+    torch.autograd.backward([y, keep], [dy, dres])
+    t = [v.detach().double().requires_grad_(True) for v in (x, *par)]
+    want = TF.layer_norm(t[0], (H,), t[1], t[2], 1e-5)
+    dx, dg, db = torch.autograd.grad(want, t, dy.double())
+    # one bf16 rounding of y and dx; fp32 sums over the rows
+    assert _rel(y, want.detach()) < 2.0 ** -8
+    assert _rel(x.grad, dx + dres.double()) < 2.0 ** -8
+    assert _rel(par[0].main_grad, dg) < 1e-5 and _rel(par[1].main_grad, db) < 1e-5
+
+
 @pytest.mark.parametrize("V,ld", [(8, 8), (1000, 1000), (1003, 1008), (51200, 51200), (57344, 57344), (57352, 57352)])
 def test_cross_entropy_rows(V, ld):
     rows = 5
