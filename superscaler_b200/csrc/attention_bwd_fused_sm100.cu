@@ -42,8 +42,8 @@
 
 namespace ssb {
 
-int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                     uint32_t box_rows, uint32_t box_cols);
+int make_tma_batched_bf16(CUtensorMap* map, const void* base, uint64_t batches, uint64_t rows, uint64_t ld,
+                          uint32_t box_rows, uint32_t box_cols);
 
 namespace {
 
@@ -146,16 +146,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     reg_dealloc<kFusedRegsIssue>();
     if (warp == 0 && elect_one() && n_it > 0) {
       // ---------------------------------------- TMA producer ----------------------------------------
-      const int qrow0 = b * p.SQ + i0 * 128;
       auto load_tile = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int col, int row) {
 #pragma unroll
-        for (int c = 0; c < CH; ++c) tma_load_2d(dst + c * 16384, tm, bar, col + c * 64, row);
+        for (int c = 0; c < CH; ++c) tma_load_3d(dst + c * 16384, tm, bar, col + c * 64, row, b);
       };
       auto load_q = [&](int i) {
         const int st = i & 1;
         if (!mbar_wait(&q_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) return false;
         mbar_arrive_expect_tx(&q_full[st], Cfg::kTile + Cfg::kStatBytes);
-        load_tile(sQ + st * Cfg::kTile, &tm_q, &q_full[st], p.q_col0 + head * HD, qrow0 + i * 128);
+        load_tile(sQ + st * Cfg::kTile, &tm_q, &q_full[st], p.q_col0 + head * HD, (i0 + i) * 128);
         bulk_load(sStat + st * 256, p.LSE + (tile0 + i) * 128, 512, &q_full[st]);
         bulk_load(sStat + st * 256 + 128, p.delta + (tile0 + i) * 128, 512, &q_full[st]);
         return true;
@@ -164,16 +163,16 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         const int st = i & 1;
         if (!mbar_wait(&do_empty[st], ((i >> 1) & 1) ^ 1, abort_flag)) return false;
         mbar_arrive_expect_tx(&do_full[st], Cfg::kTile);
-        load_tile(sdO + st * Cfg::kTile, &tm_do, &do_full[st], p.o_col0 + head * HD, qrow0 + i * 128);
+        load_tile(sdO + st * Cfg::kTile, &tm_do, &do_full[st], p.o_col0 + head * HD, (i0 + i) * 128);
         return true;
       };
       mbar_arrive_expect_tx(k_full, Cfg::kTile);
-      load_tile(sK, &tm_k, k_full, p.k_col0 + head * HD, b * p.SK + kv0);
+      load_tile(sK, &tm_k, k_full, p.k_col0 + head * HD, kv0);
       int nq = 0, ndo = 0;  // loads issued
       bool ok = load_q(0);
       nq += ok;
       mbar_arrive_expect_tx(v_full, Cfg::kTile);
-      load_tile(sV, &tm_v, v_full, p.v_col0 + head * HD, b * p.SK + kv0);
+      load_tile(sV, &tm_v, v_full, p.v_col0 + head * HD, kv0);
       if (ok) ok = load_do(0);
       ndo += ok;
       for (int i = 1; i < n_it && ok; ++i) {
@@ -403,7 +402,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           }
           a = mul_f32x2(make_float2(pr[q], pr[q + 1]), a);
           b2 = mul_f32x2(make_float2(pr[q + 2], pr[q + 3]), b2);
-          if (need_mask) {  // rows and keys outside hold another sample's data, or nothing: not even 0 x NaN may enter
+          if (need_mask) {  // rows and keys outside: not even 0 x NaN (from the padded statistics) may enter
             if (q < lo || q >= hi) a.x = 0.f;
             if (q + 1 < lo || q + 1 >= hi) a.y = 0.f;
             if (q + 2 < lo || q + 2 >= hi) b2.x = 0.f;
@@ -636,12 +635,13 @@ int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const 
   AttnParams pp = p;
   pp.delta = nd;
   pp.LSE = nlse2;
+  // Blocks past the end of a sample read zeros: P and dS are zero there, and zero times an infinity or NaN of the next
+  // sample must not enter this one's gradients.
   CUtensorMap tq, tk, tv, tdo;
-  const uint64_t rq = static_cast<uint64_t>(p.B) * p.SQ, rk = static_cast<uint64_t>(p.B) * p.SK;
-  if ((rc = make_tma_2d_bf16(&tq, q, rq, ldq, ldq, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tdo, dout, rq, lddo, lddo, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tk, k, rk, ldk, ldk, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tv, v, rk, ldv, ldv, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tq, q, p.B, p.SQ, ldq, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tdo, dout, p.B, p.SQ, lddo, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tk, k, p.B, p.SK, ldk, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tv, v, p.B, p.SK, ldv, 128, 64))) return rc;
   const bool drop = p.dropout_p > 0.f;
   if (p.bias_table != nullptr) {
     if (p.dbias_table == nullptr) return -2;

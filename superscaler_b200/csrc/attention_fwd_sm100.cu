@@ -37,8 +37,8 @@
 
 namespace ssb {
 
-int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
-                     uint32_t box_rows, uint32_t box_cols);
+int make_tma_batched_bf16(CUtensorMap* map, const void* base, uint64_t batches, uint64_t rows, uint64_t ld,
+                          uint32_t box_rows, uint32_t box_cols);
 
 namespace {
 
@@ -160,12 +160,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       Pipe pp;
       uint32_t qn[2] = {0, 0};  // items loaded per tile
       bool ok = true;
-      auto load_kv = [&](const CUtensorMap* tm, int col0, int row) {
+      auto load_kv = [&](const CUtensorMap* tm, int col0, int row, int b) {
         if (!mbar_wait(&kv_empty[pp.stage], pp.phase ^ 1, abort_flag)) return false;
         mbar_arrive_expect_tx(&kv_full[pp.stage], Cfg::kTile);
 #pragma unroll
         for (int c = 0; c < CH; ++c)
-          tma_load_2d(sKV + pp.stage * Cfg::kTile + c * 16384, tm, &kv_full[pp.stage], col0 + c * 64, row);
+          tma_load_3d(sKV + pp.stage * Cfg::kTile + c * 16384, tm, &kv_full[pp.stage], col0 + c * 64, row, b);
         pp.advance(NS);
         return true;
       };
@@ -180,15 +180,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             mbar_arrive_expect_tx(&q_full[t], Cfg::kTile);
 #pragma unroll
             for (int c = 0; c < CH; ++c)
-              tma_load_2d(sQ + t * Cfg::kTile + c * 16384, &tm_q, &q_full[t], p.q_col0 + w.head * HD + c * 64,
-                          w.b * p.SQ + w.q0 + t * 128);
+              tma_load_3d(sQ + t * Cfg::kTile + c * 16384, &tm_q, &q_full[t], p.q_col0 + w.head * HD + c * 64,
+                          w.q0 + t * 128, w.b);
             ++qn[t];
           }
-          if (t == 0) ok = load_kv(&tm_k, kcol, w.b * p.SK);
+          if (t == 0) ok = load_kv(&tm_k, kcol, 0, w.b);
         }
         for (int j = 0; j < n && ok; ++j) {
-          ok = load_kv(&tm_v, vcol, w.b * p.SK + j * 128);
-          if (ok && j + 1 < n) ok = load_kv(&tm_k, kcol, w.b * p.SK + (j + 1) * 128);
+          ok = load_kv(&tm_v, vcol, j * 128, w.b);
+          if (ok && j + 1 < n) ok = load_kv(&tm_k, kcol, (j + 1) * 128, w.b);
         }
       }
       if (!ok) {  // let the copies in flight land before the CTA leaves
@@ -516,11 +516,13 @@ int attn_fwd_launch(const void* q, int ldq, const void* k, int ldk, const void* 
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (p.ldo % 8) || (p.q_col0 % 8) || (p.k_col0 % 8) || (p.v_col0 % 8) ||
       (p.o_col0 % 8))
     return -3;
+  // Blocks past the end of a sample read zeros: a probability of zero times whatever the next sample holds there, an
+  // infinity or NaN among it, must not enter this one.
   CUtensorMap tq, tk, tv;
   int rc;
-  if ((rc = make_tma_2d_bf16(&tq, q, static_cast<uint64_t>(p.B) * p.SQ, ldq, ldq, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tk, k, static_cast<uint64_t>(p.B) * p.SK, ldk, ldk, 128, 64))) return rc;
-  if ((rc = make_tma_2d_bf16(&tv, v, static_cast<uint64_t>(p.B) * p.SK, ldv, ldv, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tq, q, p.B, p.SQ, ldq, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tk, k, p.B, p.SK, ldk, 128, 64))) return rc;
+  if ((rc = make_tma_batched_bf16(&tv, v, p.B, p.SK, ldv, 128, 64))) return rc;
   const bool drop = p.dropout_p > 0.f, bias = p.bias_table != nullptr;
 #define SSB_FWD(HD, D, BI) launch_fwd<HD, D, BI>(tq, tk, tv, p, num_sms, stream)
   if (p.HD == 128)

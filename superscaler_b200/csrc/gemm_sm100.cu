@@ -293,6 +293,27 @@ int make_tma_2d_bf16(CUtensorMap* map, const void* base, uint64_t rows, uint64_t
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
 
+// `batches` such matrices of `rows` rows one after the other: a box that reaches past the rows of its matrix is filled with
+// zeros there instead of the next matrix's rows.
+int make_tma_batched_bf16(CUtensorMap* map, const void* base, uint64_t batches, uint64_t rows, uint64_t ld,
+                          uint32_t box_rows, uint32_t box_cols) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (fn == nullptr) return -1;
+  static thread_local bool ctx_bound = false;  // as above
+  if (!ctx_bound) {
+    cudaFree(nullptr);
+    ctx_bound = true;
+  }
+  cuuint64_t dims[3] = {ld, rows, batches};
+  cuuint64_t strides[2] = {ld * 2, rows * ld * 2};
+  cuuint32_t box[3] = {box_cols, box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+
 // NHWC bf16 tensor in im2col mode: a load takes `pixels` consecutive base positions of the bounding box
 // [lower, size - 1 + upper] (stepping by `stride`, row by row, image by image) and 64 channels; zero fill outside.
 int make_tma_im2col_bf16(CUtensorMap* map, const void* base, int N, int H, int W, int C, int lower_h, int lower_w,

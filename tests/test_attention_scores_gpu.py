@@ -31,3 +31,30 @@ def test_rows_of_one_value_are_exact(HD, blocks):
     q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16().contiguous()
     o = F.flash_attention(q, k, v, 1, 1, rows, S, HD, scale=math.log(2.0))
     assert torch.equal(o, v[:1].expand(rows, HD))
+
+
+@pytest.mark.parametrize("SQ,SK,HD,causal", [(64, 128, 64, False), (192, 256, 128, False), (100, 77, 64, False),
+                                             (64, 64, 128, True), (321, 321, 64, True)])
+def test_samples_keep_their_nans(SQ, SK, HD, causal):
+    """Blocks that reach past the end of a sample must not bring in what the next one holds: with NaNs and infinities in the
+    second of three samples the results of the others stay what they are with zeros in it."""
+    B, NH = 3, 2
+    g = torch.Generator(device="cuda").manual_seed(SQ)
+    w = NH * HD
+    made = [torch.randn(B, n, w, generator=g, device="cuda") for n in (SQ, SK, SK, SQ)]
+    out = []
+    for bad in (0.0, float("nan"), float("inf")):
+        q, k, v, do = (t.clone() for t in made)
+        for t in (q, k, v, do):
+            t[1] = bad
+        q, k, v, do = (t.view(-1, w).bfloat16() for t in (q, k, v, do))
+        for t in (q, k, v):
+            t.requires_grad_(True)
+        y = F.flash_attention(q, k, v, B, NH, SQ, SK, HD, causal=causal)
+        y.backward(do)
+        out.append([t.detach().view(B, -1, w)[[0, 2]] for t in (y, q.grad, k.grad, v.grad)])
+    for other in out[1:]:
+        for a, e in zip(other, out[0]):
+            assert torch.isfinite(a).all()
+            # dq is summed over the key blocks in the order they finish: fp32 sums, then one rounding to bf16
+            assert float((a.double() - e.double()).norm()) <= 2.0 ** -9 * float(e.double().norm())
