@@ -561,10 +561,12 @@ colsum_partial_kernel(const __nv_bfloat16* __restrict__ a, int lda, float* __res
 
 constexpr int kLnStreamMaxH = 512 * kLnWarps;
 
+static bool misaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
+
 int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
                          void* sum_out, float* mean, float* rstd, int rows, int H, float eps, int num_sms,
                          cudaStream_t stream) {
-  if (H % 8) return -3;
+  if (H % 8 || misaligned(x) || misaligned(residual) || misaligned(y) || misaligned(sum_out)) return -3;
   const int blocks = min((rows + kLnWarpsPerBlock - 1) / kLnWarpsPerBlock, num_sms * 16);
   const dim3 grid(blocks), block(kLnWarpsPerBlock * 32);
   const auto* xb = reinterpret_cast<const __nv_bfloat16*>(x);
@@ -574,7 +576,7 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
 #define SSB_LN_CASE(V)                                                                                       \
   ln_fwd_kernel<V><<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
   // 16-byte loads of gamma and beta; parameters that start elsewhere take the generic kernel
-  const bool wide = ((reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta)) & 15) == 0;
+  const bool wide = !misaligned(gamma) && !misaligned(beta);
   switch (wide ? H : 0) {
     case 512: SSB_LN_CASE(2); break;
     case 1024: SSB_LN_CASE(4); break;
@@ -612,9 +614,8 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   const auto* xb = reinterpret_cast<const __nv_bfloat16*>(x);
   const auto* drb = reinterpret_cast<const __nv_bfloat16*>(dres);
   auto* dxb = reinterpret_cast<__nv_bfloat16*>(dx);
-  // 16-byte copies of the three matrices; the partial rows that ln_bwd_part_rows promised also hold the two-kernel form's
-  const bool wide = ((reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dres)) & 15) == 0;
-  if (H <= kLnStreamMaxH && wide) {
+  if (misaligned(dy) || misaligned(x) || misaligned(dres) || misaligned(dx)) return -3;  // every kernel moves 16 bytes a lane
+  if (H <= kLnStreamMaxH) {
     // dy and x are read once: dx and the per-column sums come out of the same sweep
     const int nb = ln_bwd_part_rows(rows, H, num_sms), wpr = ln_bwd_warps_per_row(H);
     const int smem = kLnStages * 3 * (kLnWarps / wpr) * H * 2 + 2 * 512 * wpr * 4;
@@ -637,7 +638,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   const int blocks = min((rows + kLnWarpsPerBlock - 1) / kLnWarpsPerBlock, num_sms * 16);
   const dim3 g(blocks), b(kLnWarpsPerBlock * 32);
   ln_bwd_dx_kernel<<<g, b, 0, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, rows, H);
-  const int slices = min(ln_bwd_slices(rows), ln_bwd_part_rows(rows, H, num_sms));
+  const int slices = ln_bwd_slices(rows);
   const int rps = (rows + slices - 1) / slices;
   dim3 grid((H / 2 + 31) / 32, slices);
   ln_bwd_gb_partial_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(dy),

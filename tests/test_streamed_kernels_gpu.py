@@ -99,3 +99,19 @@ def test_embedding_gradient_keys(V, n):
     ok = (flat >= 0) & (flat < V)
     want.index_add_(0, flat[ok], dy.double()[ok])
     assert _rel(W.main_grad, want) < 1e-6
+
+
+@pytest.mark.parametrize("H", [512, 520, 2048, 4104])
+def test_layernorm_refuses_misaligned_rows(H):
+    """The kernels move 16 bytes a lane: contiguous matrices that start elsewhere are an error on the host."""
+    rows, ext = 9, native.ext()
+    even = torch.zeros(rows, H, dtype=torch.bfloat16, device="cuda")
+    odd = torch.zeros(rows * H + 8, dtype=torch.bfloat16, device="cuda")[1:rows * H + 1].view(rows, H)
+    gamma, stat = torch.ones(H, device="cuda"), torch.ones(rows, device="cuda")
+    dg, db = torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda")
+    for x, res in ((odd, None), (even, odd)):
+        with pytest.raises(RuntimeError, match="layernorm_fwd"):
+            ext.layernorm_fwd(x, res, gamma, gamma, 1e-5)
+    for dy, x, dres in ((odd, even, None), (even, odd, None), (even, even, odd)):
+        with pytest.raises(RuntimeError, match="layernorm_bwd"):
+            ext.layernorm_bwd(dy, x, gamma, stat, stat, dres, dg, db, False)
