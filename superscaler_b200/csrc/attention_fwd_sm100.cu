@@ -287,8 +287,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t tm_s = tm_row + half * 64, tm_o = tm_row + 256 + half * (HD / 2);
     uint8_t* stage = sOut + (warp - 4) * 2048;
     float* xch = sXch + t * 256 + r;   // + half * 128
-    auto pair_sync = [&]() {  // the two warps that share these 32 rows
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory");
+    // The two warps that share these 32 rows meet once per key block and twice per item.
+    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory"); };
+    // A warp whose bounded wait ran out in its k-th item, `left` meetings before the item's end, still comes to all the
+    // meetings ahead: its partner may pass the same wait a moment later and must not be left waiting (its own next wait runs
+    // out too, P of this warp being missing).  An mbarrier with the bounded wait at every meeting costs 10 % (one sequence of
+    // 16 heads 41.0 -> 45.1 us), a barrier that tells both whether one gave up 5 % (43.0).
+    auto meet_to_the_end = [&](int k, int left) {
+      for (int idx;;) {
+        for (; left > 0; --left) pair_sync();
+        if ((idx = fwd_item_index(++k, items.total)) < 0) return;
+        if (idx >= items.total) continue;
+        const FwdItem w = fwd_item(idx, items, p);
+        left = w.q0 + t * 128 < p.SQ ? w.n[t] + 2 : 0;
+      }
     };
     const float c = p.scale * kLog2e;
     // With a bias the logits are brought into the log2 domain first (x c + bias log2 e) and everything below works on
@@ -320,7 +332,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < nt; ++j) {
         const int kv0 = j * 128 + half * 64;
-        if (!mbar_wait_warp(&s_full[t], sn & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&s_full[t], sn & 1, abort_flag)) {
+          meet_to_the_end(k, nt - j + 2);
+          ok = false;
+          break;
+        }
         ++sn;
         tc_fence_after_sync();
         const bool masked = (p.causal && kv0 + 63 > qt) || kv0 + 64 > w.kv_len;  // diagonal block or ragged end
@@ -426,7 +442,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       }
       if (!ok) break;
       if (nt > 0) {
-        if (!mbar_wait_warp(&o_full[t], on & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&o_full[t], on & 1, abort_flag)) {
+          meet_to_the_end(k, 2);
+          break;
+        }
         ++on;
         tc_fence_after_sync();
       }

@@ -1,0 +1,26 @@
+"""Every wait inside a kernel has a limit.  A named barrier has none, so where warps meet at one, a warp whose bounded wait
+ran out may not simply leave: it has to come to all the meetings that are ahead, or its partner, whose own wait may have
+succeeded a moment later, hangs."""
+import re
+from pathlib import Path
+
+import pytest
+
+import superscaler_b200
+
+CSRC = Path(superscaler_b200.__file__).parent / "csrc"
+NAMED = r'"(?:bar|barrier)(?:\.cta)?\.(?:sync|red)\b'
+
+
+def _blocks_of_failed_waits(code):
+    """What stands between each bounded wait that ran out and the `break` that follows."""
+    return [m.group(1) for m in re.finditer(r"if \(!(?:mbar_wait_warp|ring\.wait_full)\([^;{]*\)\s*\{?(.*?)\bbreak;", code, re.S)]
+
+
+@pytest.mark.parametrize("path", sorted(CSRC.glob("attention*.cu")), ids=lambda p: p.name)
+def test_warps_that_give_up_still_meet_their_partners(path):
+    code = re.sub(r"//[^\n]*", "", path.read_text())
+    for body in re.split(r"\b__global__\b", code)[1:]:
+        if re.search(NAMED, body):
+            left = _blocks_of_failed_waits(body)
+            assert left and all("meet_to_the_end(" in b for b in left)
