@@ -281,6 +281,12 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
       }
       __syncwarp();
     }
+    // The last copies land before the block may end, also where the computing warps have given up on them.
+    if (lane == 0)
+      for (int i = max(c - kLnStages, 0); i < c; ++i)
+        for (uint32_t it = 0; it < (1u << 20); ++it)
+          if (mbar_try_wait(&bars[i % kLnStages], (i / kLnStages) & 1)) break;
+    __syncwarp();
   } else {
     const float inv_h = 1.0f / static_cast<float>(H);
     float g[VPL][8];
@@ -293,12 +299,22 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         ag[i][j] = ab[i][j] = 0.f;
       }
     }
+    // The warps of a row meet once per row.  One whose bounded wait ran out at chunk `ch` still comes to the meetings ahead: the
+    // others may pass the same wait a moment later and must not be left waiting.
+    auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + rslot), "r"(32 * WPR) : "memory"); };
+    auto meet_to_the_end = [&](int ch) {
+      if (WPR > 1)
+        for (; ch * RPB + rslot < rows; ch += gridDim.x) meet();
+    };
     int c = 0;
     for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
       const int row = ch * RPB + rslot;
       const bool have = row < rows;                  // the same for all warps of a row slot
       const float mu = have ? __ldg(mean + row) : 0.f, rs = have ? __ldg(rstd + row) : 0.f;
-      if (!ring.wait_full(c)) break;
+      if (!ring.wait_full(c)) {
+        meet_to_the_end(ch);
+        break;
+      }
       if (have) {
         const uint8_t* base = ring_smem + (c % kLnStages) * stage_bytes + rslot * row_bytes;
         const uint4* pd = reinterpret_cast<const uint4*>(base);
@@ -330,7 +346,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
             slot[part * 2] = s1;
             slot[part * 2 + 1] = s2;
           }
-          asm volatile("bar.sync %0, %1;" ::"r"(1 + rslot), "r"(32 * WPR) : "memory");
+          meet();
           s1 = 0.f;
           s2 = 0.f;
 #pragma unroll

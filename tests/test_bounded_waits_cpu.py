@@ -17,10 +17,18 @@ def _blocks_of_failed_waits(code):
     return [m.group(1) for m in re.finditer(r"if \(!(?:mbar_wait_warp|ring\.wait_full)\([^;{]*\)\s*\{?(.*?)\bbreak;", code, re.S)]
 
 
-@pytest.mark.parametrize("path", sorted(CSRC.glob("attention*.cu")), ids=lambda p: p.name)
+@pytest.mark.parametrize("path", sorted(CSRC.glob("*.cu")), ids=lambda p: p.name)
 def test_warps_that_give_up_still_meet_their_partners(path):
     code = re.sub(r"//[^\n]*", "", path.read_text())
     for body in re.split(r"\b__global__\b", code)[1:]:
         if re.search(NAMED, body):
             left = _blocks_of_failed_waits(body)
             assert left and all("meet_to_the_end(" in b for b in left)
+
+
+def test_copies_of_the_layernorm_ring_land_before_the_block_ends():
+    """The thread that issues the bulk copies waits, with a limit, for the last ones of every stage after its loop."""
+    code = re.sub(r"//[^\n]*", "", (CSRC / "layernorm.cu").read_text())
+    producer = code[code.index("if (warp == kLnWarps)"):]
+    producer = producer[:producer.index("} else {")]
+    assert "bulk_load(" in producer and "mbar_try_wait(&bars[" in producer[producer.rindex("bulk_load("):]
