@@ -50,3 +50,25 @@ def test_convolution_passes(N, H, W, Cin, Cout, k, stride, pad, plan):
     assert _rel(x.grad, dx) < (2.0 ** -8 if plan & 2 else 2.0 ** -7)     # col2im adds bf16-rounded taps
     assert _rel(w.main_grad - 1.0, dw) < 2.0 ** -12                       # accumulated onto ones: one more rounding
     assert native.check_status() == 0
+
+
+@pytest.mark.parametrize("N,H,W,Cin,Cout,k,stride,pad", [
+    (61, 7, 7, 1280, 1280, 3, 1, 1),         # all three passes gather from the activation
+    (16, 28, 28, 320, 640, 3, 1, 1),         # the filter gradient builds its patch matrix in the backward
+    (2, 14, 14, 64, 64, 3, 1, 1),            # patch matrix throughout
+])
+@pytest.mark.parametrize("filter_grad", [True, False])
+def test_input_may_change_before_the_backward(N, H, W, Cin, Cout, k, stride, pad, filter_grad):
+    g = torch.Generator(device="cuda").manual_seed(N)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda").bfloat16()
+    leaf, w = r(N, H, W, Cin).requires_grad_(True), r(Cout, k * k * Cin)
+    w.requires_grad_(filter_grad)
+    got = []
+    for change in (False, True):
+        x = leaf * 1
+        y = C.conv2d(x, w, k, k, stride, pad)
+        if change:
+            x.zero_()
+        got.append(torch.autograd.grad(y, (leaf, w) if filter_grad else (leaf,), torch.ones_like(y)))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
