@@ -1,10 +1,12 @@
-"""Flash attention on scores that are not small and alike."""
+"""Flash attention on scores that are not small and alike, on samples that must not mix, and on more work items than SMs."""
 import math
 
 import pytest
 import torch
 
 from superscaler_b200.ops import functional as F
+from superscaler_b200.ops import native
+from test_attention_tiles_gpu import TOL, _oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +60,82 @@ def test_samples_keep_their_nans(SQ, SK, HD, causal):
             assert torch.isfinite(a).all()
             # dq is summed over the key blocks in the order they finish: fp32 sums, then one rounding to bf16
             assert float((a.double() - e.double()).norm()) <= 2.0 ** -9 * float(e.double().norm())
+
+
+@pytest.mark.parametrize("S,HD,causal,p,bias", [
+    (700, 64, True, 0.0, False),
+    (700, 128, True, 0.1, False),
+    (515, 64, False, 0.1, True),
+    (515, 128, False, 0.0, False),
+])
+@pytest.mark.parametrize("gain", [8.0, 32.0])
+@pytest.mark.parametrize("rising", [1, 32])              # rows of every 32 whose maximum rises with the keys
+def test_late_maxima(S, HD, causal, p, bias, gain, rising):
+    """Keys ordered along one direction that some queries follow and the others oppose: their running maximum grows in
+    every block, by more than 2^8 in probability.  The forward stays within the tolerance of small scores (fp32 scores of
+    some 2^8 are off by 2^-16).  In the backward dS = P (dP - delta) cancels where one key takes the whole row, and what
+    remains is the rounding of O in delta: e_r = 2^-9 |dO_r O_r| for row r, which enters dq_r with a weighted mean of keys
+    and dk with q_r."""
+    B, NH, seed = 2, 2, 5
+    g = torch.Generator(device="cuda").manual_seed(S + HD)
+    w, n = NH * HD, B * S
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    u = torch.nn.functional.normalize(r(HD), dim=0).repeat(NH)
+    ramp = torch.linspace(-1.0, 1.0, S, device="cuda").repeat(B)[:, None]
+    sign = torch.where(torch.arange(n, device="cuda") % 32 < rising, 1.0, -1.0)[:, None]
+    q = (0.1 * gain * r(n, w) + gain * sign * u).bfloat16()
+    k = (0.1 * r(n, w) + math.sqrt(HD) * ramp * u).bfloat16()
+    v, do = r(n, w).bfloat16(), r(n, w).bfloat16()
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    bt = r(NH, 2 * S - 1).requires_grad_(True) if bias else None
+    y = F.flash_attention(q, k, v, B, NH, S, S, HD, causal=causal, dropout_p=p, seed=seed, bias_table=bt)
+    y.backward(do)
+    o, dq, dk, dv, db = _oracle(q.detach(), k.detach(), v.detach(), do, B, NH, S, S, HD, causal, None, p, seed,
+                                bt.detach() if bias else None)
+    heads = lambda t: t.double().view(n, NH, HD)
+    e = 2.0 ** -9 * (heads(do) * heads(o)).norm(dim=-1)                       # [tokens, heads]
+    scale = HD ** -0.5
+    slack = {"dq": scale * float(e.norm() * heads(k.detach()).norm(dim=-1).max()),
+             "dk": scale * float((e * heads(q.detach()).norm(dim=-1)).norm())}
+    err = lambda a, b: float((a.double() - b).norm())
+    assert err(y.detach(), o) <= TOL * float(o.norm())
+    assert err(v.grad, dv) <= TOL * float(dv.norm())
+    assert err(q.grad, dq) <= TOL * float(dq.norm()) + 2 * slack["dq"]
+    assert err(k.grad, dk) <= TOL * float(dk.norm()) + 2 * slack["dk"]
+    if bias:
+        assert err(bt.grad, db) <= TOL * float(db.norm()) + 2 * float(e.norm())
+
+
+@pytest.mark.parametrize("SQ,SK,HD,causal,lens,p,bias", [
+    (130, 130, 64, True, False, 0.1, False),
+    (300, 300, 128, True, False, 0.1, False),
+    (300, 300, 64, False, True, 0.1, True),
+    (130, 300, 128, False, True, 0.0, False),
+    (300, 130, 64, False, True, 0.0, False),
+])
+def test_more_items_than_sms(SQ, SK, HD, causal, lens, p, bias):
+    """320 heads: every CTA of the persistent forward takes several items, some of them empty (a sample without keys)."""
+    B, NH, seed = 20, 16, 31
+    g = torch.Generator(device="cuda").manual_seed(SQ + SK + HD)
+    w = NH * HD
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    q, k, v, do = (r(B * n, w).bfloat16() for n in (SQ, SK, SK, SQ))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    bt = r(NH, SQ + SK - 1).requires_grad_(True) if bias else None
+    ln = None
+    if lens:
+        ln = torch.randint(1, SK + 1, (B,), generator=g, device="cuda", dtype=torch.int32)
+        ln[3] = ln[10] = 0
+        ln[11] = SK
+    y = F.flash_attention(q, k, v, B, NH, SQ, SK, HD, causal=causal, kv_lens=ln, dropout_p=p, seed=seed, bias_table=bt)
+    y.backward(do)
+    want = _oracle(q.detach(), k.detach(), v.detach(), do, B, NH, SQ, SK, HD, causal, ln, p, seed,
+                   bt.detach() if bias else None)
+    got = [y.detach(), q.grad, k.grad, v.grad] + ([bt.grad] if bias else [])
+    for a, e in zip(got, want):
+        e = e.double()
+        assert torch.isfinite(a).all()
+        assert float((a.double() - e).norm()) <= TOL * float(e.norm()) + HD * 2.0 ** -24 * float(do.double().norm())
+    assert native.check_status() == 0

@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _rel(a, e):
-    return float((a.double() - e).norm() / e.norm())
+    return float((a.detach().double() - e).norm() / e.norm())
 
 
 @pytest.mark.parametrize("N,H,W,Cin,Cout,k,stride,pad,plan", [

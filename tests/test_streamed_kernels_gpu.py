@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 def _rel(a, e):
-    return float((a.double() - e).norm() / e.norm().clamp_min(1e-30))
+    return float((a.detach().double() - e).norm() / e.norm().clamp_min(1e-30))
 
 
 @pytest.mark.parametrize("rows", [1, 7, 301])
@@ -115,3 +115,44 @@ def test_layernorm_refuses_misaligned_rows(H):
     for dy, x, dres in ((odd, even, None), (even, odd, None), (even, even, odd)):
         with pytest.raises(RuntimeError, match="layernorm_bwd"):
             ext.layernorm_bwd(dy, x, gamma, stat, stat, dres, dg, db, False)
+
+
+@pytest.mark.parametrize("rows,H", [(16603, 504), (8317, 1000), (4157, 2048), (2083, 4096)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_layernorm_backward_wraps_its_ring(rows, H, residual):
+    """Rows enough for every block (two per SM at most) to reuse each of the three stages of its ring at least once, the last
+    chunk ragged: one to eight warps per row."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(s, generator=g, device="cuda")
+    x, dy, dres = (r(rows, H).bfloat16() for _ in range(3))
+    gamma, beta = r(H) + 1.0, r(H)
+    y, mean, rstd = native.ext().layernorm_fwd(x, None, gamma, beta, 1e-5)
+    dg, db = torch.zeros(H, device="cuda"), torch.zeros(H, device="cuda")
+    dx = native.ext().layernorm_bwd(dy, x, gamma, mean, rstd, dres if residual else None, dg, db, True)
+    t = [v.double().requires_grad_(True) for v in (x, gamma, beta)]
+    want = torch.autograd.grad(TF.layer_norm(t[0], (H,), t[1], t[2], 1e-5), t, dy.double())
+    assert _rel(dx, want[0] + (dres.double() if residual else 0.0)) < 2.0 ** -8
+    assert _rel(dg, want[1]) < 1e-5 and _rel(db, want[2]) < 1e-5
+    assert native.check_status() == 0
+
+
+@pytest.mark.parametrize("two_pass", [False, True])       # the form of one rank alone, the one of a vocabulary over several
+def test_cross_entropy_at_the_benchmark_vocabulary(two_pass):
+    """4096 rows of 51200 bf16 logits, every entry: fp32 sums of 51200 exponentials, each off by a few units in the last
+    place (1e-5 of the loss); the gradient carries one bf16 rounding (2^-9) on top of that, so 2^-8 of each entry."""
+    T, V = 4096, 51200
+    g = torch.Generator(device="cuda").manual_seed(45)
+    logits = (torch.randn(T, V, generator=g, device="cuda") * 2).bfloat16()
+    t = torch.randint(0, V, (T,), generator=g, device="cuda")
+    work, ext = logits.clone(), native.ext()
+    if two_pass:
+        loss = ext.ce_finalize(work, t, ext.ce_stats(work, t, 0), None, 0, 0.25, True)
+    else:
+        loss = ext.ce_loss_grad(work, t, None, 0, 0.25)
+    for r in range(0, T, 512):
+        x, tt = logits[r:r + 512].double(), t[r:r + 512]
+        assert torch.allclose(loss[r:r + 512].double(), TF.cross_entropy(x, tt, reduction="none"), rtol=1e-5, atol=1e-5)
+        grad = torch.softmax(x, -1)
+        grad[torch.arange(512, device="cuda"), tt] -= 1.0
+        off = (work[r:r + 512].double() - 0.25 * grad).abs() - 2.0 ** -8 * 0.25 * grad.abs()
+        assert float(off.max()) <= 2.0 ** -126                # below the smallest normal number bf16 may round to zero
