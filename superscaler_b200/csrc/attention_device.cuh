@@ -30,10 +30,10 @@ __device__ __forceinline__ uint32_t fmix32(uint32_t x) {
 // Dropout mask: one 32-bit hash decides the four QUERIES 4t .. 4t+3 of one key; query 4t+i is kept when byte i of the
 // hash is below keep8 = round(256 (1 - p)).  The dropout probability is therefore quantised to 1/256 (the scale
 // applied to the kept values is the exact 256 / keep8), which makes the mask four times cheaper to generate than
-// one 16-bit lane per element.  The backward kernels hold one KEY per thread and sixteen consecutive queries, so
-// four hashes per thread cover a tile step without any exchange (the backward does 2.5 times the work of the
-// forward); the kernels that hold one QUERY per thread share the hashes of a key between the four lanes of a
-// query quad with shuffles.
+// one 16-bit lane per element.  The backward kernels hold one KEY per thread and consecutive queries (32 in the fused
+// kernel, 16 in the pair), so eight or four hashes per thread cover a tile step without any exchange (the backward does
+// 2.5 times the work of the forward); the kernels that hold one QUERY per thread share the hashes of a key between the
+// four lanes of a query quad with shuffles.
 __device__ __forceinline__ uint32_t attn_col_hash(uint32_t bh_seed, uint32_t key, uint32_t qquads, uint32_t qquad) {
   return fmix32((key * qquads + qquad) * 0x9E3779B1u + bh_seed);
 }
@@ -41,17 +41,6 @@ __device__ __forceinline__ bool keep_byte(uint32_t h, int i, uint32_t keep8) { r
 __host__ __device__ __forceinline__ uint32_t dropout_keep8(float p) {
   const int k = static_cast<int>((1.0f - p) * 256.0f + 0.5f);
   return static_cast<uint32_t>(k < 1 ? 1 : (k > 256 ? 256 : k));
-}
-
-// Writes 32 consecutive bf16 columns (16 packed words) of row r into a [rows][128 B] swizzled chunk.
-// piece0 = index of the first 16-byte piece inside the 128-byte row (0 or 4).
-__device__ __forceinline__ void store_row32_sw128(uint8_t* chunk, int r, int piece0, const uint32_t (&w)[16]) {
-  uint8_t* row = chunk + r * 128;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int piece = (piece0 + i) ^ (r & 7);
-    *reinterpret_cast<uint4*>(row + piece * 16) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-  }
 }
 
 // Writes 16 consecutive bf16 columns (8 packed words) of row r; piece0 = first 16-byte piece (even).

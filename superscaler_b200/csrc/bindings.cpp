@@ -376,7 +376,6 @@ void embedding_bwd(const Tensor& ids, const OptTensor& pos, const Tensor& g, con
                "embedding_bwd");
 }
 
-// dst[key - k0] += sum of the (dropout-masked) rows of g whose key equals `key`; keys ascending, order[p] = token of keys[p]
 // Keys for the sort in front of embedding_bwd_sorted: rows of a table of n rows that starts at id k0, in the narrowest type
 // that holds them (ids outside become n, which that call skips with k0 = 0).
 Tensor embedding_keys(const Tensor& ids, int64_t k0, int64_t n) {
@@ -389,6 +388,7 @@ Tensor embedding_keys(const Tensor& ids, int64_t k0, int64_t n) {
   return keys;
 }
 
+// dst[key - k0] += sum of the (dropout-masked) rows of g whose key equals `key`; keys ascending, order[p] = token of keys[p]
 void embedding_bwd_sorted(const Tensor& keys, const Tensor& order, const Tensor& g, const Tensor& dst, int64_t k0,
                           double dropout_p, int64_t seed) {
   TORCH_CHECK(g.scalar_type() == torch::kBFloat16 && g.is_contiguous() && g.is_cuda());

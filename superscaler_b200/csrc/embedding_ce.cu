@@ -252,8 +252,8 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   const int k0 = nvec * 8 + threadIdx.x;           // at most seven columns behind the last whole vector
   const float tail = k0 < V ? __bfloat162float(x[k0]) : -INFINITY;
   const long long t = targets[row] - v0;
+  // read by every thread before the barriers of the reductions, so before any thread overwrites the row
   const float tgt = (t >= 0 && t < V) ? __bfloat162float(x[t]) : 0.f;
-  __syncthreads();                                 // the target is read before any thread overwrites the row
   float tmax = tail, tsum = tail != -INFINITY ? __expf(tail - tail) : 0.f;  // this thread's maximum and sum exp(x - maximum)
   for (int v = threadIdx.x; v < nvec; v += 4 * kCeThreads) {
     uint4 q[4];

@@ -96,7 +96,7 @@ def run_layernorm(a) -> None:
 
 
 def run_embedding(a) -> None:
-    """Embedding forward (word + position + dropout) and the two forms of its backward scatter."""
+    """Embedding forward (word + position + dropout) and the forms of its backward scatter."""
     ext = native.ext()
     torch.manual_seed(0)
     T, H, V = a.tokens, a.H, a.V
@@ -108,13 +108,14 @@ def run_embedding(a) -> None:
     g = torch.randn(T, H, device="cuda").bfloat16()
     dW, dP = torch.zeros(V, H, device="cuda"), torch.zeros(seq, H, device="cuda")
 
-    def sorted_bwd():
+    def sorted_bwd(narrow):
         for keys_t, dst in ((ids, dW), (pos, dP)):
-            keys, order = torch.sort(keys_t, stable=True)
+            keys, order = torch.sort(ext.embedding_keys(keys_t, 0, dst.shape[0]) if narrow else keys_t, stable=True)
             ext.embedding_bwd_sorted(keys, order, g, dst, 0, a.dropout, 5)
 
     cases = (("fwd", lambda: ext.embedding_fwd(ids, pos, W, P, 0, a.dropout, 5), 3 * T * H * 2),
-             ("bwd sorted runs", sorted_bwd, T * H * 2 + 2 * T * H * 4),
+             ("bwd sorted runs, narrow keys", lambda: sorted_bwd(True), T * H * 2 + 2 * T * H * 4),
+             ("bwd sorted runs, 64-bit keys", lambda: sorted_bwd(False), T * H * 2 + 2 * T * H * 4),
              ("bwd float atomics", lambda: ext.embedding_bwd(ids, pos, g, dW, dP, 0, a.dropout, 5),
               T * H * 2 + 2 * T * H * 4))
     for name, fn, moved in cases:
@@ -124,14 +125,16 @@ def run_embedding(a) -> None:
 
 
 def run_crossentropy(a) -> None:
-    """Row statistics of bf16 logits, then loss + in-place gradient (the two passes of the LM-head loss)."""
+    """Loss + in-place gradient of bf16 logits: in one pass (a rank that holds the whole vocabulary), and as row statistics
+    and a second pass (tensor parallel, or rows too long for shared memory)."""
     ext = native.ext()
     torch.manual_seed(0)
     logits = (torch.randn(a.tokens, a.V, device="cuda") * 2).bfloat16()
     tg = torch.randint(0, a.V, (a.tokens,), device="cuda")
     st = ext.ce_stats(logits, tg, 0)
     nbytes = logits.numel() * 2
-    for name, fn, moved in (("stats", lambda: ext.ce_stats(logits, tg, 0), nbytes),
+    for name, fn, moved in (("one pass", lambda: ext.ce_loss_grad(logits, tg, None, 0, 1.0), 2 * nbytes),
+                            ("stats", lambda: ext.ce_stats(logits, tg, 0), nbytes),
                             ("finalize", lambda: ext.ce_finalize(logits, tg, st, None, 0, 1.0, True), 2 * nbytes)):
         ms = _time(fn, a.warmup, a.iters)
         print(f"cross-entropy {name} tokens {a.tokens} V {a.V}: {ms:.4f} ms {moved / ms / 1e6:.0f} GB/s "
@@ -166,8 +169,8 @@ def run_adam(a) -> None:
 
 
 def run_convbn(a) -> None:
-    """One Wide-ResNet bottleneck-sized k x k convolution (patch matrix + GEMM; dgrad + scatter back) and the
-    BatchNorm + ReLU around it, NHWC bf16."""
+    """One Wide-ResNet bottleneck-sized k x k convolution (implicit GEMMs for large layers, patch matrix and scatter back for
+    small ones) and the BatchNorm + ReLU around it, NHWC bf16."""
     from ..ops import conv as C
     ext = native.ext()
     torch.manual_seed(0)
