@@ -83,7 +83,7 @@ int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int
                       const GemmParams& p, int num_sms, cudaStream_t stream);
 bool ce_fused_ok(int V);
 int ce_fused_launch(void* logits, int ld, const long long* targets, const float* loss_mask, float* loss, long long rows, int V,
-                    long long v0, float grad_scale, cudaStream_t stream);
+                    long long v0, float grad_scale, int num_sms, cudaStream_t stream);
 int bn_slices(long long rows);
 int im2col_launch(const void* x, void* cols, int N, int H, int W, int C, int KH, int KW, int stride, int pad, int Kpad,
                   int num_sms, cudaStream_t stream);
@@ -452,7 +452,7 @@ Tensor ce_loss_grad(Tensor& logits, const Tensor& targets, const OptTensor& loss
                                     reinterpret_cast<const long long*>(targets.data_ptr<int64_t>()),
                                     loss_mask.has_value() ? loss_mask->data_ptr<float>() : nullptr, loss.data_ptr<float>(),
                                     logits.size(0), static_cast<int>(logits.size(1)), v0, static_cast<float>(grad_scale),
-                                    cur_stream()),
+                                    num_sms(), cur_stream()),
                "ce_loss_grad");
   return loss;
 }

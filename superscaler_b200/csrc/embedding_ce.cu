@@ -235,12 +235,12 @@ ce_finalize_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* 
 // Loss and gradient of whole rows in one pass over memory, for logits that no other rank shares.  The row is read once, into
 // shared memory; every thread keeps a running maximum and the sum of exponentials relative to it on the way, so that the
 // special-function unit works under the loads, and only the gradient is left for a second pass.  Same quantities as
-// ce_stats + ce_finalize, which read the row three times.  Two CTAs per SM: one loads while the other writes.  Head and loss
-// of 4096 rows x 51200, forward and backward: 2571 -> 2532 us; the kernel itself 232 us (3.6 TB/s, two exponentials an element).
-constexpr int kCeThreads = 512;
+// ce_stats + ce_finalize, which read the row three times.  T threads a row, 1024 per SM: one CTA loads while others write.
+// 4096 rows x 51200: 229 us (3.7 TB/s, two exponentials an element) against 263 for the two kernels.
 constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per SM
 
-__global__ void __launch_bounds__(kCeThreads, 2)
+template <int T>
+__global__ void __launch_bounds__(T, 1024 / T)
 ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __restrict__ targets,
                 const float* __restrict__ loss_mask, float* __restrict__ loss, int V, long long v0, float grad_scale) {
   extern __shared__ uint4 row_smem[];
@@ -255,15 +255,15 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   // read by every thread before the barriers of the reductions, so before any thread overwrites the row
   const float tgt = (t >= 0 && t < V) ? __bfloat162float(x[t]) : 0.f;
   float tmax = tail, tsum = tail != -INFINITY ? __expf(tail - tail) : 0.f;  // this thread's maximum and sum exp(x - maximum)
-  for (int v = threadIdx.x; v < nvec; v += 4 * kCeThreads) {
+  for (int v = threadIdx.x; v < nvec; v += 4 * T) {
     uint4 q[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (v + u * kCeThreads < nvec) q[u] = __ldcs(xv + v + u * kCeThreads);
+      if (v + u * T < nvec) q[u] = __ldcs(xv + v + u * T);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      if (v + u * kCeThreads < nvec) {
-        row_smem[v + u * kCeThreads] = q[u];       // each thread reads back what it wrote: no barrier needed
+      if (v + u * T < nvec) {
+        row_smem[v + u * T] = q[u];       // each thread reads back what it wrote: no barrier needed
         const float2 a = unpack_bf16x2(q[u].x), b = unpack_bf16x2(q[u].y), c = unpack_bf16x2(q[u].z), d = unpack_bf16x2(q[u].w);
         const float m8 = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y)), fmaxf(fmaxf(c.x, c.y), fmaxf(d.x, d.y)));
         if (m8 > tmax) {
@@ -281,7 +281,7 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   const float w = loss_mask ? loss_mask[row] : 1.0f;
   if (threadIdx.x == 0) loss[row] = (logf(s) + mx - tgt) * w;
   const float inv = 1.0f / s, gs = grad_scale * w;
-  for (int v = threadIdx.x; v < nvec; v += kCeThreads) {
+  for (int v = threadIdx.x; v < nvec; v += T) {
     const uint4 q = row_smem[v];
     const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
     float f[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
@@ -308,14 +308,21 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
 bool ce_fused_ok(int V) { return V <= kCeMaxCols; }
 
 int ce_fused_launch(void* logits, int ld, const long long* targets, const float* loss_mask, float* loss, long long rows, int V,
-                    long long v0, float grad_scale, cudaStream_t stream) {
+                    long long v0, float grad_scale, int num_sms, cudaStream_t stream) {
   if (ld % 8) return -3;
-  const int smem = (V / 8) * 16;
-  const int rc = static_cast<int>(cudaFuncSetAttribute(ce_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeMaxCols * 2));
-  if (rc) return rc;
-  ce_fused_kernel<<<static_cast<unsigned>(rows), kCeThreads, smem, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets,
-                                                                             loss_mask, loss, V, v0, grad_scale);
-  return static_cast<int>(cudaGetLastError());
+  auto launch = [&](auto kernel, int threads) {
+    const int rc = static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeMaxCols * 2));
+    if (rc) return rc;
+    kernel<<<static_cast<unsigned>(rows), threads, (V / 8) * 16, stream>>>(reinterpret_cast<__nv_bfloat16*>(logits), ld, targets,
+                                                                           loss_mask, loss, V, v0, grad_scale);
+    return static_cast<int>(cudaGetLastError());
+  };
+  // Threads of a row, 4096 rows: 128 and 256 threads take 49 and 53 us at 12288 columns, 69 and 67 at 16384; 256 and 512 take
+  // 138 and 145 at 32000, 201 and 181 at 40960 (512 throughout: 27 us at 1024 columns, where the two kernels take 15 and 128
+  // threads 9.5).  Rows that all fit on the chip at once are a matter of latency: 16 rows of 8192 take 4.6 us with 128 threads
+  // and 3.8 with 512.
+  if (rows <= 2LL * num_sms || V > 36 * 1024) return launch(ce_fused_kernel<512>, 512);
+  return V > 14 * 1024 ? launch(ce_fused_kernel<256>, 256) : launch(ce_fused_kernel<128>, 128);
 }
 
 int embedding_fwd_launch(const long long* ids, const long long* pos, const void* W, const void* P, void* out,

@@ -156,3 +156,20 @@ def test_cross_entropy_at_the_benchmark_vocabulary(two_pass):
         grad[torch.arange(512, device="cuda"), tt] -= 1.0
         off = (work[r:r + 512].double() - 0.25 * grad).abs() - 2.0 ** -8 * 0.25 * grad.abs()
         assert float(off.max()) <= 2.0 ** -126                # below the smallest normal number bf16 may round to zero
+
+
+@pytest.mark.parametrize("V", [8, 1003, 2048, 14336, 14344, 36864, 36872])     # 128, 256 and 512 threads a row
+def test_cross_entropy_of_many_rows(V):
+    """More rows than fit on the chip at once, where the width of the row chooses the number of threads."""
+    rows = 2 * torch.cuda.get_device_properties(0).multi_processor_count + 5
+    g = torch.Generator(device="cuda").manual_seed(V)
+    buf = (torch.randn(rows, (V + 7) // 8 * 8, generator=g, device="cuda") * 4).bfloat16()
+    t = torch.randint(0, V, (rows,), generator=g, device="cuda")
+    x = buf[:, :V].double()
+    work = buf.clone()
+    loss = native.ext().ce_loss_grad(work[:, :V], t, None, 0, 0.5)
+    assert torch.allclose(loss.double(), TF.cross_entropy(x, t, reduction="none"), rtol=1e-5, atol=1e-5)
+    grad = torch.softmax(x, -1)
+    grad[torch.arange(rows, device="cuda"), t] -= 1.0
+    assert _rel(work[:, :V], 0.5 * grad) < 2.0 ** -8
+    assert torch.equal(work[:, V:], buf[:, V:])
