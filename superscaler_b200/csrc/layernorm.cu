@@ -252,8 +252,6 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row_bytes = H * 2, part_bytes = RPB * row_bytes, stage_bytes = 3 * part_bytes, nvec = H / 8;
   const int chunks = (rows + RPB - 1) / RPB;
-  float* fold_g = reinterpret_cast<float*>(ring_smem + kLnStages * stage_bytes);  // [512 WPR] each
-  float* fold_b = fold_g + 512 * WPR;
   if (threadIdx.x == 0) {
     for (int i = 0; i < kLnStages; ++i) {
       mbar_init(&bars[i], 1);
@@ -381,24 +379,32 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
     }
   }
   __syncthreads();
-  // fold the row slots of the block in the order 0, 1, ...: slot s adds its warps' sums to the columns they own
-  for (int sl = 0; sl < RPB; ++sl) {
-    if (warp < kLnWarps && rslot == sl) {
+  // Every copy has landed and been read: the ring takes the sums of the row slots, [2][RPB][H], which are then added in the order
+  // 0, 1, ...  (One slot after the other into one row of sums took eight rounds at one warp per row: 16 x 512 9.5 us.)
+  float* slots = reinterpret_cast<float*>(ring_smem);
+  if (warp < kLnWarps) {
 #pragma unroll
-      for (int i = 0; i < VPL; ++i) {
-        const int col = ((part * VPL + i) * 32 + lane) * 8;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          fold_g[col + j] = (sl == 0 ? 0.f : fold_g[col + j]) + ag[i][j];
-          fold_b[col + j] = (sl == 0 ? 0.f : fold_b[col + j]) + ab[i][j];
-        }
-      }
+    for (int i = 0; i < VPL; ++i) {
+      const int v = (part * VPL + i) * 32 + lane;
+      if (v >= nvec) break;
+      float4* pg = reinterpret_cast<float4*>(slots + rslot * H + v * 8);
+      float4* pb = reinterpret_cast<float4*>(slots + (RPB + rslot) * H + v * 8);
+      pg[0] = make_float4(ag[i][0], ag[i][1], ag[i][2], ag[i][3]);
+      pg[1] = make_float4(ag[i][4], ag[i][5], ag[i][6], ag[i][7]);
+      pb[0] = make_float4(ab[i][0], ab[i][1], ab[i][2], ab[i][3]);
+      pb[1] = make_float4(ab[i][4], ab[i][5], ab[i][6], ab[i][7]);
     }
-    __syncthreads();
   }
+  __syncthreads();
   for (int col = threadIdx.x; col < H; col += blockDim.x) {
-    part_g[static_cast<size_t>(blockIdx.x) * H + col] = fold_g[col];
-    part_b[static_cast<size_t>(blockIdx.x) * H + col] = fold_b[col];
+    float g = slots[col], b = slots[RPB * H + col];
+#pragma unroll
+    for (int sl = 1; sl < RPB; ++sl) {
+      g += slots[sl * H + col];
+      b += slots[(RPB + sl) * H + col];
+    }
+    part_g[static_cast<size_t>(blockIdx.x) * H + col] = g;
+    part_b[static_cast<size_t>(blockIdx.x) * H + col] = b;
   }
   if (threadIdx.x == 0 && aborted && status != nullptr) atomicMax(status, static_cast<int>(kStatusMbarTimeout));
 }
@@ -455,24 +461,38 @@ __global__ void fold_partials_kernel(const float* __restrict__ part, float* __re
 }
 
 // Both LayerNorm weight gradients in one launch: block (x, which) folds 32 columns of part_g (which = 0) or part_b
-// (which = 1); its 1024 threads are 32 columns x 32 groups of slices, added in a fixed order (four groups per column took
-// 11 us for 296 slices: a chain of 74 loads).
-__global__ void __launch_bounds__(1024)
+// (which = 1); its threads are 32 columns x G groups of slices, added in a fixed order.  G 32 for the many partials of the
+// one-pass kernel (with four groups a chain of 74 loads, 11 us for 296 slices), 4 for few (2 slices of 5120 columns: 1.9 us
+// instead of 2.9).
+template <int G>
+__global__ void __launch_bounds__(32 * G)
 fold_partials2_kernel(const float* __restrict__ part_g, const float* __restrict__ part_b, float* __restrict__ dgamma,
                       float* __restrict__ dbeta, int slices, int H, int accumulate) {
-  __shared__ float sm[32][33];
+  __shared__ float sm[G][33];
   const float* part = blockIdx.y == 0 ? part_g : part_b;
   float* out = blockIdx.y == 0 ? dgamma : dbeta;
   const int c = threadIdx.x & 31, sg = threadIdx.x >> 5, h = blockIdx.x * 32 + c;
   float s = 0.f;
   if (h < H)
-    for (int k = sg; k < slices; k += 32) s += part[static_cast<size_t>(k) * H + h];
+    for (int k = sg; k < slices; k += G) s += part[static_cast<size_t>(k) * H + h];
   sm[sg][c] = s;
   __syncthreads();
-  // warp w adds column w's 32 groups by a butterfly: the same order every time
-  const float t = warp_sum(sm[c][sg]);
-  const int hw = blockIdx.x * 32 + sg;
-  if (c == 0 && hw < H) out[hw] = accumulate ? out[hw] + t : t;
+  static_assert(G == 4 || G == 32, "groups");
+  if constexpr (G == 32) {  // warp w adds column w's groups by a butterfly: the same order every time
+    const float t = warp_sum(sm[c][sg]);
+    const int hw = blockIdx.x * 32 + sg;
+    if (c == 0 && hw < H) out[hw] = accumulate ? out[hw] + t : t;
+  } else if (sg == 0 && h < H) {
+    const float t = (sm[0][c] + sm[1][c]) + (sm[2][c] + sm[3][c]);
+    out[h] = accumulate ? out[h] + t : t;
+  }
+}
+
+void fold_partials2(const float* part_g, const float* part_b, float* dgamma, float* dbeta, int slices, int H, int accumulate,
+                    cudaStream_t stream) {
+  const dim3 grid((H + 31) / 32, 2);
+  if (slices > 64) fold_partials2_kernel<32><<<grid, 1024, 0, stream>>>(part_g, part_b, dgamma, dbeta, slices, H, accumulate);
+  else fold_partials2_kernel<4><<<grid, 128, 0, stream>>>(part_g, part_b, dgamma, dbeta, slices, H, accumulate);
 }
 
 // Column sum of a bf16 matrix [rows, N] (bias gradients) in ONE launch, for 16-byte aligned rows (N, lda multiples
@@ -634,7 +654,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   if (H <= kLnStreamMaxH) {
     // dy and x are read once: dx and the per-column sums come out of the same sweep
     const int nb = ln_bwd_part_rows(rows, H, num_sms), wpr = ln_bwd_warps_per_row(H);
-    const int smem = kLnStages * 3 * (kLnWarps / wpr) * H * 2 + 2 * 512 * wpr * 4;
+    const int smem = kLnStages * 3 * (kLnWarps / wpr) * H * 2;
     int rc = 0;
 #define SSB_LN_BWD(W)                                                                                                        \
   rc = static_cast<int>(cudaFuncSetAttribute(ln_bwd_stream_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));    \
@@ -647,8 +667,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
       default: SSB_LN_BWD(8); break;
     }
 #undef SSB_LN_BWD
-    fold_partials2_kernel<<<dim3((H + 31) / 32, 2), 1024, 0, stream>>>(part_g, part_b, dgamma, dbeta, nb, H,
-                                                                      accumulate_wgrad);
+    fold_partials2(part_g, part_b, dgamma, dbeta, nb, H, accumulate_wgrad, stream);
     return static_cast<int>(cudaGetLastError());
   }
   const int blocks = min((rows + kLnWarpsPerBlock - 1) / kLnWarpsPerBlock, num_sms * 16);
@@ -660,8 +679,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   ln_bwd_gb_partial_kernel<<<grid, 256, 0, stream>>>(reinterpret_cast<const __nv_bfloat16*>(dy),
                                                      reinterpret_cast<const __nv_bfloat16*>(x), mean, rstd, part_g,
                                                      part_b, rows, H, rps);
-  fold_partials2_kernel<<<dim3((H + 31) / 32, 2), 1024, 0, stream>>>(part_g, part_b, dgamma, dbeta, slices, H,
-                                                                    accumulate_wgrad);
+  fold_partials2(part_g, part_b, dgamma, dbeta, slices, H, accumulate_wgrad, stream);
   return static_cast<int>(cudaGetLastError());
 }
 
