@@ -173,3 +173,9 @@ def test_cross_entropy_of_many_rows(V):
     grad[torch.arange(rows, device="cuda"), t] -= 1.0
     assert _rel(work[:, :V], 0.5 * grad) < 2.0 ** -8
     assert torch.equal(work[:, V:], buf[:, V:])
+
+
+@pytest.mark.parametrize("per_sm,extra,start", [(1024, 0, 0), (1024, 1, 0), (1024, 7, 1), (8 * 2048, 4099, 0)])
+def test_adam_at_the_edges_of_its_forms(per_sm, extra, start):
+    """An element a thread up to 1024 elements an SM, then vectors; from 8 x 2048 an SM on every block takes several passes."""
+    test_adam_vector_and_scalar_parts(torch.cuda.get_device_properties(0).multi_processor_count * per_sm + extra, start)
