@@ -13,7 +13,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("HD", [64, 128])
 @pytest.mark.parametrize("blocks", [2, 5])
-def test_rows_of_one_value_are_exact(HD, blocks):
+@pytest.mark.parametrize("NH", [1, 80])                  # a tile per CTA; more tiles than SMs: pairs of them
+def test_rows_of_one_value_are_exact(HD, blocks, NH):
     """All values of a sequence equal one vector, so every output row is that vector, whatever the scores.  A row has one
     key of score 0 in the first block and one above it by up to 8 (log2) in the last; the other keys lie 40 below and weigh
     less than 2^-30 in all.  Both keys are their block's maximum, so their probabilities are exactly one when they are
@@ -30,9 +31,9 @@ def test_rows_of_one_value_are_exact(HD, blocks):
     k[S - 50] = 0.0
     k[S - 50, 0] = 1.0
     v = torch.randn(HD, generator=g, device="cuda").expand(S, HD)
-    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16().contiguous()
-    o = F.flash_attention(q, k, v, 1, 1, rows, S, HD, scale=math.log(2.0))
-    assert torch.equal(o, v[:1].expand(rows, HD))
+    q, k, v = (t.bfloat16().repeat(1, NH) for t in (q, k, v))
+    o = F.flash_attention(q, k, v, 1, NH, rows, S, HD, scale=math.log(2.0))
+    assert torch.equal(o, v[:1].expand(rows, NH * HD))
 
 
 @pytest.mark.parametrize("SQ,SK,HD,causal", [(64, 128, 64, False), (192, 256, 128, False), (100, 77, 64, False),
@@ -70,13 +71,14 @@ def test_samples_keep_their_nans(SQ, SK, HD, causal):
 ])
 @pytest.mark.parametrize("gain", [8.0, 32.0])
 @pytest.mark.parametrize("rising", [1, 32])              # rows of every 32 whose maximum rises with the keys
-def test_late_maxima(S, HD, causal, p, bias, gain, rising):
+@pytest.mark.parametrize("B,NH", [(2, 2), (8, 4)])       # a tile per CTA; more tiles than SMs: pairs of them
+def test_late_maxima(S, HD, causal, p, bias, gain, rising, B, NH):
     """Keys ordered along one direction that some queries follow and the others oppose: their running maximum grows in
     every block, by more than 2^8 in probability.  The forward stays within the tolerance of small scores (fp32 scores of
     some 2^8 are off by 2^-16).  In the backward dS = P (dP - delta) cancels where one key takes the whole row, and what
     remains is the rounding of O in delta: e_r = 2^-9 |dO_r O_r| for row r, which enters dq_r with a weighted mean of keys
     and dk with q_r."""
-    B, NH, seed = 2, 2, 5
+    seed = 5
     g = torch.Generator(device="cuda").manual_seed(S + HD)
     w, n = NH * HD, B * S
     r = lambda *s: torch.randn(s, generator=g, device="cuda")
@@ -113,6 +115,11 @@ def test_late_maxima(S, HD, causal, p, bias, gain, rising):
     (300, 300, 64, False, True, 0.1, True),
     (130, 300, 128, False, True, 0.0, False),
     (300, 130, 64, False, True, 0.0, False),
+    (127, 127, 64, True, False, 0.1, False),
+    (257, 257, 128, True, False, 0.0, False),
+    (255, 130, 64, False, True, 0.1, False),
+    (384, 96, 128, False, False, 0.5, False),
+    (256, 256, 64, False, True, 0.1, True),
 ])
 def test_more_items_than_sms(SQ, SK, HD, causal, lens, p, bias):
     """320 heads: every CTA of the persistent forward takes several items, some of them empty (a sample without keys)."""
