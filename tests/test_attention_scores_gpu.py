@@ -146,3 +146,23 @@ def test_more_items_than_sms(SQ, SK, HD, causal, lens, p, bias):
         assert torch.isfinite(a).all()
         assert float((a.double() - e).norm()) <= TOL * float(e.norm()) + HD * 2.0 ** -24 * float(do.double().norm())
     assert native.check_status() == 0
+
+
+@pytest.mark.parametrize("S", [31, 32, 33, 64, 65, 96, 97, 160, 225])
+@pytest.mark.parametrize("HD,causal,lens", [(64, True, False), (128, True, False), (64, False, True), (128, False, True)])
+def test_warps_without_queries_or_keys(S, HD, causal, lens):
+    """Lengths around the 32 queries and 32 keys of a backward warp, which passes over what it does not see."""
+    B, NH, seed, p = 2, 2, 9, 0.1
+    g = torch.Generator(device="cuda").manual_seed(S)
+    w = NH * HD
+    q, k, v, do = (torch.randn(B * S, w, generator=g, device="cuda").bfloat16() for _ in range(4))
+    for t in (q, k, v):
+        t.requires_grad_(True)
+    ln = torch.tensor([S, max(1, S - 40)], dtype=torch.int32, device="cuda") if lens else None
+    y = F.flash_attention(q, k, v, B, NH, S, S, HD, causal=causal, kv_lens=ln, dropout_p=p, seed=seed)
+    y.backward(do)
+    want = _oracle(q.detach(), k.detach(), v.detach(), do, B, NH, S, S, HD, causal, ln, p, seed, None)
+    for a, e in zip([y.detach(), q.grad, k.grad, v.grad], want):
+        e = e.double()
+        assert float((a.double() - e).norm()) <= TOL * float(e.norm()) + HD * 2.0 ** -24 * float(do.double().norm())
+    assert native.check_status() == 0
