@@ -277,7 +277,8 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
     }
   }
   const float mx = block_reduce(tmax, true, sm);
-  const float s = block_reduce(tmax == -INFINITY ? tsum : tsum * __expf(tmax - mx), false, sm);
+  float s = block_reduce(tmax == -INFINITY ? tsum : tsum * __expf(tmax - mx), false, sm);
+  if (mx == -INFINITY) s = NAN;                    // no finite logit: no distribution, whatever the target (as in ce_stats)
   const float w = loss_mask ? loss_mask[row] : 1.0f;
   if (threadIdx.x == 0) loss[row] = (logf(s) + mx - tgt) * w;
   const float inv = 1.0f / s, gs = grad_scale * w;

@@ -179,3 +179,23 @@ def test_cross_entropy_of_many_rows(V):
 def test_adam_at_the_edges_of_its_forms(per_sm, extra, start):
     """An element a thread up to 1024 elements an SM, then vectors; from 8 x 2048 an SM on every block takes several passes."""
     test_adam_vector_and_scalar_parts(torch.cuda.get_device_properties(0).multi_processor_count * per_sm + extra, start)
+
+
+@pytest.mark.parametrize("V", [40, 1003, 2048, 40000])
+@pytest.mark.parametrize("rows", [9, 900])
+def test_cross_entropy_of_rows_that_are_not_finite(V, rows):
+    """Rows of -inf alone, with +inf or NaN in a vector or in the ragged end, targets in and outside the row: the one-pass form
+    gives what the two-pass form gives, NaN where that gives NaN."""
+    g = torch.Generator(device="cuda").manual_seed(V)
+    buf = torch.randn(rows, (V + 7) // 8 * 8, generator=g, device="cuda").bfloat16()
+    inf, nan = float("inf"), float("nan")
+    buf[0], buf[1], buf[2, :V // 2], buf[3, V // 2:] = -inf, -inf, -inf, -inf
+    buf[4, 3], buf[5, V - 1], buf[6, 3], buf[7, V - 1] = inf, inf, nan, nan
+    buf[8, :8] = nan
+    t = torch.randint(0, V, (rows,), generator=g, device="cuda")
+    t[1] = t[7] = V + 1                                   # another rank's target
+    one, two, ext = buf.clone(), buf.clone(), native.ext()
+    a = ext.ce_loss_grad(one[:, :V], t, None, 0, 0.5)
+    b = ext.ce_finalize(two[:, :V], t, ext.ce_stats(two[:, :V], t, 0), None, 0, 0.5, True)
+    assert torch.allclose(a, b, rtol=1e-5, atol=1e-5, equal_nan=True)
+    assert torch.allclose(one.float(), two.float(), rtol=2.0 ** -7, atol=0.0, equal_nan=True)   # one unit of bf16
