@@ -199,3 +199,9 @@ def test_cross_entropy_of_rows_that_are_not_finite(V, rows):
     b = ext.ce_finalize(two[:, :V], t, ext.ce_stats(two[:, :V], t, 0), None, 0, 0.5, True)
     assert torch.allclose(a, b, rtol=1e-5, atol=1e-5, equal_nan=True)
     assert torch.allclose(one.float(), two.float(), rtol=2.0 ** -7, atol=0.0, equal_nan=True)   # one unit of bf16
+
+
+@pytest.mark.parametrize("V", [32766, 40000])
+@pytest.mark.parametrize("n", [2048, 2049])               # two sequences: the last token count of 64-bit keys, the next one
+def test_embedding_gradient_where_keys_get_narrow(V, n):
+    test_embedding_gradient_keys(V, n)
