@@ -33,11 +33,11 @@
 // one key row per thread), 5 = drain.  The math of a step is a chain of waits and dependent arithmetic: with two warpgroups
 // of twice the columns (two warps per SM sub-partition) it, and not the tensor core, set the pace.
 //
-// Measured against the kernel it replaces (query blocks of 64, dQ through shared memory and bulk reductions), 16 x 16 heads of
-// 2048 x 128, whole backward: causal with dropout 1458 -> 1127 us (1181 with eight math warps), without 1377 -> 1065,
-// unmasked 2234 -> 1698; 32 x 16 heads of 512 x 64 with bias and dropout 613 -> 363 (490 with the diagonal sums as one
-// dependent chain of shuffles).  What bounds it at head size 128: the 64 KB of dQ a step that leave the SM (a copy of the
-// kernel without the reductions takes 1364 us unmasked, with plain stores in their place 1670).
+// Measured against the kernel it replaces (query blocks of 64, dQ through shared memory and bulk reductions), both timed in
+// turn, 16 x 16 heads of 2048 x 128, whole backward: causal with dropout 1465 -> 1225 us (5 % more with eight math warps),
+// without 1379 -> 1130, unmasked 2306 -> 1825; 32 x 16 heads of 512 x 64 with bias and dropout 654 -> 365 (a third more with
+// the diagonal sums as one dependent chain of shuffles).  What bounds it at head size 128: the 64 KB of dQ a step that leave
+// the SM (a copy of the kernel without the reductions took a fifth less unmasked, with plain stores in their place 2 % less).
 #include "attention_device.cuh"
 
 namespace ssb {

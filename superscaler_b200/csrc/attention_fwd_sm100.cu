@@ -11,13 +11,15 @@
 //   softmax warps: S -> registers, running maximum, P = exp2(..) as bf16 -> TMEM, each half over its own columns of S
 //   O  += P . V_j         P is the A operand straight from TMEM; accumulator in columns [256 + 128 t, .. + HD)
 // While the tensor core runs O += P V and the next S of one tile, the softmax warps of the other tile work: both units
-// stay busy and P never passes through shared memory.
+// stay busy and P never passes through shared memory.  (Published ideas: two query tiles in ping-pong, FlashAttention-3; P as an
+// operand in tensor memory, FlashAttention-4.)
 // The accumulator O stays in TMEM in the frame of the running maximum; where that grew for a row of a warp, the warp rescales
 // its columns of O itself, after its exponentials, when the registers of the scores are free again.  The row's largest
 // probability is then exactly one when it is rounded to bf16.  A reference that may lag by 2^8 saves most of these passes, but
-// rounds that probability: 2048 keys with scores of spread 3, relative error of O 2.24e-3 instead of 1.78e-3, and no time
-// gained (training layer of 16 x 16 heads 1737 instead of 1723 us, one sequence 41.0 either way; with the pass in front of
-// the exponentials 43.6).  P is a bf16 operand; the sums of the unrounded probabilities and the products are fp32.
+// rounds that probability: 2048 keys with scores of spread 3, relative error of O 2.24e-3 instead of 1.78e-3.  It gains 3 %
+// unmasked (510 instead of 525 us, 16 x 16 heads of 2048 x 128) and nothing under the causal mask (348 instead of 340); one
+// sequence takes 41.0 either way, 43.6 with the pass in front of the exponentials.  P is a bf16 operand; the sums of the
+// unrounded probabilities and the products are fp32.
 //
 // The kernel is persistent (one CTA per SM): the loads and the first product of the next item run under the epilogue
 // of the previous one.  Under the causal mask items are numbered heavy (late) query blocks first over all heads and
@@ -26,7 +28,7 @@
 // Without the mask all items cost the same and neighbours share a head.
 //
 // Measured against the one-tile kernel it replaces (128 queries a CTA, P through shared memory, four threads a row): causal,
-// 16 x 16 heads of 2048 x 128: 588 -> 346 us (794 TFLOP/s), with dropout 807 -> 405 us, unmasked 921 -> 488 us (1126 TFLOP/s);
+// 16 x 16 heads of 2048 x 128: 589 -> 340 us (808 TFLOP/s), with dropout 803 -> 395 us, unmasked 931 -> 525 us (1045 TFLOP/s);
 // one sequence of 16 heads 58.9 -> 41.0 us.  With one thread per row and four warps per tile the dropout form took 434 to
 // 449 us and T5's (bias, dropout, head size 64) 160 instead of 137: two warps per SM sub-partition could not cover the chain
 // S -> maximum -> exponentials -> P.  Tried on top, no gain: starting P.V on three quarters of the keys; slower: a separate
