@@ -724,9 +724,10 @@ class EmbeddingFn(torch.autograd.Function):
                 for keys_t, dst, k0 in ((ids, dW, v0), (pos, dP, 0)):
                     if keys_t is not None and dst is not None:
                         flat = keys_t.contiguous().view(-1)
-                        # Narrow keys take two or four passes of the radix sort instead of eight.  Up to 4096 keys the sort is one
-                        # short kernel either way and the extra call costs more host time than it saves: forward and
-                        # backward of 4096 tokens x 2048 136 us against 150, of 6144 254 against 170, of 16384 402 against 302.
+                        # Narrow keys take two or four passes of the radix sort instead of eight.  Up to 4096 keys the
+                        # sort is one short kernel either way and the extra call costs more host time than it saves:
+                        # forward and backward of 4096 tokens x 2048 136 us against 150, of 6144 254 against 175, of
+                        # 16384 402 against 302.
                         if flat.numel() > 4096:
                             flat, first = native.ext().embedding_keys(flat, k0, dst.shape[0]), 0
                         else:
