@@ -99,6 +99,28 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
+// The same without suspending the thread between looks: for the single thread whose wake-up latency everything waits for.
+__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  uint64_t t0 = 0;
+  for (uint32_t it = 0; it < kMbarSpinLimit * 16u; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 16383u) == 16383u) {
+      if (*abort_flag) return false;
+      const uint64_t now = global_timer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > kMbarTimeLimitNs) break;
+    }
+  }
+  *abort_flag = 1;
+  return false;
+}
+
 // Register budget of a warpgroup (every warp of it executes this); the sum over the block's warpgroups must stay within
 // what the block was launched with.
 template <int N>
@@ -152,6 +174,19 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
                "r"(smem_u32(smem_src)), "r"(x), "r"(y)
                : "memory");
 }
+// Adds `bytes` of fp32 values in shared memory to global memory (both 16-byte aligned, a multiple of 16 bytes; bulk async
+// group completion).
+__device__ __forceinline__ void bulk_add_f32(float* dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst),
+               "r"(smem_u32(smem_src)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
+               : "memory");
+}
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {
@@ -160,6 +195,33 @@ __device__ __forceinline__ void tma_store_wait_read() {
 template <int N>
 __device__ __forceinline__ void tma_store_wait() {
   asm volatile("cp.async.bulk.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Takes over a block of the grid that has not started yet, if there is one: a 16-byte answer arrives in shared memory and
+// completes 16 bytes on the mbarrier.  No further request may follow an answer that says there is none.
+__device__ __forceinline__ void launch_try_cancel(void* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// The answer: true with the index of the block taken over.
+__device__ __forceinline__ bool launch_cancelled(const void* answer, uint32_t& x, uint32_t& y, uint32_t& z) {
+  uint32_t yes, unused;
+  asm volatile(
+      "{\n"
+      ".reg .b128 ans;\n"
+      ".reg .pred p;\n"
+      "ld.shared.b128 ans, [%5];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, ans;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "mov.u32 %1, 0;\nmov.u32 %2, 0;\nmov.u32 %3, 0;\nmov.u32 %4, 0;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, %3, %4}, ans;\n"
+      "}\n"
+      : "=&r"(yes), "=&r"(x), "=&r"(y), "=&r"(z), "=&r"(unused)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return yes != 0;
 }
 
 // ------------------------------- tcgen05 -------------------------------------
