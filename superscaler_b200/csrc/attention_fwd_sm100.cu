@@ -4,8 +4,11 @@
 // ParallelSoftmaxFusionOp (scaled [causal|masked] softmax), ParallelSoftmaxDropoutOp and ParallelContextOp (bmm) --
 // runtime/megatron/model/flex_ops.py:711-1015 -- without ever writing the [b, np, sq, sk] score matrix to memory.
 //
-// A work item is 256 queries of one (batch, head): two tiles of 128 (or one, where tiles are few).  Every tile has eight softmax warps; two threads share a
-// query row (64 keys of a block each) and exchange one maximum per block through shared memory.
+// A work item is 256 queries of one (batch, head), two tiles of 128; where that leaves SMs idle or unequally loaded, one tile
+// whose even and odd key blocks go to the two slots, each with a maximum, a sum and an accumulator of its own that are brought
+// together at the end (one sequence of 16 causal heads of 2048 x 128: 41.4 -> 27.5 us, 4 of 1024 22.7 -> 15.1).  Every slot has
+// eight softmax warps; two threads share a query row (64 keys of a block each) and exchange one maximum per block through
+// shared memory.
 // Per key block of 128 and tile:
 //   S   = Q . K_j^T       fp32 accumulator in TMEM columns [128 t, 128 t + 128)
 //   softmax warps: S -> registers, running maximum, P = exp2(..) as bf16 -> TMEM, each half over its own columns of S
@@ -59,13 +62,16 @@ struct FwdCfg {
   static constexpr int kOutBytes = 16 * 32 * 64;           // per softmax warp: 32 rows x 32 output columns
   static constexpr int kXchBytes = 2 * 2 * 128 * 4;        // row maxima: [tile][half][row]
   static constexpr int kBarBytes = 256;
-  static constexpr int kSmem = 2 * kTile + kStages * kTile + kOutBytes + kXchBytes + kBarBytes;
+  // Score bias, per softmax warp: the distances of its 32 queries x 64 keys (32 x 16 heads of 512 x 64 with bias and dropout 121 ->
+  // 101 us).  No room at head size 128 (read from global memory).
+  static constexpr int kBiasBytes = HD == 64 ? 16 * 96 * 4 : 0;
+  static constexpr int kSmem = 2 * kTile + kStages * kTile + kOutBytes + kXchBytes + kBarBytes + kBiasBytes;
   static constexpr int kTmemCols = 512;                    // S/P 0, S/P 1, O 0, O 1: 128 columns each
 };
 
 struct FwdItems {
   int total, n_qb, heads;  // work items, query blocks per head, B * NH
-  int span;                // queries of a block: 256 (two tiles) or 128 (one)
+  int split;               // 0: a block is two tiles of 128 queries; 1: one tile, its key blocks dealt to the two slots in turn
 };
 
 struct FwdItem {
@@ -79,13 +85,14 @@ __device__ __forceinline__ FwdItem fwd_item(int idx, const FwdItems& it, const A
   const int hh = p.causal ? inner : outer;
   w.b = hh / p.NH;
   w.head = hh - w.b * p.NH;
-  w.q0 = qb * it.span;
+  w.q0 = qb * (it.split ? 128 : 256);
   w.kv_len = p.kv_lens ? max(0, min(p.kv_lens[w.b], p.SK)) : p.SK;
   const int n_kv = (w.kv_len + 127) >> 7;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int qt = w.q0 + t * 128;
-    w.n[t] = qt >= p.SQ || t * 128 >= it.span ? 0 : (p.causal ? min(n_kv, (qt >> 7) + 1) : n_kv);
+    const int qt = w.q0 + (it.split ? 0 : t * 128);
+    const int n = qt >= p.SQ ? 0 : (p.causal ? min(n_kv, (qt >> 7) + 1) : n_kv);
+    w.n[t] = it.split ? (n + 1 - t) >> 1 : n;
   }
   return w;
 }
@@ -106,7 +113,7 @@ __device__ __forceinline__ uint32_t quad_transpose(uint32_t h, uint32_t sel1, ui
   return __byte_perm(x, r2, sel2);
 }
 
-template <int HD, bool DROPOUT, bool BIAS>
+template <int HD, bool DROPOUT, bool BIAS, bool SPLIT>
 __global__ void __launch_bounds__(kFwdThreads, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const AttnParams p, const FwdItems items) {
@@ -175,8 +182,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
         if (idx >= items.total) continue;
         const FwdItem w = fwd_item(idx, items, p);
-        const int n = max(w.n[0], w.n[1]);
         const int kcol = p.k_col0 + w.head * HD, vcol = p.v_col0 + w.head * HD;
+        if constexpr (SPLIT) {  // Q K0 K1 V0 K2 V1 K3 ...
+          const int n = w.n[0] + w.n[1];
+          if (n == 0) continue;
+          if (!mbar_wait(&q_empty[0], (qn[0] & 1) ^ 1, abort_flag)) { ok = false; break; }
+          mbar_arrive_expect_tx(&q_full[0], Cfg::kTile);
+#pragma unroll
+          for (int c = 0; c < CH; ++c)
+            tma_load_3d(sQ + c * 16384, &tm_q, &q_full[0], p.q_col0 + w.head * HD + c * 64, w.q0, w.b);
+          ++qn[0];
+          ok = load_kv(&tm_k, kcol, 0, w.b);
+          if (ok && n > 1) ok = load_kv(&tm_k, kcol, 128, w.b);
+          for (int j = 0; j < n && ok; ++j) {
+            ok = load_kv(&tm_v, vcol, j * 128, w.b);
+            if (ok && j + 2 < n) ok = load_kv(&tm_k, kcol, (j + 2) * 128, w.b);
+          }
+          continue;
+        }
+        const int n = max(w.n[0], w.n[1]);
         for (int t = 0; t < 2 && ok && n > 0; ++t) {
           if (w.n[t] > 0) {
             if (!mbar_wait(&q_empty[t], (qn[t] & 1) ^ 1, abort_flag)) { ok = false; break; }
@@ -216,8 +240,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       Pipe pp;                               // next K / V stage to consume
       uint32_t qn[2] = {0, 0}, pn[2] = {0, 0};
       bool ok = true;
-      auto issue_s = [&](int t, int stage) {
-        const uint64_t a = q_k + t * kStep, bb = kv_k + stage * kStep;
+      auto issue_s = [&](int t, int qtile, int stage) {
+        const uint64_t a = q_k + qtile * kStep, bb = kv_k + stage * kStep;
 #pragma unroll
         for (int kk = 0; kk < HD / 16; ++kk) {
           const uint64_t off = ((kk >> 2) * 16384 + (kk & 3) * 32) >> 4;
@@ -225,19 +249,54 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         }
         umma_commit(&s_full[t]);
       };
+      auto issue_o = [&](int t, int stage, bool accumulate) {
+        const uint64_t bb = kv_mn + stage * kStep;
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16 (8 TMEM columns of packed bf16 pairs)
+          umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + (kk >> 2) * 64 + (kk & 3) * 8, bb + (kk * 2048 >> 4),
+                      idesc_o, accumulate || kk != 0);
+      };
       for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
         if (idx >= items.total) continue;
         const FwdItem w = fwd_item(idx, items, p);
+        if constexpr (SPLIT) {
+          const int n = w.n[0] + w.n[1];
+          if (n == 0) continue;
+          if (!(ok = mbar_spin(&q_full[0], qn[0] & 1, abort_flag))) break;
+          ++qn[0];
+          auto next_s = [&](int j) {  // scores of key block j
+            if (!(ok = mbar_spin(&kv_full[pp.stage], pp.phase, abort_flag))) return;
+            tc_fence_after_sync();
+            issue_s(j & 1, 0, pp.stage);
+            umma_commit(&kv_empty[pp.stage]);
+            if (j + 1 == n) umma_commit(&q_empty[0]);
+            pp.advance(NS);
+          };
+          for (int j = 0; j < min(n, 2) && ok; ++j) next_s(j);
+          for (int j = 0; j < n && ok; ++j) {
+            const int t = j & 1;
+            if (!(ok = mbar_spin(&kv_full[pp.stage], pp.phase, abort_flag))) break;
+            if (!(ok = mbar_spin(&p_full[t], pn[t] & 1, abort_flag))) break;
+            ++pn[t];
+            tc_fence_after_sync();
+            issue_o(t, pp.stage, j >= 2);
+            umma_commit(&kv_empty[pp.stage]);
+            pp.advance(NS);
+            if (j + 2 < n) next_s(j + 2);  // overwrites S / P of the slot: products retire in issue order
+            else umma_commit(&o_full[t]);
+          }
+          continue;
+        }
         const int n = max(w.n[0], w.n[1]);
         if (n == 0) continue;
         int sk = pp.stage;
-        if (!mbar_wait(&kv_full[sk], pp.phase, abort_flag)) break;
+        if (!mbar_spin(&kv_full[sk], pp.phase, abort_flag)) break;
         for (int t = 0; t < 2 && ok; ++t) {
           if (w.n[t] == 0) continue;
-          if (!mbar_wait(&q_full[t], qn[t] & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_spin(&q_full[t], qn[t] & 1, abort_flag)) { ok = false; break; }
           ++qn[t];
           tc_fence_after_sync();
-          issue_s(t, sk);
+          issue_s(t, t, sk);
           if (w.n[t] == 1) umma_commit(&q_empty[t]);
         }
         if (!ok) break;
@@ -251,23 +310,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           bool have_v = false, have_k = false;
           for (int t = 0; t < 2; ++t) {
             if (j >= w.n[t]) continue;
-            if (!have_v && !mbar_wait(&kv_full[sv], phv, abort_flag)) { ok = false; break; }
+            if (!have_v && !mbar_spin(&kv_full[sv], phv, abort_flag)) { ok = false; break; }
             have_v = true;
-            if (!mbar_wait(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_spin(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
             ++pn[t];
             tc_fence_after_sync();
-            const uint64_t bb = kv_mn + sv * kStep;
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16 (8 TMEM columns of packed bf16 pairs)
-              umma_f16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + (kk >> 2) * 64 + (kk & 3) * 8,
-                          bb + (kk * 2048 >> 4), idesc_o, (j | kk) != 0);
+            issue_o(t, sv, j != 0);
             if (j + 1 == w.n[t]) {
               umma_commit(&o_full[t]);
             } else {
-              if (!have_k && !mbar_wait(&kv_full[sk], pp.phase, abort_flag)) { ok = false; break; }
+              if (!have_k && !mbar_spin(&kv_full[sk], pp.phase, abort_flag)) { ok = false; break; }
               have_k = true;
               tc_fence_after_sync();
-              issue_s(t, sk);  // overwrites S / P of the tile: products retire in issue order
+              issue_s(t, t, sk);  // overwrites S / P of the tile: products retire in issue order
               if (j + 2 == w.n[t]) umma_commit(&q_empty[t]);
             }
           }
@@ -290,19 +345,29 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const uint32_t tm_s = tm_row + half * 64, tm_o = tm_row + 256 + half * (HD / 2);
     uint8_t* stage = sOut + (warp - 4) * 2048;
     float* xch = sXch + t * 256 + r;   // + half * 128
+    float* sBias = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + Cfg::kBarBytes) + (warp - 4) * 96;
     // The two warps that share these 32 rows meet once per key block and twice per item.
     auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + t * 4 + quarter) : "memory"); };
-    // A warp whose bounded wait ran out in its k-th item, `left` meetings before the item's end, still comes to all the
+    // The end of an item: with split keys the four warps of both slots that hold partial results of these rows.
+    auto end_sync = [&]() {
+      if constexpr (SPLIT) asm volatile("bar.sync %0, 128;" ::"r"(9 + quarter) : "memory");
+      else pair_sync();
+    };
+    // A warp whose bounded wait ran out in its k-th item, `left` blocks before the item's end, still comes to all the
     // meetings ahead: its partner may pass the same wait a moment later and must not be left waiting (its own next wait runs
     // out too, P of this warp being missing).  An mbarrier with the bounded wait at every meeting costs 10 % (one sequence of
     // 16 heads 41.0 -> 45.1 us), a barrier that tells both whether one gave up 5 % (43.0).
     auto meet_to_the_end = [&](int k, int left) {
       for (int idx;;) {
         for (; left > 0; --left) pair_sync();
-        if ((idx = fwd_item_index(++k, items.total)) < 0) return;
-        if (idx >= items.total) continue;
-        const FwdItem w = fwd_item(idx, items, p);
-        left = w.q0 + t * 128 < p.SQ && t * 128 < items.span ? w.n[t] + 2 : 0;
+        end_sync();
+        end_sync();
+        FwdItem w;
+        do {
+          if ((idx = fwd_item_index(++k, items.total)) < 0) return;
+          if (idx < items.total) w = fwd_item(idx, items, p);
+        } while (idx >= items.total || (!SPLIT && w.q0 + t * 128 >= p.SQ));
+        left = w.n[t];
       }
     };
     const float c = p.scale * kLog2e;
@@ -315,13 +380,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     const int sub = lane & 3;
     const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u, sel2 = (lane & 2) ? 0x3276u : 0x5410u;
     const uint32_t drop_c = (256u - keep8) * 0x01010101u;  // byte + drop_c carries out <=> byte >= keep8
-    uint32_t sn = 0, on = 0;  // blocks and items of this tile so far
+    uint32_t sn = 0, on0 = 0, on1 = 0;  // blocks of this slot so far; items with work for slot 0 and slot 1
     bool ok = true;
     for (int k = 0, idx; ok && (idx = fwd_item_index(k, items.total)) >= 0; ++k) {
       if (idx >= items.total) continue;
       const FwdItem w = fwd_item(idx, items, p);
-      const int qt = w.q0 + t * 128, q = qt + r;
-      if (qt >= p.SQ || t * 128 >= items.span) continue;
+      const int qt = w.q0 + (SPLIT ? 0 : t * 128), q = qt + r;
+      if (qt >= p.SQ) continue;
+      const int j0 = SPLIT ? t : 0, dj = SPLIT ? 2 : 1;  // key blocks of this slot: j0, j0 + dj, ...
       const int nt = w.n[t];
       uint32_t hash_base = 0, hash_step = 0;
       if constexpr (DROPOUT) {
@@ -329,14 +395,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const uint32_t bh_seed = static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(w.b) * p.NH + w.head));
         hash_base = (static_cast<uint32_t>(half * 64 + sub) * qquads + (static_cast<uint32_t>(q) >> 2)) * 0x9E3779B1u + bh_seed;
         hash_step = 4u * qquads * 0x9E3779B1u;
+        hash_base += static_cast<uint32_t>(32 * j0) * hash_step;
       }
       const float* bias_row = BIAS ? p.bias_table + static_cast<size_t>(w.head) * (p.SQ + p.SK - 1) + (p.SQ - 1) - min(q, p.SQ - 1)
                                    : nullptr;
       float m = -INFINITY, l = 0.f;
       for (int j = 0; j < nt; ++j) {
-        const int kv0 = j * 128 + half * 64;
+        const int kv0 = (j0 + j * dj) * 128 + half * 64;
+        if constexpr (BIAS && HD == 64) {  // (the reads of the block before are behind this warp's arrival)
+          const float* head_row = p.bias_table + static_cast<size_t>(w.head) * (p.SQ + p.SK - 1);
+          const int d = p.SQ - 32 - (qt + quarter * 32) + kv0 + lane;  // distance of (query 31, key 0) of this warp, + lane
+#pragma unroll
+          for (int i = 0; i < 3; ++i) sBias[i * 32 + lane] = __ldg(head_row + min(max(d + i * 32, 0), p.SQ + p.SK - 2));
+          __syncwarp();
+        }
         if (!mbar_wait_warp(&s_full[t], sn & 1, abort_flag)) {
-          meet_to_the_end(k, nt - j + 2);
+          meet_to_the_end(k, nt - j);
           ok = false;
           break;
         }
@@ -345,7 +419,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const bool masked = (p.causal && kv0 + 63 > qt) || kv0 + 64 > w.kv_len;  // diagonal block or ragged end
         const int lim = min(w.kv_len - 1, p.causal ? q : w.kv_len) - kv0;        // last visible key of this row
         auto prepare = [&](uint32_t (&x)[32], int k0) {
-          if constexpr (BIAS) {
+          if constexpr (BIAS && HD == 64) {
+            const float* br = sBias + 31 - lane + k0;
+#pragma unroll
+            for (int i = 0; i < 32; ++i) x[i] = __float_as_uint(fmaf(__uint_as_float(x[i]), c, br[i] * kLog2e));
+          } else if constexpr (BIAS) {
             const float* br = bias_row + kv0 + k0;
             if (kv0 + 64 <= p.SK) {
 #pragma unroll
@@ -421,7 +499,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         };
         exponentials(x0, 0);
         exponentials(x1, 1);
-        hash_base += 32u * hash_step;
+        hash_base += static_cast<uint32_t>(32 * dj) * hash_step;
         if (grown) {  // into the new frame; P.V of the block before completed with s_full (products retire in issue order)
           const float2 a2 = make_float2(alpha, alpha);
 #pragma unroll
@@ -444,59 +522,100 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         l = l * alpha + ((rs[0].x + rs[0].y) + (rs[1].x + rs[1].y));
       }
       if (!ok) break;
-      if (nt > 0) {
-        if (!mbar_wait_warp(&o_full[t], on & 1, abort_flag)) {
-          meet_to_the_end(k, 2);
-          break;
-        }
-        ++on;
-        tc_fence_after_sync();
+      // (both slots' sums where they share the tile)
+      if (w.n[0] > 0 && (SPLIT || t == 0)) ok = mbar_wait_warp(&o_full[0], on0++ & 1, abort_flag);
+      if (ok && w.n[1] > 0 && (SPLIT || t == 1)) ok = mbar_wait_warp(&o_full[1], on1++ & 1, abort_flag);
+      if (!ok) {
+        meet_to_the_end(k, 0);
+        break;
       }
-      {  // row sum: the two halves, added in one order by both (in the staging tiles, which are free here)
+      tc_fence_after_sync();
+      // Row sums of the halves, added in one order by all (in the staging tiles, which are free here); with split keys also
+      // the other slot's frame: factor f[u] brings slot u's sum and O into the common one.
+      float f0 = 1.f, f1 = 0.f;
+      {
         float* mine = reinterpret_cast<float*>(stage) + lane;
-        const float* other = reinterpret_cast<const float*>(sOut + (warp - 4 + (half ? -4 : 4)) * 2048) + lane;
-        *mine = l;
-        pair_sync();
-        const float lo = *other;
-        l = half ? lo + l : l + lo;
-        pair_sync();
+        auto of = [&](int slot, int hf) { return reinterpret_cast<const float*>(sOut + (slot * 8 + hf * 4 + ((warp - 4) & 3)) * 2048) + lane; };
+        mine[0] = l;
+        mine[32] = m;
+        end_sync();
+        const int own = SPLIT ? 0 : t;
+        l = of(own, 0)[0] + of(own, 1)[0];
+        if constexpr (SPLIT) {
+          const float m0 = of(0, 0)[32], m1 = of(1, 0)[32];
+          m = fmaxf(m0, m1);
+          f0 = m0 == -INFINITY ? 0.f : ex2((m0 - m) * cc);
+          f1 = m1 == -INFINITY ? 0.f : ex2((m1 - m) * cc);
+          l = l * f0 + (of(1, 0)[0] + of(1, 1)[0]) * f1;
+        } else {
+          end_sync();
+        }
       }
       const float inv_l = l > 0.f ? inv_keep / l : 0.f;
-      // 32 columns at a time through shared memory: 64-byte row segments to memory
-      auto cell = [&](int row, int piece) { return stage + row * 64 + ((piece ^ ((row >> 1) & 3)) << 4); };
-      __nv_bfloat16* obase = reinterpret_cast<__nv_bfloat16*>(p.O) + (static_cast<size_t>(w.b) * p.SQ + qt + quarter * 32) * p.ldo +
-                             p.o_col0 + w.head * HD + half * (HD / 2) + (lane & 3) * 8;
+      // 32 (16) columns at a time through shared memory: 64- (32-)byte row segments to memory
       const int rows_left = p.SQ - qt - quarter * 32;
+      __nv_bfloat16* obase = reinterpret_cast<__nv_bfloat16*>(p.O) + (static_cast<size_t>(w.b) * p.SQ + qt + quarter * 32) * p.ldo +
+                             p.o_col0 + w.head * HD + half * (HD / 2);
+      auto put = [&](auto& oo, int col) {  // a row's values -> row segments of O from column `col` of this half
+        constexpr int W = sizeof(oo) / 4, PIECES = W / 8, RPI = 32 / PIECES;
+        auto cell = [&](int row, int piece) { return stage + row * (W * 2) + ((piece ^ ((row >> (W == 32 ? 1 : 2)) & (PIECES - 1))) << 4); };
 #pragma unroll
-      for (int ch = 0; ch < HD / 64; ++ch) {
-        uint32_t oo[32];
-        if (nt > 0) {
-          tmem_ld_32x32(tm_o + ch * 32, oo);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) oo[i] = 0u;
-        }
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < PIECES; ++i) {
           uint4 v;
-          v.x = pack_bf16x2(__uint_as_float(oo[8 * i + 0]) * inv_l, __uint_as_float(oo[8 * i + 1]) * inv_l);
-          v.y = pack_bf16x2(__uint_as_float(oo[8 * i + 2]) * inv_l, __uint_as_float(oo[8 * i + 3]) * inv_l);
-          v.z = pack_bf16x2(__uint_as_float(oo[8 * i + 4]) * inv_l, __uint_as_float(oo[8 * i + 5]) * inv_l);
-          v.w = pack_bf16x2(__uint_as_float(oo[8 * i + 6]) * inv_l, __uint_as_float(oo[8 * i + 7]) * inv_l);
+          v.x = pack_bf16x2(__uint_as_float(oo[8 * i + 0]), __uint_as_float(oo[8 * i + 1]));
+          v.y = pack_bf16x2(__uint_as_float(oo[8 * i + 2]), __uint_as_float(oo[8 * i + 3]));
+          v.z = pack_bf16x2(__uint_as_float(oo[8 * i + 4]), __uint_as_float(oo[8 * i + 5]));
+          v.w = pack_bf16x2(__uint_as_float(oo[8 * i + 6]), __uint_as_float(oo[8 * i + 7]));
           *reinterpret_cast<uint4*>(cell(lane, i)) = v;
         }
         __syncwarp();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int row = i * 8 + (lane >> 2);
-          const uint4 v = *reinterpret_cast<const uint4*>(cell(row, lane & 3));
-          if (row < rows_left) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row) * p.ldo + ch * 32) = v;
+        for (int i = 0; i < 32 / RPI; ++i) {
+          const int row = i * RPI + lane / PIECES, piece = lane % PIECES;
+          const uint4 v = *reinterpret_cast<const uint4*>(cell(row, piece));
+          if (row < rows_left) *reinterpret_cast<uint4*>(obase + static_cast<size_t>(row) * p.ldo + col + piece * 8) = v;
         }
         __syncwarp();
+      };
+      if constexpr (SPLIT) {
+        // a quarter of the columns per warp: O of both slots, added in the common frame
+        constexpr int W = HD / 4;
+        const uint32_t src = tmem_base + 256 + (static_cast<uint32_t>(quarter * 32) << 16) + half * (HD / 2) + t * W;
+        uint32_t oo[W], ot[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) oo[i] = ot[i] = 0u;
+        if (w.n[0] > 0) tmem_ld_cols<W>(src, oo);
+        if (w.n[1] > 0) tmem_ld_cols<W>(src + 128, ot);
+        tmem_ld_wait();
+        // everyone's reads of O and of the exchanged sums are done: the staging tiles and, for the next item's first P.V, O
+        // are free
+        tc_fence_before_sync();
+        end_sync();
+        tc_fence_after_sync();
+        f0 *= inv_l;
+        f1 *= inv_l;
+#pragma unroll
+        for (int i = 0; i < W; ++i)
+          oo[i] = __float_as_uint(fmaf(__uint_as_float(ot[i]), f1, __uint_as_float(oo[i]) * f0));
+        put(oo, t * W);
+      } else {
+#pragma unroll
+        for (int ch = 0; ch < HD / 64; ++ch) {
+          uint32_t oo[32];
+          if (nt > 0) {
+            tmem_ld_32x32(tm_o + ch * 32, oo);
+            tmem_ld_wait();
+          } else {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) oo[i] = 0u;
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) oo[i] = __float_as_uint(__uint_as_float(oo[i]) * inv_l);
+          put(oo, ch * 32);
+        }
       }
       // rows with no visible key get +inf so that the backward probabilities exp(s - lse) vanish
-      if (half == 0 && q < p.SQ)
+      if (half == 0 && (!SPLIT || t == 0) && q < p.SQ)
         p.LSE[(static_cast<size_t>(w.b) * p.NH + w.head) * p.SQ + q] =
             l > 0.f ? m * (BIAS ? 1.0f / kLog2e : p.scale) + logf(l) : INFINITY;
       // the reads of O are ordered before the next item's P.V by the p_full arrival of its first block
@@ -513,22 +632,41 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
 }
 
+// Pairs of query tiles or single tiles with their key blocks split over the two slots: estimated time of the busiest SM, in tile
+// steps.  A split step costs a tenth more (K and V are fetched for 128 queries instead of 256, the slots are brought together at
+// the end), an item as much as 2.5 steps.  Without the mask all items are equal and whole rounds count; under it the longest item
+// or the mean counts.  Measured, pairs / split in us, head size 128: 16 causal heads of 2048 40.2 / 27.5, 4 of 1024 22.7 / 15.1,
+// 32 of 1024 24.2 / 20.2, 64 of 512 16.1 / 16.4, 32 of 2048 45.0 / 49.8; unmasked 16 of 1024 24.1 / 15.8, 16 of 2048 40.5 / 43.8,
+// 40 of 2048 111.7 / 103.1, 256 of 1024 142.6 / 163.4.
+bool fwd_split(long long heads, int SQ, int SK, int causal, int num_sms) {
+  const long long tiles = (SQ + 127) / 128, pairs = (tiles + 1) / 2;
+  const double n = (SK + 127) / 128, item = 2.5, step = 1.1;
+  if (!causal) {
+    const double rounds_pair = static_cast<double>((heads * pairs + num_sms - 1) / num_sms);
+    const double rounds_split = static_cast<double>((heads * tiles + num_sms - 1) / num_sms);
+    return rounds_split * (step * n + item) < rounds_pair * (2 * n + item);
+  }
+  const double steps = heads * n * (n + 1) / 2;
+  const double longest = tiles % 2 ? (n > 2 * n - 3 ? n : 2 * n - 3) : 2 * n - 1;
+  const double mean_pair = (steps + item * heads * pairs) / num_sms, mean_split = (step * steps + item * heads * tiles) / num_sms;
+  const double pair = longest + item > mean_pair ? longest + item : mean_pair;
+  const double split = step * n + item > mean_split ? step * n + item : mean_split;
+  return 1.05 * split < pair;
+}
+
 template <int HD, bool DROPOUT, bool BIAS>
 int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& p, int num_sms,
                cudaStream_t stream) {
-  const int rc = static_cast<int>(cudaFuncSetAttribute(attn_fwd_kernel<HD, DROPOUT, BIAS>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<HD>::kSmem));
-  if (rc) return rc;
   FwdItems it;
   it.heads = p.B * p.NH;
-  // Where every tile finds an SM of its own, the tiles of a pair would only share one: 4 heads of 1024 x 128 22.4 us in pairs,
-  // 20.3 alone (8 blocks of 128 x 128 either way), 64 heads of 256 x 64 9.6 and 8.3.  With more tiles than SMs a pair hides
-  // one tile's chain behind the other: 64 heads of 320 x 128 11.9 in pairs, 14.4 alone, unmasked 13.7 and 19.6.
-  it.span = static_cast<long long>(it.heads) * ((p.SQ + 127) / 128) <= num_sms ? 128 : 256;
-  it.n_qb = (p.SQ + it.span - 1) / it.span;
+  it.split = fwd_split(it.heads, p.SQ, p.SK, p.causal, num_sms);
+  it.n_qb = (p.SQ + (it.split ? 127 : 255)) / (it.split ? 128 : 256);
   it.total = it.n_qb * it.heads;
   const int grid = it.total < num_sms ? it.total : num_sms;
-  attn_fwd_kernel<HD, DROPOUT, BIAS><<<grid, kFwdThreads, FwdCfg<HD>::kSmem, stream>>>(tq, tk, tv, p, it);
+  auto kernel = it.split ? attn_fwd_kernel<HD, DROPOUT, BIAS, true> : attn_fwd_kernel<HD, DROPOUT, BIAS, false>;
+  const int rc = static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdCfg<HD>::kSmem));
+  if (rc) return rc;
+  kernel<<<grid, kFwdThreads, FwdCfg<HD>::kSmem, stream>>>(tq, tk, tv, p, it);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -92,7 +92,34 @@ def _oracle(q, k, v, do, B, NH, SQ, SK, HD, causal, lens, p, seed, bias):
     (131, 131, 64, False, None, 0.1, True),
 ])
 def test_attention_tile_edges(SQ, SK, HD, causal, lens, p, bias):
-    B, NH, seed = 3, 2, 77
+    _check(3, 2, SQ, SK, HD, causal, lens, p, bias)
+
+
+@pytest.mark.parametrize("B,NH,S,HD,causal,lens,p,bias", [
+    (5, 60, 300, 128, True, None, 0.1, False),            # 900 key blocks and 600 query pairs of unequal length
+    (4, 50, 260, 64, False, (260, 0, 129, 1), 0.0, False),  # blocks and samples without a visible key in between
+    (4, 40, 250, 64, False, (250, 128, 129, 3), 0.1, True),
+    (3, 50, 129, 128, False, None, 0.0, False),
+])
+def test_attention_with_more_work_items_than_sms(B, NH, S, HD, causal, lens, p, bias):
+    """CTAs that go on with further work items: backward key blocks, forward pairs of query tiles."""
+    _check(B, NH, S, S, HD, causal, lens, p, bias)
+
+
+@pytest.mark.parametrize("SQ,SK,HD,causal,lens,p,bias", [
+    (128, 128, 128, False, None, 0.0, False),             # one key block: the second slot stays empty
+    (100, 1000, 64, False, (129, 1000, 0), 0.1, False),   # the second slot empty for one sample, both for another
+    (70, 640, 128, False, (640, 300, 257), 0.1, False),
+    (2048, 2048, 128, True, None, 0.1, False),
+    (96, 385, 64, False, (385, 128, 256), 0.0, True),
+])
+def test_attention_with_few_query_tiles(SQ, SK, HD, causal, lens, p, bias):
+    """Forward with the key blocks of a tile dealt to two slots whose sums and accumulators are brought together."""
+    _check(3, 2, SQ, SK, HD, causal, lens, p, bias)
+
+
+def _check(B, NH, SQ, SK, HD, causal, lens, p, bias):
+    seed = 77
     g = torch.Generator(device="cuda").manual_seed(SQ * 1000 + SK)
     w = NH * HD
     r = lambda *s: torch.randn(s, generator=g, device="cuda")
