@@ -148,6 +148,8 @@ embedding_keys_kernel(const long long* __restrict__ ids, Key* __restrict__ keys,
   }
 }
 
+constexpr float kLog2e = 1.4426950408889634f;
+
 __device__ __forceinline__ float block_reduce(float v, bool is_max, float* sm) {
   v = is_max ? warp_max(v) : warp_sum(v);
   __syncthreads();  // protects `sm` between successive calls
@@ -232,6 +234,15 @@ ce_finalize_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* 
   }
 }
 
+// exp(x - off) = 2^((x - off) log2 e) of two packed logits, two differences and two products per instruction
+__device__ __forceinline__ float2 exp_pair(uint32_t two, float off) {
+  const float2 d = mul_f32x2(add_f32x2(unpack_bf16x2(two), make_float2(-off, -off)), make_float2(kLog2e, kLog2e));
+  float2 e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(d.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(d.y));
+  return e;
+}
+
 // Loss and gradient of whole rows in one pass over memory, for logits that no other rank shares.  The row is read once, into
 // shared memory; every thread keeps a running maximum and the sum of exponentials relative to it on the way, so that the
 // special-function unit works under the loads, and only the gradient is left for a second pass.  Same quantities as
@@ -264,15 +275,17 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
     for (int u = 0; u < 4; ++u) {
       if (v + u * T < nvec) {
         row_smem[v + u * T] = q[u];       // each thread reads back what it wrote: no barrier needed
-        const float2 a = unpack_bf16x2(q[u].x), b = unpack_bf16x2(q[u].y), c = unpack_bf16x2(q[u].z), d = unpack_bf16x2(q[u].w);
-        const float m8 = fmaxf(fmaxf(fmaxf(a.x, a.y), fmaxf(b.x, b.y)), fmaxf(fmaxf(c.x, c.y), fmaxf(d.x, d.y)));
+        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q[u]);
+        const float2 m2 = __bfloat1622float2(__hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+        const float m8 = fmaxf(m2.x, m2.y);
         if (m8 > tmax) {
           tsum *= __expf(tmax - m8);               // tmax = -inf: 0
           tmax = m8;
         }
         const float off = tmax == -INFINITY ? 0.f : tmax;
-        tsum += ((__expf(a.x - off) + __expf(a.y - off)) + (__expf(b.x - off) + __expf(b.y - off))) +
-                ((__expf(c.x - off) + __expf(c.y - off)) + (__expf(d.x - off) + __expf(d.y - off)));
+        const float2 s2 = add_f32x2(add_f32x2(exp_pair(q[u].x, off), exp_pair(q[u].y, off)),
+                                    add_f32x2(exp_pair(q[u].z, off), exp_pair(q[u].w, off)));
+        tsum += s2.x + s2.y;
       }
     }
   }
@@ -282,19 +295,25 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   const float w = loss_mask ? loss_mask[row] : 1.0f;
   if (threadIdx.x == 0) loss[row] = (logf(s) + mx - tgt) * w;
   const float inv = 1.0f / s, gs = grad_scale * w;
+  const float2 inv2 = make_float2(inv, inv), gs2 = make_float2(gs, gs);
+  const int tv = t >= 0 && t < V ? static_cast<int>(t >> 3) : -1;  // vector of the target
   for (int v = threadIdx.x; v < nvec; v += T) {
     const uint4 q = row_smem[v];
-    const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-    float f[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
+    float2 f[4] = {mul_f32x2(exp_pair(q.x, mx), inv2), mul_f32x2(exp_pair(q.y, mx), inv2),
+                   mul_f32x2(exp_pair(q.z, mx), inv2), mul_f32x2(exp_pair(q.w, mx), inv2)};
+    if (v == tv) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float pr = __expf(f[j] - mx) * inv;
-      if (static_cast<long long>(v) * 8 + j == t) pr -= 1.0f;
-      f[j] = pr * gs;
+      for (int j = 0; j < 4; ++j) {
+        if ((t & 7) == 2 * j) f[j].x -= 1.0f;
+        if ((t & 7) == 2 * j + 1) f[j].y -= 1.0f;
+      }
     }
     uint4 o;
-    o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
-    o.z = pack_bf16x2(f[4], f[5]); o.w = pack_bf16x2(f[6], f[7]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      f[j] = mul_f32x2(f[j], gs2);
+      reinterpret_cast<uint32_t*>(&o)[j] = pack_bf16x2(f[j].x, f[j].y);
+    }
     xv[v] = o;
   }
   if (k0 < V) {
