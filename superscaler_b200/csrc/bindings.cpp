@@ -52,6 +52,11 @@ int embedding_keys_launch(const long long* ids, void* keys, int key_bytes, long 
 int embedding_bwd_sorted_launch(const void* keys, int key_bytes, const long long* order, const void* g, float* dst,
                                 long long tokens, int H, long long k0, long long k1, float dropout_p,
                                 unsigned long long seed, cudaStream_t stream);
+int embedding_group_max_tokens();
+long long embedding_group_ints(long long tokens, long long rows);
+int embedding_bwd_grouped_launch(const long long* const* ids, const long long* k0, const long long* rows, float* const* dst,
+                                 int* ws, const void* g, long long tokens, int H, float dropout_p, unsigned long long seed,
+                                 cudaStream_t stream);
 int ce_stats_launch(const void* logits, int ld, const long long* targets, float* row_max, float* row_sum,
                     float* row_tgt, long long rows, int V, long long v0, cudaStream_t stream);
 int ce_finalize_launch(void* logits, int ld, const long long* targets, const float* gmax, const float* gsum,
@@ -404,6 +409,36 @@ void embedding_bwd_sorted(const Tensor& keys, const Tensor& order, const Tensor&
                                                 static_cast<float>(dropout_p), static_cast<unsigned long long>(seed),
                                                 cur_stream()),
                "embedding_bwd_sorted");
+}
+
+// dW[id - v0] += g and dP[pos] += g for up to embedding_group_max_tokens() tokens, rows summed in token order
+void embedding_bwd_grouped(const Tensor& ids, const OptTensor& pos, const Tensor& g, const Tensor& dW, const OptTensor& dP,
+                           int64_t v0, double dropout_p, int64_t seed) {
+  TORCH_CHECK(g.scalar_type() == torch::kBFloat16 && g.is_contiguous() && g.is_cuda());
+  const OptTensor idx[2] = {ids, dP.has_value() ? pos : OptTensor()};
+  const OptTensor dst[2] = {dW, dP};
+  TORCH_CHECK(!dP.has_value() || pos.has_value(), "a position table needs positions");
+  c10::cuda::CUDAGuard guard(g.device());
+  const int64_t tokens = ids.numel(), H = g.size(-1);
+  const long long* idp[2] = {nullptr, nullptr};
+  const long long k0[2] = {v0, 0};
+  long long rows[2] = {0, 0}, ints = 0;
+  float* out[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i) {
+    if (!idx[i].has_value()) continue;
+    TORCH_CHECK(idx[i]->is_cuda() && idx[i]->scalar_type() == torch::kInt64 && idx[i]->is_contiguous() &&
+                idx[i]->numel() == tokens && tokens * H == g.numel());
+    TORCH_CHECK(dst[i]->is_cuda() && dst[i]->scalar_type() == torch::kFloat32 && dst[i]->is_contiguous() && dst[i]->size(-1) == H);
+    idp[i] = reinterpret_cast<const long long*>(idx[i]->data_ptr<int64_t>());
+    rows[i] = dst[i]->size(0);
+    out[i] = dst[i]->data_ptr<float>();
+    ints += ssb::embedding_group_ints(tokens, rows[i]);
+  }
+  Tensor ws = torch::empty({ints}, torch::dtype(torch::kInt32).device(g.device()));
+  check_launch(ssb::embedding_bwd_grouped_launch(idp, k0, rows, out, ws.data_ptr<int>(), g.data_ptr(), tokens,
+                                                 static_cast<int>(H), static_cast<float>(dropout_p),
+                                                 static_cast<unsigned long long>(seed), cur_stream()),
+               "embedding_bwd_grouped");
 }
 
 // returns [3, rows] fp32: local max, sum exp(x - max), target logit (0 when the target is not local)
@@ -922,6 +957,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_bwd", &embedding_bwd);
   m.def("embedding_keys", &embedding_keys);
   m.def("embedding_bwd_sorted", &embedding_bwd_sorted);
+  m.def("embedding_bwd_grouped", &embedding_bwd_grouped);
+  m.def("embedding_group_max_tokens", &ssb::embedding_group_max_tokens);
   m.def("ce_loss_grad", &ce_loss_grad);
   m.def("ce_stats", &ce_stats);
   m.def("ce_finalize", &ce_finalize);

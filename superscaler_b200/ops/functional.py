@@ -720,20 +720,17 @@ class EmbeddingFn(torch.autograd.Function):
             if P is not None:
                 dP = mgP if mgP is not None else torch.zeros(P.shape, dtype=torch.float32, device=g.device)
             if _DETERMINISTIC_EMBEDDING_GRAD[0]:
-                # rows are summed run by run in token order: repeated runs give bitwise equal gradients
-                for keys_t, dst, k0 in ((ids, dW, v0), (pos, dP, 0)):
-                    if keys_t is not None and dst is not None:
-                        flat = keys_t.contiguous().view(-1)
-                        # Narrow keys take two or four passes of the radix sort instead of eight.  Up to 4096 keys the
-                        # sort is one short kernel either way and the extra call costs more host time than it saves:
-                        # forward and backward of 4096 tokens x 2048 136 us against 150, of 6144 254 against 175, of
-                        # 16384 402 against 302.
-                        if flat.numel() > 4096:
-                            flat, first = native.ext().embedding_keys(flat, k0, dst.shape[0]), 0
-                        else:
-                            first = k0
-                        keys, order = torch.sort(flat, stable=True)
-                        native.ext().embedding_bwd_sorted(keys, order, g, dst, first, dropout_p, seed)
+                # every row is summed in token order: repeated runs give bitwise equal gradients
+                if ids.numel() <= native.ext().embedding_group_max_tokens():
+                    native.ext().embedding_bwd_grouped(ids.contiguous().view(-1), pos.contiguous().view(-1) if pos is not None
+                                                       else None, g, dW, dP, v0, dropout_p, seed)
+                else:
+                    for keys_t, dst, k0 in ((ids, dW, v0), (pos, dP, 0)):
+                        if keys_t is not None and dst is not None:
+                            # narrow keys take two or four passes of the radix sort instead of eight
+                            flat = native.ext().embedding_keys(keys_t.contiguous().view(-1), k0, dst.shape[0])
+                            keys, order = torch.sort(flat, stable=True)
+                            native.ext().embedding_bwd_sorted(keys, order, g, dst, 0, dropout_p, seed)
             else:
                 native.ext().embedding_bwd(ids.contiguous().view(-1), pos.contiguous().view(-1) if pos is not None
                                            else None, g, dW, dP, v0, dropout_p, seed)

@@ -1,0 +1,57 @@
+"""The grouped embedding gradient (csrc/embedding_grad.cu) against the sort-based kernel, bit for bit: both sum a row's tokens
+in order.  Sizes around the limits of the kernel: one token, a token more than the threads of a cluster, the largest batch; runs
+around the length up to which tokens are ranked one by one; ids outside the table."""
+import pytest
+import torch
+
+from superscaler_b200.ops import native
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def sorted_grad(keys_t, dst, k0, g, p, seed):
+    keys, order = torch.sort(keys_t, stable=True)
+    native.ext().embedding_bwd_sorted(keys, order, g, dst, k0, p, seed)
+    return dst
+
+
+@pytest.mark.parametrize("tokens,V,S,H", [(1, 5, 1, 8), (33, 7, 16, 64), (1024, 50, 128, 520), (8193, 51200, 1024, 64),
+                                          (16384, 300, 2048, 2048), (65536, 65600, 512, 32)])
+@pytest.mark.parametrize("p", [0.0, 0.1])
+def test_grouped_embedding_gradient_equals_the_sorted_one(tokens, V, S, H, p):
+    torch.manual_seed(tokens + H)
+    k0 = 11
+    ids = torch.randint(k0 - 5, k0 + V + 5, (tokens,), device=DEV)     # some outside the table
+    pos = torch.arange(tokens, device=DEV) % S
+    g = torch.randn(tokens, H, device=DEV).bfloat16()
+    start_w, start_p = torch.randn(V, H, device=DEV), torch.randn(S, H, device=DEV)
+    dW, dP = start_w.clone(), start_p.clone()
+    native.ext().embedding_bwd_grouped(ids, pos, g, dW, dP, k0, p, 5)
+    assert torch.equal(dW, sorted_grad(ids, start_w.clone(), k0, g, p, 5))
+    assert torch.equal(dP, sorted_grad(pos, start_p.clone(), 0, g, p, 5))
+    alone = start_w.clone()
+    native.ext().embedding_bwd_grouped(ids, None, g, alone, None, k0, p, 5)
+    assert torch.equal(alone, dW)
+
+
+@pytest.mark.parametrize("run", [2, 5, 255, 256, 257, 4000])
+def test_runs_of_one_row(run):
+    torch.manual_seed(run)
+    tokens, V, H = 4000, 900, 136
+    ids = torch.randint(0, V, (tokens,), device=DEV)
+    ids[ids == 3] = 4
+    ids[torch.randperm(tokens, device=DEV)[:run]] = 3
+    g = torch.randn(tokens, H, device=DEV).bfloat16()
+    dW = torch.zeros(V, H, device=DEV)
+    native.ext().embedding_bwd_grouped(ids, None, g, dW, None, 0, 0.0, 0)
+    assert torch.equal(dW, sorted_grad(ids, torch.zeros(V, H, device=DEV), 0, g, 0.0, 0))
+
+
+def test_no_row_of_the_table_occurs():
+    ids, g = torch.full((100,), 9, device=DEV), torch.randn(100, 64, device=DEV).bfloat16()
+    dW = torch.ones(9, 64, device=DEV)
+    native.ext().embedding_bwd_grouped(ids, None, g, dW, None, 0, 0.0, 0)
+    assert torch.equal(dW, torch.ones(9, 64, device=DEV))
+    with pytest.raises(RuntimeError):
+        native.ext().embedding_bwd_grouped(ids[:0], None, g[:0], dW, None, 0, 0.0, 0)
