@@ -932,6 +932,8 @@ int64_t comm_max_blocks() { return ssb::comm_max_blocks(); }
 
 Tensor status() { return status_tensor(); }
 
+#include "autograd_nodes.h"
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -963,6 +965,12 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ce_stats", &ce_stats);
   m.def("ce_finalize", &ce_finalize);
   m.def("attn_fwd", &attn_fwd);
+  m.def("linear_node", &linear_node);
+  m.def("mlp_node", &mlp_node);
+  m.def("layernorm_node", &layernorm_node);
+  m.def("attention_node", &attention_node);
+  m.def("node_kernels", []() { return g_node_kernels.load(); });
+  m.def("node_calls", []() { return g_node_calls.load(); });
   m.def("attn_bwd", &attn_bwd);
   m.def("set_attn_bwd_deterministic", [](bool on) { g_attn_bwd_deterministic = on; });
   m.def("attn_bwd_deterministic", []() { return g_attn_bwd_deterministic; });

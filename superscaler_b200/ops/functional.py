@@ -153,6 +153,17 @@ def dropout_bwd(g, p, seed):
     raise RuntimeError("counter-based dropout exists only on the GPU path")
 
 
+def _native_node(x) -> bool:
+    """True when a call may go to the native autograd nodes (csrc/autograd_nodes.h): CUDA tensors in plain eager autograd.
+    Traced, compiled and functorch-transformed calls keep the Python functions, which those mechanisms know."""
+    return (x.is_cuda and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
+            and not torch.compiler.is_dynamo_compiling())
+
+
+def _main_grad(p):
+    return getattr(p, "main_grad", None)
+
+
 # --------------------------------------------------------------------------------------------
 # Linear (+ bias + activation + dropout + residual), one GEMM kernel forward, two backward
 # --------------------------------------------------------------------------------------------
@@ -201,6 +212,8 @@ class LinearFn(torch.autograd.Function):
 
 
 def linear(x, weight, bias=None, residual=None, act=ACT_NONE, dropout_p=0.0, seed=0):
+    if _native_node(x):
+        return native.ext().linear_node(x, weight, bias, residual, act, dropout_p, seed, _main_grad(weight), _main_grad(bias))
     return LinearFn.apply(x, weight, bias, residual, act, dropout_p, seed)
 
 
@@ -356,6 +369,9 @@ class MLPFn(torch.autograd.Function):
 
 
 def mlp(x, w1, b1, w2, b2, residual=None, act=ACT_GELU, dropout_p=0.0, seed=0):
+    if _native_node(x):
+        return native.ext().mlp_node(x, w1, b1, w2, b2, residual, act, dropout_p, seed, _main_grad(w1), _main_grad(b1),
+                                     _main_grad(w2), _main_grad(b2))
     return MLPFn.apply(x, w1, b1, w2, b2, residual, act, dropout_p, seed)
 
 
@@ -417,11 +433,15 @@ class LayerNormFn(torch.autograd.Function):
 
 
 def layernorm(x, gamma, beta, eps=1e-5):
+    if _native_node(x):
+        return native.ext().layernorm_node(x, gamma, beta, eps, False, _main_grad(gamma), _main_grad(beta))[0]
     return LayerNormFn.apply(x, gamma, beta, eps, False)
 
 
 def layernorm_keep_input(x, gamma, beta, eps=1e-5):
     """(LayerNorm(x), x): the second value is x for the residual add behind the normalised sub-layer."""
+    if _native_node(x):
+        return tuple(native.ext().layernorm_node(x, gamma, beta, eps, True, _main_grad(gamma), _main_grad(beta)))
     return LayerNormFn.apply(x, gamma, beta, eps, True)
 
 
@@ -612,6 +632,9 @@ def flash_attention(q, k, v, B, NH, SQ, SK, HD, cols=(0, 0, 0), scale=None, caus
     bias_table[h, key - query + SQ - 1] added after the scale (a relative-position bias as a table over the distance)."""
     if scale is None:
         scale = 1.0 / math.sqrt(HD)
+    if _native_node(q):
+        return native.ext().attention_node(q, k, v, B, NH, SQ, SK, HD, *cols, float(scale), bool(causal), kv_lens,
+                                           float(dropout_p), int(seed), bias_table)
     return FlashAttnFn.apply(q, k, v, B, NH, SQ, SK, HD, tuple(cols), float(scale), bool(causal), kv_lens,
                              float(dropout_p), int(seed), bias_table)
 

@@ -49,7 +49,27 @@ KERNELS_PER_CALL = {"gemm": 1, "layernorm_fwd": 1, "layernorm_bwd": 2, "colsum":
                     "attn_fwd": 1, "attn_bwd": 3, "im2col": 1, "col2im": 1, "conv_fprop": 1, "conv_dgrad": 1, "conv_wgrad": 1, "subsample": 1, "bn_fwd": 3, "bn_bwd": 3, "bn_apply": 1,
                     "maxpool_fwd": 1, "maxpool_bwd": 1, "avgpool": 1, "allreduce_scale_f32": 1,
                     "reduce_scatter_scale_sumsq_f32": 1, "allgather_b16": 1}
-launch_counter = {"kernels": 0, "calls": 0}
+
+
+class _LaunchCounter:
+    """Kernels launched and calls made since the entry was last set: those issued through the proxy below and those of the
+    native autograd nodes, which keep their own count."""
+
+    def __init__(self):
+        self.python = {"kernels": 0, "calls": 0}
+
+    @staticmethod
+    def _native(name):
+        return 0 if _mod is None else getattr(_mod, "node_" + name)()
+
+    def __getitem__(self, name):
+        return self.python[name] + self._native(name)
+
+    def __setitem__(self, name, value):
+        self.python[name] = value - self._native(name)
+
+
+launch_counter = _LaunchCounter()
 
 
 class _Counting:
@@ -67,9 +87,9 @@ class _Counting:
             if n == 0:
                 fn = raw
             else:
-                def fn(*a, _raw=raw, _n=n):
-                    launch_counter["kernels"] += _n
-                    launch_counter["calls"] += 1
+                def fn(*a, _raw=raw, _n=n, _count=launch_counter.python):
+                    _count["kernels"] += _n
+                    _count["calls"] += 1
                     return _raw(*a)
             self._cache[name] = fn
         return fn
