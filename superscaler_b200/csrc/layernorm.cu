@@ -18,10 +18,13 @@ namespace {
 
 constexpr int kLnWarpsPerBlock = 4;
 
-// VPL = uint4 vectors (8 bf16) per lane; H = VPL * 256.  VPL == 0 selects the generic
-// path that re-reads the row (any H that is a multiple of 8).
-template <int VPL>
-__global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
+// Rows that fit in the registers of a warp, read once: up to VPL vectors of 8 bf16 per lane; FULL = false: the last one, or for
+// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  fp32 arithmetic
+// two values per instruction.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984
+// 147 -> 55 us, of 1088 83 -> 33, 512 of 704 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
+// is slower (32768 x 2048 67 us instead of 55): too few warps.
+template <int VPL, bool FULL>
+__global__ void __launch_bounds__(kLnWarpsPerBlock * 32, VPL <= 2 ? 10 : VPL <= 4 ? 8 : 1)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
               const float* __restrict__ gamma, const float* __restrict__ beta, __nv_bfloat16* __restrict__ y,
               __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
@@ -30,80 +33,134 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   const int warp_global = blockIdx.x * kLnWarpsPerBlock + (threadIdx.x >> 5);
   const int warps_total = gridDim.x * kLnWarpsPerBlock;
   const int nvec = H / 8;
+  const bool last = (VPL - 1) * 32 + lane < nvec;
+  auto mine = [&](int i) { return FULL || (VPL > 8 ? i * 32 + lane < nvec : i < VPL - 1 || last); };
+  auto unpack = [](const uint4& q, float2 (&f)[4]) {
+    f[0] = unpack_bf16x2(q.x); f[1] = unpack_bf16x2(q.y); f[2] = unpack_bf16x2(q.z); f[3] = unpack_bf16x2(q.w);
+  };
   for (int row = warp_global; row < rows; row += warps_total) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
     const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * H) : nullptr;
     uint4* sr = sum_out ? reinterpret_cast<uint4*>(sum_out + static_cast<size_t>(row) * H) : nullptr;
-    constexpr int NV = VPL > 0 ? VPL : 1;
-    float vals[NV][8];
+    constexpr bool kPacked = VPL > 8;
+    float2 f[kPacked ? 1 : VPL][4];
+    uint4 q[kPacked ? VPL : 1];
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      uint4 x0 = mine(i) ? xr[i * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
+      float2(&v)[4] = f[kPacked ? 0 : i];
+      unpack(x0, v);
+      if (rr != nullptr && mine(i)) {
+        float2 g[4];
+        unpack(rr[i * 32 + lane], g);
+        uint4 o;
+        uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 t = add_f32x2(v[j], g[j]);
+          w[j] = pack_bf16x2(t.x, t.y);
+        }
+        if (sr) sr[i * 32 + lane] = o;
+        unpack(o, v);  // statistics are taken on the rounded sum so that forward and backward see the same x
+        x0 = o;
+      }
+      if constexpr (kPacked) q[i] = x0;
+      s = add_f32x2(s, add_f32x2(add_f32x2(v[0], v[1]), add_f32x2(v[2], v[3])));
+    }
+    const float mean = warp_sum(s.x + s.y) / static_cast<float>(H);
+    const float2 nm = make_float2(-mean, -mean);
+    s = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      if (!mine(i)) continue;
+      float2(&v)[4] = f[kPacked ? 0 : i];
+      if constexpr (kPacked) unpack(q[i], v);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        v[j] = add_f32x2(v[j], nm);
+        s = fma_f32x2(v[j], v[j], s);
+      }
+    }
+    const float rstd = rsqrtf(warp_sum(s.x + s.y) / static_cast<float>(H) + eps);
+    if (lane == 0) {
+      mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+    const float2 r2 = make_float2(rstd, rstd);
+    uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int v = i * 32 + lane;
+      if (!mine(i)) continue;
+      const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * v], g1 = reinterpret_cast<const float4*>(gamma)[2 * v + 1];
+      const float4 b0 = reinterpret_cast<const float4*>(beta)[2 * v], b1 = reinterpret_cast<const float4*>(beta)[2 * v + 1];
+      const float2 g[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
+      const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
+      float2(&d)[4] = f[kPacked ? 0 : i];
+      if constexpr (kPacked) {
+        unpack(q[i], d);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) d[j] = add_f32x2(d[j], nm);
+      }
+      uint4 o;
+      uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 t = fma_f32x2(mul_f32x2(d[j], r2), g[j], b[j]);
+        w[j] = pack_bf16x2(t.x, t.y);
+      }
+      yr[v] = o;
+    }
+  }
+}
+
+// Any row length that is a multiple of 8, parameters at any address: the row is read three times.
+__global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
+ln_fwd_long_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
+                   const float* __restrict__ gamma, const float* __restrict__ beta, __nv_bfloat16* __restrict__ y,
+                   __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
+                   int rows, int H, float eps) {
+  const int lane = threadIdx.x & 31;
+  const int warp_global = blockIdx.x * kLnWarpsPerBlock + (threadIdx.x >> 5);
+  const int warps_total = gridDim.x * kLnWarpsPerBlock;
+  const int nvec = H / 8;
+  for (int row = warp_global; row < rows; row += warps_total) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
+    const uint4* rr = residual ? reinterpret_cast<const uint4*>(residual + static_cast<size_t>(row) * H) : nullptr;
+    uint4* sr = sum_out ? reinterpret_cast<uint4*>(sum_out + static_cast<size_t>(row) * H) : nullptr;
     float s = 0.f;
-    if (VPL > 0) {
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        uint4 q = xr[i * 32 + lane];
-        float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
-        vals[i][0] = f0.x; vals[i][1] = f0.y; vals[i][2] = f1.x; vals[i][3] = f1.y;
-        vals[i][4] = f2.x; vals[i][5] = f2.y; vals[i][6] = f3.x; vals[i][7] = f3.y;
-        if (rr) {
-          uint4 r = rr[i * 32 + lane];
-          float2 g0 = unpack_bf16x2(r.x), g1 = unpack_bf16x2(r.y), g2 = unpack_bf16x2(r.z), g3 = unpack_bf16x2(r.w);
-          vals[i][0] += g0.x; vals[i][1] += g0.y; vals[i][2] += g1.x; vals[i][3] += g1.y;
-          vals[i][4] += g2.x; vals[i][5] += g2.y; vals[i][6] += g3.x; vals[i][7] += g3.y;
-          uint4 o;
-          o.x = pack_bf16x2(vals[i][0], vals[i][1]); o.y = pack_bf16x2(vals[i][2], vals[i][3]);
-          o.z = pack_bf16x2(vals[i][4], vals[i][5]); o.w = pack_bf16x2(vals[i][6], vals[i][7]);
-          if (sr) sr[i * 32 + lane] = o;
-          // statistics are taken on the rounded sum so that forward and backward see the same x
-          float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y), h2 = unpack_bf16x2(o.z), h3 = unpack_bf16x2(o.w);
-          vals[i][0] = h0.x; vals[i][1] = h0.y; vals[i][2] = h1.x; vals[i][3] = h1.y;
-          vals[i][4] = h2.x; vals[i][5] = h2.y; vals[i][6] = h3.x; vals[i][7] = h3.y;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s += vals[i][j];
+    for (int v = lane; v < nvec; v += 32) {
+      uint4 q = xr[v];
+      float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
+      float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+      if (rr) {
+        uint4 r = rr[v];
+        float2 g0 = unpack_bf16x2(r.x), g1 = unpack_bf16x2(r.y), g2 = unpack_bf16x2(r.z), g3 = unpack_bf16x2(r.w);
+        e[0] += g0.x; e[1] += g0.y; e[2] += g1.x; e[3] += g1.y; e[4] += g2.x; e[5] += g2.y; e[6] += g3.x; e[7] += g3.y;
+        uint4 o;
+        o.x = pack_bf16x2(e[0], e[1]); o.y = pack_bf16x2(e[2], e[3]);
+        o.z = pack_bf16x2(e[4], e[5]); o.w = pack_bf16x2(e[6], e[7]);
+        if (sr) sr[v] = o;
+        float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y), h2 = unpack_bf16x2(o.z), h3 = unpack_bf16x2(o.w);
+        e[0] = h0.x; e[1] = h0.y; e[2] = h1.x; e[3] = h1.y; e[4] = h2.x; e[5] = h2.y; e[6] = h3.x; e[7] = h3.y;
       }
-    } else {
-      for (int v = lane; v < nvec; v += 32) {
-        uint4 q = xr[v];
-        float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
-        float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-        if (rr) {
-          uint4 r = rr[v];
-          float2 g0 = unpack_bf16x2(r.x), g1 = unpack_bf16x2(r.y), g2 = unpack_bf16x2(r.z), g3 = unpack_bf16x2(r.w);
-          e[0] += g0.x; e[1] += g0.y; e[2] += g1.x; e[3] += g1.y; e[4] += g2.x; e[5] += g2.y; e[6] += g3.x; e[7] += g3.y;
-          uint4 o;
-          o.x = pack_bf16x2(e[0], e[1]); o.y = pack_bf16x2(e[2], e[3]);
-          o.z = pack_bf16x2(e[4], e[5]); o.w = pack_bf16x2(e[6], e[7]);
-          if (sr) sr[v] = o;
-          float2 h0 = unpack_bf16x2(o.x), h1 = unpack_bf16x2(o.y), h2 = unpack_bf16x2(o.z), h3 = unpack_bf16x2(o.w);
-          e[0] = h0.x; e[1] = h0.y; e[2] = h1.x; e[3] = h1.y; e[4] = h2.x; e[5] = h2.y; e[6] = h3.x; e[7] = h3.y;
-        }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) s += e[j];
-      }
+      for (int j = 0; j < 8; ++j) s += e[j];
     }
     const float mean = warp_sum(s) / static_cast<float>(H);
     float sq = 0.f;
-    // The generic path reads the (possibly just written) sum back; make the stores visible to the warp.
-    const uint4* src = (VPL == 0 && rr && sr) ? reinterpret_cast<const uint4*>(sr) : xr;
-    if (VPL == 0 && rr && sr) __syncwarp();
-    if (VPL > 0) {
+    // reads the (just written) sum back; make the stores visible to the warp
+    const uint4* src = (rr && sr) ? reinterpret_cast<const uint4*>(sr) : xr;
+    if (rr && sr) __syncwarp();
+    for (int v = lane; v < nvec; v += 32) {
+      uint4 q = src[v];
+      float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
+      float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
 #pragma unroll
-      for (int i = 0; i < NV; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float d = vals[i][j] - mean;
-          sq += d * d;
-        }
-    } else {
-      for (int v = lane; v < nvec; v += 32) {
-        uint4 q = src[v];
-        float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
-        float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float d = e[j] - mean;
-          sq += d * d;
-        }
+      for (int j = 0; j < 8; ++j) {
+        const float d = e[j] - mean;
+        sq += d * d;
       }
     }
     const float var = warp_sum(sq) / static_cast<float>(H);
@@ -113,35 +170,17 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       rstd_out[row] = rstd;
     }
     uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
-    if (VPL > 0) {
+    for (int v = lane; v < nvec; v += 32) {
+      uint4 q = src[v];
+      float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
+      float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
+      float o[8];
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int v = i * 32 + lane;
-        const float4 g0 = reinterpret_cast<const float4*>(gamma)[2 * v], g1 = reinterpret_cast<const float4*>(gamma)[2 * v + 1];
-        const float4 b0 = reinterpret_cast<const float4*>(beta)[2 * v], b1 = reinterpret_cast<const float4*>(beta)[2 * v + 1];
-        const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-        const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = (vals[i][j] - mean) * rstd * g[j] + b[j];
-        uint4 q;
-        q.x = pack_bf16x2(o[0], o[1]); q.y = pack_bf16x2(o[2], o[3]);
-        q.z = pack_bf16x2(o[4], o[5]); q.w = pack_bf16x2(o[6], o[7]);
-        yr[v] = q;
-      }
-    } else {
-      for (int v = lane; v < nvec; v += 32) {
-        uint4 q = src[v];
-        float2 f0 = unpack_bf16x2(q.x), f1 = unpack_bf16x2(q.y), f2 = unpack_bf16x2(q.z), f3 = unpack_bf16x2(q.w);
-        float e[8] = {f0.x, f0.y, f1.x, f1.y, f2.x, f2.y, f3.x, f3.y};
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = (e[j] - mean) * rstd * gamma[v * 8 + j] + beta[v * 8 + j];
-        uint4 w;
-        w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]);
-        w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
-        yr[v] = w;
-      }
+      for (int j = 0; j < 8; ++j) o[j] = (e[j] - mean) * rstd * gamma[v * 8 + j] + beta[v * 8 + j];
+      uint4 w;
+      w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]);
+      w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
+      yr[v] = w;
     }
   }
 }
@@ -610,18 +649,30 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
   const auto* rb = reinterpret_cast<const __nv_bfloat16*>(residual);
   auto* yb = reinterpret_cast<__nv_bfloat16*>(y);
   auto* sb = reinterpret_cast<__nv_bfloat16*>(sum_out);
-#define SSB_LN_CASE(V)                                                                                       \
-  ln_fwd_kernel<V><<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
-  // 16-byte loads of gamma and beta; parameters that start elsewhere take the generic kernel
+#define SSB_LN_ARGS <<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
+#define SSB_LN_CASE(V)                                          \
+  case V:                                                       \
+    if (H == V * 256) ln_fwd_kernel<V, true> SSB_LN_ARGS;       \
+    else ln_fwd_kernel<V, false> SSB_LN_ARGS;                   \
+    break
+  // 16-byte loads of gamma and beta; parameters that start elsewhere take the kernel for any address
   const bool wide = !misaligned(gamma) && !misaligned(beta);
-  switch (wide ? H : 0) {
-    case 512: SSB_LN_CASE(2); break;
-    case 1024: SSB_LN_CASE(4); break;
-    case 2048: SSB_LN_CASE(8); break;
-    case 4096: SSB_LN_CASE(16); break;
-    default: SSB_LN_CASE(0); break;
+  switch (wide ? (H + 255) / 256 : 0) {
+    SSB_LN_CASE(1);
+    SSB_LN_CASE(2);
+    SSB_LN_CASE(3);
+    SSB_LN_CASE(4);
+    SSB_LN_CASE(5);
+    SSB_LN_CASE(6);
+    SSB_LN_CASE(7);
+    SSB_LN_CASE(8);
+    case 9: case 10: case 11: case 12: ln_fwd_kernel<12, false> SSB_LN_ARGS; break;
+    case 13: case 14: case 15: ln_fwd_kernel<16, false> SSB_LN_ARGS; break;
+    SSB_LN_CASE(16);
+    default: ln_fwd_long_kernel SSB_LN_ARGS; break;
   }
 #undef SSB_LN_CASE
+#undef SSB_LN_ARGS
   return static_cast<int>(cudaGetLastError());
 }
 
