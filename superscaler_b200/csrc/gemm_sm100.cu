@@ -417,6 +417,10 @@ int launch_variant(const void* A, int lda, const void* B, int ldb, const GemmPar
 int gemm2_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                       const GemmParams& p, int num_sms, cudaStream_t stream);
 
+void gemm_cluster_plan(int M, int N, int K, bool simple, int num_sms, int* bn, int* slices);
+int gemm_cluster_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const GemmParams& p, int bn, int slices,
+                        cudaStream_t stream);
+
 // 0 = always the one-CTA kernel, 1 = two-SM kernel where the output has enough 256 x 256 tiles.
 static int g_pair_mode = 1;
 void gemm_set_pair_mode(int mode) { g_pair_mode = mode; }
@@ -428,6 +432,11 @@ int gemm_splitk_splits(int M, int N, int K, int num_sms) {
     if (M >= 256 && N >= 256 && tiles_pair >= num_sms / 4) return 1;     // the two-SM kernel takes it
   }
   if (N % 4) return 1;
+  if (g_pair_mode && K < 64 * BK) {        // shorter reductions are split inside a cluster, without a workspace
+    int bn, slices;
+    gemm_cluster_plan(M, N, K, false, num_sms, &bn, &slices);
+    if (slices > 0) return 1;
+  }
   const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
   const bool bn128 = (N <= 128) || (tiles256 < num_sms);
   const int tiles = ((M + BM - 1) / BM) * ((N + (bn128 ? 127 : 255)) / (bn128 ? 128 : 256));
@@ -458,6 +467,11 @@ int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int 
     const int tiles_pair = ((p.M + 255) / 256) * ((p.N + 255) / 256);
     if (p.M >= 256 && p.N >= 256 && tiles_pair >= num_sms / 4)
       return gemm2_bf16_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, num_sms, stream);
+    int bn, slices;
+    const bool simple = !p.out_fp32 && !p.accumulate && p.preact_out == nullptr && p.aux == nullptr && p.residual == nullptr &&
+                        p.dropout_p == 0.f;
+    gemm_cluster_plan(p.M, p.N, p.K, simple, num_sms, &bn, &slices);
+    if (slices > 0) return gemm_cluster_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, bn, slices, stream);
   }
   // Narrow outputs use the 128-wide tile so fewer columns are wasted and more CTAs are busy.
   const int tiles256 = ((p.M + BM - 1) / BM) * ((p.N + 255) / 256);

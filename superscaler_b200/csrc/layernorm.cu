@@ -24,7 +24,7 @@ constexpr int kLnWarpsPerBlock = 4;
 // 147 -> 55 us, of 1088 83 -> 33, 512 of 704 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
 // is slower (32768 x 2048 67 us instead of 55): too few warps.
 template <int VPL, bool FULL>
-__global__ void __launch_bounds__(kLnWarpsPerBlock * 32, VPL <= 2 ? 10 : VPL <= 4 ? 8 : 1)
+__global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
               const float* __restrict__ gamma, const float* __restrict__ beta, __nv_bfloat16* __restrict__ y,
               __nv_bfloat16* __restrict__ sum_out, float* __restrict__ mean_out, float* __restrict__ rstd_out,
