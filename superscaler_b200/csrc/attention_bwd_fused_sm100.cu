@@ -465,6 +465,18 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const float* bias_head = BIAS ? p.bias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
     float* dbias_head = BIAS ? p.dbias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
 
+    // Score bias of a block, fetched a block ahead: with the loads in front of their use a step waited 700 cycles for them
+    constexpr bool kBiasStaged = BIAS && HD == 64;
+    float bias_next[2] = {0.f, 0.f};
+    auto fetch_bias = [&](int q0) {
+      if constexpr (kBiasStaged) {
+        const int d = kv0 + quarter * 32 - q0 + p.SQ - 32 + lane;  // distance of (key 0, query 31) of this warp, + lane
+        bias_next[0] = __ldg(bias_head + min(max(d, 0), n_dist - 1));
+        bias_next[1] = __ldg(bias_head + min(max(d + 32, 0), n_dist - 1));
+      }
+    };
+    fetch_bias(w.i0 * 128 + g * 32);
+
     for (int i = 0; i < w.n_it; ++i, ++n) {
       const uint32_t ph = n & 1;
       const int qblk0 = (w.i0 + i) * 128, qbase = qblk0 + g * 32;
@@ -491,6 +503,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + e) ^ (r & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
         fence_proxy_async_smem();
         warp_arrive(ds_full, lane);
+        fetch_bias(qbase + 128);
         continue;
       }
       uint32_t drop = 0u;  // bit 7 - n of byte e: query 4 n + e dropped for this key; hashed before the scores are there
@@ -504,11 +517,9 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           drop |= (((x & drop_c) | ((x | drop_c) & cs)) & 0x80808080u) >> n;
         }
       }
-      if constexpr (BIAS && HD == 64) {  // (the reads of the block before are behind this warp's arrivals)
-        const int d = kv0 + quarter * 32 - qbase + p.SQ - 32 + lane;  // distance of (key 0, query 31) of this warp, + lane
-        const float b0 = __ldg(bias_head + min(max(d, 0), n_dist - 1)), b1 = __ldg(bias_head + min(max(d + 32, 0), n_dist - 1));
-        sBias[lane] = b0;
-        sBias[lane + 32] = b1;
+      if constexpr (kBiasStaged) {  // (the reads of the block before are behind this warp's arrivals)
+        sBias[lane] = bias_next[0];
+        sBias[lane + 32] = bias_next[1];
         __syncwarp();
       }
       if (!mbar_wait_warp(&q_full[ph], (n >> 1) & 1, abort_flag)) { ok = false; break; }  // the statistics
@@ -523,7 +534,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int e = 0; e < 32; e += 4) {
           float4 nl = *reinterpret_cast<const float4*>(nlse2 + e);
-          if constexpr (BIAS && HD == 64) {
+          if constexpr (kBiasStaged) {
             const float* br = sBias + lane + 31 - e;  // entries run down as the query runs up
             nl.x = fmaf(br[0], kLog2e, nl.x);
             nl.y = fmaf(br[-1], kLog2e, nl.y);
@@ -558,6 +569,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       tmem_st_wait();
       tc_fence_before_sync();
       warp_arrive(p_full, lane);
+      fetch_bias(qbase + 128);
       if (!mbar_wait_warp(dp_full, ph, abort_flag)) { ok = false; break; }
       tc_fence_after_sync();
       float diag = 0.f, wrap = 0.f;  // BIAS: sums along the diagonals through (lane, 0) and, wrapped, 32 distances below

@@ -19,10 +19,10 @@ namespace {
 constexpr int kLnWarpsPerBlock = 4;
 
 // Rows that fit in the registers of a warp, read once: up to VPL vectors of 8 bf16 per lane; FULL = false: the last one, or for
-// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  fp32 arithmetic
-// two values per instruction.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984
+// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984
 // 147 -> 55 us, of 1088 83 -> 33, 512 of 704 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
-// is slower (32768 x 2048 67 us instead of 55): too few warps.
+// is slower (32768 x 2048 67 us instead of 55): too few warps; so is fp32 arithmetic two values per instruction (32768 x 1024
+// 28.1 -> 29.9).
 template <int VPL, bool FULL>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
@@ -45,7 +45,7 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
     constexpr bool kPacked = VPL > 8;
     float2 f[kPacked ? 1 : VPL][4];
     uint4 q[kPacked ? VPL : 1];
-    float2 s = make_float2(0.f, 0.f);
+    float s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       uint4 x0 = mine(i) ? xr[i * 32 + lane] : make_uint4(0u, 0u, 0u, 0u);
@@ -58,19 +58,18 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
         uint32_t* w = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const float2 t = add_f32x2(v[j], g[j]);
-          w[j] = pack_bf16x2(t.x, t.y);
+          w[j] = pack_bf16x2(v[j].x + g[j].x, v[j].y + g[j].y);
         }
         if (sr) sr[i * 32 + lane] = o;
         unpack(o, v);  // statistics are taken on the rounded sum so that forward and backward see the same x
         x0 = o;
       }
       if constexpr (kPacked) q[i] = x0;
-      s = add_f32x2(s, add_f32x2(add_f32x2(v[0], v[1]), add_f32x2(v[2], v[3])));
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s += v[j].x + v[j].y;
     }
-    const float mean = warp_sum(s.x + s.y) / static_cast<float>(H);
-    const float2 nm = make_float2(-mean, -mean);
-    s = make_float2(0.f, 0.f);
+    const float mean = warp_sum(s) / static_cast<float>(H);
+    s = 0.f;
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       if (!mine(i)) continue;
@@ -78,16 +77,16 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       if constexpr (kPacked) unpack(q[i], v);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        v[j] = add_f32x2(v[j], nm);
-        s = fma_f32x2(v[j], v[j], s);
+        v[j].x -= mean;
+        v[j].y -= mean;
+        s += v[j].x * v[j].x + v[j].y * v[j].y;
       }
     }
-    const float rstd = rsqrtf(warp_sum(s.x + s.y) / static_cast<float>(H) + eps);
+    const float rstd = rsqrtf(warp_sum(s) / static_cast<float>(H) + eps);
     if (lane == 0) {
       mean_out[row] = mean;
       rstd_out[row] = rstd;
     }
-    const float2 r2 = make_float2(rstd, rstd);
     uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
@@ -101,14 +100,13 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
       if constexpr (kPacked) {
         unpack(q[i], d);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) d[j] = add_f32x2(d[j], nm);
+        for (int j = 0; j < 4; ++j) d[j] = make_float2(d[j].x - mean, d[j].y - mean);
       }
       uint4 o;
       uint32_t* w = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const float2 t = fma_f32x2(mul_f32x2(d[j], r2), g[j], b[j]);
-        w[j] = pack_bf16x2(t.x, t.y);
+        w[j] = pack_bf16x2(d[j].x * rstd * g[j].x + b[j].x, d[j].y * rstd * g[j].y + b[j].y);
       }
       yr[v] = o;
     }
