@@ -37,8 +37,8 @@
 // one key row per thread), 5 = drain.  The math of a step is a chain of waits and dependent arithmetic: with two warpgroups
 // of twice the columns (two warps per SM sub-partition) it, and not the tensor core, set the pace.
 //
-// The single threads that issue loads and products look for their barriers without suspending: their wake-up (300 to 500
-// cycles from a suspended wait) is on the path of every step.
+// The thread that issues the products looks for its barriers without suspending: its wake-up (300 to 500 cycles from a suspended
+// wait) is on the path of every step (with dropout 1020 -> 970 us, whole backward; the loads' thread gains nothing by it).
 //
 // Measured (kernel alone; whole backward in brackets), with one item per CTA and dQ reduced from registers -> now: 16 x 16 heads
 // of 2048 x 128 causal with dropout 951 -> 784 us (1111 -> 985), without (1073 -> 963), 4 x 16 unmasked (427 -> 370); 32 x 16
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
                       const __grid_constant__ CUtensorMap tm_dk, const __grid_constant__ CUtensorMap tm_dv,
-                      float* __restrict__ dq_acc, const AttnParams p) {
+                      float* __restrict__ dq_acc, const AttnParams p, const int more_items) {
   using Cfg = FusedCfg<HD>;
   constexpr int CH = Cfg::kCh, NDO = Cfg::kDoStages, NKV = Cfg::kKvStages;
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -179,6 +179,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   };
   // Answer to request r: true with the item, false when no block is left (or a wait ran out).
   auto take_item = [&](int r, Item& w) {
+    if (!more_items) return false;
     if (!mbar_wait(&item_full[r & 1], (r >> 1) & 1, abort_flag)) return false;
     uint32_t x, y, z;
     const bool more = launch_cancelled(&next_item[r & 1], x, y, z);
@@ -200,14 +201,14 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       };
       auto load_kv = [&](uint8_t* dst, const CUtensorMap* tm, uint64_t* full, uint64_t* empty, int col, int& n) {
         const int st = n % NKV;
-        if (!ok || !(ok = mbar_spin(&empty[st], ((n / NKV) & 1) ^ 1, abort_flag))) return;
+        if (!ok || !(ok = mbar_wait(&empty[st], ((n / NKV) & 1) ^ 1, abort_flag))) return;
         mbar_arrive_expect_tx(&full[st], Cfg::kTile);
         load_tile(dst + st * Cfg::kTile, tm, &full[st], col + w.head * HD, w.jb * 128);
         ++n;
       };
       auto load_q = [&](int i) {
         const int st = nq & 1;
-        if (!ok || !(ok = mbar_spin(&q_empty[st], ((nq >> 1) & 1) ^ 1, abort_flag))) return;
+        if (!ok || !(ok = mbar_wait(&q_empty[st], ((nq >> 1) & 1) ^ 1, abort_flag))) return;
         mbar_arrive_expect_tx(&q_full[st], Cfg::kTile + Cfg::kStatBytes);
         load_tile(sQ + st * Cfg::kTile, &tm_q, &q_full[st], p.q_col0 + w.head * HD, (w.i0 + i) * 128);
         bulk_load(sStat + st * 256, p.LSE + (w.tile0 + i) * 128, 512, &q_full[st]);
@@ -216,7 +217,7 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       };
       auto load_do = [&](int i) {
         const int st = ndo % NDO;
-        if (!ok || !(ok = mbar_spin(&do_empty[st], ((ndo / NDO) & 1) ^ 1, abort_flag))) return;
+        if (!ok || !(ok = mbar_wait(&do_empty[st], ((ndo / NDO) & 1) ^ 1, abort_flag))) return;
         mbar_arrive_expect_tx(&do_full[st], Cfg::kTile);
         load_tile(sdO + st * Cfg::kTile, &tm_do, &do_full[st], p.o_col0 + w.head * HD, (w.i0 + i) * 128);
         ++ndo;
@@ -234,7 +235,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           }
         }
         // The next item, one or two steps ahead of the end of this one.
-        if (!ok || !(ok = mbar_spin(&item_empty[r & 1], ((r >> 1) & 1) ^ 1, abort_flag))) break;
+        if (!more_items) break;
+        if (!ok || !(ok = mbar_wait(&item_empty[r & 1], ((r >> 1) & 1) ^ 1, abort_flag))) break;
         mbar_arrive_expect_tx(&item_full[r & 1], 16);
         launch_try_cancel(&next_item[r & 1], &item_full[r & 1]);
         if (!take_item(r, w)) break;
@@ -741,12 +743,13 @@ int set_smem(K kernel, int bytes) {
 
 template <int HD, bool DROPOUT, bool BIAS>
 int launch_fused(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                 const CUtensorMap& tdk, const CUtensorMap& tdv, const AttnParams& p, float* dq_acc, cudaStream_t stream) {
+                 const CUtensorMap& tdk, const CUtensorMap& tdv, const AttnParams& p, float* dq_acc, int num_sms, cudaStream_t stream) {
   int rc;
   if ((rc = set_smem(attn_bwd_fused_kernel<HD, DROPOUT, BIAS>, FusedCfg<HD>::kSmem))) return rc;
   const int n_tiles = (p.SQ + 127) / 128;
   dim3 grid_kv((p.SK + 127) / 128, p.NH, p.B);
-  attn_bwd_fused_kernel<HD, DROPOUT, BIAS><<<grid_kv, kFusedThreads, FusedCfg<HD>::kSmem, stream>>>(tq, tk, tv, tdo, tdk, tdv, dq_acc, p);
+  attn_bwd_fused_kernel<HD, DROPOUT, BIAS><<<grid_kv, kFusedThreads, FusedCfg<HD>::kSmem, stream>>>(
+      tq, tk, tv, tdo, tdk, tdv, dq_acc, p, static_cast<long long>(grid_kv.x) * grid_kv.y * grid_kv.z > num_sms);
   dim3 grid_cv(n_tiles * (HD / 32), p.NH, p.B);
   attn_dq_convert_kernel<HD><<<grid_cv, 128, 0, stream>>>(dq_acc, reinterpret_cast<__nv_bfloat16*>(p.dQ), p.lddq,
                                                           p.dq_col0, p.NH, p.SQ, n_tiles, p.scale);
@@ -763,7 +766,7 @@ long long attn_bwd_fused_scratch_floats(int B, int NH, int SQ, int HD) {
 // dout shares the layout of O (p.ldo / p.o_col0 describe both).  `scratch` holds attn_bwd_fused_scratch_floats()
 // floats, 16-byte aligned; the accumulator part is cleared here, on `stream`.
 int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const void* dout,
-                          int lddo, const AttnParams& p, float* scratch, cudaStream_t stream) {
+                          int lddo, const AttnParams& p, float* scratch, int num_sms, cudaStream_t stream) {
   if (p.HD != 64 && p.HD != 128) return -2;
   if (p.causal && p.SQ != p.SK) return -2;
   // 16-byte granularity everywhere: TMA x coordinates (column offsets of Q / K / V / dO), the 16-byte stores of
@@ -806,16 +809,16 @@ int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const 
   if (p.bias_table != nullptr) {
     if (p.dbias_table == nullptr) return -2;
     if (p.HD == 128)
-      return drop ? launch_fused<128, true, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream)
-                  : launch_fused<128, false, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream);
-    return drop ? launch_fused<64, true, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream)
-                : launch_fused<64, false, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream);
+      return drop ? launch_fused<128, true, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream)
+                  : launch_fused<128, false, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream);
+    return drop ? launch_fused<64, true, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream)
+                : launch_fused<64, false, true>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream);
   }
   if (p.HD == 128)
-    return drop ? launch_fused<128, true, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream)
-                : launch_fused<128, false, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream);
-  return drop ? launch_fused<64, true, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream)
-              : launch_fused<64, false, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, stream);
+    return drop ? launch_fused<128, true, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream)
+                : launch_fused<128, false, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream);
+  return drop ? launch_fused<64, true, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream)
+              : launch_fused<64, false, false>(tq, tk, tv, tdo, tdk, tdv, pp, dq_acc, num_sms, stream);
 }
 
 }  // namespace ssb

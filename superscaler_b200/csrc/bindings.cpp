@@ -68,7 +68,7 @@ int attn_bwd_launch(const void* q, int ldq, const void* k, int ldk, const void* 
                     int lddo, const AttnParams& p, float* delta_scratch, cudaStream_t stream);
 long long attn_bwd_fused_scratch_floats(int B, int NH, int SQ, int HD);
 int attn_bwd_fused_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const void* dout,
-                          int lddo, const AttnParams& p, float* scratch, cudaStream_t stream);
+                          int lddo, const AttnParams& p, float* scratch, int num_sms, cudaStream_t stream);
 int comm_max_blocks();
 void comm_set_peer_timeout_ns(unsigned long long ns);
 int allreduce_scale_f32_launch(void* const* peer_ptrs, void* mc_ptr, void* const* flag_ptrs, int rank, int world,
@@ -571,7 +571,7 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
     check_launch(ssb::attn_bwd_fused_launch(q.data_ptr(), static_cast<int>(q.stride(0)), k.data_ptr(),
                                             static_cast<int>(k.stride(0)), v.data_ptr(), static_cast<int>(v.stride(0)),
                                             dout.data_ptr(), static_cast<int>(dout.stride(0)), p,
-                                            scratch.data_ptr<float>(), cur_stream()),
+                                            scratch.data_ptr<float>(), num_sms(), cur_stream()),
                  "attn_bwd_fused");
     return;
   }
