@@ -10,6 +10,7 @@
 #pragma once
 #include <torch/csrc/autograd/custom_function.h>
 
+#include <array>
 #include <atomic>
 
 std::atomic<long long> g_node_kernels{0}, g_node_calls{0};  // launches issued by nodes (the counterpart of the Python counter)
@@ -24,13 +25,40 @@ using torch::autograd::variable_list;
 
 constexpr int64_t kEwBiasGeluBwd = 1, kEwDropoutBwd = 4, kEwReluBwd = 6;
 
+// A parameter whose gradient a node takes.  Its fp32 buffer `main_grad` is an attribute of the Python object and is asked for
+// when the backward runs, as the other autograd functions do: it may be attached, replaced or taken away after the forward.
+// The reference does not own the parameter (whoever may look at its gradient does).
+struct ParamRef {
+  c10::optional<c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>> ref;
+  c10::ScalarType type = torch::kFloat32;
+};
+ParamRef param_ref(const OptTensor& param) {
+  ParamRef r;
+  if (param.has_value()) {
+    r.ref.emplace(param->getIntrusivePtr());
+    r.type = param->scalar_type();
+  }
+  return r;
+}
+
 // Gradient of a parameter: added to its fp32 buffer when it has one (nothing to return then), else returned in its type.
 struct ParamGrad {
   OptTensor main;
   c10::ScalarType type;
 };
-ParamGrad param_grad(const OptTensor& main, const OptTensor& param) {
-  return {main, param.has_value() ? param->scalar_type() : torch::kFloat32};
+template <size_t N>
+std::array<ParamGrad, N> param_grads(const ParamRef* const (&params)[N]) {
+  std::array<ParamGrad, N> out;
+  pybind11::gil_scoped_acquire gil;
+  for (size_t i = 0; i < N; ++i) {
+    out[i].type = params[i]->type;
+    if (!params[i]->ref.has_value()) continue;
+    auto impl = params[i]->ref->lock();
+    if (!impl.defined()) continue;
+    const pybind11::object main = pybind11::getattr(pybind11::cast(Tensor(std::move(impl))), "main_grad", pybind11::none());
+    if (!main.is_none()) out[i].main = main.cast<Tensor>();
+  }
+  return out;
 }
 OptTensor some(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
 const OptTensor kNone;
@@ -79,7 +107,7 @@ struct NodeArgs : torch::CustomClassHolder {
   bool want_x = false, want_w = false, want_b = false;
   int64_t act = 0, seed = 0;
   double dropout_p = 0.0;
-  ParamGrad w, b, w2, b2;
+  ParamRef w, b, w2, b2;
   // attention
   int64_t B = 0, NH = 0, SQ = 0, SK = 0, HD = 0, qc = 0, kc = 0, vc = 0;
   double scale = 1.0;
@@ -110,14 +138,17 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
     if (a->act != 0) g = node_elementwise(a->act == ssb::kActGelu ? kEwBiasGeluBwd : kEwReluBwd, pre, g, 0.0, 0);
     Tensor dx, dw, db;
     if (a->want_x) dx = node_gemm(g, w, Tensor(), false, true, kNone, 0, kNone, kNone, kNone, false, 0.0, 0);
-    if (a->want_w) dw = node_wgrad(a->w, g, x);
-    if (a->want_b) db = node_bgrad(a->b, g);
+    if (a->want_w || a->want_b) {
+      const auto pg = param_grads({&a->w, &a->b});
+      if (a->want_w) dw = node_wgrad(pg[0], g, x);
+      if (a->want_b) db = node_bgrad(pg[1], g);
+    }
     return {dx, dw, db, a->has_res ? dy : Tensor(), Tensor(), Tensor()};
   }
 };
 
 Tensor linear_node(const Tensor& x, const Tensor& w, const OptTensor& bias, const OptTensor& res, int64_t act, double dropout_p,
-                   int64_t seed, const OptTensor& main_w, const OptTensor& main_b) {
+                   int64_t seed) {
   auto a = c10::make_intrusive<NodeArgs>();
   a->has_res = res.has_value();
   a->want_x = x.requires_grad();
@@ -126,8 +157,8 @@ Tensor linear_node(const Tensor& x, const Tensor& w, const OptTensor& bias, cons
   a->act = act;
   a->dropout_p = dropout_p;
   a->seed = seed;
-  a->w = param_grad(main_w, w);
-  a->b = param_grad(main_b, bias);
+  a->w = param_ref(w);
+  a->b = param_ref(bias);
   const bool training = at::GradMode::is_enabled() && (a->want_x || a->want_w || a->want_b || wants(res));
   return LinearNode::apply(x, w, bias, res, a, training);
 }
@@ -150,20 +181,20 @@ struct MlpNode : torch::autograd::Function<MlpNode> {
     const Tensor dy = grads[0].contiguous();
     const Tensor g2 = node_dropout_bwd(dy, a->dropout_p, a->seed);
     Tensor dx, db1, db2;
-    Tensor dw2 = node_wgrad(a->w2, g2, h);
-    if (a->has_bias) db2 = node_bgrad(a->b2, g2);
+    const auto pg = param_grads({&a->w, &a->b, &a->w2, &a->b2});
+    Tensor dw2 = node_wgrad(pg[2], g2, h);
+    if (a->has_bias) db2 = node_bgrad(pg[3], g2);
     const Tensor g1 = node_gemm(g2, w2, Tensor(), false, true, kNone, a->act == ssb::kActGelu ? ssb::kActDGelu : ssb::kActDRelu,
                                 pre, kNone, kNone, false, 0.0, 0);
-    Tensor dw1 = node_wgrad(a->w, g1, x);
-    if (a->want_b) db1 = node_bgrad(a->b, g1);
+    Tensor dw1 = node_wgrad(pg[0], g1, x);
+    if (a->want_b) db1 = node_bgrad(pg[1], g1);
     if (a->want_x) dx = node_gemm(g1, w1, Tensor(), false, true, kNone, 0, kNone, kNone, kNone, false, 0.0, 0);
     return {dx, dw1, db1, dw2, db2, a->has_res ? dy : Tensor(), Tensor(), Tensor()};
   }
 };
 
 Tensor mlp_node(const Tensor& x, const Tensor& w1, const OptTensor& b1, const Tensor& w2, const OptTensor& b2,
-                const OptTensor& res, int64_t act, double dropout_p, int64_t seed, const OptTensor& main_w1,
-                const OptTensor& main_b1, const OptTensor& main_w2, const OptTensor& main_b2) {
+                const OptTensor& res, int64_t act, double dropout_p, int64_t seed) {
   auto a = c10::make_intrusive<NodeArgs>();
   a->has_res = res.has_value();
   a->has_bias = b2.has_value();   // the biases' gradients are taken whenever the layer has them
@@ -172,10 +203,10 @@ Tensor mlp_node(const Tensor& x, const Tensor& w1, const OptTensor& b1, const Te
   a->act = act;
   a->dropout_p = dropout_p;
   a->seed = seed;
-  a->w = param_grad(main_w1, w1);
-  a->b = param_grad(main_b1, b1);
-  a->w2 = param_grad(main_w2, w2);
-  a->b2 = param_grad(main_b2, b2);
+  a->w = param_ref(w1);
+  a->b = param_ref(b1);
+  a->w2 = param_ref(w2);
+  a->b2 = param_ref(b2);
   const bool training = any_grad({&x, &w1, &w2}) || (at::GradMode::is_enabled() && (wants(b1) || wants(b2) || wants(res)));
   return MlpNode::apply(x, w1, b1, w2, b2, res, a, training);
 }
@@ -199,21 +230,21 @@ struct LayerNormNode : torch::autograd::Function<LayerNormNode> {
     if (!grads[0].defined()) return {dres, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};  // only the residual branch was used
     const Tensor dy = grads[0].contiguous();
     if (dres.defined()) dres = dres.contiguous();
-    const bool accumulate = a->w.main.has_value() && a->b.main.has_value();
-    Tensor dg = accumulate ? *a->w.main : torch::empty_like(gamma, torch::kFloat32);
-    Tensor db = accumulate ? *a->b.main : torch::empty_like(gamma, torch::kFloat32);
+    const auto pg = param_grads({&a->w, &a->b});
+    const bool accumulate = pg[0].main.has_value() && pg[1].main.has_value();
+    Tensor dg = accumulate ? *pg[0].main : torch::empty_like(gamma, torch::kFloat32);
+    Tensor db = accumulate ? *pg[1].main : torch::empty_like(gamma, torch::kFloat32);
     Tensor dx = layernorm_bwd(dy, x, gamma, mean, rstd, some(dres), dg, db, accumulate);
     count_kernels(2);
     if (accumulate) return {dx, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
-    return {dx, dg.to(a->w.type), db.to(a->b.type), Tensor(), Tensor(), Tensor()};
+    return {dx, dg.to(pg[0].type), db.to(pg[1].type), Tensor(), Tensor(), Tensor()};
   }
 };
 
-variable_list layernorm_node(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, bool pass_through,
-                             const OptTensor& main_g, const OptTensor& main_b) {
+variable_list layernorm_node(const Tensor& x, const Tensor& gamma, const Tensor& beta, double eps, bool pass_through) {
   auto a = c10::make_intrusive<NodeArgs>();
-  a->w = param_grad(main_g, gamma);
-  a->b = param_grad(main_b, beta);
+  a->w = param_ref(gamma);
+  a->b = param_ref(beta);
   return LayerNormNode::apply(x, gamma, beta, eps, pass_through, a);
 }
 

@@ -160,10 +160,6 @@ def _native_node(x) -> bool:
             and not torch.compiler.is_dynamo_compiling())
 
 
-def _main_grad(p):
-    return getattr(p, "main_grad", None)
-
-
 # --------------------------------------------------------------------------------------------
 # Linear (+ bias + activation + dropout + residual), one GEMM kernel forward, two backward
 # --------------------------------------------------------------------------------------------
@@ -213,7 +209,7 @@ class LinearFn(torch.autograd.Function):
 
 def linear(x, weight, bias=None, residual=None, act=ACT_NONE, dropout_p=0.0, seed=0):
     if _native_node(x):
-        return native.ext().linear_node(x, weight, bias, residual, act, dropout_p, seed, _main_grad(weight), _main_grad(bias))
+        return native.ext().linear_node(x, weight, bias, residual, act, dropout_p, seed)
     return LinearFn.apply(x, weight, bias, residual, act, dropout_p, seed)
 
 
@@ -370,8 +366,7 @@ class MLPFn(torch.autograd.Function):
 
 def mlp(x, w1, b1, w2, b2, residual=None, act=ACT_GELU, dropout_p=0.0, seed=0):
     if _native_node(x):
-        return native.ext().mlp_node(x, w1, b1, w2, b2, residual, act, dropout_p, seed, _main_grad(w1), _main_grad(b1),
-                                     _main_grad(w2), _main_grad(b2))
+        return native.ext().mlp_node(x, w1, b1, w2, b2, residual, act, dropout_p, seed)
     return MLPFn.apply(x, w1, b1, w2, b2, residual, act, dropout_p, seed)
 
 
@@ -434,14 +429,14 @@ class LayerNormFn(torch.autograd.Function):
 
 def layernorm(x, gamma, beta, eps=1e-5):
     if _native_node(x):
-        return native.ext().layernorm_node(x, gamma, beta, eps, False, _main_grad(gamma), _main_grad(beta))[0]
+        return native.ext().layernorm_node(x, gamma, beta, eps, False)[0]
     return LayerNormFn.apply(x, gamma, beta, eps, False)
 
 
 def layernorm_keep_input(x, gamma, beta, eps=1e-5):
     """(LayerNorm(x), x): the second value is x for the residual add behind the normalised sub-layer."""
     if _native_node(x):
-        return tuple(native.ext().layernorm_node(x, gamma, beta, eps, True, _main_grad(gamma), _main_grad(beta)))
+        return tuple(native.ext().layernorm_node(x, gamma, beta, eps, True))
     return LayerNormFn.apply(x, gamma, beta, eps, True)
 
 
