@@ -14,6 +14,7 @@
 namespace ssb {
 int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                      const GemmParams& p, int num_sms, cudaStream_t stream);
+int gemm_route(const GemmParams& p, int num_sms, int* bn, int* slices);
 void gemm_set_pair_mode(int mode);
 int gemm_get_pair_mode();
 int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
@@ -206,6 +207,23 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& d, bool a_mn, bool b_mn, con
   check_launch(ssb::gemm_bf16_launch(a.data_ptr(), static_cast<int>(a.stride(0)), a_mn, b.data_ptr(),
                                      static_cast<int>(b.stride(0)), b_mn, p, num_sms(), cur_stream()),
                "gemm");
+}
+
+// (kernel, tile width, slices) that a product with these operands takes, or a negative code: see gemm_route.  Addresses are only
+// looked at, 0 = operand not there; needs no device.
+std::tuple<int64_t, int64_t, int64_t> gemm_route(int64_t M, int64_t N, int64_t K, bool out_fp32, bool accumulate, int64_t act,
+                                                 int64_t bias, int64_t aux, int64_t preact_out, int64_t residual,
+                                                 double dropout_p, int64_t sms) {
+  ssb::GemmParams p{};
+  p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
+  p.out_fp32 = out_fp32; p.accumulate = accumulate; p.act = static_cast<int>(act); p.dropout_p = static_cast<float>(dropout_p);
+  p.bias = reinterpret_cast<const void*>(bias);
+  p.aux = reinterpret_cast<const void*>(aux);
+  p.preact_out = reinterpret_cast<void*>(preact_out);
+  p.residual = reinterpret_cast<const void*>(residual);
+  int bn = 0, slices = 0;
+  const int route = ssb::gemm_route(p, static_cast<int>(sms), &bn, &slices);
+  return {route, route == 2 ? bn : 0, route == 2 ? slices : 0};
 }
 
 std::vector<Tensor> layernorm_fwd(const Tensor& x, const OptTensor& residual, const Tensor& gamma, const Tensor& beta,
@@ -937,6 +955,7 @@ Tensor status() { return status_tensor(); }
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  m.def("gemm_route", &gemm_route);
   m.def("gemm", &gemm);
   m.def("gemm_allreduce", &gemm_allreduce);
   m.def("allgather_gemm", &allgather_gemm);

@@ -449,6 +449,28 @@ int gemm_splitk_splits(int M, int N, int K, int num_sms) {
   return (num_kb + kb_per - 1) / kb_per;   // no empty slice
 }
 
+// The kernel that takes a product: 0 one CTA per tile, 1 pairs of SMs, 2 clusters (then with *bn and *slices); negative: refused.
+// Row operands of the epilogue that do not start on 16 bytes: the kernel with one CTA per tile moves them by elements where no
+// 32 columns are whole (N < 32); every other kernel and width moves 16 bytes at a time (the cluster kernel all of them, also
+// where N is small), and on the device that would be a misaligned access.  The bias is read that way by all but the cluster
+// kernel.
+int gemm_route(const GemmParams& p, int num_sms, int* bn, int* slices) {
+  auto off16 = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+  const bool derivative = p.act == kActDGelu || p.act == kActDRelu;
+  const bool rows_off = off16(p.residual) || off16(p.preact_out) || (derivative && off16(p.aux));
+  if (rows_off && p.N >= 32) return -4;
+  *slices = 0;
+  if (g_pair_mode && p.k_splits <= 1) {
+    const int tiles_pair = ((p.M + 255) / 256) * ((p.N + 255) / 256);
+    if (p.M >= 256 && p.N >= 256 && tiles_pair >= num_sms / 4) return off16(p.bias) ? -4 : 1;
+    const bool simple = !p.out_fp32 && !p.accumulate && p.preact_out == nullptr && p.aux == nullptr && p.residual == nullptr &&
+                        p.dropout_p == 0.f;
+    if (!rows_off) gemm_cluster_plan(p.M, p.N, p.K, simple, num_sms, bn, slices);
+    if (*slices > 0) return 2;
+  }
+  return off16(p.bias) && p.N >= 32 ? -4 : 0;
+}
+
 // Launches the GEMM on `stream`.  Returns 0 or a CUDA / driver error code; argument errors are negative.
 int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                      const GemmParams& p, int num_sms, cudaStream_t stream) {
@@ -463,16 +485,12 @@ int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int 
     if (!plain || p.split_ws == nullptr || (p.N % 4) || (reinterpret_cast<uintptr_t>(p.split_ws) & 15) ||
         p.k_splits > (p.K + BK - 1) / BK)
       return -5;
-  } else if (g_pair_mode) {
-    const int tiles_pair = ((p.M + 255) / 256) * ((p.N + 255) / 256);
-    if (p.M >= 256 && p.N >= 256 && tiles_pair >= num_sms / 4)
-      return gemm2_bf16_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, num_sms, stream);
-    int bn, slices;
-    const bool simple = !p.out_fp32 && !p.accumulate && p.preact_out == nullptr && p.aux == nullptr && p.residual == nullptr &&
-                        p.dropout_p == 0.f;
-    gemm_cluster_plan(p.M, p.N, p.K, simple, num_sms, &bn, &slices);
-    if (slices > 0) return gemm_cluster_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, bn, slices, stream);
   }
+  int bn, slices;
+  const int route = gemm_route(p, num_sms, &bn, &slices);
+  if (route < 0) return route;
+  if (route == 1) return gemm2_bf16_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, num_sms, stream);
+  if (route == 2) return gemm_cluster_launch(A, lda, a_mn_major, B, ldb, b_mn_major, p, bn, slices, stream);
   // Narrow outputs use the 128-wide tile so fewer columns are wasted and more CTAs are busy.
   const int tiles256 = ((p.M + BM - 1) / BM) * ((p.N + 255) / 256);
   const bool bn128 = (p.N <= 128) || (tiles256 < num_sms);

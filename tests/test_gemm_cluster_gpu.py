@@ -68,3 +68,20 @@ def test_cluster_gemm_is_repeatable():
     torch.manual_seed(4)
     a, w = torch.randn(512, 4096, device=DEV).bfloat16(), torch.randn(512, 4096, device=DEV).bfloat16()
     assert torch.equal(F.gemm(a, w), F.gemm(a, w))
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 24, 2000), (130, 16, 64), (513, 8, 512)])
+@pytest.mark.parametrize("shift", [1, 2, 4])
+def test_narrow_outputs_with_operands_off_a_boundary(M, N, K, shift):
+    """Column views that do not start on 16 bytes (refused where 32 columns are whole)."""
+    torch.manual_seed(N + shift)
+    bf = lambda *s: torch.randn(*s, device=DEV).bfloat16()
+    view = lambda t: t[:, shift:shift + N]
+    a, w, res, x, pre = bf(M, K), bf(N, K) * 0.05, view(bf(M, 64)), view(bf(M, 64)), view(bf(M, 64))
+    want = a.double() @ w.double().t()
+    assert rel(F.gemm(a, w, residual=res), want + res.double()) < 2.0 ** -8
+    assert rel(F.gemm(a, w, act=F.ACT_DRELU, aux=x), want * (x > 0)) < 2.0 ** -8
+    y = F.gemm(a, w, act=F.ACT_RELU, preact_out=pre)
+    assert rel(pre, want) < 2.0 ** -8 and rel(y, want.relu()) < 2.0 ** -8
+    with pytest.raises(RuntimeError, match="gemm"):
+        F.gemm(a, bf(40, K), residual=bf(M, 64)[:, shift:shift + 40])

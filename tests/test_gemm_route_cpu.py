@@ -1,0 +1,45 @@
+"""Which GEMM kernel takes a product (csrc/gemm_sm100.cu, gemm_route): a function of sizes, options and addresses that needs no
+device.  Epilogue operands that start off a 16-byte boundary may only reach the kernel that moves them by elements."""
+import pytest
+
+from superscaler_b200.ops import functional as F
+from superscaler_b200.ops import native
+
+native._load()
+pytestmark = pytest.mark.skipif(native._mod is None, reason="native extension not built")
+SMS = 148
+EVEN, ODD = 0x1000, 0x1008            # addresses on and off a 16-byte boundary
+ONE_CTA, PAIR, CLUSTER, REFUSED = 0, 1, 2, -4
+
+
+def route(M, N, K, *, act=F.ACT_NONE, bias=0, aux=0, preact_out=0, residual=0, sms=SMS):
+    return native.ext().gemm_route(M, N, K, False, False, act, bias, aux, preact_out, residual, 0.0, sms)
+
+
+@pytest.mark.parametrize("operand,act", [("residual", F.ACT_NONE), ("preact_out", F.ACT_GELU), ("aux", F.ACT_DGELU),
+                                         ("aux", F.ACT_DRELU)])
+@pytest.mark.parametrize("M,N,K", [(16, 8, 64), (300, 24, 2000), (4096, 31, 512), (300, 32, 2000), (512, 1024, 1024),
+                                   (200, 72, 64), (4096, 4096, 1024), (30000, 40, 64)])
+def test_row_operands_off_a_boundary(operand, act, M, N, K):
+    kernel, bn, slices = route(M, N, K, act=act, **{operand: EVEN})
+    assert kernel in (ONE_CTA, PAIR, CLUSTER) and (kernel != CLUSTER or (bn in (64, 128) and slices in (1, 2, 4, 8)))
+    for start in range(EVEN + 2, EVEN + 16, 2):
+        assert route(M, N, K, act=act, **{operand: start})[0] == (ONE_CTA if N < 32 else REFUSED)
+
+
+def test_narrow_outputs_do_take_the_cluster_kernel():
+    """(what makes the test above one of the addresses, not of the sizes)"""
+    assert route(300, 24, 2000, residual=EVEN)[0] == CLUSTER
+
+
+def test_an_operand_that_is_not_read_may_lie_anywhere():
+    assert route(512, 1024, 1024, aux=ODD)[0] == route(512, 1024, 1024, aux=EVEN)[0]
+
+
+@pytest.mark.parametrize("M,N,K,odd", [(300, 24, 2000, None), (200, 31, 64, None), (512, 1024, 1024, None),
+                                       (4096, 4096, 1024, REFUSED), (30000, 40, 64, REFUSED)])
+def test_bias_off_a_boundary(M, N, K, odd):
+    """The cluster kernel reads the bias by elements, the others 32 (16) columns at a time in 16-byte pieces."""
+    even = route(M, N, K, bias=EVEN)
+    assert even[0] >= 0
+    assert route(M, N, K, bias=ODD) == (even if odd is None else (odd, 0, 0))
