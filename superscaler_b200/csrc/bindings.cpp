@@ -3,13 +3,17 @@
 // returns 0 or an error code; a non-zero code raises, so a missing or failing native path is
 // never silent.
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
+
+#include <atomic>
 
 #include "attention_sm100.cuh"
 #include "gemm_sm100.cuh"
 #include "gemm_ar_sm100.cuh"
 #include "gemm_ag_sm100.cuh"
+#include "per_device.h"
 
 namespace ssb {
 int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
@@ -119,27 +123,32 @@ using OptTensor = c10::optional<Tensor>;
 cudaStream_t cur_stream() { return at::cuda::getCurrentCUDAStream().stream(); }
 
 int num_sms() {
-  static int n[64] = {0};
-  int dev = at::cuda::current_device();
-  if (n[dev] == 0) n[dev] = at::cuda::getDeviceProperties(dev)->multiProcessorCount;
-  return n[dev];
+  static ssb::PerDevice<int> n;
+  const int dev = at::cuda::current_device();
+  return n.get(dev, [&] { return at::cuda::getDeviceProperties(dev)->multiProcessorCount; });
+}
+
+// Zeros on the device, which are there when the call returns: the next user may be another thread on another stream.  (Inside a
+// capture the clearing becomes part of the graph, as it always did.)
+Tensor device_zeros(int dev, int64_t n) {
+  Tensor t = torch::zeros({n}, torch::dtype(torch::kInt32).device(torch::kCUDA, dev));
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None)
+    C10_CUDA_CHECK(cudaStreamSynchronize(cur_stream()));
+  return t;
 }
 
 // One status word per device, written by kernels whose bounded waits run out.
 Tensor& status_tensor() {
-  static std::vector<Tensor> st(64);
-  int dev = at::cuda::current_device();
-  if (!st[dev].defined()) st[dev] = torch::zeros({1}, torch::dtype(torch::kInt32).device(torch::kCUDA, dev));
-  return st[dev];
+  static ssb::PerDevice<Tensor> st;
+  const int dev = at::cuda::current_device();
+  return st.get(dev, [&] { return device_zeros(dev, 1); });
 }
 
 // Zero-initialised ticket counters of the one-launch column sum (one set per device; every call leaves them zero).
 Tensor& ticket_tensor() {
-  static std::vector<Tensor> st(64);
-  int dev = at::cuda::current_device();
-  if (!st[dev].defined())
-    st[dev] = torch::zeros({ssb::colsum_tickets()}, torch::dtype(torch::kInt32).device(torch::kCUDA, dev));
-  return st[dev];
+  static ssb::PerDevice<Tensor> st;
+  const int dev = at::cuda::current_device();
+  return st.get(dev, [&] { return device_zeros(dev, ssb::colsum_tickets()); });
 }
 
 void check_launch(int rc, const char* what) { TORCH_CHECK(rc == 0, what, ": native launcher failed with code ", rc); }
@@ -555,7 +564,7 @@ std::vector<Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, 
 
 // false (default): the fused backward kernel, whose dQ is accumulated with floating-point reductions in arrival
 // order; true: the dK/dV + dQ kernel pair, bitwise reproducible.
-bool g_attn_bwd_deterministic = false;
+std::atomic<bool> g_attn_bwd_deterministic{false};  // (read by the threads that run a backward)
 
 // dq, dk, dv are written into caller-provided 2-D matrices (same conventions as q, k, v).
 void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& dout,
@@ -992,7 +1001,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("node_calls", []() { return g_node_calls.load(); });
   m.def("attn_bwd", &attn_bwd);
   m.def("set_attn_bwd_deterministic", [](bool on) { g_attn_bwd_deterministic = on; });
-  m.def("attn_bwd_deterministic", []() { return g_attn_bwd_deterministic; });
+  m.def("attn_bwd_deterministic", []() { return g_attn_bwd_deterministic.load(); });
   m.def("conv_plan", &conv_plan);
   m.def("conv_fprop", &conv_fprop);
   m.def("conv_dgrad", &conv_dgrad);

@@ -17,6 +17,8 @@
 #include "gemm_sm100.cuh"
 #include "gemm_epilogue.cuh"
 
+#include <atomic>
+
 namespace ssb {
 
 namespace {
@@ -422,7 +424,7 @@ int gemm_cluster_launch(const void* A, int lda, int a_mn, const void* B, int ldb
                         cudaStream_t stream);
 
 // 0 = always the one-CTA kernel, 1 = two-SM kernel where the output has enough 256 x 256 tiles.
-static int g_pair_mode = 1;
+static std::atomic<int> g_pair_mode{1};  // (read by the threads that run a backward)
 void gemm_set_pair_mode(int mode) { g_pair_mode = mode; }
 int gemm_get_pair_mode() { return g_pair_mode; }
 

@@ -1,4 +1,8 @@
 """The native autograd nodes of linear, MLP, LayerNorm and attention (csrc/autograd_nodes.h)."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -58,3 +62,27 @@ def test_the_gradient_buffer_is_the_one_of_the_backward(op, change):
         else:
             # the same sums, rounded to the parameter's type (bf16: 2^-9) in `want` only
             assert p.grad is None and rel(p.main_grad, want[k]) < 2.0 ** -8
+
+
+def test_first_use_of_the_device_values_in_a_backward():
+    """The status word is made by whichever thread comes first: here Python threads and the backward's, each on a stream of its
+    own, in a fresh process.  (Products only: column sums share their ticket counters between the streams of a device.)"""
+    code = """
+import threading, torch
+from superscaler_b200.ops import functional as F, native
+x = torch.randn(256, 512, device="cuda").bfloat16().requires_grad_(True)
+w = torch.nn.Parameter(torch.randn(256, 512, device="cuda").bfloat16() * 0.05)
+torch.cuda.synchronize()
+out = {}
+def work(i):
+    with torch.cuda.stream(torch.cuda.Stream()):
+        g = torch.autograd.grad(F.linear(x, w, act=F.ACT_GELU).float().sum(), [x, w])
+        torch.cuda.current_stream().synchronize()
+        out[i] = g
+threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+assert len(out) == 4 and all(torch.equal(a, e) for o in out.values() for a, e in zip(o, out[0]))
+assert native.check_status() == 0
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=Path(__file__).parent.parent)
