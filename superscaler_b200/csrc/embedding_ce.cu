@@ -234,12 +234,19 @@ ce_finalize_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* 
   }
 }
 
-// exp(x - off) = 2^((x - off) log2 e) of two packed logits, two differences and two products per instruction
+// exp(x - off) = 2^((x - off) log2 e) of two packed logits, two differences and two products per instruction.  kTiny: results
+// below 2^-126 are kept (a gradient is scaled afterwards); in a sum next to a term of one they are nothing, and zero will do.
+template <bool kTiny>
 __device__ __forceinline__ float2 exp_pair(uint32_t two, float off) {
   const float2 d = mul_f32x2(add_f32x2(unpack_bf16x2(two), make_float2(-off, -off)), make_float2(kLog2e, kLog2e));
   float2 e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(d.x));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(d.y));
+  if constexpr (kTiny) {
+    asm("ex2.approx.f32 %0, %1;" : "=f"(e.x) : "f"(d.x));
+    asm("ex2.approx.f32 %0, %1;" : "=f"(e.y) : "f"(d.y));
+  } else {
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(d.x));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(d.y));
+  }
   return e;
 }
 
@@ -247,7 +254,8 @@ __device__ __forceinline__ float2 exp_pair(uint32_t two, float off) {
 // shared memory; every thread keeps a running maximum and the sum of exponentials relative to it on the way, so that the
 // special-function unit works under the loads, and only the gradient is left for a second pass.  Same quantities as
 // ce_stats + ce_finalize, which read the row three times.  T threads a row, 1024 per SM: one CTA loads while others write.
-// 4096 rows x 51200: 229 us (3.7 TB/s, two exponentials an element) against 263 for the two kernels.
+// 4096 rows x 51200: 199 us (4.2 TB/s, two exponentials an element) against 263 for the two kernels; results below the normal
+// range are 6 us of it.
 constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per SM
 
 template <int T>
@@ -283,8 +291,8 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
           tmax = m8;
         }
         const float off = tmax == -INFINITY ? 0.f : tmax;
-        const float2 s2 = add_f32x2(add_f32x2(exp_pair(q[u].x, off), exp_pair(q[u].y, off)),
-                                    add_f32x2(exp_pair(q[u].z, off), exp_pair(q[u].w, off)));
+        const float2 s2 = add_f32x2(add_f32x2(exp_pair<false>(q[u].x, off), exp_pair<false>(q[u].y, off)),
+                                    add_f32x2(exp_pair<false>(q[u].z, off), exp_pair<false>(q[u].w, off)));
         tsum += s2.x + s2.y;
       }
     }
@@ -299,8 +307,8 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   const int tv = t >= 0 && t < V ? static_cast<int>(t >> 3) : -1;  // vector of the target
   for (int v = threadIdx.x; v < nvec; v += T) {
     const uint4 q = row_smem[v];
-    float2 f[4] = {mul_f32x2(exp_pair(q.x, mx), inv2), mul_f32x2(exp_pair(q.y, mx), inv2),
-                   mul_f32x2(exp_pair(q.z, mx), inv2), mul_f32x2(exp_pair(q.w, mx), inv2)};
+    float2 f[4] = {mul_f32x2(exp_pair<true>(q.x, mx), inv2), mul_f32x2(exp_pair<true>(q.y, mx), inv2),
+                   mul_f32x2(exp_pair<true>(q.z, mx), inv2), mul_f32x2(exp_pair<true>(q.w, mx), inv2)};
     if (v == tv) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {

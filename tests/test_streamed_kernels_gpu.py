@@ -205,3 +205,23 @@ def test_cross_entropy_of_rows_that_are_not_finite(V, rows):
 @pytest.mark.parametrize("n", [2048, 2049])               # two sequences: the last token count of 64-bit keys, the next one
 def test_embedding_gradient_where_keys_get_narrow(V, n):
     test_embedding_gradient_keys(V, n)
+
+
+@pytest.mark.parametrize("V", [40, 1003, 40000, 60000])   # the one-pass form at each number of threads, the two-pass form
+def test_cross_entropy_keeps_probabilities_below_the_normal_range(V):
+    """Probabilities of 1e-39 to 1e-42 times a large gradient scale (a loss scale) are ordinary gradients: exp is good to 2^-16
+    there (the exponent is near 140, in fp32), a subnormal of 5e-42 holds eleven bits, and bf16 rounds by 2^-9: below 2^-8."""
+    rows, scale = 6, 2.0 ** 100
+    buf = torch.zeros(rows, (V + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)
+    for r, low in enumerate((-80.0, -86.0, -88.0, -90.0, -92.0, -95.0)):
+        buf[r] = low
+    t = torch.tensor([0, 1, V // 2, V - 1, V - 2, 7], device="cuda")
+    buf[torch.arange(rows, device="cuda"), t] = 0.0
+    work = buf.clone()
+    native.ext().ce_loss_grad(work[:, :V], t, None, 0, scale)
+    x = buf[:, :V].double()
+    grad = torch.softmax(x, -1) * scale
+    grad[torch.arange(rows, device="cuda"), t] = 0.0     # p - 1 of the target rounds to nothing
+    work[torch.arange(rows, device="cuda"), t] = 0.0
+    off = (work[:, :V].double() - grad).abs() - 2.0 ** -8 * grad
+    assert float(off.max()) <= 0.0
