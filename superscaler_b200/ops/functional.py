@@ -16,6 +16,7 @@ import os
 
 import torch
 import torch.nn.functional as F
+from torch.autograd import forward_ad
 
 from . import native
 
@@ -155,9 +156,11 @@ def dropout_bwd(g, p, seed):
 
 def _native_node(x) -> bool:
     """True when a call may go to the native autograd nodes (csrc/autograd_nodes.h): CUDA tensors in plain eager autograd.
-    Traced, compiled and functorch-transformed calls keep the Python functions, which those mechanisms know."""
+    Other calls keep the Python functions: Dynamo and the tracer look into them, functorch transforms and forward-mode
+    differentiation refuse them with the errors of an autograd function that does not support them.  Both forms launch the same
+    kernels in the same order (tests/test_autograd_nodes_gpu.py compares them bit for bit)."""
     return (x.is_cuda and not torch._C._are_functorch_transforms_active() and torch._C._get_tracing_state() is None
-            and not torch.compiler.is_dynamo_compiling())
+            and forward_ad._current_level < 0 and not torch.compiler.is_dynamo_compiling())
 
 
 # --------------------------------------------------------------------------------------------
