@@ -7,11 +7,9 @@
 // has to share with the main thread); a node costs the kernels' launches and allocations.  Back to back on the host: scoring one
 // prompt of 512 tokens with four layers 779 -> 456 us, a step of a two-layer model with two micro-batches 3387 -> 2797, forward
 // and backward of one attention call 112 -> 85.
+//
+// (Included inside the anonymous namespace of bindings.cpp, so it includes nothing itself.)
 #pragma once
-#include <torch/csrc/autograd/custom_function.h>
-
-#include <array>
-#include <atomic>
 
 std::atomic<long long> g_node_kernels{0}, g_node_calls{0};  // launches issued by nodes (the counterpart of the Python counter)
 

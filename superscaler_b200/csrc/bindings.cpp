@@ -5,8 +5,10 @@
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <atomic>
 
 #include "attention_sm100.cuh"
