@@ -1,4 +1,4 @@
-// bf16 GEMM for outputs of few tiles (at most one per SM): a cluster of S CTAs shares an output tile of 128 x BN, each reduces
+// bf16 GEMM for outputs of few tiles (at most one per SM; gemm_cluster_plan says which): a cluster of S CTAs shares an output tile of 128 x BN, each reduces
 // its slice of K on its own SM, and the partial tiles meet in the epilogue over distributed shared memory.  Same operands
 // and the same operations in the epilogue as the other GEMM kernels (gemm_sm100.cuh).
 //
@@ -425,31 +425,54 @@ int launch(const void* A, int lda, const void* B, int ldb, const GemmParams& p, 
 
 }  // namespace
 
-// Tile width and slices for an output, or slices = 0 where the kernel with one thread per output row is the better one: more
-// tiles of 128 x 128 than SMs, or an epilogue without row operands (`simple`) whose reduction is not split.
-void gemm_cluster_plan(int M, int N, int K, bool simple, int num_sms, int* bn_out, int* slices_out) {
-  const int num_m = (M + BM - 1) / BM, num_kb = (K + BK - 1) / BK;
+// Tile width and slices for an output, or slices = 0 where the kernel with one thread per output row is the better one.
+//
+// That kernel takes 220 ns a K block and its epilogue goes by chunks of 32 columns: 470 ns each for a plain bf16 result, more with
+// operands, a column of a chunk that is not whole 60; with a single warp of rows 0.6 of it.  Here the chain is shorter by the
+// slices and the epilogue does not grow with the columns, but the whole starts 2000 ns later (the partial tile, the operands),
+// and the meeting costs 500 to 1700.  So outputs of few columns and short reductions stay there: 2048 x 8 x 200 5.4 us, here 6.4;
+// 64 x 4096 x 512 plain 7.1, here 8.4; 1000 x 32 x 64 with GeLU and pre-activation 5.5, here 6.4.  Reductions that are long and not
+// split are fed by four stages instead of six, 64 ns a K block beyond the 32nd: 512 x 4096 x 16384 with GeLU 68.7, here 89.9.
+// Over 8447 calls (2 to 8192 in each size, nine epilogues) 29 are slower by more than 3 % than with that kernel alone; with a rule
+// that only asked for few tiles 534 were.
+void gemm_cluster_plan(const GemmParams& p, int num_sms, int* bn_out, int* slices_out) {
+  const int M = p.M, N = p.N, num_m = (M + BM - 1) / BM, num_kb = (p.K + BK - 1) / BK;
   *slices_out = 0;
   *bn_out = 128;
   if (static_cast<long long>(num_m) * ((N + 127) / 128) > num_sms) return;
-  int best = 0;
-  for (int bn = 64; bn <= 128; bn += 64) {
-    const long long tiles = static_cast<long long>(num_m) * ((N + bn - 1) / bn);
+  int best = 0, bn = 128, slices = 0;
+  for (int width = 64; width <= 128; width += 64) {
+    const long long tiles = static_cast<long long>(num_m) * ((N + width - 1) / width);
     for (int s = 1; s <= kMaxCluster; s *= 2) {
       const int per = (num_kb + s - 1) / s;
       // clusters of four and more do not fill every last SM of a GPC
       if (tiles * s > (s == 8 ? num_sms * 2 / 3 : s == 4 ? num_sms * 7 / 8 : num_sms) || (s > 1 && (per < 2 || (s - 1) * per >= num_kb))) continue;
       // cycles: the operands of a K block (an SM receives about 70 bytes a clock: 24 KB 345, 32 KB 462), the meeting over
       // distributed shared memory, the epilogue
-      const int cost = per * (bn == 64 ? 345 : 462) + (s > 1 ? 800 : 0) + 2400 * bn / 128 / s;
-      if (*slices_out == 0 || cost < best) {
+      const int cost = per * (width == 64 ? 345 : 462) + (s > 1 ? 800 : 0) + 2400 * width / 128 / s;
+      if (slices == 0 || cost < best) {
         best = cost;
-        *bn_out = bn;
-        *slices_out = s;
+        bn = width;
+        slices = s;
       }
     }
   }
-  if (simple && *slices_out == 1) *slices_out = 0;
+  if (slices == 0) return;
+  const bool row_operand = p.residual != nullptr || p.aux != nullptr;
+  // nothing to gain but the epilogue, and that one is simple
+  if (slices == 1 && !p.out_fp32 && !p.accumulate && p.preact_out == nullptr && !row_operand && p.dropout_p == 0.f) return;
+  const int chunk = 470 + (p.bias != nullptr ? 300 : 0) + (p.preact_out != nullptr ? 230 : 0) + (row_operand ? 540 : 0) +
+                    (p.out_fp32 ? 250 : 0) + (p.accumulate ? (p.out_fp32 ? 1350 : 900) : 0);
+  int epilogue = chunk * (((N < 128 ? N : 128) + 31) / 32) + (N < 128 ? 60 * (N % 32) : 0);
+  if (M <= 32) epilogue = epilogue * 6 / 10;
+  const int per = (num_kb + slices - 1) / slices;
+  int late = 2000;
+  if (slices == 1) late += num_kb > 32 ? 64 * (num_kb - 32) : 0;
+  else if (bn == 64) late += slices == 2 ? 500 : 1100;
+  else late += slices == 4 ? 1700 : 1000;
+  if (epilogue + 220 * (num_kb - per) + (bn == 64 ? 40 * per : 0) <= late) return;
+  *bn_out = bn;
+  *slices_out = slices;
 }
 
 int gemm_cluster_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const GemmParams& p, int bn, int slices,

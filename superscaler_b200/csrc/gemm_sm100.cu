@@ -419,7 +419,7 @@ int launch_variant(const void* A, int lda, const void* B, int ldb, const GemmPar
 int gemm2_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                       const GemmParams& p, int num_sms, cudaStream_t stream);
 
-void gemm_cluster_plan(int M, int N, int K, bool simple, int num_sms, int* bn, int* slices);
+void gemm_cluster_plan(const GemmParams& p, int num_sms, int* bn, int* slices);
 int gemm_cluster_launch(const void* A, int lda, int a_mn, const void* B, int ldb, int b_mn, const GemmParams& p, int bn, int slices,
                         cudaStream_t stream);
 
@@ -435,8 +435,11 @@ int gemm_splitk_splits(int M, int N, int K, int num_sms) {
   }
   if (N % 4) return 1;
   if (g_pair_mode && K < 64 * BK) {        // shorter reductions are split inside a cluster, without a workspace
+    GemmParams p{};
+    p.M = M; p.N = N; p.K = K;
+    p.out_fp32 = 1;
     int bn, slices;
-    gemm_cluster_plan(M, N, K, false, num_sms, &bn, &slices);
+    gemm_cluster_plan(p, num_sms, &bn, &slices);
     if (slices > 0) return 1;
   }
   const int tiles256 = ((M + BM - 1) / BM) * ((N + 255) / 256);
@@ -465,9 +468,7 @@ int gemm_route(const GemmParams& p, int num_sms, int* bn, int* slices) {
   if (g_pair_mode && p.k_splits <= 1) {
     const int tiles_pair = ((p.M + 255) / 256) * ((p.N + 255) / 256);
     if (p.M >= 256 && p.N >= 256 && tiles_pair >= num_sms / 4) return off16(p.bias) ? -4 : 1;
-    const bool simple = !p.out_fp32 && !p.accumulate && p.preact_out == nullptr && p.aux == nullptr && p.residual == nullptr &&
-                        p.dropout_p == 0.f;
-    if (!rows_off) gemm_cluster_plan(p.M, p.N, p.K, simple, num_sms, bn, slices);
+    if (!rows_off) gemm_cluster_plan(p, num_sms, bn, slices);
     if (*slices > 0) return 2;
   }
   return off16(p.bias) && p.N >= 32 ? -4 : 0;

@@ -12,8 +12,8 @@ EVEN, ODD = 0x1000, 0x1008            # addresses on and off a 16-byte boundary
 ONE_CTA, PAIR, CLUSTER, REFUSED = 0, 1, 2, -4
 
 
-def route(M, N, K, *, act=F.ACT_NONE, bias=0, aux=0, preact_out=0, residual=0, sms=SMS):
-    return native.ext().gemm_route(M, N, K, False, False, act, bias, aux, preact_out, residual, 0.0, sms)
+def route(M, N, K, *, act=F.ACT_NONE, bias=0, aux=0, preact_out=0, residual=0, fp32=False, accumulate=False, sms=SMS):
+    return native.ext().gemm_route(M, N, K, fp32, accumulate, act, bias, aux, preact_out, residual, 0.0, sms)
 
 
 @pytest.mark.parametrize("operand,act", [("residual", F.ACT_NONE), ("preact_out", F.ACT_GELU), ("aux", F.ACT_DGELU),
@@ -43,3 +43,18 @@ def test_bias_off_a_boundary(M, N, K, odd):
     even = route(M, N, K, bias=EVEN)
     assert even[0] >= 0
     assert route(M, N, K, bias=ODD) == (even if odd is None else (odd, 0, 0))
+
+
+PLAIN, GELU = {}, dict(act=F.ACT_GELU, bias=EVEN, preact_out=EVEN)
+RESIDUAL, DGELU, WGRAD = dict(bias=EVEN, residual=EVEN), dict(act=F.ACT_DGELU, aux=EVEN), dict(fp32=True, accumulate=True)
+
+
+@pytest.mark.parametrize("M,N,K,call,one_cta,cluster", [       # microseconds with either kernel, captured
+    (2048, 8, 200, PLAIN, 5.4, 6.4), (64, 4096, 512, PLAIN, 7.1, 8.4), (512, 2048, 512, PLAIN, 7.4, 8.2),
+    (1000, 8, 64, GELU, 5.4, 6.0), (200, 32, 64, GELU, 5.4, 6.4), (200, 32, 128, DGELU, 5.7, 6.6),
+    (512, 4096, 16384, GELU, 68.7, 89.9), (2048, 1024, 12288, GELU, 54.2, 69.8), (2048, 1024, 16384, RESIDUAL, 69.8, 91.2),
+    (512, 1024, 1024, RESIDUAL, 12.7, 9.1), (512, 1024, 4096, RESIDUAL, 23.0, 12.0), (512, 4096, 1024, GELU, 13.1, 11.4),
+    (1024, 512, 512, WGRAD, 15.0, 8.6), (1000, 8, 8192, PLAIN, 32.4, 9.1), (1024, 1024, 512, WGRAD, 15.0, 8.6),
+])
+def test_the_faster_kernel_takes_the_call(M, N, K, call, one_cta, cluster):
+    assert route(M, N, K, **call)[0] == (CLUSTER if cluster < one_cta else ONE_CTA)
