@@ -118,6 +118,17 @@ def test_attention_with_few_query_tiles(SQ, SK, HD, causal, lens, p, bias):
     _check(3, 2, SQ, SK, HD, causal, lens, p, bias)
 
 
+@pytest.mark.parametrize("HD", [64, 128])
+@pytest.mark.parametrize("S,lens,p,bias", [(100, True, 0.1, False), (128, False, 0.0, True), (33, True, 0.0, False)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_attention_backward_with_a_key_block_per_sm(HD, S, lens, p, bias, extra):
+    """As many key blocks as SMs: every CTA has one and its math warps write dV and dK; with one more, CTAs go on and the drain
+    warps write them."""
+    heads = torch.cuda.get_device_properties(0).multi_processor_count + extra
+    B = next(b for b in (4, 3, 2, 1) if heads % b == 0)
+    _check(B, heads // B, S, S, HD, False, ((S, 0, S - 32, 1)[:B] if lens else None), p, bias)
+
+
 def _check(B, NH, SQ, SK, HD, causal, lens, p, bias):
     seed = 77
     g = torch.Generator(device="cuda").manual_seed(SQ * 1000 + SK)
