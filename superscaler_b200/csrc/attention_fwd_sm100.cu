@@ -699,6 +699,9 @@ int launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& 
 
 }  // namespace
 
+// Which form the forward takes: true where the key blocks of a query tile are split over the two slots.
+bool attn_fwd_split(long long heads, int SQ, int SK, int causal, int num_sms) { return fwd_split(heads, SQ, SK, causal, num_sms); }
+
 // q/k/v: base pointers of the 2-D matrices that hold the heads (see AttnParams); ld in elements.
 int attn_fwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const AttnParams& p,
                     int num_sms, cudaStream_t stream) {

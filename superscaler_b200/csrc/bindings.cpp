@@ -69,6 +69,7 @@ int ce_stats_launch(const void* logits, int ld, const long long* targets, float*
 int ce_finalize_launch(void* logits, int ld, const long long* targets, const float* gmax, const float* gsum,
                        const float* gtgt, const float* loss_mask, float* loss, long long rows, int V, long long v0,
                        float grad_scale, int write_grad, cudaStream_t stream);
+bool attn_fwd_split(long long heads, int SQ, int SK, int causal, int num_sms);
 int attn_fwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const AttnParams& p,
                     int num_sms, cudaStream_t stream);
 int attn_bwd_launch(const void* q, int ldq, const void* k, int ldk, const void* v, int ldv, const void* dout,
@@ -995,6 +996,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ce_stats", &ce_stats);
   m.def("ce_finalize", &ce_finalize);
   m.def("attn_fwd", &attn_fwd);
+  m.def("attn_fwd_split", &ssb::attn_fwd_split);
   m.def("linear_node", &linear_node);
   m.def("mlp_node", &mlp_node);
   m.def("layernorm_node", &layernorm_node);

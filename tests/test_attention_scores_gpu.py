@@ -11,9 +11,14 @@ from test_attention_tiles_gpu import TOL, _oracle
 pytestmark = pytest.mark.gpu
 
 
+def _split(heads, SQ, SK, causal):
+    """True where the forward deals the key blocks of a query tile to two slots, False where it works on pairs of tiles."""
+    return native.ext().attn_fwd_split(heads, SQ, SK, causal, torch.cuda.get_device_properties(0).multi_processor_count)
+
+
 @pytest.mark.parametrize("HD", [64, 128])
 @pytest.mark.parametrize("blocks", [2, 5])
-@pytest.mark.parametrize("NH", [1, 80])                  # a tile per CTA; more tiles than SMs: pairs of them
+@pytest.mark.parametrize("NH", [1, 80, 120])             # (which form of the forward each takes: see below)
 def test_rows_of_one_value_are_exact(HD, blocks, NH):
     """All values of a sequence equal one vector, so every output row is that vector, whatever the scores.  A row has one
     key of score 0 in the first block and one above it by up to 8 (log2) in the last; the other keys lie 40 below and weigh
@@ -21,6 +26,7 @@ def test_rows_of_one_value_are_exact(HD, blocks, NH):
     rounded to bf16, and sums and products are fp32: the result is off by less than 2^-18 before it is rounded to bf16, which
     returns the vector itself.  A probability rounded away from one (by up to 2^-9) would show."""
     S, rows = 128 * blocks, 128 * blocks
+    assert _split(NH, rows, S, False) == ((NH, blocks) in {(1, 2), (1, 5), (80, 5)})
     g = torch.Generator(device="cuda").manual_seed(HD + blocks)
     q = torch.zeros(rows, HD, device="cuda")
     q[:, 0] = (torch.arange(rows, device="cuda") % 128 + 1) / 16.0        # score of the late key: up to 8
@@ -71,13 +77,14 @@ def test_samples_keep_their_nans(SQ, SK, HD, causal):
 ])
 @pytest.mark.parametrize("gain", [8.0, 32.0])
 @pytest.mark.parametrize("rising", [1, 32])              # rows of every 32 whose maximum rises with the keys
-@pytest.mark.parametrize("B,NH", [(2, 2), (8, 4)])       # a tile per CTA; more tiles than SMs: pairs of them
+@pytest.mark.parametrize("B,NH", [(2, 2), (8, 4)])       # split keys; split keys if causal, else pairs of tiles
 def test_late_maxima(S, HD, causal, p, bias, gain, rising, B, NH):
     """Keys ordered along one direction that some queries follow and the others oppose: their running maximum grows in
     every block, by more than 2^8 in probability.  The forward stays within the tolerance of small scores (fp32 scores of
     some 2^8 are off by 2^-16).  In the backward dS = P (dP - delta) cancels where one key takes the whole row, and what
     remains is the rounding of O in delta: e_r = 2^-9 |dO_r O_r| for row r, which enters dq_r with a weighted mean of keys
     and dk with q_r."""
+    assert _split(B * NH, S, S, causal) == (B * NH == 4 or (B * NH == 32 and causal))
     seed = 5
     g = torch.Generator(device="cuda").manual_seed(S + HD)
     w, n = NH * HD, B * S
@@ -107,6 +114,42 @@ def test_late_maxima(S, HD, causal, p, bias, gain, rising, B, NH):
     assert err(k.grad, dk) <= TOL * float(dk.norm()) + 2 * slack["dk"]
     if bias:
         assert err(bt.grad, db) <= TOL * float(db.norm()) + 2 * float(e.norm())
+
+
+@pytest.mark.parametrize("HD,p", [(64, 0.0), (128, 0.1)])
+@pytest.mark.parametrize("gain,rising", [(8.0, 1), (32.0, 1), (32.0, 32)])
+def test_late_maxima_in_causal_pairs(HD, p, gain, rising):
+    """Pairs of query tiles of unequal length under the mask: more heads than those above."""
+    test_late_maxima(700, HD, True, p, False, gain, rising, 8, 12)
+
+
+@pytest.mark.parametrize("NH", [2, 120])                 # split keys; pairs of tiles
+@pytest.mark.parametrize("HD", [64, 128])
+@pytest.mark.parametrize("first", [0, 1])                # the even or the odd key blocks: one slot or the other
+@pytest.mark.parametrize("bad", [-math.inf, math.inf, math.nan])
+def test_scores_that_are_not_finite_in_one_slot(NH, HD, first, bad):
+    """Whole key blocks of scores -inf (rows with a first component of one) or +inf (minus one), a single NaN key: rows come out
+    as softmax gives them, NaN where that is NaN, and the others stay what they are."""
+    S = 640
+    assert _split(NH, S, S, False) == (NH == 2)
+    g = torch.Generator(device="cuda").manual_seed(HD)
+    q, k, v = (torch.randn(S, HD, generator=g, device="cuda").bfloat16() for _ in range(3))
+    q[:, 0] = 1.0
+    if bad == math.inf:
+        q[::3, 0] = -1.0                                 # their scores of those keys are -inf: no weight
+    k[:, 0] = 0.0
+    if math.isnan(bad):
+        k[128 * first + 5, 0] = bad
+    else:
+        for b in range(first, 5, 2):
+            k[128 * b:128 * (b + 1), 0] = bad
+    s = (q.double() @ k.double().t()) / math.sqrt(HD)
+    want = torch.softmax(s, -1) @ v.double()
+    o = F.flash_attention(*(t.repeat(1, NH) for t in (q, k, v)), 1, NH, S, S, HD).double().view(S, NH, HD)
+    ok = torch.isfinite(want).all(-1)
+    assert bool(ok.any()) == (not math.isnan(bad)) and bool(torch.isnan(o[~ok]).all())
+    err = (o[ok] - want[ok][:, None]).norm()
+    assert float(err) <= TOL * float(want[ok].norm()) * math.sqrt(NH)
 
 
 @pytest.mark.parametrize("SQ,SK,HD,causal,lens,p,bias", [

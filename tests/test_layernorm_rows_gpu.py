@@ -1,5 +1,5 @@
-"""LayerNorm forward for rows held in registers: lengths that do not fill the last vector of every lane, one row at a time and
-two (csrc/layernorm.cu), against 64-bit LayerNorm.  Tolerance: one rounding to bf16 (2^-9) of every result."""
+"""LayerNorm forward for rows held in the registers of a warp: lengths that do not fill the last vector of every lane, values kept
+as fp32 and packed (csrc/layernorm.cu), against 64-bit LayerNorm.  Tolerance: one rounding to bf16 (2^-9) of every result."""
 import pytest
 import torch
 

@@ -81,10 +81,11 @@ def test_adam_vector_and_scalar_parts(n, start):
     assert torch.equal(p16, p.bfloat16()) and not grad.any()
 
 
-@pytest.mark.parametrize("n", [300, 4096])                # below and at the token count that takes them
-@pytest.mark.parametrize("V", [3, 32766, 32767, 40000])   # 16-bit keys up to 32766 rows, 32-bit beyond
-def test_embedding_gradient_keys(V, n):
-    H, v0 = 64, 5
+@pytest.mark.parametrize("n", [300, 4096])
+@pytest.mark.parametrize("V", [3, 32766, 32767, 40000])
+def test_embedding_gradient_keys(V, n, H=64):
+    """Two sequences of n tokens: grouped by row up to 65536 tokens, sorted beyond."""
+    v0 = 5
     g = torch.Generator(device="cuda").manual_seed(V)
     ids = torch.randint(v0, v0 + V, (2, n), generator=g, device="cuda")
     ids[0, :4] = torch.tensor([0, v0 - 1, v0 + V, 2 ** 40], device="cuda")    # outside the table, one past 32 bits
@@ -201,10 +202,35 @@ def test_cross_entropy_of_rows_that_are_not_finite(V, rows):
     assert torch.allclose(one.float(), two.float(), rtol=2.0 ** -7, atol=0.0, equal_nan=True)   # one unit of bf16
 
 
-@pytest.mark.parametrize("V", [32766, 40000])
-@pytest.mark.parametrize("n", [2048, 2049])               # two sequences: the last token count of 64-bit keys, the next one
-def test_embedding_gradient_where_keys_get_narrow(V, n):
-    test_embedding_gradient_keys(V, n)
+@pytest.mark.parametrize("V", [3, 32766, 32767, 40000])   # sort keys of 16 bits up to 32766 rows, of 32 beyond
+@pytest.mark.parametrize("n", [32768, 32769, 40000])      # two sequences: the last token count that is grouped, then sorted ones
+def test_embedding_gradient_of_many_tokens(V, n):
+    test_embedding_gradient_keys(V, n, H=8)
+
+
+@pytest.mark.parametrize("V", [1, 32766, 32767, 40000])
+@pytest.mark.parametrize("n", [1, 257, 5000])
+def test_sorted_embedding_gradient_with_narrow_keys(V, n):
+    """The sorted form itself, with the keys it is given above 65536 tokens: every row summed in token order."""
+    H, k0, ext = 24, 7, native.ext()
+    g = torch.Generator(device="cuda").manual_seed(V + n)
+    ids = torch.randint(k0 - 3, k0 + V + 3, (n,), generator=g, device="cuda")
+    ids[0] = 2 ** 40 + k0                                 # one past 32 bits
+    if n > 100:
+        ids[10:90] = k0 + V - 1                           # a run at the last row
+    dy, start = torch.randn(n, H, generator=g, device="cuda").bfloat16(), torch.randn(V, H, generator=g, device="cuda")
+    keys = ext.embedding_keys(ids, k0, V)
+    assert keys.dtype == (torch.int16 if V <= 32766 else torch.int32)
+    inside = (ids >= k0) & (ids < k0 + V)
+    assert torch.equal(keys.long(), torch.where(inside, ids - k0, V))
+    keys, order = torch.sort(keys, stable=True)
+    dst = start.clone()
+    ext.embedding_bwd_sorted(keys, order, dy, dst, 0, 0.0, 0)
+    want = start.double().index_add_(0, (ids - k0)[inside], dy.double()[inside])
+    assert _rel(dst, want) < 1e-6
+    again = start.clone()
+    ext.embedding_bwd_sorted(keys, order, dy, again, 0, 0.0, 0)
+    assert torch.equal(dst, again)
 
 
 @pytest.mark.parametrize("V", [40, 1003, 40000, 60000])   # the one-pass form at each number of threads, the two-pass form
