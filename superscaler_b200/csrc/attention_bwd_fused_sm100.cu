@@ -57,6 +57,7 @@ namespace {
 
 using namespace attn;
 
+constexpr MbarLook kIssueLook = MbarLook::kPoll;  // of the thread that issues the products (see above)
 constexpr int kFusedThreads = 768;
 constexpr int kFusedMathWarps = 16;
 // Register split of the 768 x 80 registers the block is launched with: 128 (56 + 4 * 80 + 104) = 61440.
@@ -282,13 +283,13 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           const int kst = m % NKV;
           const uint32_t kph = (m / NKV) & 1;
           const uint64_t kk_k = k_k + kst * kStage, kk_mn = k_mn + kst * kStage, vv_k = v_k + kst * kStage;
-          ok = mbar_spin(&k_full[kst], kph, abort_flag) && mbar_spin(&q_full[n & 1], (n >> 1) & 1, abort_flag);
+          ok = mbar_wait<kIssueLook>(&k_full[kst], kph, abort_flag) && mbar_wait<kIssueLook>(&q_full[n & 1], (n >> 1) & 1, abort_flag);
           if (!ok) break;
           tc_fence_after_sync();
           product(tmem_s, kk_k, q_k + (n & 1) * kStage);
           umma_commit(s_full);
-          ok = mbar_spin(&v_full[kst], kph, abort_flag) && mbar_spin(&do_full[n % NDO], (n / NDO) & 1, abort_flag) &&
-               (HD == 64 || n == 0 || mbar_spin(dq_empty, (n - 1) & 1, abort_flag));  // dP^T takes the columns of dQ
+          ok = mbar_wait<kIssueLook>(&v_full[kst], kph, abort_flag) && mbar_wait<kIssueLook>(&do_full[n % NDO], (n / NDO) & 1, abort_flag) &&
+               (HD == 64 || n == 0 || mbar_wait<kIssueLook>(dq_empty, (n - 1) & 1, abort_flag));  // dP^T takes the columns of dQ
           if (!ok) break;
           tc_fence_after_sync();
           product(tmem_dp, vv_k, do_k + (n % NDO) * kStage);
@@ -297,8 +298,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             const int st = n & 1, nx = st ^ 1, dst = n % NDO, dnx = (n + 1) % NDO;
             const uint32_t ph = n & 1;
             const bool last = i + 1 == w.n_it;
-            if (!(ok = mbar_spin(p_full, ph, abort_flag))) break;
-            if (i == 0 && m > 0 && !(ok = mbar_spin(acc_empty, (m - 1) & 1, abort_flag))) break;
+            if (!(ok = mbar_wait<kIssueLook>(p_full, ph, abort_flag))) break;
+            if (i == 0 && m > 0 && !(ok = mbar_wait<kIssueLook>(acc_empty, (m - 1) & 1, abort_flag))) break;
             tc_fence_after_sync();
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)  // 128 queries = 8 steps of 16; the warpgroups' shares of P^T start 32 columns apart
@@ -306,15 +307,15 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                           (i | kk) != 0);
             umma_commit(&do_empty[dst]);
             if (!last) {
-              if (!(ok = mbar_spin(&q_full[nx], ((n + 1) >> 1) & 1, abort_flag))) break;
+              if (!(ok = mbar_wait<kIssueLook>(&q_full[nx], ((n + 1) >> 1) & 1, abort_flag))) break;
               tc_fence_after_sync();
               product(tmem_s, kk_k, q_k + nx * kStage);
               umma_commit(s_full);
             } else {
               umma_commit(&v_empty[kst]);
             }
-            if (!(ok = mbar_spin(ds_full, ph, abort_flag))) break;
-            if (HD == 64 && n >= 1 && !(ok = mbar_spin(dq_empty, (n - 1) & 1, abort_flag))) break;
+            if (!(ok = mbar_wait<kIssueLook>(ds_full, ph, abort_flag))) break;
+            if (HD == 64 && n >= 1 && !(ok = mbar_wait<kIssueLook>(dq_empty, (n - 1) & 1, abort_flag))) break;
             tc_fence_after_sync();
 #pragma unroll
             for (int kk = 0; kk < 8; ++kk)  // 128 keys = 8 steps of 16
@@ -327,8 +328,8 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
                           idesc_acc, (i | kk) != 0);
             umma_commit(&q_empty[st]);
             if (!last) {
-              if (!(ok = mbar_spin(&do_full[dnx], ((n + 1) / NDO) & 1, abort_flag))) break;
-              if (HD == 128 && !(ok = mbar_spin(dq_empty, ph, abort_flag))) break;
+              if (!(ok = mbar_wait<kIssueLook>(&do_full[dnx], ((n + 1) / NDO) & 1, abort_flag))) break;
+              if (HD == 128 && !(ok = mbar_wait<kIssueLook>(dq_empty, ph, abort_flag))) break;
               tc_fence_after_sync();
               product(tmem_dp, vv_k, do_k + dnx * kStage);
               umma_commit(dp_full);
@@ -461,184 +462,184 @@ attn_bwd_fused_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     uint32_t n = 0;
     bool ok = true;
     for (int t = 0;; ++t) {
-    const int kv0 = w.jb * 128, kv = kv0 + r, kv_len = w.kv_len;
-    const uint32_t bh_seed = DROPOUT ? static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(w.b) * p.NH + w.head)) : 0u;
-    // attn_col_hash mixes (key quads + quad) * 0x9E3779B1 + seed: linear in the quad
-    const uint32_t hash0 = (static_cast<uint32_t>(kv) * ((p.SQ + 3) >> 2) + static_cast<uint32_t>(w.i0 * 32 + g * 8)) * 0x9E3779B1u + bh_seed;
-    const bool kv_ok = kv < kv_len;
-    // score bias: bias_table[head][kv - q + SQ - 1] log2(e); its gradient is dS summed along the diagonals
-    const float* bias_head = BIAS ? p.bias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
-    float* dbias_head = BIAS ? p.dbias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
+      const int kv0 = w.jb * 128, kv = kv0 + r, kv_len = w.kv_len;
+      const uint32_t bh_seed = DROPOUT ? static_cast<uint32_t>(hash64(p.dropout_seed, static_cast<uint64_t>(w.b) * p.NH + w.head)) : 0u;
+      // attn_col_hash mixes (key quads + quad) * 0x9E3779B1 + seed: linear in the quad
+      const uint32_t hash0 = (static_cast<uint32_t>(kv) * ((p.SQ + 3) >> 2) + static_cast<uint32_t>(w.i0 * 32 + g * 8)) * 0x9E3779B1u + bh_seed;
+      const bool kv_ok = kv < kv_len;
+      // score bias: bias_table[head][kv - q + SQ - 1] log2(e); its gradient is dS summed along the diagonals
+      const float* bias_head = BIAS ? p.bias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
+      float* dbias_head = BIAS ? p.dbias_table + static_cast<size_t>(w.head) * n_dist : nullptr;
 
-    // Score bias of a block, fetched a block ahead: with the loads in front of their use a step waited 700 cycles for them
-    constexpr bool kBiasStaged = BIAS && HD == 64;
-    float bias_next[2] = {0.f, 0.f};
-    auto fetch_bias = [&](int q0) {
-      if constexpr (kBiasStaged) {
-        const int d = kv0 + quarter * 32 - q0 + p.SQ - 32 + lane;  // distance of (key 0, query 31) of this warp, + lane
-        bias_next[0] = __ldg(bias_head + min(max(d, 0), n_dist - 1));
-        bias_next[1] = __ldg(bias_head + min(max(d + 32, 0), n_dist - 1));
-      }
-    };
-    fetch_bias(w.i0 * 128 + g * 32);
+      // Score bias of a block, fetched a block ahead: with the loads in front of their use a step waited 700 cycles for them
+      constexpr bool kBiasStaged = BIAS && HD == 64;
+      float bias_next[2] = {0.f, 0.f};
+      auto fetch_bias = [&](int q0) {
+        if constexpr (kBiasStaged) {
+          const int d = kv0 + quarter * 32 - q0 + p.SQ - 32 + lane;  // distance of (key 0, query 31) of this warp, + lane
+          bias_next[0] = __ldg(bias_head + min(max(d, 0), n_dist - 1));
+          bias_next[1] = __ldg(bias_head + min(max(d + 32, 0), n_dist - 1));
+        }
+      };
+      fetch_bias(w.i0 * 128 + g * 32);
 
-    for (int i = 0; i < w.n_it; ++i, ++n) {
-      const uint32_t ph = n & 1;
-      const int qblk0 = (w.i0 + i) * 128, qbase = qblk0 + g * 32;
-      const float* nlse2 = sStat + ph * 256 + g * 32;
-      const float* nd = nlse2 + 128;
-      const bool need_mask = (p.causal && kv0 + 127 > qblk0) || qblk0 + 128 > p.SQ || kv0 + 128 > kv_len;
-      // queries lo .. hi - 1 of this thread's 32 see its key
-      const int lo = p.causal ? kv - qbase : 0, hi = kv_ok ? p.SQ - qbase : 0;
-      // Nothing to see for the whole warp (above the diagonal or past an end): zeros for P and dS, no arithmetic.  In a
-      // last block of 64 queries these are half of the warps: 256 heads of 64 x 64 15.6 -> 13.7 us.
-      if (need_mask && (qbase >= p.SQ || kv0 + quarter * 32 >= (p.causal ? min(kv_len, qbase + 32) : kv_len))) {
-        uint32_t zero[16];
+      for (int i = 0; i < w.n_it; ++i, ++n) {
+        const uint32_t ph = n & 1;
+        const int qblk0 = (w.i0 + i) * 128, qbase = qblk0 + g * 32;
+        const float* nlse2 = sStat + ph * 256 + g * 32;
+        const float* nd = nlse2 + 128;
+        const bool need_mask = (p.causal && kv0 + 127 > qblk0) || qblk0 + 128 > p.SQ || kv0 + 128 > kv_len;
+        // queries lo .. hi - 1 of this thread's 32 see its key
+        const int lo = p.causal ? kv - qbase : 0, hi = kv_ok ? p.SQ - qbase : 0;
+        // Nothing to see for the whole warp (above the diagonal or past an end): zeros for P and dS, no arithmetic.  In a
+        // last block of 64 queries these are half of the warps: 256 heads of 64 x 64 15.6 -> 13.7 us.
+        if (need_mask && (qbase >= p.SQ || kv0 + quarter * 32 >= (p.causal ? min(kv_len, qbase + 32) : kv_len))) {
+          uint32_t zero[16];
 #pragma unroll
-        for (int e = 0; e < 16; ++e) zero[e] = 0u;
+          for (int e = 0; e < 16; ++e) zero[e] = 0u;
+          if (!mbar_wait_warp(s_full, ph, abort_flag)) { ok = false; break; }
+          tc_fence_after_sync();
+          tmem_st_32x16(my_s, zero);
+          tmem_st_wait();
+          tc_fence_before_sync();
+          warp_arrive(p_full, lane);
+          if (!mbar_wait_warp(dp_full, ph, abort_flag)) { ok = false; break; }
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + e) ^ (r & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+          fence_proxy_async_smem();
+          warp_arrive(ds_full, lane);
+          fetch_bias(qbase + 128);
+          continue;
+        }
+        uint32_t drop = 0u;  // bit 7 - n of byte e: query 4 n + e dropped for this key; hashed before the scores are there
+        if constexpr (DROPOUT) {
+          uint32_t h = hash0 + static_cast<uint32_t>(i) * (32u * 0x9E3779B1u);
+#pragma unroll
+          for (int n = 0; n < 8; ++n) {
+            const uint32_t x = fmix32(h);
+            h += 0x9E3779B1u;
+            const uint32_t cs = (x & 0x7f7f7f7fu) + (drop_c & 0x7f7f7f7fu);
+            drop |= (((x & drop_c) | ((x | drop_c) & cs)) & 0x80808080u) >> n;
+          }
+        }
+        if constexpr (kBiasStaged) {  // (the reads of the block before are behind this warp's arrivals)
+          sBias[lane] = bias_next[0];
+          sBias[lane + 32] = bias_next[1];
+          __syncwarp();
+        }
+        if (!mbar_wait_warp(&q_full[ph], (n >> 1) & 1, abort_flag)) { ok = false; break; }  // the statistics
         if (!mbar_wait_warp(s_full, ph, abort_flag)) { ok = false; break; }
         tc_fence_after_sync();
-        tmem_st_32x16(my_s, zero);
+        float pr[32];
+        {
+          uint32_t rs[32], w[16];
+          tmem_ld_32x32(my_s, rs);
+          tmem_ld_wait();
+          const float2 c2 = make_float2(c, c);
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {
+            float4 nl = *reinterpret_cast<const float4*>(nlse2 + e);
+            if constexpr (kBiasStaged) {
+              const float* br = sBias + lane + 31 - e;  // entries run down as the query runs up
+              nl.x = fmaf(br[0], kLog2e, nl.x);
+              nl.y = fmaf(br[-1], kLog2e, nl.y);
+              nl.z = fmaf(br[-2], kLog2e, nl.z);
+              nl.w = fmaf(br[-3], kLog2e, nl.w);
+            } else if constexpr (BIAS) {
+              const int d = kv - (qbase + e) + p.SQ - 1;  // entries run down as the query runs up
+              nl.x = fmaf(__ldg(bias_head + min(max(d, 0), n_dist - 1)), kLog2e, nl.x);
+              nl.y = fmaf(__ldg(bias_head + min(max(d - 1, 0), n_dist - 1)), kLog2e, nl.y);
+              nl.z = fmaf(__ldg(bias_head + min(max(d - 2, 0), n_dist - 1)), kLog2e, nl.z);
+              nl.w = fmaf(__ldg(bias_head + min(max(d - 3, 0), n_dist - 1)), kLog2e, nl.w);
+            }
+            const float2 a = fma_f32x2(make_float2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), c2, make_float2(nl.x, nl.y));
+            const float2 b2 = fma_f32x2(make_float2(__uint_as_float(rs[e + 2]), __uint_as_float(rs[e + 3])), c2, make_float2(nl.z, nl.w));
+            pr[e] = ex2(a.x);
+            pr[e + 1] = ex2(a.y);
+            pr[e + 2] = ex2(b2.x);
+            pr[e + 3] = ex2(b2.y);
+          }
+          if (need_mask) {  // uniform branch: only blocks on the diagonal or at the ragged ends pay for the tests
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              if (e < lo || e >= hi) pr[e] = 0.f;
+          }
+#pragma unroll
+          for (int e = 0; e < 16; ++e) {
+            w[e] = pack_bf16x2(pr[2 * e], pr[2 * e + 1]);
+            if constexpr (DROPOUT) w[e] &= ~spread_sign_bytes(drop << (e >> 1), (e & 1) ? 0xBBAA : 0x9988);
+          }
+          tmem_st_32x16(my_s, w);
+        }
         tmem_st_wait();
         tc_fence_before_sync();
         warp_arrive(p_full, lane);
-        if (!mbar_wait_warp(dp_full, ph, abort_flag)) { ok = false; break; }
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + e) ^ (r & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        fence_proxy_async_smem();
-        warp_arrive(ds_full, lane);
         fetch_bias(qbase + 128);
-        continue;
-      }
-      uint32_t drop = 0u;  // bit 7 - n of byte e: query 4 n + e dropped for this key; hashed before the scores are there
-      if constexpr (DROPOUT) {
-        uint32_t h = hash0 + static_cast<uint32_t>(i) * (32u * 0x9E3779B1u);
+        if (!mbar_wait_warp(dp_full, ph, abort_flag)) { ok = false; break; }
+        tc_fence_after_sync();
+        float diag = 0.f, wrap = 0.f;  // BIAS: sums along the diagonals through (lane, 0) and, wrapped, 32 distances below
 #pragma unroll
-        for (int n = 0; n < 8; ++n) {
-          const uint32_t x = fmix32(h);
-          h += 0x9E3779B1u;
-          const uint32_t cs = (x & 0x7f7f7f7fu) + (drop_c & 0x7f7f7f7fu);
-          drop |= (((x & drop_c) | ((x | drop_c) & cs)) & 0x80808080u) >> n;
-        }
-      }
-      if constexpr (kBiasStaged) {  // (the reads of the block before are behind this warp's arrivals)
-        sBias[lane] = bias_next[0];
-        sBias[lane + 32] = bias_next[1];
-        __syncwarp();
-      }
-      if (!mbar_wait_warp(&q_full[ph], (n >> 1) & 1, abort_flag)) { ok = false; break; }  // the statistics
-      if (!mbar_wait_warp(s_full, ph, abort_flag)) { ok = false; break; }
-      tc_fence_after_sync();
-      float pr[32];
-      {
-        uint32_t rs[32], w[16];
-        tmem_ld_32x32(my_s, rs);
-        tmem_ld_wait();
-        const float2 c2 = make_float2(c, c);
+        for (int ch = 0; ch < 2; ++ch) {
+          uint32_t rp[16], w[8];
+          tmem_ld_32x16(my_dp + ch * 16, rp);
+          tmem_ld_wait();
+          const float2 k2 = make_float2(inv_keep, inv_keep);
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          float4 nl = *reinterpret_cast<const float4*>(nlse2 + e);
-          if constexpr (kBiasStaged) {
-            const float* br = sBias + lane + 31 - e;  // entries run down as the query runs up
-            nl.x = fmaf(br[0], kLog2e, nl.x);
-            nl.y = fmaf(br[-1], kLog2e, nl.y);
-            nl.z = fmaf(br[-2], kLog2e, nl.z);
-            nl.w = fmaf(br[-3], kLog2e, nl.w);
-          } else if constexpr (BIAS) {
-            const int d = kv - (qbase + e) + p.SQ - 1;  // entries run down as the query runs up
-            nl.x = fmaf(__ldg(bias_head + min(max(d, 0), n_dist - 1)), kLog2e, nl.x);
-            nl.y = fmaf(__ldg(bias_head + min(max(d - 1, 0), n_dist - 1)), kLog2e, nl.y);
-            nl.z = fmaf(__ldg(bias_head + min(max(d - 2, 0), n_dist - 1)), kLog2e, nl.z);
-            nl.w = fmaf(__ldg(bias_head + min(max(d - 3, 0), n_dist - 1)), kLog2e, nl.w);
-          }
-          const float2 a = fma_f32x2(make_float2(__uint_as_float(rs[e]), __uint_as_float(rs[e + 1])), c2, make_float2(nl.x, nl.y));
-          const float2 b2 = fma_f32x2(make_float2(__uint_as_float(rs[e + 2]), __uint_as_float(rs[e + 3])), c2, make_float2(nl.z, nl.w));
-          pr[e] = ex2(a.x);
-          pr[e + 1] = ex2(a.y);
-          pr[e + 2] = ex2(b2.x);
-          pr[e + 3] = ex2(b2.y);
-        }
-        if (need_mask) {  // uniform branch: only blocks on the diagonal or at the ragged ends pay for the tests
+          for (int e = 0; e < 16; e += 4) {
+            const int q = ch * 16 + e;
+            const float4 n4 = *reinterpret_cast<const float4*>(nd + q);
+            if constexpr (DROPOUT) {
+              const uint32_t d = drop << (q >> 2);
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (e < lo || e >= hi) pr[e] = 0.f;
-        }
+              for (int u = 0; u < 4; ++u) rp[e + u] &= ~spread_sign_bytes(d, 0x8888 + 0x1111 * u);
+            }
+            float2 a = make_float2(__uint_as_float(rp[e]), __uint_as_float(rp[e + 1]));
+            float2 b2 = make_float2(__uint_as_float(rp[e + 2]), __uint_as_float(rp[e + 3]));
+            if constexpr (DROPOUT) {
+              a = fma_f32x2(a, k2, make_float2(n4.x, n4.y));
+              b2 = fma_f32x2(b2, k2, make_float2(n4.z, n4.w));
+            } else {
+              a = add_f32x2(a, make_float2(n4.x, n4.y));
+              b2 = add_f32x2(b2, make_float2(n4.z, n4.w));
+            }
+            a = mul_f32x2(make_float2(pr[q], pr[q + 1]), a);
+            b2 = mul_f32x2(make_float2(pr[q + 2], pr[q + 3]), b2);
+            if (need_mask) {  // rows and keys outside: not even 0 x NaN (from the padded statistics) may enter
+              if (q < lo || q >= hi) a.x = 0.f;
+              if (q + 1 < lo || q + 1 >= hi) a.y = 0.f;
+              if (q + 2 < lo || q + 2 >= hi) b2.x = 0.f;
+              if (q + 3 < lo || q + 3 >= hi) b2.y = 0.f;
+            }
+            w[e >> 1] = pack_bf16x2(a.x, a.y);
+            w[(e >> 1) + 1] = pack_bf16x2(b2.x, b2.y);
+            if constexpr (BIAS) {
+              // Gradient of the bias table: dS (before the softmax scale) summed along the diagonals key - query.  Lane l
+              // takes entry (l + q, q) from lane l + q: all on its own diagonal, or 32 distances below it where the
+              // lane index wraps.  Independent shuffles, two coalesced reductions per warp and step.
+              const float v4[4] = {a.x, a.y, b2.x, b2.y};
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-          w[e] = pack_bf16x2(pr[2 * e], pr[2 * e + 1]);
-          if constexpr (DROPOUT) w[e] &= ~spread_sign_bytes(drop << (e >> 1), (e & 1) ? 0xBBAA : 0x9988);
-        }
-        tmem_st_32x16(my_s, w);
-      }
-      tmem_st_wait();
-      tc_fence_before_sync();
-      warp_arrive(p_full, lane);
-      fetch_bias(qbase + 128);
-      if (!mbar_wait_warp(dp_full, ph, abort_flag)) { ok = false; break; }
-      tc_fence_after_sync();
-      float diag = 0.f, wrap = 0.f;  // BIAS: sums along the diagonals through (lane, 0) and, wrapped, 32 distances below
-#pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        uint32_t rp[16], w[8];
-        tmem_ld_32x16(my_dp + ch * 16, rp);
-        tmem_ld_wait();
-        const float2 k2 = make_float2(inv_keep, inv_keep);
-#pragma unroll
-        for (int e = 0; e < 16; e += 4) {
-          const int q = ch * 16 + e;
-          const float4 n4 = *reinterpret_cast<const float4*>(nd + q);
-          if constexpr (DROPOUT) {
-            const uint32_t d = drop << (q >> 2);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) rp[e + u] &= ~spread_sign_bytes(d, 0x8888 + 0x1111 * u);
-          }
-          float2 a = make_float2(__uint_as_float(rp[e]), __uint_as_float(rp[e + 1]));
-          float2 b2 = make_float2(__uint_as_float(rp[e + 2]), __uint_as_float(rp[e + 3]));
-          if constexpr (DROPOUT) {
-            a = fma_f32x2(a, k2, make_float2(n4.x, n4.y));
-            b2 = fma_f32x2(b2, k2, make_float2(n4.z, n4.w));
-          } else {
-            a = add_f32x2(a, make_float2(n4.x, n4.y));
-            b2 = add_f32x2(b2, make_float2(n4.z, n4.w));
-          }
-          a = mul_f32x2(make_float2(pr[q], pr[q + 1]), a);
-          b2 = mul_f32x2(make_float2(pr[q + 2], pr[q + 3]), b2);
-          if (need_mask) {  // rows and keys outside: not even 0 x NaN (from the padded statistics) may enter
-            if (q < lo || q >= hi) a.x = 0.f;
-            if (q + 1 < lo || q + 1 >= hi) a.y = 0.f;
-            if (q + 2 < lo || q + 2 >= hi) b2.x = 0.f;
-            if (q + 3 < lo || q + 3 >= hi) b2.y = 0.f;
-          }
-          w[e >> 1] = pack_bf16x2(a.x, a.y);
-          w[(e >> 1) + 1] = pack_bf16x2(b2.x, b2.y);
-          if constexpr (BIAS) {
-            // Gradient of the bias table: dS (before the softmax scale) summed along the diagonals key - query.  Lane l
-            // takes entry (l + q, q) from lane l + q: all on its own diagonal, or 32 distances below it where the
-            // lane index wraps.  Independent shuffles, two coalesced reductions per warp and step.
-            const float v4[4] = {a.x, a.y, b2.x, b2.y};
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const float y = __shfl_sync(0xffffffffu, v4[u], (lane + q + u) & 31);
-              if (lane + q + u < 32) diag += y;
-              else wrap += y;
+              for (int u = 0; u < 4; ++u) {
+                const float y = __shfl_sync(0xffffffffu, v4[u], (lane + q + u) & 31);
+                if (lane + q + u < 32) diag += y;
+                else wrap += y;
+              }
             }
           }
-        }
 #pragma unroll
-        for (int e = 0; e < 2; ++e)
-          *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + ch * 2 + e) ^ (r & 7)) << 4)) =
-              make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+          for (int e = 0; e < 2; ++e)
+            *reinterpret_cast<uint4*>(ds_row + ((((g & 1) * 4 + ch * 2 + e) ^ (r & 7)) << 4)) =
+                make_uint4(w[4 * e], w[4 * e + 1], w[4 * e + 2], w[4 * e + 3]);
+        }
+        tc_fence_before_sync();
+        fence_proxy_async_smem();
+        warp_arrive(ds_full, lane);
+        if constexpr (BIAS) {
+          const int d = kv - qbase + p.SQ - 1;
+          if (d >= 0 && d < n_dist) atomicAdd(dbias_head + d, diag);
+          if (lane > 0 && d - 32 >= 0 && d - 32 < n_dist) atomicAdd(dbias_head + d - 32, wrap);
+        }
       }
-      tc_fence_before_sync();
-      fence_proxy_async_smem();
-      warp_arrive(ds_full, lane);
-      if constexpr (BIAS) {
-        const int d = kv - qbase + p.SQ - 1;
-        if (d >= 0 && d < n_dist) atomicAdd(dbias_head + d, diag);
-        if (lane > 0 && d - 32 >= 0 && d - 32 < n_dist) atomicAdd(dbias_head + d - 32, wrap);
-      }
-    }
       if (!ok || !MORE) break;
       const bool more = take_item(t, w);
       if (!__all_sync(0xffffffffu, more)) break;

@@ -48,29 +48,10 @@ int make_tma_batched_bf16(CUtensorMap* map, const void* base, uint64_t batches, 
 namespace {
 
 using namespace attn;
-// mbar_wait without a suspend-time hint, for the thread that issues the products: its wake-up is on the path of every step
+// The thread that issues the products looks at its barriers without a suspend-time hint: its wake-up is on the path of every step
 // (16 x 16 heads of 2048 x 128 causal 346 -> 342 us; looking without suspending at all takes issue slots from the softmax warps,
 // 384 -> 400 with dropout).
-__device__ __forceinline__ bool mbar_nohint(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  uint64_t t0 = 0;
-  for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok)
-                 : "r"(smem_u32(bar)), "r"(parity)
-                 : "memory");
-    if (ok) return true;
-    if ((it & 1023u) == 1023u) {
-      if (*abort_flag) return false;
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kMbarTimeLimitNs) break;
-    }
-  }
-  *abort_flag = 1;
-  return false;
-}
-
+constexpr MbarLook kIssueLook = MbarLook::kBrief;
 
 constexpr int kFwdThreads = 640;   // five warpgroups: {TMA, MMA, 2 idle}, then two (column halves) per tile
 // Register split: 640 threads are launched with 96 registers each (61440 in all); the first warpgroup keeps 64 and the four
@@ -285,10 +266,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if constexpr (SPLIT) {
           const int n = w.n[0] + w.n[1];
           if (n == 0) continue;
-          if (!(ok = mbar_nohint(&q_full[0], qn[0] & 1, abort_flag))) break;
+          if (!(ok = mbar_wait<kIssueLook>(&q_full[0], qn[0] & 1, abort_flag))) break;
           ++qn[0];
           auto next_s = [&](int j) {  // scores of key block j
-            if (!(ok = mbar_nohint(&kv_full[pp.stage], pp.phase, abort_flag))) return;
+            if (!(ok = mbar_wait<kIssueLook>(&kv_full[pp.stage], pp.phase, abort_flag))) return;
             tc_fence_after_sync();
             issue_s(j & 1, 0, pp.stage);
             umma_commit(&kv_empty[pp.stage]);
@@ -298,8 +279,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           for (int j = 0; j < min(n, 2) && ok; ++j) next_s(j);
           for (int j = 0; j < n && ok; ++j) {
             const int t = j & 1;
-            if (!(ok = mbar_nohint(&kv_full[pp.stage], pp.phase, abort_flag))) break;
-            if (!(ok = mbar_nohint(&p_full[t], pn[t] & 1, abort_flag))) break;
+            if (!(ok = mbar_wait<kIssueLook>(&kv_full[pp.stage], pp.phase, abort_flag))) break;
+            if (!(ok = mbar_wait<kIssueLook>(&p_full[t], pn[t] & 1, abort_flag))) break;
             ++pn[t];
             tc_fence_after_sync();
             issue_o(t, pp.stage, j >= 2);
@@ -313,10 +294,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         const int n = max(w.n[0], w.n[1]);
         if (n == 0) continue;
         int sk = pp.stage;
-        if (!mbar_nohint(&kv_full[sk], pp.phase, abort_flag)) break;
+        if (!mbar_wait<kIssueLook>(&kv_full[sk], pp.phase, abort_flag)) break;
         for (int t = 0; t < 2 && ok; ++t) {
           if (w.n[t] == 0) continue;
-          if (!mbar_nohint(&q_full[t], qn[t] & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait<kIssueLook>(&q_full[t], qn[t] & 1, abort_flag)) { ok = false; break; }
           ++qn[t];
           tc_fence_after_sync();
           issue_s(t, t, sk);
@@ -333,16 +314,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           bool have_v = false, have_k = false;
           for (int t = 0; t < 2; ++t) {
             if (j >= w.n[t]) continue;
-            if (!have_v && !mbar_nohint(&kv_full[sv], phv, abort_flag)) { ok = false; break; }
+            if (!have_v && !mbar_wait<kIssueLook>(&kv_full[sv], phv, abort_flag)) { ok = false; break; }
             have_v = true;
-            if (!mbar_nohint(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait<kIssueLook>(&p_full[t], pn[t] & 1, abort_flag)) { ok = false; break; }
             ++pn[t];
             tc_fence_after_sync();
             issue_o(t, sv, j != 0);
             if (j + 1 == w.n[t]) {
               umma_commit(&o_full[t]);
             } else {
-              if (!have_k && !mbar_nohint(&kv_full[sk], pp.phase, abort_flag)) { ok = false; break; }
+              if (!have_k && !mbar_wait<kIssueLook>(&kv_full[sk], pp.phase, abort_flag)) { ok = false; break; }
               have_k = true;
               tc_fence_after_sync();
               issue_s(t, t, sk);  // overwrites S / P of the tile: products retire in issue order

@@ -66,29 +66,48 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// How a thread looks at a phase: suspended by the hardware for up to a time it is given (2 us) or of its own choosing, or not at
+// all.  The shorter, the sooner it goes on and the more issue slots it takes from the other warps.
+enum class MbarLook { kSuspend, kBrief, kPoll };
+
+template <MbarLook kLook = MbarLook::kSuspend>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n"  // suspend-time hint: 2 us
-      "selp.u32 %0, 1, 0, p;\n"
-      "}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if constexpr (kLook == MbarLook::kSuspend) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 2000;\n"  // suspend-time hint: 2 us
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+  } else if constexpr (kLook == MbarLook::kBrief) {
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+  } else {
+    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(ok)
+                 : "r"(smem_u32(bar)), "r"(parity)
+                 : "memory");
+  }
   return ok != 0;
 }
 
 // Bounded wait on an mbarrier phase.  Returns false when the limit ran out or
 // when another role of the CTA already raised `*abort_flag` (shared memory).
+template <MbarLook kLook = MbarLook::kSuspend>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   // The global timer is slow to read (microseconds), so it is only consulted once in a while and
   // never on the fast path; the iteration limit alone already bounds the loop.
+  constexpr uint32_t kEvery = kLook == MbarLook::kPoll ? 16384u : 1024u, kLimit = kMbarSpinLimit * (kEvery / 1024u);
   uint64_t t0 = 0;
-  for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 1023u) == 1023u) {
+  for (uint32_t it = 0; it < kLimit; ++it) {
+    if (mbar_try_wait<kLook>(bar, parity)) return true;
+    if ((it & (kEvery - 1u)) == kEvery - 1u) {
       if (*abort_flag) return false;
       const uint64_t now = global_timer_ns();
       if (t0 == 0) t0 = now;
@@ -99,26 +118,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return false;
 }
 
-// The same without suspending the thread between looks: for the single thread whose wake-up latency everything waits for.
-__device__ __forceinline__ bool mbar_spin(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  uint64_t t0 = 0;
-  for (uint32_t it = 0; it < kMbarSpinLimit * 16u; ++it) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    if (ok) return true;
-    if ((it & 16383u) == 16383u) {
-      if (*abort_flag) return false;
-      const uint64_t now = global_timer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > kMbarTimeLimitNs) break;
-    }
-  }
-  *abort_flag = 1;
-  return false;
+// Every thread of every CTA of the cluster; orders memory accesses on both sides.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // Register budget of a warpgroup (every warp of it executes this); the sum over the block's warpgroups must stay within
@@ -440,13 +443,6 @@ __device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
       : "=f"(d.x), "=f"(d.y)
       : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
-}
-
-// Four fp32 additions to 16 aligned bytes of global memory (no result; performed in the L2).
-__device__ __forceinline__ void red_add_v4(float* dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "f"(__uint_as_float(a)),
-               "f"(__uint_as_float(b)), "f"(__uint_as_float(c)), "f"(__uint_as_float(d))
-               : "memory");
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

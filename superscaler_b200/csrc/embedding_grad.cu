@@ -35,11 +35,6 @@ struct GroupArgs {
   GroupTable t[2];
 };
 
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 __global__ void __cluster_dims__(kGroupCtas, 1, 1) __launch_bounds__(kGroupThreads)
 embedding_group_kernel(const GroupArgs args, int tokens) {
   const GroupTable& a = args.t[blockIdx.x / kGroupCtas];
