@@ -66,9 +66,9 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// How a thread looks at a phase: suspended by the hardware for up to a time it is given (2 us) or of its own choosing, or not at
-// all.  The shorter, the sooner it goes on and the more issue slots it takes from the other warps.
-enum class MbarLook { kSuspend, kBrief, kPoll };
+// How a thread looks at a phase: suspended by the hardware for up to a time it is given (2 us) or of the hardware's choosing,
+// after which it goes on sooner and takes more issue slots from the other warps.
+enum class MbarLook { kSuspend, kBrief };
 
 template <MbarLook kLook = MbarLook::kSuspend>
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
@@ -83,13 +83,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
-  } else if constexpr (kLook == MbarLook::kBrief) {
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(ok)
-                 : "r"(smem_u32(bar)), "r"(parity)
-                 : "memory");
   } else {
-    asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
                  : "=r"(ok)
                  : "r"(smem_u32(bar)), "r"(parity)
                  : "memory");
@@ -103,11 +98,10 @@ template <MbarLook kLook = MbarLook::kSuspend>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   // The global timer is slow to read (microseconds), so it is only consulted once in a while and
   // never on the fast path; the iteration limit alone already bounds the loop.
-  constexpr uint32_t kEvery = kLook == MbarLook::kPoll ? 16384u : 1024u, kLimit = kMbarSpinLimit * (kEvery / 1024u);
   uint64_t t0 = 0;
-  for (uint32_t it = 0; it < kLimit; ++it) {
+  for (uint32_t it = 0; it < kMbarSpinLimit; ++it) {
     if (mbar_try_wait<kLook>(bar, parity)) return true;
-    if ((it & (kEvery - 1u)) == kEvery - 1u) {
+    if ((it & 1023u) == 1023u) {
       if (*abort_flag) return false;
       const uint64_t now = global_timer_ns();
       if (t0 == 0) t0 = now;
