@@ -443,7 +443,7 @@ void gemm_cluster_plan(const GemmParams& p, int num_sms, int* bn_out, int* slice
       const int per = (num_kb + s - 1) / s;
       // clusters of four and more do not fill every last SM of a GPC
       if (tiles * s > (s == 8 ? num_sms * 2 / 3 : s == 4 ? num_sms * 7 / 8 : num_sms) || (s > 1 && (per < 2 || (s - 1) * per >= num_kb))) continue;
-      // cycles: the operands of a K block (an SM receives about 70 bytes a clock: 24 KB 345, 32 KB 462), the meeting over
+      // cycles: the operands of a K block (an SM receives 70 to 80 bytes a clock: 24 KB 345, 32 KB 462), the meeting over
       // distributed shared memory, the epilogue
       const int cost = per * (width == 64 ? 345 : 462) + (s > 1 ? 800 : 0) + 2400 * width / 128 / s;
       if (slices == 0 || cost < best) {

@@ -19,10 +19,12 @@ namespace {
 constexpr int kLnWarpsPerBlock = 4;
 
 // Rows that fit in the registers of a warp, read once: up to VPL vectors of 8 bf16 per lane; FULL = false: the last one, or for
-// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984
-// 147 -> 55 us, of 1088 83 -> 33, 512 of 704 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
+// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  Lengths that are
+// not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984 147 -> 55 us, of 1088 83 -> 33, 512 of 704
+// 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
 // is slower (32768 x 2048 67 us instead of 55): too few warps; so is fp32 arithmetic two values per instruction (32768 x 1024
-// 28.1 -> 29.9).
+// 28.1 -> 29.9).  What bounds it is the latency of the loads with 15 warps an SM (125 registers): 32768 x 2048 keeps the DRAM 47 %
+// busy, the issue slots 35 %, and hardly ever waits for a math pipe.
 template <int VPL, bool FULL>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
@@ -274,8 +276,7 @@ __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
 // and the block writes ONE row of partials (part_g[block][h], part_b[block][h]); fold_partials2_kernel adds the blocks.
 // The result does not depend on the order of execution.  32768 x 2048 with residual gradient, this kernel and the fold:
 // 134 -> 107 us (register-staged form, H 1024 and 2048 only; other H took two kernels that read dy and x twice: 32768 x 1536
-// 173 -> 81, 512 x 768 11.5 -> 5.9).  The
-// same ring under the forward changed nothing (68 us: bound by its arithmetic), so that stays as it was.
+// 173 -> 81, 512 x 768 11.5 -> 5.9).  The same ring under the forward of that time changed nothing (68 us).
 template <int WPR>
 __global__ void __launch_bounds__((kLnWarps + 1) * 32, 2)
 ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,

@@ -3,7 +3,8 @@
 All activations are 2-D ``[tokens, features]`` bf16 matrices with tokens in batch-major order
 (``row = b * seq + s``).  Weight gradients are accumulated by the kernels straight into the fp32
 ``main_grad`` buffer attached to each parameter (gradient-accumulation fusion), so ``backward``
-returns ``None`` for parameters that carry a ``main_grad``.
+returns ``None`` for parameters that carry a ``main_grad``.  The attribute is looked up when the
+backward runs.
 
 On CUDA tensors the native kernels always run (a missing extension raises).  CPU tensors take a
 plain PyTorch implementation of the same math, which is what the multi-process gloo tests and the
@@ -769,13 +770,14 @@ class EmbeddingFn(torch.autograd.Function):
 
 
 def set_deterministic_embedding_grad(on: bool) -> None:
-    """Selects how the embedding gradient is scattered on the GPU: sorted runs with plain stores (order
-    independent, the default) or float atomics (order dependent in the last bit)."""
+    """Selects how the embedding gradient is scattered on the GPU: every row summed in token order by one block, tokens grouped by
+    row (sorted above 65536 tokens; independent of the order of execution, the default), or float atomics (order dependent
+    in the last bit)."""
     _DETERMINISTIC_EMBEDDING_GRAD[0] = bool(on)
 
 
 def set_deterministic(on: bool) -> None:
-    """Bitwise-reproducible training steps on the GPU.  On: the embedding gradient is summed in sorted runs (the
+    """Bitwise-reproducible training steps on the GPU.  On: the embedding gradient is summed in token order (the
     default anyway) and the attention backward runs as the dK/dV + dQ kernel pair.  Off (the default for attention):
     the fused attention backward kernel, which sums the key blocks' shares of dQ in an fp32 buffer in the order
     they arrive, so dQ may differ in the last bit between two runs of the same step."""
