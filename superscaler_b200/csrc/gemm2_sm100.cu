@@ -466,6 +466,61 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         flush(p.D, p.ldd);
         continue;
       }
+      // fp32 output: 16 columns at a time through the staging tile, 64-byte row segments to memory; what is there already
+      // (gradients are added to) is read in the same pieces, one ahead; the first while the tensor cores still work on this tile.
+      // A thread with a row of its own moved 16 of every 32-byte sector at a time and waited for each 16 columns of old values
+      // in turn; with a reduction of 4096 that took longer than the main loop of the next tile.  Alone / sustained under the power
+      // cap: weight gradients 51200 x 2048 over 4096 rows 649 -> 600 / 805 -> 754 us, 8192 x 2048 over 8192 216 -> 209 / 255 -> 248.
+      if (p.out_fp32 && col0 + 64 <= p.N && !has_operand && p.preact_out == nullptr) {
+        const int srow = lane >> 2, spiece = lane & 3;
+        float* out = reinterpret_cast<float*>(p.D) + static_cast<size_t>(row0 + srow) * p.ldd + col0 + spiece * 4;
+        auto cell = [&](int rr, int piece) { return stg + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4); };
+        auto old_values = [&](float4 (&o)[4], int c) {
+#pragma unroll
+          for (int it = 0; it < 4; ++it)
+            if (row0 + it * 8 + srow < p.M) o[it] = *reinterpret_cast<const float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16);
+        };
+        float4 old[4] = {}, next[4] = {};
+        if (p.accumulate) old_values(old, 0);
+        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
+          ok = false;
+          break;
+        }
+        tc_fence_after_sync();
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          if (p.accumulate && c < 3) old_values(next, c + 1);
+          uint32_t r[16];
+          tmem_ld_32x16(taddr + c * 16, r);
+          tmem_ld_wait();
+          if (c == 3) {  // the accumulator stage is free once its last columns are in registers
+            tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(mapa_smem(smem_u32(&tmem_empty_bar[acc]), 0));
+          }
+          const uint4 none[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+          float pre[16], v[16];
+          gemm_epilogue_math16(p, row, col0 + c * 16, r, none, keep16, drop_scale, pre, v);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(cell(lane, i)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          __syncwarp();
+#pragma unroll
+          for (int it = 0; it < 4; ++it) {
+            const int rr = it * 8 + srow;
+            float4 q = *reinterpret_cast<const float4*>(cell(rr, spiece));
+            if (row0 + rr < p.M) {
+              if (p.accumulate) {
+                q.x += old[it].x; q.y += old[it].y; q.z += old[it].z; q.w += old[it].w;
+              }
+              *reinterpret_cast<float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16) = q;
+            }
+          }
+#pragma unroll
+          for (int it = 0; it < 4; ++it) old[it] = next[it];
+          __syncwarp();
+        }
+        continue;
+      }
       if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
         ok = false;
         break;
