@@ -21,6 +21,7 @@ namespace ssb {
 int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                      const GemmParams& p, int num_sms, cudaStream_t stream);
 int gemm_route(const GemmParams& p, int num_sms, int* bn, int* slices);
+int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms);
 void gemm_set_pair_mode(int mode);
 int gemm_get_pair_mode();
 int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
@@ -968,6 +969,9 @@ Tensor status() { return status_tensor(); }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_route", &gemm_route);
+  m.def("gemm_pair_columns", [](int64_t M, int64_t N, int64_t K, bool out_fp32, int64_t sms) {
+    return ssb::gemm2_tile_columns(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), out_fp32, static_cast<int>(sms));
+  });
   m.def("gemm", &gemm);
   m.def("gemm_allreduce", &gemm_allreduce);
   m.def("allgather_gemm", &allgather_gemm);

@@ -14,6 +14,10 @@
 //                longer than the K = 2048 main loop of the next tile (measured 643 us against 407 us for the same
 //                GEMM with a plain epilogue)
 //
+// Wide tile (NH = 2): 256 x 512, two accumulators of 256 columns that take the whole TMEM.  Long products run into the power cap,
+// where what a product costs in energy sets the pace, not idle cycles: a quarter less traffic from the L2 for the same
+// arithmetic lets the clock rise (4096 x 2048 over 51200: 1310 -> 1417 MHz at 990 W, tensor pipe 77 % busy either way).
+//
 // Barriers: `full` lives in the leader and counts the bytes of both CTAs' loads (the peer's TMA signals it
 // through the cluster address); `empty` and `tmem_full` exist in both CTAs and are signalled together by a
 // multicast tcgen05.commit; `tmem_empty` lives in the leader and collects the epilogue warps of both CTAs.
@@ -41,6 +45,8 @@ constexpr int BN2 = 256;
 constexpr int BK2 = 64;
 constexpr int kStagesPlain = 5;
 constexpr int kStagesGather = 4;                 // one stage (32 KB) becomes the pusher's staging area
+constexpr int kStagesWide = 4;                   // of 48 KB
+constexpr int kSwitchGroup = 2;                  // wide tile: K blocks at both ends of a tile that are taken half by half
 constexpr int kPushChunk2 = 16384;
 constexpr int kEpiWarps = 16;
 constexpr int kThreads2 = 64 + kEpiWarps * 32;
@@ -50,8 +56,9 @@ constexpr int kConvNone = 0, kConvA = 1, kConvB = 2;
 constexpr int kABytes2 = BM2 * BK2 * 2;
 constexpr int kBBytes2 = BNH * BK2 * 2;
 constexpr int kStageBytes2 = kABytes2 + kBBytes2;
-constexpr int kEpiStage = 32 * 128;                 // per epilogue warp: 32 rows x 64 bf16 columns, 128-byte swizzle
-constexpr int kSmem2 = kStagesPlain * kStageBytes2 + kEpiWarps * kEpiStage + 1024 + 256;  // both variants
+constexpr int kEpiStage = 32 * 128;                 // per epilogue warp: 32 rows x 64 bf16 columns (wide tile: 32 columns)
+constexpr int kSmem2 = kStagesPlain * kStageBytes2 + kEpiWarps * kEpiStage + 1024 + 256;  // all variants
+static_assert(kStagesWide * (kABytes2 + 2 * kBBytes2) + kEpiWarps * kEpiStage / 2 + 1024 + 256 <= kSmem2, "wide tile");
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -172,18 +179,20 @@ __device__ __forceinline__ TileCoord2 tile_coord2(int tile, int num_m, int num_n
 //           input gradient (A = output gradient, taps flipped, B = filter read MN-major).  A channel block that reaches past C
 //           is zero-filled, so what the filter's block holds there (the next tap) does not matter.
 //   kConvB: filter gradient; the reduction runs over the pixels, B's columns are (tap, channel), C a multiple of 64.
-template <bool A_MN, bool B_MN, bool GATHER, int CONV>
+template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
 __global__ void __launch_bounds__(GATHER ? kThreadsGather : kThreads2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a2,
                   const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv) {
-  constexpr int kStages2 = GATHER ? kStagesGather : kStagesPlain;
+  constexpr int kStages2 = NH == 2 ? kStagesWide : GATHER ? kStagesGather : kStagesPlain;
+  constexpr int BNT = NH * BN2;                     // columns of a tile
+  constexpr int kStageAll = kABytes2 + NH * kBBytes2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + kStages2 * kABytes2;
-  uint8_t* push_buf = smem + kStages2 * kStageBytes2;              // GATHER only: 2 x 16 KB
+  uint8_t* push_buf = smem + kStages2 * kStageAll;              // GATHER only: 2 x 16 KB
   uint8_t* epi_stage = push_buf + (GATHER ? 2 * kPushChunk2 : 0);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(epi_stage + kEpiWarps * kEpiStage);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi_stage + kEpiWarps * kEpiStage / NH);
   uint64_t* full_bar = bars;                       // leader's are used
   uint64_t* empty_bar = bars + kStages2;           // both CTAs
   uint64_t* tmem_full_bar = bars + 2 * kStages2;   // both CTAs
@@ -200,7 +209,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const int num_clusters = gridDim.x >> 1;
 
   const int num_m = (p.M + 2 * BM2 - 1) / (2 * BM2);
-  const int num_n = (p.N + BN2 - 1) / BN2;
+  const int num_n = (p.N + BNT - 1) / BNT;
   const int num_tiles = num_m * num_n;
   const int conv_cblk = CONV == kConvA ? (cv.C + BK2 - 1) / BK2 : 1;  // channel blocks per tap
   const int num_kb = CONV == kConvA ? cv.KH * cv.KW * conv_cblk : (p.K + BK2 - 1) / BK2;
@@ -244,7 +253,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
         const TileCoord2 tc = tile_coord2(tile, num_m, num_n);
         int m0 = pblk_of(tc.m_blk) * 2 * BM2 + static_cast<int>(cta_rank) * BM2;
-        const int n0 = tc.n_blk * BN2 + static_cast<int>(cta_rank) * BNH;
+        const int n0 = tc.n_blk * BNT + static_cast<int>(cta_rank) * BNH;
         const CUtensorMap* ta = &tma_a;
         if (GATHER) {
           if (src_of(tc.m_blk) == cm.rank) {
@@ -281,10 +290,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             ok = false;
             break;
           }
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * kStageBytes2);
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * kStageAll);
           const uint32_t bar = mapa_smem(smem_u32(&full_bar[stage]), 0);
           uint8_t* sa = smem_a + stage * kABytes2;
-          uint8_t* sb = smem_b + stage * kBBytes2;
+          uint8_t* sb = smem_b + stage * (NH * kBBytes2);
           if (CONV == kConvA) {
             const int tap = tap_r * cv.KW + tap_s;
             const int ow = cv.flip ? cv.KW - 1 - tap_s : tap_s, oh = cv.flip ? cv.KH - 1 - tap_r : tap_r;
@@ -315,11 +324,15 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             for (int c = 0; c < BNH / 64; ++c)
               tma_load_im2col_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, bc[c], pw, ph, pn, bs[c], br[c]);
           } else if (CONV == kConvNone) {
-            if (!B_MN) {
-              tma_load_2d_pair(sb, &tma_b, bar, kb * BK2, n0);
-            } else {
 #pragma unroll
-              for (int c = 0; c < BNH / 64; ++c) tma_load_2d_pair(sb + c * (64 * BK2 * 2), &tma_b, bar, n0 + c * 64, kb * BK2);
+            for (int h = 0; h < NH; ++h) {
+              if (!B_MN) {
+                tma_load_2d_pair(sb + h * kBBytes2, &tma_b, bar, kb * BK2, n0 + h * BN2);
+              } else {
+#pragma unroll
+                for (int c = 0; c < BNH / 64; ++c)
+                  tma_load_2d_pair(sb + h * kBBytes2 + c * (64 * BK2 * 2), &tma_b, bar, n0 + h * BN2 + c * 64, kb * BK2);
+              }
             }
           }
           if (++stage == kStages2) {
@@ -340,6 +353,51 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       int iter = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters, ++iter) {
+        // D (+)= A . B of one stage, 64 of the reduction
+        auto products = [&](uint32_t tmem_d, int st, int h, bool first) {
+          const uint32_t sa = smem_u32(smem_a + st * kABytes2);
+          const uint32_t sb = smem_u32(smem_b + (st * NH + h) * kBBytes2);
+#pragma unroll
+          for (int k = 0; k < BK2 / 16; ++k) {
+            const uint64_t da = A_MN ? umma_desc_sw128(sa + k * 2048, 64 * BK2 * 2, 1024)
+                                     : umma_desc_sw128(sa + k * 32, 16, 1024);
+            const uint64_t db = B_MN ? umma_desc_sw128(sb + k * 2048, 64 * BK2 * 2, 1024)
+                                     : umma_desc_sw128(sb + k * 32, 16, 1024);
+            umma_f16_ss_pair(tmem_d, da, db, idesc, !first || k != 0 ? 1u : 0u);
+          }
+        };
+        if constexpr (NH == 2) {
+          // Both halves take the whole TMEM, so the next tile waits for the epilogue.  The first and the last K blocks of a tile
+          // are taken half by half: the first half is complete, and its columns wanted again, that much earlier.
+          for (int kb = 0; kb < num_kb && ok;) {
+            const bool last = kb + kSwitchGroup >= num_kb;
+            const int g = last ? num_kb - kb : kb == 0 ? kSwitchGroup : 1;
+            int st = stage;
+            uint32_t ph = phase;
+#pragma unroll
+            for (int h = 0; h < NH; ++h) {
+              if (kb == 0 && !(ok = ok && mbar_wait(&tmem_empty_bar[h], (iter & 1) ^ 1, abort_flag))) break;
+              st = stage;
+              ph = phase;
+              for (int j = 0; j < g; ++j) {
+                if (h == 0 && !(ok = mbar_wait(&full_bar[st], ph, abort_flag))) break;
+                tc_fence_after_sync();
+                products(tmem_base + h * BN2, st, h, kb + j == 0);
+                if (h == NH - 1) umma_commit_pair(&empty_bar[st]);
+                if (++st == kStages2) {
+                  st = 0;
+                  ph ^= 1;
+                }
+              }
+              if (!ok) break;
+              if (last) umma_commit_pair(&tmem_full_bar[h]);
+            }
+            stage = st;
+            phase = ph;
+            kb += g;
+          }
+          continue;
+        }
         const int acc = iter & 1;
         const uint32_t acc_phase = (iter >> 1) & 1;
         if (!mbar_wait(&tmem_empty_bar[acc], acc_phase ^ 1, abort_flag)) {
@@ -347,23 +405,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           break;
         }
         tc_fence_after_sync();
-        const uint32_t tmem_d = tmem_base + acc * BN2;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
             ok = false;
             break;
           }
           tc_fence_after_sync();
-          const uint32_t sa = smem_u32(smem_a + stage * kABytes2);
-          const uint32_t sb = smem_u32(smem_b + stage * kBBytes2);
-#pragma unroll
-          for (int k = 0; k < BK2 / 16; ++k) {
-            const uint64_t da = A_MN ? umma_desc_sw128(sa + k * 2048, 64 * BK2 * 2, 1024)
-                                     : umma_desc_sw128(sa + k * 32, 16, 1024);
-            const uint64_t db = B_MN ? umma_desc_sw128(sb + k * 2048, 64 * BK2 * 2, 1024)
-                                     : umma_desc_sw128(sb + k * 32, 16, 1024);
-            umma_f16_ss_pair(tmem_d, da, db, idesc, (kb | k) != 0 ? 1u : 0u);
-          }
+          products(tmem_base + acc * BN2, stage, 0, kb == 0);
           umma_commit_pair(&empty_bar[stage]);
           if (++stage == kStages2) {
             stage = 0;
@@ -377,111 +425,159 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     // -------------------------------- epilogue --------------------------------
     const int quarter = warp & 3;
     const int grp = (warp - 2) >> 2;  // 64-column group of the 256-column tile
-    uint8_t* stg = epi_stage + (warp - 2) * kEpiStage;
+    constexpr int kCols = 64 / NH, kPieces = kCols / 8, kRows = 32 / kPieces;  // columns staged at a time, 16-byte pieces of a row, rows per pass
+    uint8_t* stg = epi_stage + (warp - 2) * (kEpiStage / NH);
     const uint32_t keep16 = dropout_keep16(p.dropout_p);
     const float drop_scale = p.dropout_p > 0.f ? 65536.0f / static_cast<float>(keep16) : 1.0f;
     int iter = 0;
     bool ok = true;
     for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters, ++iter) {
       const TileCoord2 tc = tile_coord2(tile, num_m, num_n);
-      const int acc = iter & 1;
-      const uint32_t acc_phase = (iter >> 1) & 1;
       const int row0 = pblk_of(tc.m_blk) * 2 * BM2 + static_cast<int>(cta_rank) * BM2 + quarter * 32;  // first row of this warp
-      const int col0 = tc.n_blk * BN2 + grp * 64;                                              // first column
       const int row = row0 + lane;
       const bool row_ok = row < p.M;
-      const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN2 + grp * 64;
-      // Staged path: bf16 output, no accumulate, the warp's 64 columns inside the matrix, at most one row operand.
-      // Row operands enter and results leave through a 4 KB swizzled staging tile, so every global access of the
-      // warp is four full 128-byte row segments instead of 32 scattered 32-byte pieces.
-      const bool has_operand = p.residual != nullptr || p.act == kActDGelu || p.act == kActDRelu;
-      const bool staged = !p.out_fp32 && !p.accumulate && col0 + 64 <= p.N &&
-                          !(p.residual != nullptr && (p.act == kActDGelu || p.act == kActDRelu)) &&
-                          !(p.preact_out != nullptr && has_operand);
-      if (staged) {
-        const int srow = lane >> 3, spiece = lane & 7;  // coalesced phase: 4 rows x 8 sixteen-byte pieces per pass
-        auto cell = [&](int rr, int piece) { return stg + rr * 128 + ((piece ^ (rr & 7)) << 4); };
-        if (has_operand) {  // fetched while the tensor cores still work on this tile
-          const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.residual != nullptr ? p.residual : p.aux);
-          const int ld = p.residual != nullptr ? p.ldres : p.ldaux;
-#pragma unroll
-          for (int it = 0; it < 8; ++it) {
-            const int rr = it * 4 + srow;
-            if (row0 + rr < p.M)
-              *reinterpret_cast<uint4*>(cell(rr, spiece)) =
-                  __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(row0 + rr) * ld + col0) + spiece);
-          }
+#pragma unroll 1
+      for (int h = 0; h < NH && ok; ++h) {
+        const int acc = NH == 2 ? h : iter & 1;
+        const uint32_t acc_phase = (NH == 2 ? iter : iter >> 1) & 1;
+        const int col0 = tc.n_blk * BNT + h * BN2 + grp * 64;  // first column
+        const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN2 + grp * 64;
+        auto release = [&]() {  // the accumulator columns are free
+          tc_fence_before_sync();
           __syncwarp();
-        }
-        if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
-          ok = false;
-          break;
-        }
-        tc_fence_after_sync();
-        auto flush = [&](void* base, int ld) {  // staging tile -> global, 4 rows x 128 bytes per instruction
-          __syncwarp();
-#pragma unroll
-          for (int it = 0; it < 8; ++it) {
-            const int rr = it * 4 + srow;
-            if (row0 + rr < p.M)
-              *(reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(base) + static_cast<size_t>(row0 + rr) * ld + col0) +
-                spiece) = *reinterpret_cast<const uint4*>(cell(rr, spiece));
-          }
-          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(mapa_smem(smem_u32(&tmem_empty_bar[acc]), 0));
         };
-        if (p.preact_out != nullptr) {  // first pass: the pre-activation tile
+        // Staged path: bf16 output, no accumulate, the warp's 64 columns inside the matrix, at most one row operand.
+        // Row operands enter and results leave through a swizzled staging tile, so every global access of the warp is four
+        // full 128-byte row segments (wide tile: eight of 64 bytes) instead of 32 scattered 32-byte pieces.
+        const bool has_operand = p.residual != nullptr || p.act == kActDGelu || p.act == kActDRelu;
+        const bool staged = !p.out_fp32 && !p.accumulate && col0 + 64 <= p.N &&
+                            !(p.residual != nullptr && (p.act == kActDGelu || p.act == kActDRelu)) &&
+                            !(p.preact_out != nullptr && has_operand);
+        if (staged) {
+          const int srow = lane / kPieces, spiece = lane % kPieces;  // coalesced phase
+          auto cell = [&](int rr, int piece) {
+            return stg + rr * (kCols * 2) + ((piece ^ ((NH == 2 ? rr >> 1 : rr) & (kPieces - 1))) << 4);
+          };
+          auto fetch = [&](int c0) {
+            const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(p.residual != nullptr ? p.residual : p.aux);
+            const int ld = p.residual != nullptr ? p.ldres : p.ldaux;
+#pragma unroll
+            for (int it = 0; it < kPieces; ++it) {
+              const int rr = it * kRows + srow;
+              if (row0 + rr < p.M)
+                *reinterpret_cast<uint4*>(cell(rr, spiece)) =
+                    __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(row0 + rr) * ld + c0) + spiece);
+            }
+            __syncwarp();
+          };
+          auto flush = [&](void* base, int ld, int c0) {  // staging tile -> global
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < kPieces; ++it) {
+              const int rr = it * kRows + srow;
+              if (row0 + rr < p.M)
+                *(reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(base) + static_cast<size_t>(row0 + rr) * ld + c0) +
+                  spiece) = *reinterpret_cast<const uint4*>(cell(rr, spiece));
+            }
+            __syncwarp();
+          };
+          if (has_operand) fetch(col0);  // while the tensor cores still work on this tile
+          if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
+#pragma unroll 1
+          for (int part = 0; part < NH; ++part) {
+            const int c0 = col0 + part * kCols;
+            if (part > 0 && has_operand) fetch(c0);
+            if (p.preact_out != nullptr) {  // first pass: the pre-activation tile
+#pragma unroll 1
+              for (int c = 0; c < kCols / 16; ++c) {
+                uint32_t r[16];
+                tmem_ld_32x16(taddr + part * kCols + c * 16, r);
+                tmem_ld_wait();
+                const uint4 none[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+                float pre[16], v[16];
+                gemm_epilogue_math16(p, row, c0 + c * 16, r, none, keep16, drop_scale, pre, v);
+                *reinterpret_cast<uint4*>(cell(lane, 2 * c)) = pack8(pre);
+                *reinterpret_cast<uint4*>(cell(lane, 2 * c + 1)) = pack8(pre + 8);
+              }
+              flush(p.preact_out, p.ldpre, c0);
+            }
+#pragma unroll 1
+            for (int c = 0; c < kCols / 16; ++c) {
+              uint32_t r[16];
+              tmem_ld_32x16(taddr + part * kCols + c * 16, r);
+              tmem_ld_wait();
+              if (part == NH - 1 && c == kCols / 16 - 1) release();  // its last columns are in registers
+              uint4 operand[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
+              if (has_operand) {
+                operand[0] = *reinterpret_cast<const uint4*>(cell(lane, 2 * c));
+                operand[1] = *reinterpret_cast<const uint4*>(cell(lane, 2 * c + 1));
+              }
+              float pre[16], v[16];
+              gemm_epilogue_math16(p, row, c0 + c * 16, r, operand, keep16, drop_scale, pre, v);
+              *reinterpret_cast<uint4*>(cell(lane, 2 * c)) = pack8(v);
+              *reinterpret_cast<uint4*>(cell(lane, 2 * c + 1)) = pack8(v + 8);
+            }
+            flush(p.D, p.ldd, c0);
+          }
+          continue;
+        }
+        // fp32 output: 16 columns at a time through the staging tile, 64-byte row segments to memory; what is there already
+        // (gradients are added to) is read in the same pieces, one ahead; the first while the tensor cores still work on this tile.
+        // A thread with a row of its own moved 16 of every 32-byte sector at a time and waited for each 16 columns of old values
+        // in turn; with a reduction of 4096 that took longer than the main loop of the next tile.  Alone / sustained under the
+        // power cap: weight gradients 51200 x 2048 over 4096 rows 649 -> 600 / 805 -> 754 us, 8192 x 2048 over 8192 216 -> 209 /
+        // 255 -> 248.
+        if (p.out_fp32 && col0 + 64 <= p.N && !has_operand && p.preact_out == nullptr) {
+          const int srow = lane >> 2, spiece = lane & 3;
+          float* out = reinterpret_cast<float*>(p.D) + static_cast<size_t>(row0 + srow) * p.ldd + col0 + spiece * 4;
+          auto cell = [&](int rr, int piece) { return stg + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4); };
+          auto old_values = [&](float4 (&o)[4], int c) {
+#pragma unroll
+            for (int it = 0; it < 4; ++it)
+              if (row0 + it * 8 + srow < p.M) o[it] = *reinterpret_cast<const float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16);
+          };
+          float4 old[4] = {}, next[4] = {};
+          if (p.accumulate) old_values(old, 0);
+          if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
+            ok = false;
+            break;
+          }
+          tc_fence_after_sync();
 #pragma unroll 1
           for (int c = 0; c < 4; ++c) {
+            if (p.accumulate && c < 3) old_values(next, c + 1);
             uint32_t r[16];
             tmem_ld_32x16(taddr + c * 16, r);
             tmem_ld_wait();
+            if (c == 3) release();
             const uint4 none[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
             float pre[16], v[16];
             gemm_epilogue_math16(p, row, col0 + c * 16, r, none, keep16, drop_scale, pre, v);
-            *reinterpret_cast<uint4*>(cell(lane, 2 * c)) = pack8(pre);
-            *reinterpret_cast<uint4*>(cell(lane, 2 * c + 1)) = pack8(pre + 8);
-          }
-          flush(p.preact_out, p.ldpre);
-        }
-#pragma unroll 1
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[16];
-          tmem_ld_32x16(taddr + c * 16, r);
-          tmem_ld_wait();
-          if (c == 3) {  // the accumulator stage is free once its last columns are in registers
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_smem(smem_u32(&tmem_empty_bar[acc]), 0));
-          }
-          uint4 operand[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-          if (has_operand) {
-            operand[0] = *reinterpret_cast<const uint4*>(cell(lane, 2 * c));
-            operand[1] = *reinterpret_cast<const uint4*>(cell(lane, 2 * c + 1));
-          }
-          float pre[16], v[16];
-          gemm_epilogue_math16(p, row, col0 + c * 16, r, operand, keep16, drop_scale, pre, v);
-          *reinterpret_cast<uint4*>(cell(lane, 2 * c)) = pack8(v);
-          *reinterpret_cast<uint4*>(cell(lane, 2 * c + 1)) = pack8(v + 8);
-        }
-        flush(p.D, p.ldd);
-        continue;
-      }
-      // fp32 output: 16 columns at a time through the staging tile, 64-byte row segments to memory; what is there already
-      // (gradients are added to) is read in the same pieces, one ahead; the first while the tensor cores still work on this tile.
-      // A thread with a row of its own moved 16 of every 32-byte sector at a time and waited for each 16 columns of old values
-      // in turn; with a reduction of 4096 that took longer than the main loop of the next tile.  Alone / sustained under the power
-      // cap: weight gradients 51200 x 2048 over 4096 rows 649 -> 600 / 805 -> 754 us, 8192 x 2048 over 8192 216 -> 209 / 255 -> 248.
-      if (p.out_fp32 && col0 + 64 <= p.N && !has_operand && p.preact_out == nullptr) {
-        const int srow = lane >> 2, spiece = lane & 3;
-        float* out = reinterpret_cast<float*>(p.D) + static_cast<size_t>(row0 + srow) * p.ldd + col0 + spiece * 4;
-        auto cell = [&](int rr, int piece) { return stg + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4); };
-        auto old_values = [&](float4 (&o)[4], int c) {
 #pragma unroll
-          for (int it = 0; it < 4; ++it)
-            if (row0 + it * 8 + srow < p.M) o[it] = *reinterpret_cast<const float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16);
-        };
-        float4 old[4] = {}, next[4] = {};
-        if (p.accumulate) old_values(old, 0);
+            for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(cell(lane, i)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int it = 0; it < 4; ++it) {
+              const int rr = it * 8 + srow;
+              float4 q = *reinterpret_cast<const float4*>(cell(rr, spiece));
+              if (row0 + rr < p.M) {
+                if (p.accumulate) {
+                  q.x += old[it].x; q.y += old[it].y; q.z += old[it].z; q.w += old[it].w;
+                }
+                *reinterpret_cast<float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16) = q;
+              }
+            }
+#pragma unroll
+            for (int it = 0; it < 4; ++it) old[it] = next[it];
+            __syncwarp();
+          }
+          continue;
+        }
         if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
           ok = false;
           break;
@@ -489,56 +585,16 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         tc_fence_after_sync();
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
-          if (p.accumulate && c < 3) old_values(next, c + 1);
+          const int n0 = col0 + c * 16;
+          if (n0 >= p.N) break;  // uniform across the warp
           uint32_t r[16];
           tmem_ld_32x16(taddr + c * 16, r);
           tmem_ld_wait();
-          if (c == 3) {  // the accumulator stage is free once its last columns are in registers
-            tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(mapa_smem(smem_u32(&tmem_empty_bar[acc]), 0));
-          }
-          const uint4 none[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-          float pre[16], v[16];
-          gemm_epilogue_math16(p, row, col0 + c * 16, r, none, keep16, drop_scale, pre, v);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) *reinterpret_cast<float4*>(cell(lane, i)) = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          __syncwarp();
-#pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int rr = it * 8 + srow;
-            float4 q = *reinterpret_cast<const float4*>(cell(rr, spiece));
-            if (row0 + rr < p.M) {
-              if (p.accumulate) {
-                q.x += old[it].x; q.y += old[it].y; q.z += old[it].z; q.w += old[it].w;
-              }
-              *reinterpret_cast<float4*>(out + static_cast<size_t>(it * 8) * p.ldd + c * 16) = q;
-            }
-          }
-#pragma unroll
-          for (int it = 0; it < 4; ++it) old[it] = next[it];
-          __syncwarp();
+          if (!row_ok) continue;
+          gemm_epilogue_chunk<16>(p, row, n0, r, keep16, drop_scale);
         }
-        continue;
+        release();
       }
-      if (!__all_sync(0xffffffffu, mbar_wait(&tmem_full_bar[acc], acc_phase, abort_flag))) {
-        ok = false;
-        break;
-      }
-      tc_fence_after_sync();
-#pragma unroll 1
-      for (int c = 0; c < 4; ++c) {
-        const int n0 = col0 + c * 16;
-        if (n0 >= p.N) break;  // uniform across the warp
-        uint32_t r[16];
-        tmem_ld_32x16(taddr + c * 16, r);
-        tmem_ld_wait();
-        if (!row_ok) continue;
-        gemm_epilogue_chunk<16>(p, row, n0, r, keep16, drop_scale);
-      }
-      tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_smem(smem_u32(&tmem_empty_bar[acc]), 0));
     }
   } else if (GATHER) {
     // --------------------------------- pusher ---------------------------------
@@ -612,10 +668,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   }
 }
 
-template <bool A_MN, bool B_MN, bool GATHER, int CONV>
+template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
 int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap& tb, const GemmParams& p,
                 const GemmAgComm& cm, const ConvLoad& cv, int num_sms, cudaStream_t stream) {
-  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV>;
+  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV, NH>;
   constexpr int threads = GATHER ? kThreadsGather : kThreads2;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -640,7 +696,7 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
     }
     max_clusters = n;
   }
-  const int num_tiles = ((p.M + 2 * BM2 - 1) / (2 * BM2)) * ((p.N + BN2 - 1) / BN2);
+  const int num_tiles = ((p.M + 2 * BM2 - 1) / (2 * BM2)) * ((p.N + NH * BN2 - 1) / (NH * BN2));
   int clusters = num_sms / 2;
   if (clusters > max_clusters) clusters = max_clusters;
   if (clusters > num_tiles) clusters = num_tiles;
@@ -652,6 +708,18 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, ta2, tb, p, cm, cv));
+}
+
+// The tile of 256 x 512 takes a product with a long reduction, where its end (the next tile waits for the epilogue) weighs little,
+// and where counting in whole rounds of 256 columns costs nothing.  us alone / sustained under the power cap, 256 -> 512 columns:
+// 8192 x 2048 bf16 over 4096: 109 -> 117 / 116 -> 119; 6144: 155 -> 160 / 175 -> 172; 8192: 204 -> 204 / 234 -> 225; 12288: 301 -> 291 /
+// 349 -> 330; 4096 x 2048 over 51200: 594 -> 568 / 708 -> 652.  fp32, added to: over 8192 210 -> 224 / 251 -> 246; 16384: 403 -> 416 /
+// 481 -> 455; 32768: 804 -> 751 / 944 -> 875.
+constexpr int kWideK = 8192, kWideKFp32 = 16384;
+bool wide_tile(int M, int N, int K, bool out_fp32, int num_sms) {
+  const long long m = (M + 255LL) / 256, narrow = m * ((N + 255LL) / 256), wide = m * ((N + 511LL) / 512);
+  const int pairs = num_sms / 2;
+  return N >= 512 && K >= (out_fp32 ? kWideKFp32 : kWideK) && 2 * ((wide + pairs - 1) / pairs) <= (narrow + pairs - 1) / pairs;
 }
 
 template <bool A_MN, bool B_MN, bool GATHER>
@@ -670,10 +738,15 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
   if (rc != 0) return rc;
   rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, BNH, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
   if (rc != 0) return rc;
-  return launch_maps<A_MN, B_MN, GATHER, kConvNone>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
+  if constexpr (!GATHER)
+    if (wide_tile(p.M, p.N, p.K, p.out_fp32, num_sms)) return launch_maps<A_MN, B_MN, false, kConvNone, 2>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
+  return launch_maps<A_MN, B_MN, GATHER, kConvNone, 1>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
 }
 
 }  // namespace
+
+// Columns of the output tile for a product that this kernel takes: 256 or 512.
+int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms) { return wide_tile(M, N, K, out_fp32, num_sms) ? 512 : 256; }
 
 // Same contract as gemm_bf16_launch; callers pick this variant for outputs of at least 256 x 256.
 int gemm2_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
@@ -711,7 +784,7 @@ int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, 
   if ((rc = make_tma_im2col_bf16(&ta, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BM2))) return rc;
   if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, BNH, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<false, false, false, kConvA>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<false, false, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
 }
 
 // dx[N, H, W, C] of a stride-1 convolution from dy[N, Ho, Wo, K]; p describes the GEMM [N H W, C] with K = KH * KW * K.
@@ -724,7 +797,7 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
   if ((rc = make_tma_im2col_bf16(&ta, dy, N, Ho, Wo, Kout, lh, lw, -pad, -pad, 1, BM2))) return rc;
   if ((rc = make_tma_2d_bf16(&tb, w, Kout, static_cast<uint64_t>(KH) * KW * C, ldw, BK2, 64))) return rc;
   ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
-  return launch_maps<false, true, false, kConvA>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
 }
 
 // dw[K, KH * KW * C] from dy[N Ho Wo, K] and x; p describes the GEMM [K, KH * KW * C] with K = N Ho Wo.
@@ -735,7 +808,7 @@ int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int
   if ((rc = make_tma_2d_bf16(&ta, dy, p.K, p.M, lddy, BK2, 64))) return rc;
   if ((rc = make_tma_im2col_bf16(&tb, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<true, true, false, kConvB>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<true, true, false, kConvB, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
 }
 
 }  // namespace ssb

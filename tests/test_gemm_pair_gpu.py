@@ -52,3 +52,49 @@ def test_fp32_outputs(M, N, K, a_mn, b_mn, accumulate, bias):
         want = want + d.double()
     F.gemm(a, b, out=d, a_mn=a_mn, b_mn=b_mn, bias=bb, accumulate=accumulate)
     check(d, whole, want, bound + 2.0 ** -22 * (want.abs() + 4))
+
+
+# Tiles of 256 x 512: (M, N, K, fp32) with both halves whole, the second half cut or empty, rows and reduction that end inside.
+WIDE = [(2048, 4608, 8192, False), (1901, 4456, 8264, False), (2040, 4200, 8200, False), (2044, 4360, 8192, False),
+        (1904, 4424, 16456, True)]
+
+
+@pytest.mark.parametrize("M,N,K,fp32", WIDE)
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_wide_tiles(M, N, K, fp32, a_mn, b_mn):
+    assert native.ext().gemm_pair_columns(M, N, K, fp32, 148) == 512
+    a, b, want, bound = operands(M, N, K, a_mn, b_mn)
+    d, whole = padded(M, N, torch.float32 if fp32 else torch.bfloat16)
+    if fp32:
+        want = want + d.double()
+    F.gemm(a, b, out=d, a_mn=a_mn, b_mn=b_mn, accumulate=fp32)
+    check(d, whole, want, bound + (2.0 ** -22 if fp32 else 2.0 ** -8) * (want.abs() + 2.0 ** -20))
+
+
+@pytest.mark.parametrize("M,N,K", [(2048, 4608, 8192), (1901, 4452, 8264)])
+@pytest.mark.parametrize("kind", ["bias_residual_dropout", "gelu_preact", "dgelu", "accumulate"])
+def test_wide_tile_epilogues(M, N, K, kind):
+    """Against the kernel with one CTA per tile: the same products in the same order of the reduction, the same epilogue."""
+    a, b, _, _ = operands(M, N, K, False, False)
+    a = a * 0.02
+    bias, rows = torch.randn(N, device=DEV).bfloat16(), [padded(M, N)[0] for _ in range(2)]
+    results = []
+    for mode in (0, 1):
+        native.ext().gemm_set_pair_mode(mode)
+        try:
+            d = rows[1].clone() if kind == "accumulate" else torch.empty(M, N, device=DEV, dtype=torch.bfloat16)
+            pre = torch.zeros(M, (N + 7) // 8 * 8, device=DEV, dtype=torch.bfloat16)[:, :N]
+            call = dict(bias_residual_dropout=dict(bias=bias, residual=rows[0], dropout_p=0.1, seed=5), accumulate=dict(accumulate=True),
+                        gelu_preact=dict(bias=bias, act=F.ACT_GELU, preact_out=pre), dgelu=dict(act=F.ACT_DGELU, aux=rows[0]))[kind]
+            if kind == "bias_residual_dropout" and N % 8:
+                d = torch.empty(M, N + 4, device=DEV, dtype=torch.bfloat16)[:, :N]
+                call.pop("dropout_p")
+            elif N % 8:
+                d = torch.empty(M, N + 4, device=DEV, dtype=torch.bfloat16)[:, :N].copy_(rows[1])
+            F.gemm(a, b, out=d, **call)
+            results.append((d.clone(), pre.clone()))
+        finally:
+            native.ext().gemm_set_pair_mode(1)
+    assert native.check_status() == 0
+    for one, pair in zip(*results):
+        assert torch.equal(one, pair)
