@@ -18,13 +18,18 @@ namespace {
 
 constexpr int kLnWarpsPerBlock = 4;
 
+__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
+  const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
+}
+
 // Rows that fit in the registers of a warp, read once: up to VPL vectors of 8 bf16 per lane; FULL = false: the last one, or for
 // VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  Lengths that are
 // not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984 147 -> 55 us, of 1088 83 -> 33, 512 of 704
 // 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
 // is slower (32768 x 2048 67 us instead of 55): too few warps; so is fp32 arithmetic two values per instruction (32768 x 1024
 // 28.1 -> 29.9).  What bounds it is the latency of the loads with 15 warps an SM (125 registers): 32768 x 2048 keeps the DRAM 47 %
-// busy, the issue slots 35 %, and hardly ever waits for a math pipe.
+// busy, the issue slots 35 %, and hardly ever waits for a math pipe.  Many rows of some lengths go to ln_fwd_group_kernel below.
 template <int VPL, bool FULL>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
@@ -111,6 +116,162 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
         w[j] = pack_bf16x2(d[j].x * rstd * g[j].x + b[j].x, d[j].y * rstd * g[j].y + b[j].y);
       }
       yr[v] = o;
+    }
+  }
+}
+
+// Many rows of up to 2048: WPR warps share a row and take R rows at a time, the next R on their way meanwhile.  gamma and beta stay in
+// registers; a warp per row read them from the L1 for every row, and its loads, sums and stores came one after the other
+// (warps an SM and loads in flight were what bounded it: DRAM 47 %, issue slots 35 %).  The warps of a row exchange their means and
+// sums of squares about them once per R rows; these are brought together about the common mean, which is no less exact than sums
+// over the whole row.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
+// Measured, a warp per row -> this: 32768 x 2048 55.7 -> 49.0 us, x 1536 49.1 -> 38.9, x 512 16.5 -> 13.8, 4096 x 2048 11.6 -> 10.5; a copy
+// takes 42.5, 32.8, 12.4, 7.3.  Rows of 513 to 1280 columns stay with a warp each: two or three warps are idle in part there
+// (32768 x 768 22.6 -> 29, x 1152 34.1 -> 37.3, x 1280 37.0 -> 37.5).
+template <int WPR>
+struct LnGroup {
+  static constexpr int kRows = 3, kGroups = WPR == 1 ? 4 : 1, kThreads = 32 * WPR * kGroups, kBlocks = 512 / kThreads;  // per SM
+};
+bool ln_fwd_grouped(int rows, int H, int num_sms) {  // every group has all of its rows at least once
+  const int groups = num_sms * (H <= 512 ? LnGroup<1>::kBlocks * 4 : H <= 1536 ? LnGroup<3>::kBlocks : LnGroup<4>::kBlocks);
+  return (H <= 512 || (H > 1280 && H <= 2048)) && rows >= groups * 3;
+}
+template <int WPR>
+__global__ void __launch_bounds__(LnGroup<WPR>::kThreads, LnGroup<WPR>::kBlocks)
+ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int H,
+                    float eps) {
+  constexpr int VPL = 2, G = LnGroup<WPR>::kGroups, R = LnGroup<WPR>::kRows;
+  __shared__ float2 xch[2][G][WPR][R];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slot = warp / WPR, part = warp % WPR;
+  const int nvec = H / 8;
+  float g[VPL][8], b[VPL][8];
+  bool mine[VPL];
+  int at[VPL], count = 0;  // this lane's vectors; columns of this warp
+#pragma unroll
+  for (int i = 0; i < VPL; ++i) {
+    at[i] = (i * WPR + part) * 32 + lane;
+    mine[i] = at[i] < nvec;
+    count += 8 * max(0, min(32, nvec - (i * WPR + part) * 32));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      g[i][j] = mine[i] ? __ldg(gamma + at[i] * 8 + j) : 0.f;  // once: any alignment
+      b[i][j] = mine[i] ? __ldg(beta + at[i] * 8 + j) : 0.f;
+    }
+  }
+  const float inv_count = count > 0 ? 1.0f / static_cast<float>(count) : 0.f, inv_h = 1.0f / static_cast<float>(H);
+  uint4 next[R][VPL];
+  auto fetch = [&](int row0) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int i = 0; i < VPL; ++i)
+        if (mine[i] && row0 + r < rows) next[r][i] = __ldg(reinterpret_cast<const uint4*>(x + static_cast<size_t>(row0 + r) * H) + at[i]);
+  };
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) next[r][i] = make_uint4(0u, 0u, 0u, 0u);
+  const int step = gridDim.x * G * R;
+  int row0 = (blockIdx.x * G + slot) * R, turn = 0;
+  fetch(row0);
+  for (; row0 < rows; row0 += step, turn ^= 1) {
+    uint4 q[R][VPL];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) q[r][i] = next[r][i];
+    fetch(row0 + step);
+    // The rows stay packed: each of the three uses unpacks them again (kept as fp32 they would not fit and be spilled).
+    auto packed = [&]() {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int i = 0; i < VPL; ++i) asm volatile("" : "+r"(q[r][i].x), "+r"(q[r][i].y), "+r"(q[r][i].z), "+r"(q[r][i].w));
+    };
+    float m[R], s2[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        float v[8];
+        unpack8(q[r][i], v);
+        t += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+      }
+      m[r] = t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < R; ++r) m[r] += __shfl_xor_sync(0xffffffffu, m[r], o);
+    packed();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      m[r] *= inv_count;
+      float t = 0.f;
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        float v[8];
+        unpack8(q[r][i], v);
+        float u = 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) u = fmaf(v[j] - m[r], v[j] - m[r], u);
+        if (mine[i]) t += u;
+      }
+      s2[r] = t;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < R; ++r) s2[r] += __shfl_xor_sync(0xffffffffu, s2[r], o);
+    packed();
+    if constexpr (WPR > 1) {
+      float2(&slots)[WPR][R] = xch[turn][slot];
+      if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) slots[part][r] = make_float2(m[r] * static_cast<float>(count), s2[r]);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(32 * WPR) : "memory");
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        float2 e[WPR];
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < WPR; ++w) {
+          e[w] = slots[w][r];
+          sum += e[w].x;
+        }
+        m[r] = sum * inv_h;
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < WPR; ++w) {
+          const float n = static_cast<float>(8 * (max(0, min(32, nvec - w * 32)) + max(0, min(32, nvec - (WPR + w) * 32))));
+          const float d = n > 0.f ? e[w].x / n - m[r] : 0.f;
+          t += fmaf(d * n, d, e[w].y);
+        }
+        s2[r] = t;
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int row = row0 + r;
+      if (row >= rows) break;
+      const float rs = rsqrtf(s2[r] * inv_h + eps);
+      if (part == 0 && lane == 0) {
+        mean_out[row] = m[r];
+        rstd_out[row] = rs;
+      }
+      uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
+#pragma unroll
+      for (int i = 0; i < VPL; ++i) {
+        if (!mine[i]) continue;
+        float v[8];
+        unpack8(q[r][i], v);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = (v[j] - m[r]) * rs * g[i][j] + b[i][j];
+        yr[at[i]] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+      }
     }
   }
 }
@@ -264,11 +425,6 @@ struct LnRing {
   }
 };
 
-__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
-  const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-
 // One pass over dy, x and dres for any H <= 512 * WPR: dx, and in the same sweep every lane keeps running sums of
 // dy * xhat and dy for its 16 columns over all rows its warp visits (their gamma stays in registers).  A chunk is
 // 8 / WPR consecutive rows of the three matrices; WPR warps share a row (each owns 512 columns) and exchange their two
@@ -344,10 +500,24 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         for (; ch * RPB + rslot < rows; ch += gridDim.x) meet();
     };
     int c = 0;
+    // Statistics of the row: with many rows in a chunk loaded a chunk ahead, like the rows themselves (32768 x 512 33.0 -> 29.8 us,
+    // x 1024 55.4 -> 53.4; four warps a row 100.6 -> 102.5).
+    constexpr bool kStatsAhead = WPR <= 2;
+    float mu_next = 0.f, rs_next = 0.f;
+    auto fetch_stats = [&](int ch) {
+      const int row = ch * RPB + rslot;
+      if (ch < chunks && row < rows) {
+        mu_next = __ldg(mean + row);
+        rs_next = __ldg(rstd + row);
+      }
+    };
+    if (kStatsAhead) fetch_stats(blockIdx.x);
     for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
       const int row = ch * RPB + rslot;
       const bool have = row < rows;                  // the same for all warps of a row slot
-      const float mu = have ? __ldg(mean + row) : 0.f, rs = have ? __ldg(rstd + row) : 0.f;
+      if (!kStatsAhead) fetch_stats(ch);
+      const float mu = mu_next, rs = rs_next;
+      if (kStatsAhead) fetch_stats(ch + gridDim.x);
       if (!ring.wait_full(c)) {
         meet_to_the_end(ch);
         break;
@@ -648,6 +818,16 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
   const auto* rb = reinterpret_cast<const __nv_bfloat16*>(residual);
   auto* yb = reinterpret_cast<__nv_bfloat16*>(y);
   auto* sb = reinterpret_cast<__nv_bfloat16*>(sum_out);
+  if (residual == nullptr && ln_fwd_grouped(rows, H, num_sms)) {
+    auto launch = [&](auto kernel, auto cfg) {
+      using Cfg = decltype(cfg);
+      kernel<<<num_sms * Cfg::kBlocks, Cfg::kThreads, 0, stream>>>(xb, gamma, beta, yb, mean, rstd, rows, H, eps);
+    };
+    if (H <= 512) launch(ln_fwd_group_kernel<1>, LnGroup<1>{});
+    else if (H <= 1536) launch(ln_fwd_group_kernel<3>, LnGroup<3>{});
+    else launch(ln_fwd_group_kernel<4>, LnGroup<4>{});
+    return static_cast<int>(cudaGetLastError());
+  }
 #define SSB_LN_ARGS <<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
 #define SSB_LN_CASE(V)                                          \
   case V:                                                       \

@@ -28,3 +28,26 @@ def test_layernorm_forward_row_lengths(H, rows, with_residual):
     assert float((out[1].double() - d.mean(-1)).abs().max()) < 1e-5
     rstd = 1.0 / torch.sqrt(d.var(-1, unbiased=False) + 1e-5)
     assert float(((out[2].double() - rstd) / rstd).abs().max()) < 1e-4
+
+
+@pytest.mark.parametrize("H,rows", [(8, 7104), (248, 7105), (264, 7106), (512, 9001),              # a warp per row, three at a time
+                                    (1288, 2220), (1472, 2221), (1536, 2370),                      # three warps per row
+                                    (1544, 1776), (1800, 1777), (2048, 1778), (2048, 5003),        # four
+                                    (512, 7103), (1536, 2219), (2048, 1775)])                      # one row short of it
+@pytest.mark.parametrize("offset", [3.0, 300.0])
+def test_layernorm_forward_of_many_rows(H, rows, offset):
+    """Mean and 1/std from parts of a row.  fp32 sums of values near `offset`: off by 2^-22 offset at most per value, hence the mean by
+    that, the sum of squares about it by its square; results round to bf16 once (2^-9)."""
+    torch.manual_seed(H + rows)
+    x = (torch.randn(rows, H, device=DEV) * 2 + offset).bfloat16()
+    flat = torch.randn(2 * H + 1, device=DEV)
+    for g, b in ((flat[:H], flat[H:2 * H]), (flat[1:H + 1], flat[H + 1:])):      # on and off a 16-byte boundary
+        y, mean, rstd = native.ext().layernorm_fwd(x, None, g, b, 1e-5)[:3]
+        d = x.double()
+        mu = d.mean(-1)
+        want = torch.nn.functional.layer_norm(d, (H,), g.double(), b.double(), 1e-5)
+        r = 1.0 / torch.sqrt(d.var(-1, unbiased=False) + 1e-5)
+        assert float((mean.double() - mu).abs().max()) <= 2.0 ** -20 * offset
+        assert float(((rstd.double() - r) / r).abs().max()) <= 2.0 ** -18
+        slip = 2.0 ** -20 * offset * r[:, None] * g.double().abs()
+        assert float(((y.double() - want).abs() - 2.0 ** -8 * (want.abs() + b.double().abs()) - slip).max()) <= 0
