@@ -55,3 +55,21 @@ def test_no_row_of_the_table_occurs():
     assert torch.equal(dW, torch.ones(9, 64, device=DEV))
     with pytest.raises(RuntimeError):
         native.ext().embedding_bwd_grouped(ids[:0], None, g[:0], dW, None, 0, 0.0, 0)
+
+
+@pytest.mark.parametrize("H", [8, 264, 2040, 2048, 2056, 2560, 4104])          # one pass of 32 .. 256 threads, two, three
+@pytest.mark.parametrize("tokens", [1, 887, 889, 2500])                         # around a token for every block; further rounds
+@pytest.mark.parametrize("places", [False, True])
+def test_lookup(H, tokens, places):
+    """Ids outside [v0, v1) give no word; a sum of two bf16 values rounds once."""
+    torch.manual_seed(H + tokens)
+    V, v0 = 300, 50
+    W, P = torch.randn(V, H, device=DEV).bfloat16(), torch.randn(77, H, device=DEV).bfloat16()
+    ids = torch.randint(0, v0 + V + 40, (tokens,), device=DEV)
+    pos = torch.randint(0, 77, (tokens,), device=DEV)
+    y = native.ext().embedding_fwd(ids, pos if places else None, W, P if places else None, v0, 0.0, 1)
+    here = ((ids >= v0) & (ids < v0 + V))[:, None]
+    want = torch.where(here, W[(ids - v0).clamp(0, V - 1)].float(), torch.zeros((), device=DEV))
+    if places:
+        want = want + P[pos].float()
+    assert torch.equal(y, want.bfloat16())
