@@ -20,6 +20,7 @@ constexpr int kGroupCtas = 8, kGroupThreads = 1024;
 constexpr int kMaxTokens = 65536;                                   // bitmap of a batch: 8 KB of shared memory
 constexpr int kPerThread = kMaxTokens / (kGroupCtas * kGroupThreads);
 constexpr int kRankMax = 256;
+constexpr int kSumBlocks = 5;  // per SM: with the 63 registers the compiler likes there were four, with six it spills
 
 struct GroupTable {
   const long long* ids;
@@ -95,8 +96,9 @@ embedding_group_kernel(const GroupArgs args, int tokens) {
 }
 
 // What a block does is a chain of loads (row, its tokens, their gradients); the values that are added to are fetched in front of it,
-// four gradients at a time.  16384 tokens x 2048, V 51200, with positions: 84 -> 78 us, V 2048 52 -> 38; x 576 29 -> 23.
-__global__ void __launch_bounds__(256)
+// four gradients at a time.  16384 tokens x 2048, V 51200, with positions: 84 -> 70 us (78 with four blocks an SM, 85 with six),
+// V 2048 52 -> 35; x 576 29 -> 20.
+__global__ void __launch_bounds__(256, kSumBlocks)
 embedding_sum_kernel(const GroupArgs args, const __nv_bfloat16* __restrict__ g, int tokens, int H, float dropout_p,
                      unsigned long long seed) {
   __shared__ uint32_t bits[kMaxTokens / 32];   // kRankMax or fewer tokens: [unordered | ordered]
@@ -109,6 +111,7 @@ embedding_sum_kernel(const GroupArgs args, const __nv_bfloat16* __restrict__ g, 
   const int key = run.x, base = run.y, n = run.z, t = run.w;
   const int* list = a.list + base;
   const int nvec = H / 8;
+  const uint4* gradients = reinterpret_cast<const uint4*>(g);
   float4* out = reinterpret_cast<float4*>(a.dst + static_cast<size_t>(key) * H);
   float4 lo, hi;  // what is there already: on its way while the tokens are put in order
   if (static_cast<int>(threadIdx.x) < nvec) {
@@ -159,12 +162,13 @@ embedding_sum_kernel(const GroupArgs args, const __nv_bfloat16* __restrict__ g, 
       lo = out[2 * c];
       hi = out[2 * c + 1];
     }
-    auto add = [&](long long v, const uint4& q) {
+    auto at = [&](int token) { return static_cast<size_t>(token) * nvec + c; };
+    auto add = [&](int token, const uint4& q) {
       const float2 x0 = unpack_bf16x2(q.x), x1 = unpack_bf16x2(q.y), x2 = unpack_bf16x2(q.z), x3 = unpack_bf16x2(q.w);
       float f[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
       if (dropout_p > 0.f) {
-        const uint32_t m0 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2, keep16);
-        const uint32_t m1 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16);
+        const uint64_t v = at(token);
+        const uint32_t m0 = dropout_keep4(seed, v * 2, keep16), m1 = dropout_keep4(seed, v * 2 + 1, keep16);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           f[i] = ((m0 >> i) & 1u) ? f[i] * scale : 0.f;
@@ -175,20 +179,19 @@ embedding_sum_kernel(const GroupArgs args, const __nv_bfloat16* __restrict__ g, 
       for (int i = 0; i < 8; ++i) acc[i] += f[i];
     };
     if (n == 1) {
-      const long long v = static_cast<long long>(t) * nvec + c;
-      add(v, *reinterpret_cast<const uint4*>(g + v * 8));
+      add(t, gradients[at(t)]);
     } else {
       for (int j = 0; j < n; j += 4) {           // four rows under way at a time, added in token order
-        long long v[4];
+        int token[4];
         uint4 q[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          v[i] = static_cast<long long>(sorted[min(j + i, n - 1)]) * nvec + c;
-          if (j + i < n) q[i] = *reinterpret_cast<const uint4*>(g + v[i] * 8);
+          token[i] = sorted[min(j + i, n - 1)];
+          if (j + i < n) q[i] = gradients[at(token[i])];
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
-          if (j + i < n) add(v[i], q[i]);
+          if (j + i < n) add(token[i], q[i]);
       }
     }
     lo.x += acc[0]; lo.y += acc[1]; lo.z += acc[2]; lo.w += acc[3];
