@@ -402,7 +402,6 @@ ln_bwd_dx_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __re
   }
 }
 
-constexpr int kLnWarps = 8;        // warps that compute; one more issues the copies
 constexpr int kLnStages = 3;
 
 // Ring of stages filled by one thread; `chunk` c of this block sits in stage c % kLnStages.
@@ -427,21 +426,30 @@ struct LnRing {
 
 // One pass over dy, x and dres for any H <= 512 * WPR: dx, and in the same sweep every lane keeps running sums of
 // dy * xhat and dy for its 16 columns over all rows its warp visits (their gamma stays in registers).  A chunk is
-// 8 / WPR consecutive rows of the three matrices; WPR warps share a row (each owns 512 columns) and exchange their two
+// NW / WPR consecutive rows of the three matrices; WPR warps share a row (each owns 512 columns) and exchange their two
 // row sums through shared memory.  The warps of a block fold their column sums through shared memory in a fixed order
 // and the block writes ONE row of partials (part_g[block][h], part_b[block][h]); fold_partials2_kernel adds the blocks.
-// The result does not depend on the order of execution.  32768 x 2048 with residual gradient, this kernel and the fold:
-// 134 -> 107 us (register-staged form, H 1024 and 2048 only; other H took two kernels that read dy and x twice: 32768 x 1536
-// 173 -> 81, 512 x 768 11.5 -> 5.9).  The same ring under the forward of that time changed nothing (68 us).
-template <int WPR>
-__global__ void __launch_bounds__((kLnWarps + 1) * 32, 2)
+// The result does not depend on the order of execution.  dy and x are kept packed over the warps' meeting and unpacked again behind it:
+// fewer registers, less spilled.  What bounds it is the chain of a chunk (copies, sums, meeting, stores), two blocks an SM; more
+// stages, more and smaller blocks, or two rows of a warp at a time are slower.  Three warps a row up to 1536 columns, where four
+// were idle in part.  32768 rows with residual gradient, this kernel and the fold, before -> now: x 2048 100 -> 93 us, x 1536 87 -> 68,
+// x 1152 82 -> 65, x 1024 55 -> 50, x 512 33 -> 29 (a copy of two such matrices: 84, 65, 50, 45, 24).
+// NW warps compute, WPR of them on a row; one more issues the copies.  Two blocks an SM.
+template <int WPR_, int NW_>
+struct LnBwd {
+  static constexpr int WPR = WPR_, NW = NW_, kRows = NW / WPR, kThreads = (NW + 1) * 32;  // kRows: of a chunk
+  static constexpr bool kStatsAhead = WPR <= 3;
+};
+template <class Cfg>
+__global__ void __launch_bounds__(Cfg::kThreads, 2)
 ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                      const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ part_g, float* __restrict__ part_b, int rows, int H, int* __restrict__ status) {
-  constexpr int VPL = 2, RPB = kLnWarps / WPR;       // vectors per lane, rows of a chunk
+  constexpr int WPR = Cfg::WPR, NW = Cfg::NW, RPB = Cfg::kRows;
+  constexpr int VPL = 2;       // vectors per lane
   extern __shared__ __align__(128) uint8_t ring_smem[];
-  __shared__ float xch[2][RPB][WPR][2];
+  __shared__ float2 xch[2][RPB][WPR];
   __shared__ uint64_t bars[2 * kLnStages];
   __shared__ int aborted;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -450,7 +458,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kLnStages; ++i) {
       mbar_init(&bars[i], 1);
-      mbar_init(&bars[kLnStages + i], kLnWarps);
+      mbar_init(&bars[kLnStages + i], NW);
     }
     aborted = 0;
     fence_mbar_init();
@@ -459,7 +467,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   const LnRing ring{bars, bars + kLnStages, &aborted};
   float ag[VPL][8], ab[VPL][8];
   const int rslot = warp / WPR, part = warp % WPR;
-  if (warp == kLnWarps) {
+  if (warp == NW) {
     int c = 0;
     for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
       if (!ring.wait_empty(c)) break;
@@ -492,7 +500,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         ag[i][j] = ab[i][j] = 0.f;
       }
     }
-    // The warps of a row meet once per row.  One whose bounded wait ran out at chunk `ch` still comes to the meetings ahead: the
+    // The warps of a row meet once per chunk.  One whose bounded wait ran out at chunk `ch` still comes to the meetings ahead: the
     // others may pass the same wait a moment later and must not be left waiting.
     auto meet = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + rslot), "r"(32 * WPR) : "memory"); };
     auto meet_to_the_end = [&](int ch) {
@@ -500,66 +508,65 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         for (; ch * RPB + rslot < rows; ch += gridDim.x) meet();
     };
     int c = 0;
-    // Statistics of the row: with many rows in a chunk loaded a chunk ahead, like the rows themselves (32768 x 512 33.0 -> 29.8 us,
-    // x 1024 55.4 -> 53.4; four warps a row 100.6 -> 102.5).
-    constexpr bool kStatsAhead = WPR <= 2;
+    // Statistics of the row: loaded a chunk ahead, like the row itself (32768 x 512 33.0 -> 29.8 us, x 1024 55.4 -> 53.4, x 1536 72.8 ->
+    // 67.7; with four warps a row 93.0 -> 96.3).
     float mu_next = 0.f, rs_next = 0.f;
     auto fetch_stats = [&](int ch) {
       const int row = ch * RPB + rslot;
-      if (ch < chunks && row < rows) {
-        mu_next = __ldg(mean + row);
-        rs_next = __ldg(rstd + row);
-      }
+      const bool have = ch < chunks && row < rows;
+      mu_next = have ? __ldg(mean + row) : 0.f;
+      rs_next = have ? __ldg(rstd + row) : 0.f;
     };
-    if (kStatsAhead) fetch_stats(blockIdx.x);
+    if (Cfg::kStatsAhead) fetch_stats(blockIdx.x);
     for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
-      const int row = ch * RPB + rslot;
-      const bool have = row < rows;                  // the same for all warps of a row slot
-      if (!kStatsAhead) fetch_stats(ch);
+      const int row = ch * RPB + rslot;              // the same for all warps of a row slot
+      if (!Cfg::kStatsAhead) fetch_stats(ch);
       const float mu = mu_next, rs = rs_next;
-      if (kStatsAhead) fetch_stats(ch + gridDim.x);
+      if (Cfg::kStatsAhead) fetch_stats(ch + gridDim.x);
       if (!ring.wait_full(c)) {
         meet_to_the_end(ch);
         break;
       }
-      if (have) {
+      if (row < rows) {
         const uint8_t* base = ring_smem + (c % kLnStages) * stage_bytes + rslot * row_bytes;
         const uint4* pd = reinterpret_cast<const uint4*>(base);
         const uint4* px = reinterpret_cast<const uint4*>(base + part_bytes);
         const uint4* pr = reinterpret_cast<const uint4*>(base + 2 * part_bytes);
-        float d[VPL][8], xh[VPL][8], s1 = 0.f, s2 = 0.f;
+        uint4 qd[VPL], qx[VPL];
+        float s1 = 0.f, s2 = 0.f;
 #pragma unroll
         for (int i = 0; i < VPL; ++i) {
           const int v = (part * VPL + i) * 32 + lane;
           const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-          float xv[8];
-          unpack8(v < nvec ? pd[v] : zero, d[i]);
-          unpack8(v < nvec ? px[v] : zero, xv);
+          float d[8], xv[8];
+          qd[i] = v < nvec ? pd[v] : zero;
+          qx[i] = v < nvec ? px[v] : zero;
+          unpack8(qd[i], d);
+          unpack8(qx[i], xv);
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
-            xh[i][j] = (xv[j] - mu) * rs;
-            const float dg = d[i][j] * g[i][j];
+            const float xh = (xv[j] - mu) * rs, dg = d[j] * g[i][j];
             s1 += dg;
-            s2 += dg * xh[i][j];
-            ag[i][j] += d[i][j] * xh[i][j];
-            ab[i][j] += d[i][j];
+            s2 += dg * xh;
+            ag[i][j] += d[j] * xh;
+            ab[i][j] += d[j];
           }
         }
-        s1 = warp_sum(s1);
-        s2 = warp_sum(s2);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+          s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        }
         if constexpr (WPR > 1) {
-          float* slot = &xch[c & 1][rslot][0][0];
-          if (lane == 0) {
-            slot[part * 2] = s1;
-            slot[part * 2 + 1] = s2;
-          }
+          float2(&slot)[WPR] = xch[c & 1][rslot];
+          if (lane == 0) slot[part] = make_float2(s1, s2);
           meet();
-          s1 = 0.f;
-          s2 = 0.f;
+          s1 = s2 = 0.f;
 #pragma unroll
           for (int w = 0; w < WPR; ++w) {
-            s1 += slot[w * 2];
-            s2 += slot[w * 2 + 1];
+            const float2 e = slot[w];
+            s1 += e.x;
+            s2 += e.y;
           }
         }
         s1 *= inv_h;
@@ -569,19 +576,21 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
         for (int i = 0; i < VPL; ++i) {
           const int v = (part * VPL + i) * 32 + lane;
           if (v >= nvec) break;
-          float o[8];
+          float d[8], xv[8], o[8];
+          unpack8(qd[i], d);
+          unpack8(qx[i], xv);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = rs * (d[i][j] * g[i][j] - s1 - xh[i][j] * s2);
-          if (dres) {
-            float r[8];
-            unpack8(pr[v], r);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += r[j];
+          for (int j = 0; j < 8; ++j) {
+            const float xh = (xv[j] - mu) * rs;
+            o[j] = rs * (d[j] * g[i][j] - s1 - xh * s2);
           }
-          uint4 w;
-          w.x = pack_bf16x2(o[0], o[1]); w.y = pack_bf16x2(o[2], o[3]);
-          w.z = pack_bf16x2(o[4], o[5]); w.w = pack_bf16x2(o[6], o[7]);
-          dxr[v] = w;
+          if (dres) {
+            float t[8];
+            unpack8(pr[v], t);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += t[j];
+          }
+          dxr[v] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
         }
       }
       ring.release(c, lane);
@@ -591,7 +600,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   // Every copy has landed and been read: the ring takes the sums of the row slots, [2][RPB][H], which are then added in the order
   // 0, 1, ...  (One slot after the other into one row of sums took eight rounds at one warp per row: 16 x 512 9.5 us instead of 5.5.)
   float* slots = reinterpret_cast<float*>(ring_smem);
-  if (warp < kLnWarps) {
+  if (warp < NW) {
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       const int v = (part * VPL + i) * 32 + lane;
@@ -804,7 +813,7 @@ colsum_partial_kernel(const __nv_bfloat16* __restrict__ a, int lda, float* __res
 
 }  // namespace
 
-constexpr int kLnStreamMaxH = 512 * kLnWarps;
+constexpr int kLnStreamMaxH = 4096;
 
 static bool misaligned(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) != 0; }
 
@@ -861,15 +870,24 @@ int ln_bwd_slices(int rows) {
   return s < 1 ? 1 : (s > 128 ? 128 : s);
 }
 
-static int ln_bwd_warps_per_row(int H) { return H <= 512 ? 1 : H <= 1024 ? 2 : H <= 2048 ? 4 : 8; }
+// Calls fn with the form of the one-pass backward for rows of H.
+template <class Fn>
+static auto ln_bwd_form(int H, Fn fn) {
+  if (H <= 512) return fn(LnBwd<1, 8>{});
+  if (H <= 1024) return fn(LnBwd<2, 8>{});
+  if (H <= 1536) return fn(LnBwd<3, 6>{});
+  if (H <= 2048) return fn(LnBwd<4, 8>{});
+  return fn(LnBwd<8, 8>{});
+}
 
 // Rows of partial sums the backward needs in each of part_g / part_b (then H floats per row).
 int ln_bwd_part_rows(int rows, int H, int num_sms) {
-  if (H <= kLnStreamMaxH) {  // one-pass kernel: one row of partials per block, two resident blocks per SM
-    const int rpb = kLnWarps / ln_bwd_warps_per_row(H);
-    const int want = (rows + rpb - 1) / rpb;
-    return want < num_sms * 2 ? want : num_sms * 2;
-  }
+  if (H <= kLnStreamMaxH)  // one-pass kernel: one row of partials per block
+    return ln_bwd_form(H, [&](auto cfg) {
+      using Cfg = decltype(cfg);
+      const int want = (rows + Cfg::kRows - 1) / Cfg::kRows;
+      return want < num_sms * 2 ? want : num_sms * 2;
+    });
   return ln_bwd_slices(rows);
 }
 
@@ -884,20 +902,16 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   if (misaligned(dy) || misaligned(x) || misaligned(dres) || misaligned(dx)) return -3;  // every kernel moves 16 bytes a lane
   if (H <= kLnStreamMaxH) {
     // dy and x are read once: dx and the per-column sums come out of the same sweep
-    const int nb = ln_bwd_part_rows(rows, H, num_sms), wpr = ln_bwd_warps_per_row(H);
-    const int smem = kLnStages * 3 * (kLnWarps / wpr) * H * 2;
-    int rc = 0;
-#define SSB_LN_BWD(W)                                                                                                        \
-  rc = static_cast<int>(cudaFuncSetAttribute(ln_bwd_stream_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));    \
-  if (rc) return rc;                                                                                                         \
-  ln_bwd_stream_kernel<W><<<nb, (kLnWarps + 1) * 32, smem, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, part_g, part_b, rows, H, status)
-    switch (wpr) {
-      case 1: SSB_LN_BWD(1); break;
-      case 2: SSB_LN_BWD(2); break;
-      case 4: SSB_LN_BWD(4); break;
-      default: SSB_LN_BWD(8); break;
-    }
-#undef SSB_LN_BWD
+    const int nb = ln_bwd_part_rows(rows, H, num_sms);
+    const int rc = ln_bwd_form(H, [&](auto cfg) {
+      using Cfg = decltype(cfg);
+      const int smem = kLnStages * 3 * Cfg::kRows * H * 2;
+      const int e = static_cast<int>(cudaFuncSetAttribute(ln_bwd_stream_kernel<Cfg>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (e == 0)
+        ln_bwd_stream_kernel<Cfg><<<nb, Cfg::kThreads, smem, stream>>>(dyb, xb, gamma, mean, rstd, drb, dxb, part_g, part_b, rows, H, status);
+      return e;
+    });
+    if (rc) return rc;
     fold_partials2(part_g, part_b, dgamma, dbeta, nb, H, accumulate_wgrad, stream);
     return static_cast<int>(cudaGetLastError());
   }

@@ -251,3 +251,20 @@ def test_cross_entropy_keeps_probabilities_below_the_normal_range(V):
     work[torch.arange(rows, device="cuda"), t] = 0.0
     off = (work[:, :V].double() - grad).abs() - 2.0 ** -8 * grad
     assert float(off.max()) <= 0.0
+
+
+@pytest.mark.parametrize("rows,H", [(1, 1032), (7, 1536), (1777, 1288), (2500, 1536), (1200, 1544), (2401, 1800)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_layernorm_backward_with_three_and_four_warps_a_row(rows, H, residual):
+    torch.manual_seed(rows + H)
+    x, dy = (torch.randn(rows, H, device="cuda") * 2 + 1).bfloat16(), torch.randn(rows, H, device="cuda").bfloat16()
+    g, b = torch.randn(H, device="cuda"), torch.randn(H, device="cuda")
+    dres = torch.randn(rows, H, device="cuda").bfloat16() if residual else None
+    _, mean, rstd = native.ext().layernorm_fwd(x, None, g, b, 1e-5)[:3]
+    dg, db = torch.ones(H, device="cuda"), torch.ones(H, device="cuda")
+    dx = native.ext().layernorm_bwd(dy, x, g, mean, rstd, dres, dg, db, True)
+    t = [v.double().requires_grad_(True) for v in (x, g, b)]
+    want = torch.autograd.grad(torch.nn.functional.layer_norm(t[0], (H,), t[1], t[2], 1e-5), t, dy.double())
+    assert _rel(dx, want[0] + (dres.double() if residual else 0)) < 2.0 ** -8       # one rounding to bf16
+    assert _rel(dg - 1, want[1]) < 1e-5 and _rel(db - 1, want[2]) < 1e-5            # fp32 sums
+    assert native.check_status() == 0
