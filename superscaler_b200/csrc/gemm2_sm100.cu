@@ -182,9 +182,9 @@ __device__ __forceinline__ TileCoord2 tile_coord2(int tile, int num_m, int num_n
 template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
 __global__ void __launch_bounds__(GATHER ? kThreadsGather : kThreads2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a2,
-                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv) {
+                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv, const int bn) {
   constexpr int kStages2 = NH == 2 ? kStagesWide : GATHER ? kStagesGather : kStagesPlain;
-  constexpr int BNT = NH * BN2;                     // columns of a tile
+  const int BNT = NH == 2 ? 2 * BN2 : bn;           // columns of a tile
   constexpr int kStageAll = kABytes2 + NH * kBBytes2;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -253,7 +253,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
         const TileCoord2 tc = tile_coord2(tile, num_m, num_n);
         int m0 = pblk_of(tc.m_blk) * 2 * BM2 + static_cast<int>(cta_rank) * BM2;
-        const int n0 = tc.n_blk * BNT + static_cast<int>(cta_rank) * BNH;
+        const int n0 = tc.n_blk * BNT + static_cast<int>(cta_rank) * (bn / 2);
         const CUtensorMap* ta = &tma_a;
         if (GATHER) {
           if (src_of(tc.m_blk) == cm.rank) {
@@ -290,7 +290,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             ok = false;
             break;
           }
-          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * kStageAll);
+          if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * (B_MN ? kStageAll : kABytes2 + NH * (bn / 2) * (BK2 * 2)));
           const uint32_t bar = mapa_smem(smem_u32(&full_bar[stage]), 0);
           uint8_t* sa = smem_a + stage * kABytes2;
           uint8_t* sb = smem_b + stage * (NH * kBBytes2);
@@ -347,7 +347,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   } else if (warp == 1) {
     // ------------------------------- MMA issuer -------------------------------
     if (leader && elect_one()) {
-      constexpr uint32_t idesc = umma_idesc_bf16(2 * BM2, BN2, A_MN, B_MN);
+      const uint32_t idesc = umma_idesc_bf16(2 * BM2, bn, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;
       int iter = 0;
@@ -441,6 +441,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         const int acc = NH == 2 ? h : iter & 1;
         const uint32_t acc_phase = (NH == 2 ? iter : iter >> 1) & 1;
         const int col0 = tc.n_blk * BNT + h * BN2 + grp * 64;  // first column
+        const int col_end = min(p.N, tc.n_blk * BNT + h * BN2 + bn);
         const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * BN2 + grp * 64;
         auto release = [&]() {  // the accumulator columns are free
           tc_fence_before_sync();
@@ -451,7 +452,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         // Row operands enter and results leave through a swizzled staging tile, so every global access of the warp is four
         // full 128-byte row segments (wide tile: eight of 64 bytes) instead of 32 scattered 32-byte pieces.
         const bool has_operand = p.residual != nullptr || p.act == kActDGelu || p.act == kActDRelu;
-        const bool staged = !p.out_fp32 && !p.accumulate && col0 + 64 <= p.N &&
+        const bool staged = !p.out_fp32 && !p.accumulate && col0 + 64 <= col_end &&
                             !(p.residual != nullptr && (p.act == kActDGelu || p.act == kActDRelu)) &&
                             !(p.preact_out != nullptr && has_operand);
         if (staged) {
@@ -532,7 +533,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         // in turn; with a reduction of 4096 that took longer than the main loop of the next tile.  Alone / sustained under the
         // power cap: weight gradients 51200 x 2048 over 4096 rows 649 -> 600 / 805 -> 754 us, 8192 x 2048 over 8192 216 -> 209 /
         // 255 -> 248.
-        if (p.out_fp32 && col0 + 64 <= p.N && !has_operand && p.preact_out == nullptr) {
+        if (p.out_fp32 && col0 + 64 <= col_end && !has_operand && p.preact_out == nullptr) {
           const int srow = lane >> 2, spiece = lane & 3;
           float* out = reinterpret_cast<float*>(p.D) + static_cast<size_t>(row0 + srow) * p.ldd + col0 + spiece * 4;
           auto cell = [&](int rr, int piece) { return stg + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4); };
@@ -586,7 +587,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 #pragma unroll 1
         for (int c = 0; c < 4; ++c) {
           const int n0 = col0 + c * 16;
-          if (n0 >= p.N) break;  // uniform across the warp
+          if (n0 >= col_end) break;  // uniform across the warp
           uint32_t r[16];
           tmem_ld_32x16(taddr + c * 16, r);
           tmem_ld_wait();
@@ -670,7 +671,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
 template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
 int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap& tb, const GemmParams& p,
-                const GemmAgComm& cm, const ConvLoad& cv, int num_sms, cudaStream_t stream) {
+                const GemmAgComm& cm, const ConvLoad& cv, int bn, int num_sms, cudaStream_t stream) {
   auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV, NH>;
   constexpr int threads = GATHER ? kThreadsGather : kThreads2;
   cudaLaunchAttribute attr[1];
@@ -696,7 +697,7 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
     }
     max_clusters = n;
   }
-  const int num_tiles = ((p.M + 2 * BM2 - 1) / (2 * BM2)) * ((p.N + NH * BN2 - 1) / (NH * BN2));
+  const int num_tiles = ((p.M + 2 * BM2 - 1) / (2 * BM2)) * ((p.N + NH * bn - 1) / (NH * bn));
   int clusters = num_sms / 2;
   if (clusters > max_clusters) clusters = max_clusters;
   if (clusters > num_tiles) clusters = num_tiles;
@@ -707,7 +708,7 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, ta2, tb, p, cm, cv));
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, ta, ta2, tb, p, cm, cv, bn));
 }
 
 // The tile of 256 x 512 takes a product with a long reduction, where its end (the next tile waits for the epilogue) weighs little,
@@ -720,6 +721,18 @@ bool wide_tile(int M, int N, int K, bool out_fp32, int num_sms) {
   const long long m = (M + 255LL) / 256, narrow = m * ((N + 255LL) / 256), wide = m * ((N + 511LL) / 512);
   const int pairs = num_sms / 2;
   return N >= 512 && K >= (out_fp32 ? kWideKFp32 : kWideK) && 2 * ((wide + pairs - 1) / pairs) <= (narrow + pairs - 1) / pairs;
+}
+
+// Columns of a tile, in steps of the 32 that a pair's instruction takes: fewer than 256 where the rounds of narrower tiles are shorter
+// by a tenth at least (a narrower tile moves more per operation).  640 output channels in three tiles: a sixth of 256-column tiles
+// is padding.  16 x 28 x 28 of 640 channels, 3 x 3, with 256 -> 224 columns: forward 67.6 -> 62.0 us, input gradient 68.5 -> 64.4.
+int tile_columns(int M, int N, int num_sms) {
+  const int pairs = num_sms / 2;
+  auto time = [&](int bn) { return ((M + 255LL) / 256 * ((N + bn - 1) / bn) + pairs - 1) / pairs * bn; };
+  int best = BN2;
+  for (int bn = BN2 - 32; bn >= 160; bn -= 32)
+    if (10 * time(bn) <= 9 * time(BN2) && time(bn) < time(best)) best = bn;
+  return best;
 }
 
 template <bool A_MN, bool B_MN, bool GATHER>
@@ -736,17 +749,21 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
     ta2 = ta;
   }
   if (rc != 0) return rc;
-  rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, BNH, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
+  const bool wide = !GATHER && wide_tile(p.M, p.N, p.K, p.out_fp32, num_sms);
+  const int bn = GATHER || wide ? BN2 : tile_columns(p.M, p.N, num_sms);
+  rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, bn / 2, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
   if (rc != 0) return rc;
   if constexpr (!GATHER)
-    if (wide_tile(p.M, p.N, p.K, p.out_fp32, num_sms)) return launch_maps<A_MN, B_MN, false, kConvNone, 2>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
-  return launch_maps<A_MN, B_MN, GATHER, kConvNone, 1>(ta, ta2, tb, p, cm, ConvLoad{}, num_sms, stream);
+    if (wide) return launch_maps<A_MN, B_MN, false, kConvNone, 2>(ta, ta2, tb, p, cm, ConvLoad{}, bn, num_sms, stream);
+  return launch_maps<A_MN, B_MN, GATHER, kConvNone, 1>(ta, ta2, tb, p, cm, ConvLoad{}, bn, num_sms, stream);
 }
 
 }  // namespace
 
-// Columns of the output tile for a product that this kernel takes: 256 or 512.
-int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms) { return wide_tile(M, N, K, out_fp32, num_sms) ? 512 : 256; }
+// Columns of the output tile for a product that this kernel takes.
+int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms) {
+  return wide_tile(M, N, K, out_fp32, num_sms) ? 2 * BN2 : tile_columns(M, N, num_sms);
+}
 
 // Same contract as gemm_bf16_launch; callers pick this variant for outputs of at least 256 x 256.
 int gemm2_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
@@ -782,9 +799,10 @@ int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, 
   CUtensorMap ta, tb;
   int rc;
   if ((rc = make_tma_im2col_bf16(&ta, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BM2))) return rc;
-  if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, BNH, BK2))) return rc;
+  const int bn = tile_columns(p.M, p.N, num_sms);
+  if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, bn / 2, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<false, false, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<false, false, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
 }
 
 // dx[N, H, W, C] of a stride-1 convolution from dy[N, Ho, Wo, K]; p describes the GEMM [N H W, C] with K = KH * KW * K.
@@ -797,7 +815,7 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
   if ((rc = make_tma_im2col_bf16(&ta, dy, N, Ho, Wo, Kout, lh, lw, -pad, -pad, 1, BM2))) return rc;
   if ((rc = make_tma_2d_bf16(&tb, w, Kout, static_cast<uint64_t>(KH) * KW * C, ldw, BK2, 64))) return rc;
   ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
-  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, tile_columns(p.M, p.N, num_sms), num_sms, stream);
 }
 
 // dw[K, KH * KW * C] from dy[N Ho Wo, K] and x; p describes the GEMM [K, KH * KW * C] with K = N Ho Wo.
@@ -808,7 +826,7 @@ int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int
   if ((rc = make_tma_2d_bf16(&ta, dy, p.K, p.M, lddy, BK2, 64))) return rc;
   if ((rc = make_tma_im2col_bf16(&tb, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<true, true, false, kConvB, 1>(ta, ta, tb, p, GemmAgComm{}, cv, num_sms, stream);
+  return launch_maps<true, true, false, kConvB, 1>(ta, ta, tb, p, GemmAgComm{}, cv, BN2, num_sms, stream);
 }
 
 }  // namespace ssb

@@ -98,3 +98,26 @@ def test_wide_tile_epilogues(M, N, K, kind):
     assert native.check_status() == 0
     for one, pair in zip(*results):
         assert torch.equal(one, pair)
+
+
+# Tiles of 224, 192 and 160 columns, whose last 64 columns are 32 (or none): N at and around the ends of tiles.
+NARROW = [(12544, 640, 200, 224), (12541, 645, 136, 224), (9472, 384, 192, 192), (9470, 381, 72, 192), (9472, 320, 64, 160),
+          (9400, 317, 200, 160)]
+
+
+@pytest.mark.parametrize("M,N,K,columns", NARROW)
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("fp32", [False, True])
+def test_narrow_tiles(M, N, K, columns, a_mn, b_mn, fp32):
+    assert native.ext().gemm_pair_columns(M, N, K, fp32, 148) == columns
+    if a_mn:
+        M = M // 8 * 8
+    a, b, want, bound = operands(M, N, K, a_mn, b_mn)
+    d, whole = padded(M, N, torch.float32 if fp32 else torch.bfloat16)
+    if fp32:
+        want = want + d.double()
+    bias = torch.randn(N, device=DEV).bfloat16() if not fp32 else None
+    if bias is not None:
+        want = want + bias.double()
+    F.gemm(a, b, out=d, a_mn=a_mn, b_mn=b_mn, bias=bias, accumulate=fp32)
+    check(d, whole, want, bound + (2.0 ** -22 if fp32 else 2.0 ** -8) * (want.abs() + 4))
