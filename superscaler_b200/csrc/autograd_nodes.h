@@ -1,12 +1,13 @@
-// The differentiable ops of a transformer layer as native autograd nodes: LayerNorm, linear (+ activation, dropout, residual),
-// MLP and flash attention.  Included by bindings.cpp behind the wrappers it calls; the same kernels in the same order as the
+// The differentiable ops of a transformer as native autograd nodes: LayerNorm, linear (+ activation, dropout, residual), MLP, flash
+// attention, the embedding lookup and the head with its loss.  Included by bindings.cpp behind the wrappers it calls; the same kernels in the same order as the
 // autograd functions of ops/functional.py, which stay the path of CPU tensors and of traced or transformed calls.
 //
 // Why: a layer of a small model spends more time on the host than on the GPU.  A Python autograd function costs 20 to 40 us a
 // call in either direction (argument checks, context, a kernel call each through the interpreter, which the backward thread
 // has to share with the main thread); a node costs the kernels' launches and allocations.  Back to back on the host: scoring one
 // prompt of 512 tokens with four layers 779 -> 456 us, a step of a two-layer model with two micro-batches 3387 -> 2797, forward
-// and backward of one attention call 112 -> 85.
+// and backward of one attention call 112 -> 85; with the lookup and the head as nodes too the step 2501 -> 2195 and the scoring
+// 433 -> 400.
 //
 // (Included inside the anonymous namespace of bindings.cpp, so it includes nothing itself.)
 #pragma once
@@ -110,6 +111,9 @@ struct NodeArgs : torch::CustomClassHolder {
   int64_t B = 0, NH = 0, SQ = 0, SK = 0, HD = 0, qc = 0, kc = 0, vc = 0;
   double scale = 1.0;
   bool causal = false;
+  // embedding: the tables, whose gradients need their sizes and gradient buffers; not saved tensors, which may not change in place
+  Tensor table, places;
+  int64_t v0 = 0;
 };
 using NodeArgsPtr = c10::intrusive_ptr<NodeArgs>;
 void keep_args(AutogradContext* ctx, const NodeArgsPtr& a) { ctx->saved_data["args"] = c10::IValue::make_capsule(a); }
@@ -295,4 +299,101 @@ Tensor attention_node(const Tensor& q, const Tensor& k, const Tensor& v, int64_t
   a->same_kv = k.data_ptr() == v.data_ptr() && k.sizes() == v.sizes();
   a->same_qkv = a->same_kv && q.data_ptr() == k.data_ptr() && q.sizes() == k.sizes();
   return AttentionNode::apply(q, k, v, kv_lens, table, a);
+}
+
+// Which kernel sums the embedding gradient (see set_deterministic_embedding_grad of ops/functional.py): rows in token order, or
+// float atomics.  Read by the threads that run a backward.
+std::atomic<bool> g_embedding_in_order{[] {
+  const char* atomics = std::getenv("SSB_EMBEDDING_GRAD_ATOMICS");
+  return atomics == nullptr || std::string(atomics) != "1";
+}()};
+
+struct EmbeddingNode : torch::autograd::Function<EmbeddingNode> {
+  // The tables are passed for the graph alone; the values come with the arguments.
+  static Tensor forward(AutogradContext* ctx, const Tensor& ids, const OptTensor& pos, const Tensor& W, const OptTensor& P,
+                        const NodeArgsPtr& a) {
+    Tensor flat_pos;
+    if (pos.has_value()) flat_pos = pos->contiguous().view(-1);
+    Tensor y = embedding_fwd(ids.contiguous().view(-1), some(flat_pos), W, P, a->v0, a->dropout_p, a->seed);
+    count_kernels(1);
+    ctx->save_for_backward({ids, pos.has_value() ? *pos : Tensor()});
+    keep_args(ctx, a);
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const auto saved = ctx->get_saved_variables();
+    const NodeArgsPtr a = args_of(ctx);
+    const Tensor g = grads[0].contiguous(), ids = saved[0].contiguous().view(-1);
+    Tensor pos;
+    if (saved[1].defined()) pos = saved[1].contiguous().view(-1);
+    const auto pg = param_grads({&a->w, &a->b});
+    auto buffer = [&](const ParamGrad& p, const Tensor& t) {
+      return p.main.has_value() ? *p.main : torch::zeros(t.sizes(), g.options().dtype(torch::kFloat32));
+    };
+    Tensor dW = buffer(pg[0], a->table), dP;
+    if (a->places.defined()) dP = buffer(pg[1], a->places);
+    if (!g_embedding_in_order) {
+      embedding_bwd(ids, some(pos), g, dW, some(dP), a->v0, a->dropout_p, a->seed);
+      count_kernels(1);
+    } else if (ids.numel() <= ssb::embedding_group_max_tokens()) {
+      embedding_bwd_grouped(ids, some(pos), g, dW, some(dP), a->v0, a->dropout_p, a->seed);
+      count_kernels(2);
+    } else {
+      auto sorted = [&](const Tensor& keys_of, const Tensor& dst, int64_t k0) {
+        const auto order = torch::sort(embedding_keys(keys_of, k0, dst.size(0)), /*stable=*/true, 0, false);
+        count_kernels(1);
+        embedding_bwd_sorted(std::get<0>(order), std::get<1>(order), g, dst, 0, a->dropout_p, a->seed);
+      };
+      sorted(ids, dW, a->v0);
+      if (pos.defined() && dP.defined()) sorted(pos, dP, 0);
+    }
+    return {Tensor(), Tensor(), pg[0].main.has_value() ? Tensor() : dW.to(a->table.scalar_type()),
+            !dP.defined() || pg[1].main.has_value() ? Tensor() : dP.to(a->places.scalar_type()), Tensor()};
+  }
+};
+
+Tensor embedding_node(const Tensor& ids, const OptTensor& pos, const Tensor& W, const OptTensor& P, int64_t v0, double dropout_p,
+                      int64_t seed) {
+  auto a = c10::make_intrusive<NodeArgs>();
+  a->v0 = v0;
+  a->dropout_p = dropout_p;
+  a->seed = seed;
+  a->table = W;
+  a->w = param_ref(W);
+  if (P.has_value()) {
+    a->places = *P;
+    a->b = param_ref(P);
+  }
+  return EmbeddingNode::apply(ids, pos, W, P, a);
+}
+
+struct HeadLossNode : torch::autograd::Function<HeadLossNode> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& W, const Tensor& targets, const OptTensor& mask,
+                        const NodeArgsPtr& a) {
+    Tensor logits = node_gemm(x, W, Tensor(), false, false, kNone, 0, kNone, kNone, kNone, false, 0.0, 0);
+    const Tensor losses = ce_loss_grad(logits, targets.contiguous().view(-1), mask, a->v0, a->scale);
+    count_kernels(1);
+    ctx->save_for_backward({x, W, logits});
+    keep_args(ctx, a);
+    return losses.sum() * a->scale;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list) {
+    const auto saved = ctx->get_saved_variables();
+    const Tensor &x = saved[0], &W = saved[1], &g = saved[2];
+    const NodeArgsPtr a = args_of(ctx);
+    Tensor dx, dw;
+    if (a->want_x) dx = node_gemm(g, W, Tensor(), false, true, kNone, 0, kNone, kNone, kNone, false, 0.0, 0);
+    if (a->want_w) dw = node_wgrad(param_grads({&a->w})[0], g, x);
+    return {dx, dw, Tensor(), Tensor(), Tensor()};
+  }
+};
+
+Tensor head_loss_node(const Tensor& x, const Tensor& W, const Tensor& targets, const OptTensor& mask, int64_t v0, double loss_scale) {
+  auto a = c10::make_intrusive<NodeArgs>();
+  a->v0 = v0;
+  a->scale = loss_scale;
+  a->want_x = x.requires_grad();
+  a->want_w = W.requires_grad();
+  a->w = param_ref(W);
+  return HeadLossNode::apply(x, W, targets, mask, a);
 }

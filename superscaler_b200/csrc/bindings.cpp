@@ -10,6 +10,8 @@
 
 #include <array>
 #include <atomic>
+#include <cstdlib>
+#include <string>
 
 #include "attention_sm100.cuh"
 #include "gemm_sm100.cuh"
@@ -1005,6 +1007,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("mlp_node", &mlp_node);
   m.def("layernorm_node", &layernorm_node);
   m.def("attention_node", &attention_node);
+  m.def("embedding_node", &embedding_node);
+  m.def("head_loss_node", &head_loss_node);
+  m.def("set_embedding_in_order", [](bool on) { g_embedding_in_order = on; });
   m.def("node_kernels", []() { return g_node_kernels.load(); });
   m.def("node_calls", []() { return g_node_calls.load(); });
   m.def("attn_bwd", &attn_bwd);

@@ -774,6 +774,8 @@ def set_deterministic_embedding_grad(on: bool) -> None:
     row (sorted above 65536 tokens; independent of the order of execution, the default), or float atomics (order dependent
     in the last bit)."""
     _DETERMINISTIC_EMBEDDING_GRAD[0] = bool(on)
+    if native.available():
+        native.ext().set_embedding_in_order(bool(on))
 
 
 def set_deterministic(on: bool) -> None:
@@ -787,6 +789,8 @@ def set_deterministic(on: bool) -> None:
 
 
 def embedding(ids, pos, W, P=None, v0=0, dropout_p=0.0, seed=0):
+    if _native_node(W):
+        return native.ext().embedding_node(ids, pos, W, P, v0, dropout_p, seed)
     return EmbeddingFn.apply(ids, pos, W, P, v0, dropout_p, seed)
 
 
@@ -848,6 +852,8 @@ class LMHeadCrossEntropyFn(torch.autograd.Function):
 
 
 def lm_head_cross_entropy(x, W, targets, loss_mask=None, v0=0, loss_scale=1.0, group=None):
+    if _native_node(x) and (group is None or torch.distributed.get_world_size(group) == 1):
+        return native.ext().head_loss_node(x, W, targets, loss_mask, v0, float(loss_scale))
     return LMHeadCrossEntropyFn.apply(x, W, targets, loss_mask, v0, float(loss_scale), group)
 
 

@@ -1,4 +1,4 @@
-"""The native autograd nodes of linear, MLP, LayerNorm and attention (csrc/autograd_nodes.h)."""
+"""The native autograd nodes of linear, MLP, LayerNorm, attention, embedding and the head with its loss (csrc/autograd_nodes.h)."""
 import subprocess
 import sys
 import warnings
@@ -145,7 +145,29 @@ def _attention(form, causal, lens, p, table):
     return t, (), lambda t: F.flash_attention(*operands(t), *tail(t)), lambda t: F.FlashAttnFn.apply(*operands(t), *tail(t))
 
 
+def _embedding(places, v0, p):
+    ids = torch.randint(v0 - 4, v0 + 54, (5, 24), device=DEV)           # some outside the table
+    pos = torch.arange(24, device=DEV).repeat(5)
+    t = {"W": _bf(50, 264)}
+    if places:
+        t["P"] = _bf(24, 264)
+    args = lambda t: (ids, pos if places else None, t["W"], t.get("P"), v0, p, 7)
+    return t, ("W", "P"), lambda t: F.embedding(*args(t)), lambda t: F.EmbeddingFn.apply(*args(t))
+
+
+def _head(mask, v0):
+    t = {"x": _bf(136, 192), "W": _bf(264, 192, scale=0.1)}
+    targets = torch.randint(v0, v0 + 264, (8, 17), device=DEV)
+    weights = torch.rand(136, device=DEV) if mask else None
+    args = lambda t: (t["x"], t["W"], targets, weights, v0, 1.0 / 136, None)
+    return t, ("W",), lambda t: F.lm_head_cross_entropy(*args(t)), lambda t: F.LMHeadCrossEntropyFn.apply(*args(t))
+
+
 CASES = {
+    "embedding": (_embedding, False, 11, 0.0),
+    "embedding_places_dropout": (_embedding, True, 0, 0.1),
+    "head_loss": (_head, False, 0),
+    "head_loss_mask": (_head, True, 5),
     "linear": (_linear, F.ACT_NONE, True, True, 0.0),
     "linear_gelu_dropout": (_linear, F.ACT_GELU, True, True, 0.1),
     "linear_relu": (_linear, F.ACT_RELU, True, False, 0.0),
@@ -278,3 +300,27 @@ def test_compiled_calls(name):
         warnings.simplefilter("ignore")                  # the graph breaks at the kernels' bindings
         compiled = _outcome(tensors, params, torch.compile(node, backend="eager"), buffers=params)
     _same(compiled, _outcome(tensors, params, node, buffers=params))
+
+
+@pytest.mark.parametrize("in_order,tokens", [(True, 70000), (False, 120)])      # sorted above 65536 tokens; float atomics
+def test_embedding_node_takes_the_other_gradient_kernels(in_order, tokens):
+    torch.manual_seed(3)
+    ids, pos = torch.randint(0, 300, (tokens,), device=DEV), torch.arange(tokens, device=DEV) % 64
+    g = torch.randn(tokens, 64, device=DEV).bfloat16()
+    grads = []
+    for call in (F.embedding, F.EmbeddingFn.apply):
+        W, P = (torch.nn.Parameter(torch.zeros(n, 64, device=DEV).bfloat16()) for n in (300, 64))
+        P.main_grad = torch.ones(64, 64, device=DEV)
+        y = call(ids, pos, W, P, 0, 0.0, 0)
+        F.set_deterministic_embedding_grad(in_order)                            # what counts is the switch at the backward
+        try:
+            y.backward(g)
+        finally:
+            F.set_deterministic_embedding_grad(True)
+        assert P.grad is None
+        grads.append((W.grad, P.main_grad))
+    for a, b in zip(*grads):
+        if in_order:
+            assert torch.equal(a, b)
+        else:
+            assert rel(a, b) < 2.0 ** -8
