@@ -273,11 +273,14 @@ __device__ __forceinline__ float2 exp_pair(uint32_t two, float off) {
 // shared memory; every thread keeps a running maximum and the sum of exponentials relative to it on the way, so that the
 // special-function unit works under the loads, and only the gradient is left for a second pass.  Same quantities as
 // ce_stats + ce_finalize, which read the row three times.  T threads a row, 1024 per SM: one CTA loads while others write.
-// 4096 rows x 51200: 199 us (4.2 TB/s, two exponentials an element) against 263 for the two kernels; results below the normal
+// 4096 rows x 51200: 177 us (4.7 TB/s, two exponentials an element) against 263 for the two kernels; results below the normal
 // range are 6 us of it.
 constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per SM
 
-template <int T>
+// AHEAD: the next four loads of a thread are under way while it works on the last four, in rows of which it has several rounds:
+// 4096 rows x 51200 193 -> 177 us, x 40000 150 -> 134, x 32000 116 -> 106 (eight loads at a time instead: 201, 152, 109; one round
+// is slower for it, x 2048 12.3 -> 13.1).
+template <int T, bool AHEAD>
 __global__ void __launch_bounds__(T, 1024 / T)
 ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __restrict__ targets,
                 const float* __restrict__ loss_mask, float* __restrict__ loss, int V, long long v0, float grad_scale) {
@@ -293,11 +296,22 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __r
   // read by every thread before the barriers of the reductions, so before any thread overwrites the row
   const float tgt = (t >= 0 && t < V) ? __bfloat162float(x[t]) : 0.f;
   float tmax = tail, tsum = tail != -INFINITY ? __expf(tail - tail) : 0.f;  // this thread's maximum and sum exp(x - maximum)
-  for (int v = threadIdx.x; v < nvec; v += 4 * T) {
-    uint4 q[4];
+  uint4 next[4];
+  auto fetch = [&](int v, uint4 (&q)[4]) {
 #pragma unroll
     for (int u = 0; u < 4; ++u)
       if (v + u * T < nvec) q[u] = __ldcs(xv + v + u * T);
+  };
+  if (AHEAD) fetch(threadIdx.x, next);
+  for (int v = threadIdx.x; v < nvec; v += 4 * T) {
+    uint4 q[4];
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = next[u];
+      fetch(v + 4 * T, next);
+    } else {
+      fetch(v, q);
+    }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (v + u * T < nvec) {
@@ -368,8 +382,10 @@ int ce_fused_launch(void* logits, int ld, const long long* targets, const float*
   // 138 and 145 at 32000, 201 and 181 at 40960 (512 throughout: 27 us at 1024 columns, where the two kernels take 15 and 128
   // threads 9.5).  Rows that all fit on the chip at once are a matter of latency: 16 rows of 8192 take 4.6 us with 128 threads
   // and 3.8 with 512.
-  if (rows <= 2LL * num_sms || V > 36 * 1024) return launch(ce_fused_kernel<512>, 512);
-  return V > 14 * 1024 ? launch(ce_fused_kernel<256>, 256) : launch(ce_fused_kernel<128>, 128);
+  const bool few = rows <= 2LL * num_sms;
+  if (V > 36 * 1024 || (few && V > 14 * 1024)) return launch(ce_fused_kernel<512, true>, 512);
+  if (few) return launch(ce_fused_kernel<512, false>, 512);
+  return V > 14 * 1024 ? launch(ce_fused_kernel<256, true>, 256) : launch(ce_fused_kernel<128, false>, 128);
 }
 
 int embedding_fwd_launch(const long long* ids, const long long* pos, const void* W, const void* P, void* out,
