@@ -35,6 +35,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
                          const void* dres, void* dx, float* dgamma, float* dbeta, float* part_g, float* part_b,
                          int accumulate_wgrad, int rows, int H, int* status, int num_sms, cudaStream_t stream);
 int colsum_tickets();
+int colsum_part_rows(int rows);
 int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N,
                   cudaStream_t stream);
 int elementwise_launch(int op, const void* x, const void* a, const void* bias, void* out, long long rows, int N,
@@ -284,7 +285,7 @@ void colsum(const Tensor& a, Tensor& out, bool accumulate) {
   TORCH_CHECK(out.scalar_type() == torch::kFloat32 && out.numel() == a.size(1) && out.is_contiguous());
   c10::cuda::CUDAGuard guard(a.device());
   const int rows = static_cast<int>(a.size(0)), N = static_cast<int>(a.size(1));
-  Tensor part = torch::empty({ssb::ln_bwd_slices(rows), N}, torch::dtype(torch::kFloat32).device(a.device()));
+  Tensor part = torch::empty({ssb::colsum_part_rows(rows), N}, torch::dtype(torch::kFloat32).device(a.device()));
   check_launch(ssb::colsum_launch(a.data_ptr(), static_cast<int>(a.stride(0)), out.data_ptr<float>(),
                                   part.data_ptr<float>(), ticket_tensor().data_ptr<int>(), accumulate, rows, N,
                                   cur_stream()),

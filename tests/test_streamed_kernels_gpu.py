@@ -268,3 +268,21 @@ def test_layernorm_backward_with_three_and_four_warps_a_row(rows, H, residual):
     assert _rel(dx, want[0] + (dres.double() if residual else 0)) < 2.0 ** -8       # one rounding to bf16
     assert _rel(dg - 1, want[1]) < 1e-5 and _rel(db - 1, want[2]) < 1e-5            # fp32 sums
     assert native.check_status() == 0
+
+
+@pytest.mark.parametrize("rows,N", [(1, 8), (63, 264), (64, 256), (65, 2048), (129, 520), (1000, 1000), (8192, 72), (8193, 640), (20000, 8192)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_column_sums(rows, N, accumulate):
+    """One slice of rows, a few, as many as there may be; fp32 sums of `rows` values: off by rows 2^-24 of their magnitudes at most,
+    far less for the tree they are added in."""
+    torch.manual_seed(rows + N)
+    a = torch.randn(rows, N + 8, device="cuda").bfloat16()[:, :N]
+    out = torch.randn(N, device="cuda")
+    want = a.double().sum(0) + (out.double() if accumulate else 0)
+    for _ in range(2):                                   # the counters are as they were after a call
+        got = out.clone()
+        native.ext().colsum(a, got, accumulate)
+        assert float(((got.double() - want).abs() - (rows + 8) * 2.0 ** -24 * (a.double().abs().sum(0) + out.double().abs())).max()) <= 0
+    again = out.clone()
+    native.ext().colsum(a, again, accumulate)
+    assert torch.equal(got, again)
