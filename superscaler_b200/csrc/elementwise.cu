@@ -70,16 +70,11 @@ ew_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__
       for (int j = 0; j < 8; ++j) o[j] = f[j] + g[j];
     } else {
       // dropout family: element index = v*8 + j, hash groups of 4
-      uint32_t m0 = 0xF, m1 = 0xF;
-      if (dropout_p > 0.f) {
-        m0 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2, keep16);
-        m1 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16);
-      }
-      const float sc = dropout_p > 0.f ? scale : 1.0f;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        o[j] = ((m0 >> j) & 1u) ? f[j] * sc : 0.f;
-        o[4 + j] = ((m1 >> j) & 1u) ? f[4 + j] * sc : 0.f;
+      for (int j = 0; j < 8; ++j) o[j] = f[j];
+      if (dropout_p > 0.f) {
+        dropout_apply4(o, dropout_drop4(seed, static_cast<uint64_t>(v) * 2, keep16), scale);
+        dropout_apply4(o + 4, dropout_drop4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16), scale);
       }
       if (OP == kEwBiasDropAdd) {
 #pragma unroll

@@ -57,13 +57,8 @@ embedding_fwd_kernel(const long long* __restrict__ ids, const long long* __restr
       }
       const long long v = t * nvec + c;
       if (dropout_p > 0.f) {
-        const uint32_t m0 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2, keep16);
-        const uint32_t m1 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          f[j] = ((m0 >> j) & 1u) ? f[j] * scale : 0.f;
-          f[4 + j] = ((m1 >> j) & 1u) ? f[4 + j] * scale : 0.f;
-        }
+        dropout_apply4(f, dropout_drop4(seed, static_cast<uint64_t>(v) * 2, keep16), scale);
+        dropout_apply4(f + 4, dropout_drop4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16), scale);
       }
       uint4 o;
       o.x = pack_bf16x2(f[0], f[1]); o.y = pack_bf16x2(f[2], f[3]);
@@ -90,13 +85,8 @@ embedding_bwd_kernel(const long long* __restrict__ ids, const long long* __restr
     float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), cc = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
     float f[8] = {a.x, a.y, b.x, b.y, cc.x, cc.y, d.x, d.y};
     if (dropout_p > 0.f) {
-      const uint32_t m0 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2, keep16);
-      const uint32_t m1 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        f[j] = ((m0 >> j) & 1u) ? f[j] * scale : 0.f;
-        f[4 + j] = ((m1 >> j) & 1u) ? f[4 + j] * scale : 0.f;
-      }
+      dropout_apply4(f, dropout_drop4(seed, static_cast<uint64_t>(v) * 2, keep16), scale);
+      dropout_apply4(f + 4, dropout_drop4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16), scale);
     }
     const long long id = ids[t];
     if (dW != nullptr && id >= v0 && id < v1) {
@@ -136,13 +126,8 @@ embedding_bwd_sorted_kernel(const Key* __restrict__ keys, const long long* __res
       float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), cc = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
       float f[8] = {a.x, a.y, b.x, b.y, cc.x, cc.y, d.x, d.y};
       if (dropout_p > 0.f) {
-        const uint32_t m0 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2, keep16);
-        const uint32_t m1 = dropout_keep4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          f[i] = ((m0 >> i) & 1u) ? f[i] * scale : 0.f;
-          f[4 + i] = ((m1 >> i) & 1u) ? f[4 + i] * scale : 0.f;
-        }
+        dropout_apply4(f, dropout_drop4(seed, static_cast<uint64_t>(v) * 2, keep16), scale);
+        dropout_apply4(f + 4, dropout_drop4(seed, static_cast<uint64_t>(v) * 2 + 1, keep16), scale);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] += f[i];

@@ -168,12 +168,8 @@ embedding_sum_kernel(const GroupArgs args, const __nv_bfloat16* __restrict__ g, 
       float f[8] = {x0.x, x0.y, x1.x, x1.y, x2.x, x2.y, x3.x, x3.y};
       if (dropout_p > 0.f) {
         const uint64_t v = at(token);
-        const uint32_t m0 = dropout_keep4(seed, v * 2, keep16), m1 = dropout_keep4(seed, v * 2 + 1, keep16);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          f[i] = ((m0 >> i) & 1u) ? f[i] * scale : 0.f;
-          f[4 + i] = ((m1 >> i) & 1u) ? f[4 + i] * scale : 0.f;
-        }
+        dropout_apply4(f, dropout_drop4(seed, v * 2, keep16), scale);
+        dropout_apply4(f + 4, dropout_drop4(seed, v * 2 + 1, keep16), scale);
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] += f[i];

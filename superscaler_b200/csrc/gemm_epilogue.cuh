@@ -103,9 +103,7 @@ __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row
     const uint64_t g0 = (static_cast<uint64_t>(row) * static_cast<uint64_t>(p.N) + n0) >> 2;
 #pragma unroll
     for (int g = 0; g < W / 4; ++g) {
-      const uint32_t m = dropout_keep4(p.dropout_seed, g0 + g, keep16);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[4 * g + i] = ((m >> i) & 1u) ? v[4 * g + i] * drop_scale : 0.f;
+      dropout_apply4(v + 4 * g, dropout_drop4(p.dropout_seed, g0 + g, keep16), drop_scale);
     }
   }
   if (p.residual != nullptr) {
@@ -212,9 +210,7 @@ __device__ __forceinline__ void gemm_epilogue_math16(const GemmParams& p, int ro
     const uint64_t g0 = (static_cast<uint64_t>(row) * static_cast<uint64_t>(p.N) + n0) >> 2;
 #pragma unroll
     for (int g = 0; g < 4; ++g) {
-      const uint32_t m = dropout_keep4(p.dropout_seed, g0 + g, keep16);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[4 * g + i] = ((m >> i) & 1u) ? v[4 * g + i] * drop_scale : 0.f;
+      dropout_apply4(v + 4 * g, dropout_drop4(p.dropout_seed, g0 + g, keep16), drop_scale);
     }
   }
   if (p.residual != nullptr) {
