@@ -125,8 +125,8 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 // (warps an SM and loads in flight were what bounded it: DRAM 47 %, issue slots 35 %).  The warps of a row exchange their means and
 // sums of squares about them once per R rows; these are brought together about the common mean, which is no less exact than sums
 // over the whole row.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
-// Measured, a warp per row -> this: 32768 x 2048 55.7 -> 49.0 us, x 1536 49.1 -> 38.9, x 512 16.5 -> 13.8, 4096 x 2048 11.6 -> 10.5; a copy
-// takes 42.5, 32.8, 12.4, 7.3.  Rows of 513 to 1280 columns stay with a warp each: two or three warps are idle in part there
+// Measured, a warp per row -> this: 32768 x 2048 55.7 -> 47.6 us, x 1536 49.1 -> 37.3, x 512 16.5 -> 13.8, 4096 x 2048 11.6 -> 9.5 (48.3,
+// 38.6, 10.3 with a division per warp and row in the combination); a copy takes 42.0, 32.4, 12.3, 7.3.  Issue slots are 74 % busy.  Rows of 513 to 1280 columns stay with a warp each: two or three warps are idle in part there
 // (32768 x 768 22.6 -> 29, x 1152 34.1 -> 37.3, x 1280 37.0 -> 37.5).
 template <int WPR>
 struct LnGroup {
@@ -159,6 +159,9 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       b[i][j] = mine[i] ? __ldg(beta + at[i] * 8 + j) : 0.f;
     }
   }
+  __shared__ float columns[WPR];  // of every warp of a row
+  if (WPR > 1 && lane == 0) columns[part] = static_cast<float>(count);
+  if (WPR > 1) __syncthreads();
   const float inv_count = count > 0 ? 1.0f / static_cast<float>(count) : 0.f, inv_h = 1.0f / static_cast<float>(H);
   uint4 next[R][VPL];
   auto fetch = [&](int row0) {
@@ -230,25 +233,21 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       float2(&slots)[WPR][R] = xch[turn][slot];
       if (lane == 0) {
 #pragma unroll
-        for (int r = 0; r < R; ++r) slots[part][r] = make_float2(m[r] * static_cast<float>(count), s2[r]);
+        for (int r = 0; r < R; ++r) slots[part][r] = make_float2(m[r], s2[r]);
       }
       __syncthreads();  // (one row slot per block: all warps have the same rows)
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        float2 e[WPR];
         float sum = 0.f;
 #pragma unroll
-        for (int w = 0; w < WPR; ++w) {
-          e[w] = slots[w][r];
-          sum += e[w].x;
-        }
+        for (int w = 0; w < WPR; ++w) sum = fmaf(slots[w][r].x, columns[w], sum);
         m[r] = sum * inv_h;
         float t = 0.f;
 #pragma unroll
-        for (int w = 0; w < WPR; ++w) {
-          const float n = static_cast<float>(8 * (max(0, min(32, nvec - w * 32)) + max(0, min(32, nvec - (WPR + w) * 32))));
-          const float d = n > 0.f ? e[w].x / n - m[r] : 0.f;
-          t += fmaf(d * n, d, e[w].y);
+        for (int w = 0; w < WPR; ++w) {  // (read again: held, they are spilled)
+          const volatile float* e = &slots[w][r].x;
+          const float d = e[0] - m[r];
+          t += fmaf(d * columns[w], d, e[1]);
         }
         s2[r] = t;
       }
