@@ -126,15 +126,17 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
 // sums of squares about them once per R rows; these are brought together about the common mean, which is no less exact than sums
 // over the whole row.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
 // Measured, a warp per row -> this: 32768 x 2048 55.7 -> 47.6 us, x 1536 49.1 -> 37.3, x 512 16.5 -> 13.8, 4096 x 2048 11.6 -> 9.5 (48.3,
-// 38.6, 10.3 with a division per warp and row in the combination); a copy takes 42.0, 32.4, 12.3, 7.3.  Issue slots are 74 % busy.  Rows of 513 to 1280 columns stay with a warp each: two or three warps are idle in part there
-// (32768 x 768 22.6 -> 29, x 1152 34.1 -> 37.3, x 1280 37.0 -> 37.5).
+// 38.6, 10.3 with a division per warp and row in the combination); a copy takes 42.0, 32.4, 12.3, 7.3.  Issue slots are 74 % busy.
+// 32768 x 1024 28.4 -> 24.9, x 896 27.6 -> 23.5, x 1280 36.8 -> 34.7, 8192 x 1024 10.2 -> 9.2.  Rows of 513 to 768 columns stay with a warp each
+// (x 640 20.0 -> 20.7, x 768 22.3 -> 22.0: the second warp is idle in part), and so do 4096 x 1024 (6.3 -> 6.6: the last groups have none).
 template <int WPR>
 struct LnGroup {
   static constexpr int kRows = 3, kGroups = WPR == 1 ? 4 : 1, kThreads = 32 * WPR * kGroups, kBlocks = 512 / kThreads;  // per SM
 };
-bool ln_fwd_grouped(int rows, int H, int num_sms) {  // every group has all of its rows at least once
-  const int groups = num_sms * (H <= 512 ? LnGroup<1>::kBlocks * 4 : H <= 1536 ? LnGroup<3>::kBlocks : LnGroup<4>::kBlocks);
-  return (H <= 512 || (H > 1280 && H <= 2048)) && rows >= groups * 3;
+bool ln_fwd_grouped(int rows, int H, int num_sms) {  // every group has all of its rows at least once, of 769 to 1280 columns twice
+  if (H > 2048 || (H > 512 && H <= 768)) return false;
+  const int groups = num_sms * (H <= 512 ? LnGroup<1>::kBlocks * 4 : H <= 1024 ? LnGroup<2>::kBlocks : H <= 1536 ? LnGroup<3>::kBlocks : LnGroup<4>::kBlocks);
+  return rows >= groups * 3 * (H > 768 && H <= 1280 ? 2 : 1);
 }
 template <int WPR>
 __global__ void __launch_bounds__(LnGroup<WPR>::kThreads, LnGroup<WPR>::kBlocks)
@@ -848,6 +850,7 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
       kernel<<<num_sms * Cfg::kBlocks, Cfg::kThreads, 0, stream>>>(xb, gamma, beta, yb, mean, rstd, rows, H, eps);
     };
     if (H <= 512) launch(ln_fwd_group_kernel<1>, LnGroup<1>{});
+    else if (H <= 1024) launch(ln_fwd_group_kernel<2>, LnGroup<2>{});
     else if (H <= 1536) launch(ln_fwd_group_kernel<3>, LnGroup<3>{});
     else launch(ln_fwd_group_kernel<4>, LnGroup<4>{});
     return static_cast<int>(cudaGetLastError());

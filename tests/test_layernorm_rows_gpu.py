@@ -33,7 +33,8 @@ def test_layernorm_forward_row_lengths(H, rows, with_residual):
 @pytest.mark.parametrize("H,rows", [(8, 7104), (248, 7105), (264, 7106), (512, 9001),              # a warp per row, three at a time
                                     (1288, 2220), (1472, 2221), (1536, 2370),                      # three warps per row
                                     (1544, 1776), (1800, 1777), (2048, 1778), (2048, 5003),        # four
-                                    (512, 7103), (1536, 2219), (2048, 1775)])                      # one row short of it
+                                    (776, 7104), (960, 7105), (1024, 7999), (1032, 4440), (1280, 5003),  # two and three, of two rounds
+                                    (512, 7103), (1536, 2219), (2048, 1775), (1024, 7103)])        # one row short of it
 @pytest.mark.parametrize("offset", [3.0, 300.0])
 def test_layernorm_forward_of_many_rows(H, rows, offset):
     """Mean and 1/std from parts of a row.  fp32 sums of values near `offset`: off by 2^-22 offset at most per value, hence the mean by
