@@ -377,6 +377,7 @@ int embedding_fwd_launch(const long long* ids, const long long* pos, const void*
                          long long tokens, int H, long long v0, long long v1, float dropout_p,
                          unsigned long long seed, int num_sms, cudaStream_t stream) {
   if (H % 8) return -3;
+  if (H == 0) return 0;  // rows of no columns: nothing to look up
   const int nvec = H / 8, passes = (nvec + 255) / 256;
   const int tpr = ((nvec + passes - 1) / passes + 31) / 32 * 32, slots = 256 / tpr;
   const long long want = (tokens + slots - 1) / slots, most = static_cast<long long>(num_sms) * kEmbedBlocks;

@@ -4,6 +4,7 @@ around the length up to which tokens are ranked one by one; ids outside the tabl
 import pytest
 import torch
 
+from superscaler_b200.ops import functional as F
 from superscaler_b200.ops import native
 
 pytestmark = pytest.mark.gpu
@@ -73,3 +74,17 @@ def test_lookup(H, tokens, places):
     if places:
         want = want + P[pos].float()
     assert torch.equal(y, want.bfloat16())
+
+
+@pytest.mark.parametrize("places", [False, True])
+def test_tables_of_no_columns(places):
+    """Accepted: no values, no gradients, no division by the length of a row."""
+    ids = torch.tensor([[1, 7, 2]], device=DEV)
+    W, P = (torch.nn.Parameter(torch.empty(n, 0, device=DEV, dtype=torch.bfloat16)) for n in (5, 3))
+    args = (ids, torch.arange(3, device=DEV) if places else None, W, P if places else None, 0, 0.1, 7)
+    for call in (F.embedding, F.EmbeddingFn.apply):
+        y = call(*args)
+        assert y.shape == (3, 0)
+        y.backward(torch.empty_like(y))
+        assert W.grad.shape == W.shape and (not places or P.grad.shape == P.shape)
+    assert native.check_status() == 0
