@@ -1,4 +1,4 @@
-// LayerNorm forward / backward for bf16 activations with fp32 statistics, one warp per row.
+// LayerNorm forward / backward for bf16 activations with fp32 statistics, one to eight warps per row.
 // Covers the role of the reference's mixed-precision fused LayerNorm extension
 // (runtime/megatron/fused_kernels/layer_norm_cuda_kernel.cu:290-334 forward,
 // :415-651 backward): y = (x - mean) * rstd * gamma + beta, saving mean and rstd;
@@ -23,13 +23,11 @@ __device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
   f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
 }
 
-// Rows that fit in the registers of a warp, read once: up to VPL vectors of 8 bf16 per lane; FULL = false: the last one, or for
-// VPL > 8 the last few, are not there for every lane.  Values are kept as fp32 up to VPL 8, packed beyond that.  Lengths that are
-// not 512, 1024, 2048 or 4096 used to take the kernel below: 32768 rows of 1984 147 -> 55 us, of 1088 83 -> 33, 512 of 704
-// 4.1 -> 2.8.  Two rows at a time, to read gamma and beta from the L1 once for both,
-// is slower (32768 x 2048 67 us instead of 55): too few warps; so is fp32 arithmetic two values per instruction (32768 x 1024
-// 28.1 -> 29.9).  What bounds it is the latency of the loads with 15 warps an SM (125 registers): 32768 x 2048 keeps the DRAM 47 %
-// busy, the issue slots 35 %, and hardly ever waits for a math pipe.  Many rows of some lengths go to ln_fwd_group_kernel below.
+// Rows with a residual, and rows of 513 to 768 and of more than 2048 columns, that fit in the registers of a warp, read once: up to VPL
+// vectors of 8 bf16 per lane; FULL = false: the last one, or for VPL > 8 the last few, are not there for every lane.  Values are
+// kept as fp32 up to VPL 8, packed beyond that.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel for any
+// length: 512 rows of 704 4.1 -> 2.8 us.  What bounds it is the latency of the loads with few warps an SM (125 registers for
+// 2048 columns: 15 warps).  Two rows at a time leave too few of them; fp32 arithmetic two values per instruction is slower, too.
 template <int VPL, bool FULL>
 __global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
 ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual,
@@ -120,21 +118,143 @@ ln_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restri
   }
 }
 
+// Rows without a residual of up to 512 and of 769 to 2048 columns are taken by two kernels, few of them by ln_fwd_parts_kernel, many by
+// ln_fwd_group_kernel.  A row has the same bits in either, so its result does not depend on how many there are: vector 32 j + lane
+// belongs to part j % parts of the row; a part has its sum and the sum of its squares about (nearly) its own mean, which are brought
+// together about the row's.  The pieces, with every rounding spelled out:
+__device__ __forceinline__ float ln_add8(float sum, const float (&v)[8]) {
+  return sum + (((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+}
+__device__ __forceinline__ float ln_add_squares8(float sum, const float (&v)[8], float m) {
+  float u = 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) u = fmaf(v[j] - m, v[j] - m, u);
+  return sum + u;
+}
+__device__ __forceinline__ float ln_part_mean(float sum, float inv_columns) { return __fmul_rn(sum, inv_columns); }
+// Squares about the row's mean from those about m, the value of ln_part_mean: sum (v - mean)^2 = squares + 2 (m - mean) sum (v - m) +
+// columns (m - mean)^2.  The middle term is what the rounding of m leaves; with it a row of parts is as exact as one summed whole
+// (rows of 1000 columns about 300, 1 / std: 5.8e-8 whole, 1.5e-7 without it, 4.3e-8 with it).
+__device__ __forceinline__ float ln_part_squares(float sum, float squares, float columns, float inv_columns, float mean) {
+  const float m = ln_part_mean(sum, inv_columns), d = m - mean, rest = fmaf(-m, columns, sum);
+  return fmaf(d, fmaf(columns, d, rest + rest), squares);
+}
+// a / n for n > 0 and inv near 1 / n: the product, and once its residual (Newton's method), which is left out of infinities.  The
+// products alone put the means of rows that are no power of two off by half as much again as a division does.
+__device__ __forceinline__ float ln_quotient(float a, float n, float inv) {
+  const float q = __fmul_rn(a, inv), rest = fmaf(-q, n, a);
+  return rest - rest == 0.f ? fmaf(rest, inv, q) : q;
+}
+__device__ __forceinline__ uint4 ln_values8(const float (&v)[8], float mean, float rstd, const float (&g)[8], const float (&b)[8]) {
+  float o[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) o[j] = fmaf((v[j] - mean) * rstd, g[j], b[j]);
+  return make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+}
+
+// A warp per row, up to VPL vectors per lane.  FULL, WIDE: every lane has all of them, gamma and beta start on 16 bytes.  HOLD: gamma and
+// beta are fetched in front of the row, where all rows are on the chip at once anyway; otherwise where they are used.
+template <int VPL, bool FULL, bool WIDE, bool HOLD>
+__global__ void __launch_bounds__(kLnWarpsPerBlock * 32)
+ln_fwd_parts_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ gamma, const float* __restrict__ beta,
+                    __nv_bfloat16* __restrict__ y, float* __restrict__ mean_out, float* __restrict__ rstd_out, int rows, int H,
+                    float eps) {
+  constexpr int kParts = (VPL + 1) / 2;
+  const int lane = threadIdx.x & 31, nvec = H / 8;
+  auto mine = [&](int i) { return FULL || i < VPL - 1 || i * 32 + lane < nvec; };
+  const float h = static_cast<float>(H), inv_h = 1.0f / h;
+  float columns[kParts], inv_columns[kParts];
+#pragma unroll
+  for (int p = 0; p < kParts; ++p) {
+    int n = 0;
+#pragma unroll
+    for (int i = p; i < VPL; i += kParts) n += FULL || i < VPL - 1 ? 256 : 8 * min(32, nvec - i * 32);
+    columns[p] = static_cast<float>(n);
+    inv_columns[p] = 1.0f / columns[p];
+  }
+  auto parameters = [&](const float* from, int i, float (&v)[8]) {
+    const int at = i * 32 + lane;
+    if constexpr (WIDE) {
+      const float4 a = reinterpret_cast<const float4*>(from)[2 * at], c = reinterpret_cast<const float4*>(from)[2 * at + 1];
+      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+      v[4] = c.x; v[5] = c.y; v[6] = c.z; v[7] = c.w;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = from[8 * at + j];
+    }
+  };
+  float g[HOLD ? VPL : 1][8], b[HOLD ? VPL : 1][8];
+  if constexpr (HOLD) {
+#pragma unroll
+    for (int i = 0; i < VPL; ++i)
+      if (mine(i)) {
+        parameters(gamma, i, g[i]);
+        parameters(beta, i, b[i]);
+      }
+  }
+  for (int row = blockIdx.x * kLnWarpsPerBlock + (threadIdx.x >> 5); row < rows; row += gridDim.x * kLnWarpsPerBlock) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
+    float f[VPL][8], m[kParts] = {}, s2[kParts] = {};  // m: sums
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) unpack8(mine(i) ? xr[i * 32 + lane] : make_uint4(0u, 0u, 0u, 0u), f[i]);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) m[i % kParts] = ln_add8(m[i % kParts], f[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) m[p] += __shfl_xor_sync(0xffffffffu, m[p], o);
+    float mean = kParts == 1 ? ln_quotient(m[0], h, inv_h) : 0.f;
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      const int p = i % kParts;
+      if (mine(i)) s2[p] = ln_add_squares8(s2[p], f[i], kParts == 1 ? mean : ln_part_mean(m[p], inv_columns[p]));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) s2[p] += __shfl_xor_sync(0xffffffffu, s2[p], o);
+    float squares = s2[0];
+    if constexpr (kParts > 1) {
+      squares = 0.f;
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) mean += m[p];
+      mean = ln_quotient(mean, h, inv_h);
+#pragma unroll
+      for (int p = 0; p < kParts; ++p) squares += ln_part_squares(m[p], s2[p], columns[p], inv_columns[p], mean);
+    }
+    const float rstd = rsqrtf(ln_quotient(squares, h, inv_h) + eps);
+    if (lane == 0) {
+      mean_out[row] = mean;
+      rstd_out[row] = rstd;
+    }
+    uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
+#pragma unroll
+    for (int i = 0; i < VPL; ++i) {
+      if (!mine(i)) continue;
+      if constexpr (!HOLD) {
+        parameters(gamma, i, g[0]);
+        parameters(beta, i, b[0]);
+      }
+      yr[i * 32 + lane] = ln_values8(f[i], mean, rstd, g[HOLD ? i : 0], b[HOLD ? i : 0]);
+    }
+  }
+}
+
 // Many rows of up to 2048: WPR warps share a row and take R rows at a time, the next R on their way meanwhile.  gamma and beta stay in
 // registers; a warp per row read them from the L1 for every row, and its loads, sums and stores came one after the other
-// (warps an SM and loads in flight were what bounded it: DRAM 47 %, issue slots 35 %).  The warps of a row exchange their means and
-// sums of squares about them once per R rows; these are brought together about the common mean, which is no less exact than sums
-// over the whole row.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
-// Measured, a warp per row -> this: 32768 x 2048 55.7 -> 47.6 us, x 1536 49.1 -> 37.3, x 512 16.5 -> 13.8, 4096 x 2048 11.6 -> 9.5 (48.3,
-// 38.6, 10.3 with a division per warp and row in the combination); a copy takes 42.0, 32.4, 12.3, 7.3.  Issue slots are 74 % busy.
-// 32768 x 1024 28.4 -> 24.9, x 896 27.6 -> 23.5, x 1280 36.8 -> 34.7, 8192 x 1024 10.2 -> 9.2.  Rows of 513 to 768 columns stay with a warp each
-// (x 640 20.0 -> 20.7, x 768 22.3 -> 22.0: the second warp is idle in part), and so do 4096 x 1024 (6.3 -> 6.6: the last groups have none).
+// (warps an SM and loads in flight were what bounded it: DRAM 47 %, issue slots 35 %).  The warps of a row exchange their sums and sums
+// of squares once per R rows.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
+// Bounded by issue slots: what is done once per row is done by a lane per row, not by every lane for all of them (47.6 -> 45.2, x 1800
+// 46.0 -> 43.3, x 512 12.3 -> 12.0).  Measured, a warp per row -> this: 32768 x 2048 55.7 -> 45.2 us, x 1536 49.1 -> 36.5, 4096 x 2048
+// 11.6 -> 8.7; a copy takes 42.0, 32.4, 7.3.  32768 x 1024 28.4 -> 24.6, x 896 27.6 -> 23.5, x 1280 36.8 -> 33.6, 8192 x 1024 10.2 -> 9.2.
+// Rows of 513 to 768 columns stay with a warp each (x 640 20.0 -> 20.7, x 768 22.3 -> 22.0: the second warp is idle in part), and so do 4096 x
+// 1024 (6.3 -> 6.6: the last groups have none).
 template <int WPR>
 struct LnGroup {
   static constexpr int kRows = 3, kGroups = WPR == 1 ? 4 : 1, kThreads = 32 * WPR * kGroups, kBlocks = 512 / kThreads;  // per SM
 };
+bool ln_fwd_in_parts(int H) { return H > 0 && (H <= 512 || (H > 768 && H <= 2048)); }
 bool ln_fwd_grouped(int rows, int H, int num_sms) {  // every group has all of its rows at least once, of 769 to 1280 columns twice
-  if (H > 2048 || (H > 512 && H <= 768)) return false;
   const int groups = num_sms * (H <= 512 ? LnGroup<1>::kBlocks * 4 : H <= 1024 ? LnGroup<2>::kBlocks : H <= 1536 ? LnGroup<3>::kBlocks : LnGroup<4>::kBlocks);
   return rows >= groups * 3 * (H > 768 && H <= 1280 ? 2 : 1);
 }
@@ -161,10 +281,10 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       b[i][j] = mine[i] ? __ldg(beta + at[i] * 8 + j) : 0.f;
     }
   }
-  __shared__ float columns[WPR];  // of every warp of a row
-  if (WPR > 1 && lane == 0) columns[part] = static_cast<float>(count);
+  const float n = static_cast<float>(count), inv_n = 1.0f / n, h = static_cast<float>(H), inv_h = 1.0f / h;
+  __shared__ float2 columns[WPR];  // of every warp of a row, and their reciprocal
+  if (WPR > 1 && lane == 0) columns[part] = make_float2(n, inv_n);
   if (WPR > 1) __syncthreads();
-  const float inv_count = count > 0 ? 1.0f / static_cast<float>(count) : 0.f, inv_h = 1.0f / static_cast<float>(H);
   uint4 next[R][VPL];
   auto fetch = [&](int row0) {
 #pragma unroll
@@ -202,7 +322,7 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
       for (int i = 0; i < VPL; ++i) {
         float v[8];
         unpack8(q[r][i], v);
-        t += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
+        t = ln_add8(t, v);
       }
       m[r] = t;
     }
@@ -211,18 +331,30 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
 #pragma unroll
       for (int r = 0; r < R; ++r) m[r] += __shfl_xor_sync(0xffffffffu, m[r], o);
     packed();
+    // What is done per row is done by the lane of its number, for all R at once.
+    auto of_lane = [&](const float (&v)[R]) { return lane == 1 ? v[1] : lane == 2 ? v[2] : v[0]; };
+    auto to_all = [&](float v, float (&all)[R]) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) all[r] = __shfl_sync(0xffffffffu, v, r);
+    };
+    static_assert(R == 3, "rows at a time");
+    float centre[R], rs[R], mean;
+    if constexpr (WPR == 1) {
+      mean = ln_quotient(of_lane(m), h, inv_h);
+      to_all(mean, centre);
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) centre[r] = ln_part_mean(m[r], inv_n);
+    }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      m[r] *= inv_count;
       float t = 0.f;
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
         float v[8];
         unpack8(q[r][i], v);
-        float u = 0.f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) u = fmaf(v[j] - m[r], v[j] - m[r], u);
-        if (mine[i]) t += u;
+        const float with = ln_add_squares8(t, v, centre[r]);
+        if (mine[i]) t = with;
       }
       s2[r] = t;
     }
@@ -231,47 +363,42 @@ ln_fwd_group_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
 #pragma unroll
       for (int r = 0; r < R; ++r) s2[r] += __shfl_xor_sync(0xffffffffu, s2[r], o);
     packed();
-    if constexpr (WPR > 1) {
+    float squares;
+    if constexpr (WPR == 1) {
+      squares = of_lane(s2);
+    } else {
       float2(&slots)[WPR][R] = xch[turn][slot];
       if (lane == 0) {
 #pragma unroll
         for (int r = 0; r < R; ++r) slots[part][r] = make_float2(m[r], s2[r]);
       }
       __syncthreads();  // (one row slot per block: all warps have the same rows)
+      const int r = lane < R ? lane : 0;
+      mean = squares = 0.f;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float sum = 0.f;
+      for (int w = 0; w < WPR; ++w) mean += slots[w][r].x;
+      mean = ln_quotient(mean, h, inv_h);
 #pragma unroll
-        for (int w = 0; w < WPR; ++w) sum = fmaf(slots[w][r].x, columns[w], sum);
-        m[r] = sum * inv_h;
-        float t = 0.f;
-#pragma unroll
-        for (int w = 0; w < WPR; ++w) {  // (read again: held, they are spilled)
-          const volatile float* e = &slots[w][r].x;
-          const float d = e[0] - m[r];
-          t += fmaf(d * columns[w], d, e[1]);
-        }
-        s2[r] = t;
-      }
+      for (int w = 0; w < WPR; ++w) squares += ln_part_squares(slots[w][r].x, slots[w][r].y, columns[w].x, columns[w].y, mean);
+      to_all(mean, centre);
+    }
+    const float rstd = rsqrtf(ln_quotient(squares, h, inv_h) + eps);
+    to_all(rstd, rs);
+    if (part == 0 && lane < R && row0 + lane < rows) {
+      mean_out[row0 + lane] = mean;
+      rstd_out[row0 + lane] = rstd;
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int row = row0 + r;
       if (row >= rows) break;
-      const float rs = rsqrtf(s2[r] * inv_h + eps);
-      if (part == 0 && lane == 0) {
-        mean_out[row] = m[r];
-        rstd_out[row] = rs;
-      }
       uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
 #pragma unroll
       for (int i = 0; i < VPL; ++i) {
         if (!mine[i]) continue;
         float v[8];
         unpack8(q[r][i], v);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = (v[j] - m[r]) * rs * g[i][j] + b[i][j];
-        yr[at[i]] = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        yr[at[i]] = ln_values8(v, centre[r], rs[r], g[i], b[i]);
       }
     }
   }
@@ -844,15 +971,42 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
   const auto* rb = reinterpret_cast<const __nv_bfloat16*>(residual);
   auto* yb = reinterpret_cast<__nv_bfloat16*>(y);
   auto* sb = reinterpret_cast<__nv_bfloat16*>(sum_out);
-  if (residual == nullptr && ln_fwd_grouped(rows, H, num_sms)) {
-    auto launch = [&](auto kernel, auto cfg) {
-      using Cfg = decltype(cfg);
-      kernel<<<num_sms * Cfg::kBlocks, Cfg::kThreads, 0, stream>>>(xb, gamma, beta, yb, mean, rstd, rows, H, eps);
+  const bool wide = !misaligned(gamma) && !misaligned(beta);  // 16-byte loads of both
+  if (residual == nullptr && ln_fwd_in_parts(H)) {
+    if (ln_fwd_grouped(rows, H, num_sms)) {
+      auto launch = [&](auto kernel, auto cfg) {
+        using Cfg = decltype(cfg);
+        kernel<<<num_sms * Cfg::kBlocks, Cfg::kThreads, 0, stream>>>(xb, gamma, beta, yb, mean, rstd, rows, H, eps);
+      };
+      if (H <= 512) launch(ln_fwd_group_kernel<1>, LnGroup<1>{});
+      else if (H <= 1024) launch(ln_fwd_group_kernel<2>, LnGroup<2>{});
+      else if (H <= 1536) launch(ln_fwd_group_kernel<3>, LnGroup<3>{});
+      else launch(ln_fwd_group_kernel<4>, LnGroup<4>{});
+      return static_cast<int>(cudaGetLastError());
+    }
+    // HOLD takes three times the registers.  592 rows of 1024 2.86 -> 2.29 us, of 2048 3.48 -> 2.92, one row of 1536 3.14 -> 2.04; where
+    // the rows then wait for one another it loses: 4096 of 1024 4.9 -> 5.8, 1700 of 1280 3.9 -> 4.05, of 2048 5.0 -> 6.4.
+    const bool hold = rows <= num_sms * (H <= 1024 ? 16 : 4);
+    auto launch = [&](auto full, auto any, auto any_hold, auto full_hold, auto off) {
+      auto kernel = !wide ? off : H % 256 ? (hold ? any_hold : any) : hold ? full_hold : full;
+      kernel<<<grid, block, 0, stream>>>(xb, gamma, beta, yb, mean, rstd, rows, H, eps);
     };
-    if (H <= 512) launch(ln_fwd_group_kernel<1>, LnGroup<1>{});
-    else if (H <= 1024) launch(ln_fwd_group_kernel<2>, LnGroup<2>{});
-    else if (H <= 1536) launch(ln_fwd_group_kernel<3>, LnGroup<3>{});
-    else launch(ln_fwd_group_kernel<4>, LnGroup<4>{});
+#define SSB_LN_CASE(V)                                                                                                       \
+  case V:                                                                                                                    \
+    launch(ln_fwd_parts_kernel<V, true, true, false>, ln_fwd_parts_kernel<V, false, true, false>,                            \
+           ln_fwd_parts_kernel<V, false, true, true>, ln_fwd_parts_kernel<V, true, true, true>,                              \
+           ln_fwd_parts_kernel<V, false, false, false>);                                                                     \
+    break
+    switch ((H + 255) / 256) {
+      SSB_LN_CASE(1);
+      SSB_LN_CASE(2);
+      SSB_LN_CASE(4);
+      SSB_LN_CASE(5);
+      SSB_LN_CASE(6);
+      SSB_LN_CASE(7);
+      SSB_LN_CASE(8);
+    }
+#undef SSB_LN_CASE
     return static_cast<int>(cudaGetLastError());
   }
 #define SSB_LN_ARGS <<<grid, block, 0, stream>>>(xb, rb, gamma, beta, yb, sb, mean, rstd, rows, H, eps)
@@ -861,8 +1015,7 @@ int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma
     if (H == V * 256) ln_fwd_kernel<V, true> SSB_LN_ARGS;       \
     else ln_fwd_kernel<V, false> SSB_LN_ARGS;                   \
     break
-  // 16-byte loads of gamma and beta; parameters that start elsewhere take the kernel for any address
-  const bool wide = !misaligned(gamma) && !misaligned(beta);
+  // parameters that start elsewhere take the kernel for any address
   switch (wide ? (H + 255) / 256 : 0) {
     SSB_LN_CASE(1);
     SSB_LN_CASE(2);

@@ -52,3 +52,20 @@ def test_layernorm_forward_of_many_rows(H, rows, offset):
         assert float(((rstd.double() - r) / r).abs().max()) <= 2.0 ** -18
         slip = 2.0 ** -20 * offset * r[:, None] * g.double().abs()
         assert float(((y.double() - want).abs() - 2.0 ** -8 * (want.abs() + b.double().abs()) - slip).max()) <= 0
+
+
+@pytest.mark.parametrize("H,rows", [(8, 7104), (264, 7105), (512, 9001), (520, 4000), (776, 7104), (1000, 7999), (1024, 8000), (1032, 4440),
+                                    (1280, 5003), (1288, 2220), (1536, 2370), (1544, 1776), (1800, 2500), (2048, 5003), (3000, 300)])
+@pytest.mark.parametrize("with_residual", [False, True])
+def test_layernorm_forward_of_a_row_does_not_depend_on_how_many_there_are(H, rows, with_residual):
+    """Which kernel takes a call depends on the number of rows; the result of a row does not, in any bit."""
+    torch.manual_seed(H)
+    x = (torch.randn(rows, H, device=DEV) * 2 + 1).bfloat16()
+    res = torch.randn(rows, H, device=DEV).bfloat16() if with_residual else None
+    flat = torch.randn(2 * H + 1, device=DEV)
+    for g, b in ((flat[:H], flat[H:2 * H]), (flat[1:H + 1], flat[H + 1:])):      # on and off a 16-byte boundary
+        call = lambda a, e: native.ext().layernorm_fwd(x[a:e], None if res is None else res[a:e], g, b, 1e-5)[:3]
+        whole = call(0, rows)
+        for a, e in ((0, 1), (8, 19), (rows // 2, rows // 2 + 700), (0, min(rows, 2400)), (rows - 300, rows)):
+            for part, want in zip(call(a, e), whole):
+                assert torch.equal(part, want[a:e])
