@@ -301,12 +301,9 @@ Tensor attention_node(const Tensor& q, const Tensor& k, const Tensor& v, int64_t
   return AttentionNode::apply(q, k, v, kv_lens, table, a);
 }
 
-// Which kernel sums the embedding gradient (see set_deterministic_embedding_grad of ops/functional.py): rows in token order, or
-// float atomics.  Read by the threads that run a backward.
-std::atomic<bool> g_embedding_in_order{[] {
-  const char* atomics = std::getenv("SSB_EMBEDDING_GRAD_ATOMICS");
-  return atomics == nullptr || std::string(atomics) != "1";
-}()};
+// Which kernel sums the embedding gradient (set_deterministic_embedding_grad of ops/functional.py): rows in token order, or float
+// atomics.  Read by the threads that run a backward.
+std::atomic<bool> g_embedding_in_order{true};
 
 struct EmbeddingNode : torch::autograd::Function<EmbeddingNode> {
   // The tables are passed for the graph alone; the values come with the arguments.

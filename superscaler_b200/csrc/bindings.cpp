@@ -10,8 +10,6 @@
 
 #include <array>
 #include <atomic>
-#include <cstdlib>
-#include <string>
 
 #include "attention_sm100.cuh"
 #include "gemm_sm100.cuh"
@@ -1011,6 +1009,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding_node", &embedding_node);
   m.def("head_loss_node", &head_loss_node);
   m.def("set_embedding_in_order", [](bool on) { g_embedding_in_order = on; });
+  m.def("embedding_in_order", []() { return g_embedding_in_order.load(); });
   m.def("node_kernels", []() { return g_node_kernels.load(); });
   m.def("node_calls", []() { return g_node_calls.load(); });
   m.def("attn_bwd", &attn_bwd);

@@ -703,9 +703,6 @@ def scaled_softmax(x, scale=1.0, mode=0, mask=None):
 # --------------------------------------------------------------------------------------------
 # Embedding and LM head + cross entropy
 # --------------------------------------------------------------------------------------------
-_DETERMINISTIC_EMBEDDING_GRAD = [os.environ.get("SSB_EMBEDDING_GRAD_ATOMICS", "0") != "1"]
-
-
 class EmbeddingFn(torch.autograd.Function):
     """dropout(W[ids - v0] (0 outside the local vocab range) + P[pos]).  Vocab-parallel ranks all-reduce the
     result outside (reference: runtime/megatron/mpu/layers.py:136-205, flex_ops.py:229-380)."""
@@ -741,7 +738,7 @@ class EmbeddingFn(torch.autograd.Function):
             dP = None
             if P is not None:
                 dP = mgP if mgP is not None else torch.zeros(P.shape, dtype=torch.float32, device=g.device)
-            if _DETERMINISTIC_EMBEDDING_GRAD[0]:
+            if native.ext().embedding_in_order():
                 # every row is summed in token order: repeated runs give bitwise equal gradients
                 if ids.numel() <= native.ext().embedding_group_max_tokens():
                     native.ext().embedding_bwd_grouped(ids.contiguous().view(-1), pos.contiguous().view(-1) if pos is not None
@@ -772,10 +769,12 @@ class EmbeddingFn(torch.autograd.Function):
 def set_deterministic_embedding_grad(on: bool) -> None:
     """Selects how the embedding gradient is scattered on the GPU: every row summed in token order by one block, tokens grouped by
     row (sorted above 65536 tokens; independent of the order of execution, the default), or float atomics (order dependent
-    in the last bit)."""
-    _DETERMINISTIC_EMBEDDING_GRAD[0] = bool(on)
-    if native.available():
-        native.ext().set_embedding_in_order(bool(on))
+    in the last bit).  Set to float atomics at first by SSB_EMBEDDING_GRAD_ATOMICS=1 when this module is imported.  The switch is
+    the extension's: the Python function and the native node read the same one, when a backward runs."""
+    native.when_loaded(lambda ext: ext.set_embedding_in_order(bool(on)))
+
+
+set_deterministic_embedding_grad(os.environ.get("SSB_EMBEDDING_GRAD_ATOMICS", "0") != "1")
 
 
 def set_deterministic(on: bool) -> None:

@@ -16,6 +16,7 @@ import torch
 _PKG_DIR = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 _mod = None
 _err = None
+_on_load = []                             # what was asked of the extension before it was there
 
 
 def _load():
@@ -31,9 +32,19 @@ def _load():
         spec = importlib.util.spec_from_file_location("superscaler_b200._C", cands[0])
         mod = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(mod)
+        for fn in _on_load:
+            fn(mod)
         _mod = mod
     except Exception as e:  # noqa: BLE001 - reported verbatim by ext()
         _err = e
+
+
+def when_loaded(fn) -> None:
+    """Calls ``fn(extension)``: at once when it is loaded, else as soon as it is."""
+    if _mod is not None:
+        fn(_mod)
+    else:
+        _on_load.append(fn)
 
 
 def available() -> bool:
