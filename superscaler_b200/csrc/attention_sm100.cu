@@ -14,6 +14,7 @@
 //             dV += P^T.dO and dK += dS^T.Q accumulate in TMEM.
 //   dQ      : CTA = 128 queries; key blocks of 64; dQ += dS.K accumulates in TMEM.
 #include "attention_device.cuh"
+#include "launch_once.cuh"
 
 namespace ssb {
 
@@ -613,11 +614,6 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, int ldo, int o_col0, cons
   }
 }
 
-template <typename K>
-int set_smem(K kernel, int bytes) {
-  return static_cast<int>(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-}
-
 }  // namespace
 
 // delta[b, h, q] = rowsum(dO * O), the first step of both backward paths.
@@ -655,21 +651,15 @@ int attn_bwd_launch(const void* q, int ldq, const void* k, int ldk, const void* 
   if ((rc = make_tma_2d_bf16(&tv64, v, rk, ldv, ldv, 64, 64))) return rc;
   dim3 grid_kv((p.SK + 127) / 128, p.NH, p.B), grid_q((p.SQ + 127) / 128, p.NH, p.B);
   if (p.HD == 128) {
-    static bool done = false;
-    if (!done) {
-      if ((rc = set_smem(attn_bwd_dkv_kernel<128>, DkvCfg<128>::kSmem))) return rc;
-      if ((rc = set_smem(attn_bwd_dq_kernel<128>, DqCfg<128>::kSmem))) return rc;
-      done = true;
-    }
+    static OncePerDevice<> smem_allowed[2];
+    if ((rc = allow_smem_once(smem_allowed[0], attn_bwd_dkv_kernel<128>, DkvCfg<128>::kSmem))) return rc;
+    if ((rc = allow_smem_once(smem_allowed[1], attn_bwd_dq_kernel<128>, DqCfg<128>::kSmem))) return rc;
     attn_bwd_dkv_kernel<128><<<grid_kv, kAttnThreads, DkvCfg<128>::kSmem, stream>>>(tq64, tk128, tv128, tdo64, pp);
     attn_bwd_dq_kernel<128><<<grid_q, kAttnThreads, DqCfg<128>::kSmem, stream>>>(tq128, tk64, tv64, tdo128, pp);
   } else {
-    static bool done = false;
-    if (!done) {
-      if ((rc = set_smem(attn_bwd_dkv_kernel<64>, DkvCfg<64>::kSmem))) return rc;
-      if ((rc = set_smem(attn_bwd_dq_kernel<64>, DqCfg<64>::kSmem))) return rc;
-      done = true;
-    }
+    static OncePerDevice<> smem_allowed[2];
+    if ((rc = allow_smem_once(smem_allowed[0], attn_bwd_dkv_kernel<64>, DkvCfg<64>::kSmem))) return rc;
+    if ((rc = allow_smem_once(smem_allowed[1], attn_bwd_dq_kernel<64>, DqCfg<64>::kSmem))) return rc;
     attn_bwd_dkv_kernel<64><<<grid_kv, kAttnThreads, DkvCfg<64>::kSmem, stream>>>(tq64, tk128, tv128, tdo64, pp);
     attn_bwd_dq_kernel<64><<<grid_q, kAttnThreads, DqCfg<64>::kSmem, stream>>>(tq128, tk64, tv64, tdo128, pp);
   }

@@ -29,6 +29,7 @@
 #include "gemm_ag_sm100.cuh"
 #include "gemm_epilogue.cuh"
 #include "gemm_sm100.cuh"
+#include "launch_once.cuh"
 
 namespace ssb {
 
@@ -679,8 +680,10 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  static int max_clusters = 0;
-  if (max_clusters == 0) {
+  static OncePerDevice<> resident;
+  int dev = 0, max_clusters = 0;
+  if (const cudaError_t e = cudaGetDevice(&dev)) return static_cast<int>(e);
+  const int rc = resident.get(dev, &max_clusters, [&](int* clusters) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem2);
     if (e != cudaSuccess) return static_cast<int>(e);
     cudaLaunchConfig_t q = {};
@@ -689,14 +692,14 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
     q.dynamicSmemBytes = kSmem2;
     q.attrs = attr;
     q.numAttrs = 1;
-    int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, kernel, &q);
-    if (e != cudaSuccess || n < 1) {
+    e = cudaOccupancyMaxActiveClusters(clusters, kernel, &q);
+    if (e != cudaSuccess || *clusters < 1) {
       (void)cudaGetLastError();
       return -5;
     }
-    max_clusters = n;
-  }
+    return 0;
+  });
+  if (rc) return rc;
   const int num_tiles = ((p.M + 2 * BM2 - 1) / (2 * BM2)) * ((p.N + NH * bn - 1) / (NH * bn));
   int clusters = num_sms / 2;
   if (clusters > max_clusters) clusters = max_clusters;

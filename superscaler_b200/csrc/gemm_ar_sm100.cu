@@ -42,6 +42,7 @@
 #include "common.cuh"
 #include "gemm_ar_sm100.cuh"
 #include "gemm_sm100.cuh"
+#include "launch_once.cuh"
 
 namespace ssb {
 
@@ -523,14 +524,9 @@ int gemm_ar_launch(const void* A, int lda, const void* B, int ldb, int b_mn_majo
   if (rc != 0) return rc;
   rc = !b_mn_major ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, BN, BK) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK, 64);
   if (rc != 0) return rc;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_ar_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(gemm_ar_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    attr_done = true;
-  }
+  static OncePerDevice<> smem_allowed[2];
+  if ((rc = allow_smem_once(smem_allowed[0], gemm_ar_kernel<false>, kSmemBytes))) return rc;
+  if ((rc = allow_smem_once(smem_allowed[1], gemm_ar_kernel<true>, kSmemBytes))) return rc;
   const int grid = num_tiles < num_sms ? num_tiles : num_sms;
   GemmArComm c2 = cm;
   c2.grid = grid;  // the same on every rank: it enters the tile -> owner map

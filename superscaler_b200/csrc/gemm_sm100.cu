@@ -15,6 +15,7 @@
 // epilogue of tile i overlaps the main loop of tile i+1.
 #include "common.cuh"
 #include "gemm_sm100.cuh"
+#include "launch_once.cuh"
 #include "gemm_epilogue.cuh"
 
 #include <atomic>
@@ -387,12 +388,8 @@ int launch_variant(const void* A, int lda, const void* B, int ldb, const GemmPar
   if (rc != 0) return rc;
 
   auto kernel = gemm_bf16_kernel<BN, A_MN, B_MN>;
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    attr_done = true;
-  }
+  static OncePerDevice<> smem_allowed;
+  if ((rc = allow_smem_once(smem_allowed, kernel, Cfg::kSmemBytes))) return rc;
   const int num_tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   if (p.k_splits > 1) {
     // every slice writes a plain fp32 [M, N] block of the workspace; the fold adds them, in slice order, into D

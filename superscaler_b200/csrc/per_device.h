@@ -1,4 +1,4 @@
-// One value per device, made at its first use and kept for the life of the process.
+// Values per device, made at their first use and kept for the life of the process.
 #pragma once
 #include <atomic>
 #include <memory>
@@ -33,6 +33,25 @@ class PerDevice {
     std::unique_ptr<T> value;
   };
   Slot slots_[kDevices];
+};
+
+// A positive number per device that the CUDA runtime is asked for once, or what has to be set there once (a kernel's attributes
+// belong to a device).  `make(int* value)` returns an error code, which is handed on and not kept; threads that come together
+// may each ask.  A value of 0 means: not asked yet.
+template <int kDevices = 64>
+class OncePerDevice {
+ public:
+  template <class Make>
+  int get(int device, int* value, Make make) {
+    std::atomic<int>& kept = values_[device];
+    if ((*value = kept.load(std::memory_order_acquire)) != 0) return 0;
+    const int rc = make(value);
+    if (rc == 0) kept.store(*value, std::memory_order_release);
+    return rc;
+  }
+
+ private:
+  std::atomic<int> values_[kDevices] = {};
 };
 
 }  // namespace ssb

@@ -67,3 +67,45 @@ def test_lazily_made_device_values_go_through_it():
         body = body[:body.index("\n}")]
         assert "PerDevice<" in body and ".get(" in body
     assert not re.search(r"static\s+std::vector<\s*Tensor\s*>", code)
+
+
+ONCE = r"""
+#include "per_device.h"
+#include <cstdio>
+#include <thread>
+#include <vector>
+int main() {
+  static ssb::OncePerDevice<> once;
+  int asked[3] = {}, value = 0;
+  auto ask = [&](int device, int rc, int answer) {
+    return once.get(device, &value, [&](int* v) { asked[device]++; *v = answer; return rc; });
+  };
+  if (ask(0, 0, 7) != 0 || value != 7 || ask(0, 0, 9) != 0 || value != 7 || asked[0] != 1) std::puts("not kept");
+  if (ask(1, 0, 8) != 0 || value != 8 || asked[1] != 1) std::puts("the other device was not asked");
+  if (ask(2, -5, 3) != -5 || ask(2, 0, 4) != 0 || value != 4 || asked[2] != 2) std::puts("an error was kept");
+  static ssb::OncePerDevice<> shared;
+  std::vector<std::thread> threads;
+  for (int t = 0; t < 16; ++t)
+    threads.emplace_back([&] {
+      for (int d = 0; d < 64; ++d) {
+        int v = 0;
+        if (shared.get(d, &v, [&](int* x) { *x = d + 1; return 0; }) != 0 || v != d + 1) std::puts("wrong value");
+      }
+    });
+  for (auto& t : threads) t.join();
+  std::puts("done");
+}
+"""
+
+
+def test_what_is_set_once_is_set_on_every_device(tmp_path):
+    (tmp_path / "t.cpp").write_text(ONCE)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-pthread", f"-I{CSRC}", str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    assert subprocess.run([str(tmp_path / "t")], capture_output=True, text=True, check=True, timeout=60).stdout == "done\n"
+
+
+def test_launchers_keep_no_flag_of_the_process():
+    """A function-local number or flag that a launcher sets belongs to the process; what it stands for belongs to a device."""
+    for path in sorted(CSRC.glob("*.cu")):
+        code = re.sub(r"//[^\n]*", "", path.read_text())
+        assert not re.search(r"^\s+static\s+(?:bool|int)\s+\w+\s*=", code, re.M), path.name
