@@ -19,3 +19,15 @@ def pytest_collection_modifyitems(config, items):
     for item in items:
         if "gpu" in item.keywords:
             item.add_marker(skip)
+
+
+@pytest.fixture(autouse=True)
+def embedding_switch_as_found():
+    """`set_deterministic(False)` also selects the float atomics of the embedding gradient, which the tests that follow must not
+    inherit: training runs that are compared with one another would differ in the last bits."""
+    native = sys.modules.get("superscaler_b200.ops.native")
+    ext = getattr(native, "_mod", None)
+    before = ext.embedding_in_order() if ext is not None else None
+    yield
+    if before is not None:
+        ext.set_embedding_in_order(before)
