@@ -21,7 +21,7 @@ namespace ssb {
 int gemm_bf16_launch(const void* A, int lda, int a_mn_major, const void* B, int ldb, int b_mn_major,
                      const GemmParams& p, int num_sms, cudaStream_t stream);
 int gemm_route(const GemmParams& p, int num_sms, int* bn, int* slices);
-int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms);
+int gemm2_tile_columns(int M, int N, int K, bool b_mn, bool whole_lines, bool out_fp32, int num_sms);
 void gemm_set_pair_mode(int mode);
 int gemm_get_pair_mode();
 int layernorm_fwd_launch(const void* x, const void* residual, const float* gamma, const float* beta, void* y,
@@ -238,6 +238,13 @@ std::tuple<int64_t, int64_t, int64_t> gemm_route(int64_t M, int64_t N, int64_t K
   int bn = 0, slices = 0;
   const int route = ssb::gemm_route(p, static_cast<int>(sms), &bn, &slices);
   return {route, route == 2 ? bn : 0, route == 2 ? slices : 0};
+}
+
+// Columns of the output tile of a product that goes to the pairs of SMs (whole_lines: the operands' rows start on 128 bytes); needs
+// no device.
+int64_t gemm_pair_columns(int64_t M, int64_t N, int64_t K, bool out_fp32, int64_t sms, bool b_mn, bool whole_lines) {
+  return ssb::gemm2_tile_columns(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), b_mn, whole_lines, out_fp32,
+                                 static_cast<int>(sms));
 }
 
 std::vector<Tensor> layernorm_fwd(const Tensor& x, const OptTensor& residual, const Tensor& gamma, const Tensor& beta,
@@ -970,9 +977,8 @@ Tensor status() { return status_tensor(); }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_route", &gemm_route);
-  m.def("gemm_pair_columns", [](int64_t M, int64_t N, int64_t K, bool out_fp32, int64_t sms) {
-    return ssb::gemm2_tile_columns(static_cast<int>(M), static_cast<int>(N), static_cast<int>(K), out_fp32, static_cast<int>(sms));
-  });
+  m.def("gemm_pair_columns", &gemm_pair_columns, py::arg("M"), py::arg("N"), py::arg("K"), py::arg("out_fp32"), py::arg("sms"),
+        py::arg("b_mn") = false, py::arg("whole_lines") = true);
   m.def("gemm", &gemm);
   m.def("gemm_allreduce", &gemm_allreduce);
   m.def("allgather_gemm", &allgather_gemm);

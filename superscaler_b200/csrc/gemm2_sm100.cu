@@ -726,17 +726,33 @@ bool wide_tile(int M, int N, int K, bool out_fp32, int num_sms) {
   return N >= 512 && K >= (out_fp32 ? kWideKFp32 : kWideK) && 2 * ((wide + pairs - 1) / pairs) <= (narrow + pairs - 1) / pairs;
 }
 
-// Columns of a tile, in steps of the 32 that a pair's instruction takes: fewer than 256 where the rounds of narrower tiles are shorter
-// by a tenth at least (a narrower tile moves more per operation).  640 output channels in three tiles: a sixth of 256-column tiles
-// is padding.  16 x 28 x 28 of 640 channels, 3 x 3, with 256 -> 224 columns: forward 67.6 -> 62.0 us, input gradient 68.5 -> 64.4.
-int tile_columns(int M, int N, int num_sms) {
-  const int pairs = num_sms / 2;
-  auto time = [&](int bn) { return ((M + 255LL) / 256 * ((N + bn - 1) / bn) + pairs - 1) / pairs * bn; };
+// Columns of a tile, in steps of the 32 that a pair's instruction takes: fewer than 256 where the rounds of narrower tiles are enough
+// shorter.  A round costs its columns and a part that does not shrink with them (A's rows, the epilogue; of a B read MN-major
+// always 128 columns a CTA), measured like BN2 more columns or twice that.  Single call / sustained under the power cap, 256
+// columns -> fewer, us:
+//   taken      K-major B: 2048 x 3072 over 2048 34.8 -> 30.7 / 28.7 -> 26.3 (192), 2560 x 2048 over 4096 56.3 -> 47.1 / 47.1 -> 40.7 (160),
+//              4096 x 5120 over 4096 134 -> 120 / 145 -> 141 (224), 12544 x 640 64.4 -> 60.3 / 67.5 -> 62.8 (224: a sixth was padding);
+//              MN-major: 2560 x 4096 over 4096 82.9 -> 72.7 / 79.1 -> 75.8 (192), fp32 and added to 91.0 -> 82.9 / 90.1 -> 89.2
+//   not taken  8192 x 2560 over 2048 72.7 -> 76.8 / 75.8 -> 79.8 (160: seven rounds for five), 16384 x 1536 MN-major over 4096 216 -> 194 /
+//              174 -> 178 (192: seven for six), 2048 x 8192 MN-major fp32 over 4096 136 -> 116 / 130 -> 134 (224: more tiles, no padding)
+//   short      reductions end before a tile's epilogue does: 4096 x 5120 over 512 28.6 -> 29.1 sustained, 2048 x 10240 28.7 -> 29.3
+//   off lines  rows off 128 bytes cost the narrower tile of an MN-major B more than it saves: 3064 x 1984 over 4096 57.4 -> 65.3 (192),
+//              with 3072 rows 54.3 -> 53.1
+// 16 x 28 x 28 of 640 channels, 3 x 3, 256 -> 224: forward 67.6 -> 62.0, input gradient 68.5 -> 64.4.
+int tile_columns(int M, int N, int K, bool b_mn, bool whole_lines, int num_sms) {
+  if (b_mn && !whole_lines) return BN2;
+  const long long pairs = num_sms / 2, m = (M + 255LL) / 256;
+  auto n = [&](int bn) { return (N + bn - 1LL) / bn; };
+  auto rounds = [&](int bn) { return (m * n(bn) + pairs - 1) / pairs; };
+  auto cost = [&](int bn) { return rounds(bn) * (bn + (b_mn ? 2 * BN2 : BN2)); };
   int best = BN2;
   for (int bn = BN2 - 32; bn >= 160; bn -= 32)
-    if (10 * time(bn) <= 9 * time(BN2) && time(bn) < time(best)) best = bn;
-  return best;
+    if (cost(bn) < cost(best)) best = bn;
+  const bool less_padding = 10 * n(best) * best <= 9 * n(BN2) * BN2;
+  const int percent = K < 1024 && rounds(BN2) > 2 ? 90 : !b_mn ? 95 : less_padding ? 96 : 93;
+  return 100 * cost(best) <= percent * cost(BN2) ? best : BN2;
 }
+bool whole_lines(int lda, int ldb) { return lda % 64 == 0 && ldb % 64 == 0; }
 
 template <bool A_MN, bool B_MN, bool GATHER>
 int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams& p, const GemmAgComm& cm, int num_sms,
@@ -753,7 +769,7 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
   }
   if (rc != 0) return rc;
   const bool wide = !GATHER && wide_tile(p.M, p.N, p.K, p.out_fp32, num_sms);
-  const int bn = GATHER || wide ? BN2 : tile_columns(p.M, p.N, num_sms);
+  const int bn = GATHER || wide ? BN2 : tile_columns(p.M, p.N, p.K, B_MN, whole_lines(lda, ldb), num_sms);
   rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, bn / 2, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
   if (rc != 0) return rc;
   if constexpr (!GATHER)
@@ -764,8 +780,8 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
 }  // namespace
 
 // Columns of the output tile for a product that this kernel takes.
-int gemm2_tile_columns(int M, int N, int K, bool out_fp32, int num_sms) {
-  return wide_tile(M, N, K, out_fp32, num_sms) ? 2 * BN2 : tile_columns(M, N, num_sms);
+int gemm2_tile_columns(int M, int N, int K, bool b_mn, bool whole_lines, bool out_fp32, int num_sms) {
+  return wide_tile(M, N, K, out_fp32, num_sms) ? 2 * BN2 : tile_columns(M, N, K, b_mn, whole_lines, num_sms);
 }
 
 // Same contract as gemm_bf16_launch; callers pick this variant for outputs of at least 256 x 256.
@@ -802,7 +818,7 @@ int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, 
   CUtensorMap ta, tb;
   int rc;
   if ((rc = make_tma_im2col_bf16(&ta, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BM2))) return rc;
-  const int bn = tile_columns(p.M, p.N, num_sms);
+  const int bn = tile_columns(p.M, p.N, p.K, false, true, num_sms);
   if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, bn / 2, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
   return launch_maps<false, false, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
@@ -818,7 +834,8 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
   if ((rc = make_tma_im2col_bf16(&ta, dy, N, Ho, Wo, Kout, lh, lw, -pad, -pad, 1, BM2))) return rc;
   if ((rc = make_tma_2d_bf16(&tb, w, Kout, static_cast<uint64_t>(KH) * KW * C, ldw, BK2, 64))) return rc;
   ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
-  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, tile_columns(p.M, p.N, num_sms), num_sms, stream);
+  const int bn = tile_columns(p.M, p.N, p.K, true, whole_lines(Kout, ldw), num_sms);
+  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
 }
 
 // dw[K, KH * KW * C] from dy[N Ho Wo, K] and x; p describes the GEMM [K, KH * KW * C] with K = N Ho Wo.

@@ -58,3 +58,23 @@ RESIDUAL, DGELU, WGRAD = dict(bias=EVEN, residual=EVEN), dict(act=F.ACT_DGELU, a
 ])
 def test_the_faster_kernel_takes_the_call(M, N, K, call, one_cta, cluster):
     assert route(M, N, K, **call)[0] == (CLUSTER if cluster < one_cta else ONE_CTA)
+
+
+@pytest.mark.parametrize("M,N,K,b_mn,lines,columns", [
+    # rounds a fifth shorter and more, in either layout
+    (2048, 3072, 2048, False, True, 192), (2560, 2048, 4096, False, True, 160), (2560, 4096, 4096, True, True, 192),
+    (4096, 1280, 4096, True, True, 160), (4096, 768, 512, False, True, 192),
+    # an eighth shorter: less of the output is padding, or B is read K-major
+    (12544, 640, 5760, False, True, 224), (12544, 640, 5760, True, True, 224), (4096, 5120, 4096, False, True, 224),
+    (4096, 5120, 4096, True, True, 256), (2048, 8192, 4096, True, True, 256),
+    # more rounds of narrower tiles, which move more for each operation
+    (8192, 2560, 2048, False, True, 256), (16384, 1280, 4096, True, True, 256), (4096, 6144, 4096, False, True, 256),
+    (8192, 3072, 4096, True, True, 256), (16384, 1536, 2048, False, True, 256),
+    # a reduction that ends before the epilogue does, over several rounds
+    (4096, 5120, 512, False, True, 256), (2048, 10240, 512, False, True, 256),
+    # operands whose rows start off 128 bytes
+    (2560, 4096, 4096, True, False, 256), (2560, 2048, 4096, False, False, 160),
+])
+def test_columns_of_a_tile_on_pairs(M, N, K, b_mn, lines, columns):
+    """Narrower tiles only where they are the faster ones, also under the power cap (times in csrc/gemm2_sm100.cu)."""
+    assert native.ext().gemm_pair_columns(M, N, K, False, SMS, b_mn, lines) == columns
