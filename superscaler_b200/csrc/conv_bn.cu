@@ -248,20 +248,16 @@ bn_stats_final_kernel(const float* __restrict__ part, int slices, int C, long lo
 // reads (a kilobyte per warp and array) kept the L1 busy while DRAM ran at 11 % of its peak.
 constexpr int kBnRowsPerBlock = 32;
 
-// Eight per-channel values, c0 a multiple of 8: two loads where the array starts on 16 bytes.
-__device__ __forceinline__ void ldc8(const float* __restrict__ p, int c0, float (&v)[8]) {
-  if ((reinterpret_cast<uintptr_t>(p) & 15) == 0) {
-    const float4 a = __ldg(reinterpret_cast<const float4*>(p + c0)), b = __ldg(reinterpret_cast<const float4*>(p + c0) + 1);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __ldg(p + c0 + j);
-  }
+// Eight per-channel values from 16 bytes on.
+__device__ __forceinline__ void ldc8(const float* p, float (&v)[8]) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+  v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 
-// per_sm: blocks an SM.  Six where a block's constants weigh as much as its rows (forward, 12544 x 640 12.0 -> 7.3 us together with the loads
-// above); the backward's pass is faster with the two rounds of sixteen (23.4 against 26 us with its column sums).
+// per_sm: blocks an SM.  Six where a block's constants weigh as much as its rows: forward, 12544 x 640 12.0 -> 7.0 us together with 16-byte
+// loads of the constants, one branch for all of them and the first row ahead of it (784 x 512 2.3; 2.8 with a branch for each array,
+// 2.5 with 4-byte loads).  The backward's pass is faster with the two rounds of sixteen (23.4 against 26 us with its column sums).
 inline dim3 bn_grid(long long rows, int C, int num_sms, int per_sm) {
   const int gx = (C / 8 + 7) / 8;
   long long gy = (rows + kBnRowsPerBlock - 1) / kBnRowsPerBlock;
@@ -280,21 +276,36 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
   const int cv = blockIdx.x * 8 + (threadIdx.x & 7);
   if (cv >= C / 8) return;
   const int c0 = cv * 8;
+  const long long stride = static_cast<long long>(gridDim.y) * kBnRowsPerBlock;
+  long long r = static_cast<long long>(blockIdx.y) * kBnRowsPerBlock + (threadIdx.x >> 3);
+  if (r >= rows) return;
+  const uint4 first = ldq8(x + r * C + c0);  // on its way with the constants: short calls are this chain
   float a[8], b[8];
   {
     float g[8], m[8];
-    ldc8(rstd, c0, a);
-    ldc8(gamma, c0, g);
-    ldc8(beta, c0, b);
-    ldc8(mean, c0, m);
+    const uintptr_t any = reinterpret_cast<uintptr_t>(rstd) | reinterpret_cast<uintptr_t>(gamma) |
+                          reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(mean);
+    if ((any & 15) == 0) {
+      ldc8(rstd + c0, a);
+      ldc8(gamma + c0, g);
+      ldc8(beta + c0, b);
+      ldc8(mean + c0, m);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        a[j] = __ldg(rstd + c0 + j);
+        g[j] = __ldg(gamma + c0 + j);
+        b[j] = __ldg(beta + c0 + j);
+        m[j] = __ldg(mean + c0 + j);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       a[j] = a[j] * g[j];
       b[j] = b[j] - m[j] * a[j];
     }
   }
-  const long long stride = static_cast<long long>(gridDim.y) * kBnRowsPerBlock;
-  long long r = static_cast<long long>(blockIdx.y) * kBnRowsPerBlock + (threadIdx.x >> 3);
+  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
   auto finish = [&](long long row, const uint4& qx, const uint4& qr) {
     float f[8], res[8];
     unpack8(qx, f);
@@ -306,17 +317,18 @@ bn_apply_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __rest
     }
     st8(y + row * C + c0, f);
   };
-  const uint4 none = make_uint4(0u, 0u, 0u, 0u);
-  for (; r + 3 * stride < rows; r += 4 * stride) {   // four independent rows in flight per thread, packed until they are used
+  auto other = [&](long long row) { return residual != nullptr ? ldq8(residual + row * C + c0) : none; };
+  finish(r, first, other(r));
+  for (r += stride; r + 3 * stride < rows; r += 4 * stride) {   // four independent rows in flight per thread, packed until they are used
     uint4 f[4], q[4];
 #pragma unroll
     for (int u = 0; u < 4; ++u) f[u] = ldq8(x + (r + u * stride) * C + c0);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) q[u] = residual != nullptr ? ldq8(residual + (r + u * stride) * C + c0) : none;
+    for (int u = 0; u < 4; ++u) q[u] = other(r + u * stride);
 #pragma unroll
     for (int u = 0; u < 4; ++u) finish(r + u * stride, f[u], q[u]);
   }
-  for (; r < rows; r += stride) finish(r, ldq8(x + r * C + c0), residual != nullptr ? ldq8(residual + r * C + c0) : none);
+  for (; r < rows; r += stride) finish(r, ldq8(x + r * C + c0), other(r));
 }
 
 // Backward partials over a row slice: sum g and sum g * xhat, with g = dy masked by (y > 0) when relu.

@@ -91,3 +91,24 @@ def test_pooling(shape):
     ya.backward(torch.ones_like(ya))
     hw = shape[1] * shape[2]
     assert rel(ya, x.float().mean((1, 2))) < 8e-3 and rel(xa.grad, torch.full_like(x.float(), 1 / hw)) < 8e-3
+
+
+@pytest.mark.parametrize("rows,Cn", [(1, 8), (33, 72), (784, 512), (4096, 24), (30000, 640)])      # one row a thread to several
+@pytest.mark.parametrize("res", [False, True])
+def test_batch_norm_constants_start_anywhere(rows, Cn, res):
+    """The element-wise pass reads the constants in pieces of 16 bytes, or one by one where any of them starts elsewhere: the same
+    bits, within a rounding to bf16 (2^-8 of the terms' magnitudes) of 64-bit arithmetic."""
+    torch.manual_seed(rows)
+    x = torch.randn(rows, Cn, device=DEV).bfloat16()
+    r = torch.randn(rows, Cn, device=DEV).bfloat16() if res else None
+    flat = torch.rand(4, Cn + 1, device=DEV) + 0.5
+    odd = [torch.empty(Cn + 1, device=DEV)[1:].copy_(f[:Cn]) for f in flat]
+    even = [f[:Cn].clone() for f in flat]
+    want = native.ext().bn_apply(x, r, *even, True)
+    for i in range(4):
+        one = even[:i] + odd[i:i + 1] + even[i + 1:]
+        assert torch.equal(native.ext().bn_apply(x, r, *one, True), want)
+    mean, rstd, g, b = (t.double() for t in even)
+    terms = ((x.double() - mean) * rstd * g, b, r.double() if res else torch.zeros((), device=DEV).double())
+    size = x.double().abs() * rstd * g + mean * rstd * g + b + terms[2].abs()
+    assert float(((want.double() - sum(terms).clamp_min(0)).abs() - 2.0 ** -8 * size).max()) <= 0
