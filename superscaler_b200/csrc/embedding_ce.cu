@@ -264,7 +264,8 @@ constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per 
 
 // AHEAD: the next four loads of a thread are under way while it works on the last four, in rows of which it has several rounds:
 // 4096 rows x 51200 193 -> 177 us, x 40000 150 -> 134, x 32000 116 -> 106 (eight loads at a time instead: 201, 152, 109; one round
-// is slower for it, x 2048 12.3 -> 13.1).
+// is slower for it, x 2048 12.3 -> 13.1).  Few rows, 512 threads (one round up to 16384 columns): 8 x 16000 3.99 -> 4.16, 64 x 16384 4.10 ->
+// 4.19, but 148 x 16000 5.54 -> 5.43, 296 x 16384 8.09 -> 7.78; 8 x 18432 4.41 -> 4.51, 148 x 18432 6.65 -> 6.03, 64 x 32000 6.66 -> 6.13.
 template <int T, bool AHEAD>
 __global__ void __launch_bounds__(T, 1024 / T)
 ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __restrict__ targets,
@@ -368,7 +369,7 @@ int ce_fused_launch(void* logits, int ld, const long long* targets, const float*
   // threads 9.5).  Rows that all fit on the chip at once are a matter of latency: 16 rows of 8192 take 4.6 us with 128 threads
   // and 3.8 with 512.
   const bool few = rows <= 2LL * num_sms;
-  if (V > 36 * 1024 || (few && V > 14 * 1024)) return launch(ce_fused_kernel<512, true>, 512);
+  if (V > 36 * 1024 || (few && (V > 16 * 1024 || (V > 14 * 1024 && rows >= num_sms)))) return launch(ce_fused_kernel<512, true>, 512);
   if (few) return launch(ce_fused_kernel<512, false>, 512);
   return V > 14 * 1024 ? launch(ce_fused_kernel<256, true>, 256) : launch(ce_fused_kernel<128, false>, 128);
 }
