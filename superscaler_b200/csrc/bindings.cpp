@@ -34,7 +34,7 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
                          int accumulate_wgrad, int rows, int H, int* status, int num_sms, cudaStream_t stream);
 int colsum_tickets();
 int colsum_part_rows(int rows);
-int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N,
+int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N, int num_sms,
                   cudaStream_t stream);
 int elementwise_launch(int op, const void* x, const void* a, const void* bias, void* out, long long rows, int N,
                        float dropout_p, unsigned long long seed, int num_sms, cudaStream_t stream);
@@ -292,7 +292,7 @@ void colsum(const Tensor& a, Tensor& out, bool accumulate) {
   const int rows = static_cast<int>(a.size(0)), N = static_cast<int>(a.size(1));
   Tensor part = torch::empty({ssb::colsum_part_rows(rows), N}, torch::dtype(torch::kFloat32).device(a.device()));
   check_launch(ssb::colsum_launch(a.data_ptr(), static_cast<int>(a.stride(0)), out.data_ptr<float>(),
-                                  part.data_ptr<float>(), ticket_tensor().data_ptr<int>(), accumulate, rows, N,
+                                  part.data_ptr<float>(), ticket_tensor().data_ptr<int>(), accumulate, rows, N, num_sms(),
                                   cur_stream()),
                "colsum");
 }

@@ -10,7 +10,9 @@
 #include "common.cuh"
 
 namespace ssb {
-int ln_bwd_slices(int rows);  // the row partition of the regular column sum, so both variants add in one order
+// Slices of the rows (of 256 at least, 128 at most).  The regular column sum takes them too for matrices it cannot read 16 bytes at a
+// time, and adds in this order there; elsewhere it has slices of its own.
+int ln_bwd_slices(int rows);
 }
 
 namespace {

@@ -1099,16 +1099,16 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   return static_cast<int>(cudaGetLastError());
 }
 
-// out[N] (+)= column sums of a[rows, N]; `part` is scratch of ln_bwd_slices(rows) x N floats; `tickets` holds
-// kColsumTickets zero-initialised counters that every call leaves at zero.
-// Rows of N partial sums that a call needs as scratch (16-byte aligned).
+// Rows of N partial sums that a call of colsum_launch needs as scratch, whichever of its kernels takes it.
 int colsum_part_rows(int rows) {
   const int most = (rows + kColsumMinRows - 1) / kColsumMinRows, two_pass = ln_bwd_slices(rows);
   const int one_pass = most < kColsumMaxSlices ? most : kColsumMaxSlices;
   return one_pass > two_pass ? one_pass : two_pass;
 }
 
-int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N,
+// out[N] (+)= column sums of a[rows, N]; `part` is scratch of colsum_part_rows(rows) x N floats, 16-byte aligned; `tickets` holds
+// kColsumTickets zero-initialised counters that every call leaves at zero.
+int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets, int accumulate, int rows, int N, int num_sms,
                   cudaStream_t stream) {
   if (N % 2 || lda % 2) return -3;
   const int slices = ln_bwd_slices(rows);
@@ -1116,7 +1116,7 @@ int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets,
   const int colblocks = (N + 255) / 256;
   if (N % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && colblocks <= kColsumTickets &&
       tickets != nullptr) {
-    int sl = 148 * kColsumBlocks / colblocks;
+    int sl = num_sms * kColsumBlocks / colblocks;
     const int most = (rows + kColsumMinRows - 1) / kColsumMinRows;
     sl = sl > kColsumMaxSlices ? kColsumMaxSlices : sl;
     sl = sl > most ? most : sl;
