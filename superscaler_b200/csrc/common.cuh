@@ -408,7 +408,8 @@ __device__ __forceinline__ uint32_t spread_sign_bytes(uint32_t x, uint32_t sel) 
 }
 
 // The mask of dropout_keep4 as the carries of four byte additions: bit 7 of byte i set, element 4 * group + i is dropped (the other
-// bits mean nothing).  No extraction and comparison per element: lookup of 16384 x 2048 with dropout 34.4 -> 33.7 us, its
+// bits mean nothing).  No extraction and comparison per element, which only the epilogue of the cluster GEMM is faster with (512 x
+// 1024 over 1024 8.63 us, 8.77 with this): lookup of 16384 x 2048 with dropout 34.4 -> 33.7 us, its
 // gradient 71.6 -> 70.7.
 __device__ __forceinline__ uint32_t dropout_drop4(uint64_t seed, uint64_t group, uint32_t keep16) {
   const uint32_t s32 = static_cast<uint32_t>(seed) ^ (static_cast<uint32_t>(seed >> 32) * 0x85EBCA6Bu);
@@ -423,6 +424,23 @@ __device__ __forceinline__ void dropout_apply4(float* v, uint32_t drop, float sc
 #pragma unroll
   for (int i = 0; i < 4; ++i)
     v[i] = __uint_as_float(__float_as_uint(v[i] * scale) & ~spread_sign_bytes(drop, 0x8888u + 0x1111u * i));
+}
+
+// 8 bf16 values <-> 8 floats
+__device__ __forceinline__ void unpack8(const uint4 q, float* f) {
+  float2 t;
+  t = unpack_bf16x2(q.x); f[0] = t.x; f[1] = t.y;
+  t = unpack_bf16x2(q.y); f[2] = t.x; f[3] = t.y;
+  t = unpack_bf16x2(q.z); f[4] = t.x; f[5] = t.y;
+  t = unpack_bf16x2(q.w); f[6] = t.x; f[7] = t.y;
+}
+__device__ __forceinline__ uint4 pack8(const float* f) {
+  uint4 q;
+  q.x = pack_bf16x2(f[0], f[1]);
+  q.y = pack_bf16x2(f[2], f[3]);
+  q.z = pack_bf16x2(f[4], f[5]);
+  q.w = pack_bf16x2(f[6], f[7]);
+  return q;
 }
 
 // Two fp32 operations per instruction (the same rounding as the scalar forms).

@@ -18,17 +18,8 @@ namespace ssb {
 namespace {
 
 __device__ __forceinline__ uint4 ldq8(const __nv_bfloat16* p) { return *reinterpret_cast<const uint4*>(p); }
-__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
-  float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
 __device__ __forceinline__ void ld8(const __nv_bfloat16* p, float (&f)[8]) { unpack8(ldq8(p), f); }
-__device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) {
-  uint4 q;
-  q.x = pack_bf16x2(f[0], f[1]); q.y = pack_bf16x2(f[2], f[3]);
-  q.z = pack_bf16x2(f[4], f[5]); q.w = pack_bf16x2(f[6], f[7]);
-  *reinterpret_cast<uint4*>(p) = q;
-}
+__device__ __forceinline__ void st8(__nv_bfloat16* p, const float (&f)[8]) { *reinterpret_cast<uint4*>(p) = pack8(f); }
 
 struct ConvGeom {
   int N, H, W, C, KH, KW, stride, pad, Ho, Wo, Kpad;  // Kpad = row length of the patch matrix (>= KH*KW*C)

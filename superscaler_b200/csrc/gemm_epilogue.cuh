@@ -7,23 +7,6 @@
 
 namespace ssb {
 
-// 8 bf16 values <-> 8 floats
-__device__ __forceinline__ void unpack8(const uint4 q, float* f) {
-  float2 t;
-  t = unpack_bf16x2(q.x); f[0] = t.x; f[1] = t.y;
-  t = unpack_bf16x2(q.y); f[2] = t.x; f[3] = t.y;
-  t = unpack_bf16x2(q.z); f[4] = t.x; f[5] = t.y;
-  t = unpack_bf16x2(q.w); f[6] = t.x; f[7] = t.y;
-}
-__device__ __forceinline__ uint4 pack8(const float* f) {
-  uint4 q;
-  q.x = pack_bf16x2(f[0], f[1]);
-  q.y = pack_bf16x2(f[2], f[3]);
-  q.z = pack_bf16x2(f[4], f[5]);
-  q.w = pack_bf16x2(f[6], f[7]);
-  return q;
-}
-
 template <int W>
 __device__ __forceinline__ void gemm_epilogue_chunk(const GemmParams& p, int row, int n0, const uint32_t (&r)[W],
                                                     uint32_t keep16, float drop_scale) {

@@ -18,11 +18,6 @@ namespace {
 
 constexpr int kLnWarpsPerBlock = 4;
 
-__device__ __forceinline__ void unpack8(const uint4& q, float (&f)[8]) {
-  const float2 a = unpack_bf16x2(q.x), b = unpack_bf16x2(q.y), c = unpack_bf16x2(q.z), d = unpack_bf16x2(q.w);
-  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y; f[4] = c.x; f[5] = c.y; f[6] = d.x; f[7] = d.y;
-}
-
 // Rows with a residual, and rows of 513 to 768 and of more than 2048 columns, that fit in the registers of a warp, read once: up to VPL
 // vectors of 8 bf16 per lane; FULL = false: the last one, or for VPL > 8 the last few, are not there for every lane.  Values are
 // kept as fp32 up to VPL 8, packed beyond that.  Lengths that are not 512, 1024, 2048 or 4096 used to take the kernel for any
@@ -149,7 +144,7 @@ __device__ __forceinline__ uint4 ln_values8(const float (&v)[8], float mean, flo
   float o[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) o[j] = fmaf((v[j] - mean) * rstd, g[j], b[j]);
-  return make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+  return pack8(o);
 }
 
 // A warp per row, up to VPL vectors per lane.  FULL, WIDE: every lane has all of them, gamma and beta start on 16 bytes.  HOLD: gamma and
@@ -722,7 +717,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] += t[j];
           }
-          dxr[v] = make_uint4(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]), pack_bf16x2(o[4], o[5]), pack_bf16x2(o[6], o[7]));
+          dxr[v] = pack8(o);
         }
       }
       ring.release(c, lane);
