@@ -29,6 +29,6 @@ def test_warps_that_give_up_still_meet_their_partners(path):
 def test_copies_of_the_layernorm_ring_land_before_the_block_ends():
     """The thread that issues the bulk copies waits, with a limit, for the last ones of every stage after its loop."""
     code = re.sub(r"//[^\n]*", "", (CSRC / "layernorm.cu").read_text())
-    producer = code[code.index("if (warp == kLnWarps)"):]
-    producer = producer[:producer.index("} else {")]
-    assert "bulk_load(" in producer and "mbar_try_wait(&bars[" in producer[producer.rindex("bulk_load("):]
+    (kernel,) = [k for k in re.split(r"\b__global__\b", code)[1:] if "bulk_load(" in k]
+    behind = kernel[kernel.rindex("bulk_load("):]
+    assert "mbar_try_wait(&bars[" in behind[:behind.index("} else {")]

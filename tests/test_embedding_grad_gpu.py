@@ -88,3 +88,28 @@ def test_tables_of_no_columns(places):
         y.backward(torch.empty_like(y))
         assert W.grad.shape == W.shape and (not places or P.grad.shape == P.shape)
     assert native.check_status() == 0
+
+
+@pytest.mark.parametrize("H", [8, 264, 2048, 2056, 4104])                       # several tokens a block, one pass, two, three
+@pytest.mark.parametrize("tokens", [1, 889, 2500])
+@pytest.mark.parametrize("p", [0.1, 0.996])
+def test_lookup_dropout(H, tokens, p):
+    """The mask is the element-wise kernel's for the same seed and flat index; sum and scale are fp32, rounded once; every gradient
+    kernel drops what the forward dropped."""
+    torch.manual_seed(H + tokens)
+    ext = native.ext()
+    W, P = torch.randn(3000, H, device=DEV).bfloat16(), torch.randn(77, H, device=DEV).bfloat16()
+    ids, pos = torch.randperm(3000, device=DEV)[:tokens], torch.randint(0, 77, (tokens,), device=DEV)
+    ones = torch.ones(tokens, H, device=DEV).bfloat16()
+    kept = ext.elementwise(F.EW_DROPOUT, ones, None, None, p, 9) != 0
+    scale = torch.tensor(256.0 / max(1, int((1 - p) * 256 + 0.5)), device=DEV)
+    zero = torch.zeros((), device=DEV)
+    y = ext.embedding_fwd(ids, pos, W, P, 0, p, 9)
+    assert torch.equal(y, torch.where(kept, (W[ids].float() + P[pos].float()) * scale, zero).bfloat16())
+    want = torch.zeros(3000, H, device=DEV)
+    want[ids] = torch.where(kept, scale, zero)
+    grouped, atomic = torch.zeros_like(want), torch.zeros_like(want)
+    ext.embedding_bwd_grouped(ids, None, ones, grouped, None, 0, p, 9)
+    ext.embedding_bwd(ids, None, ones, atomic, None, 0, p, 9)
+    for dW in (grouped, atomic, sorted_grad(ids, torch.zeros_like(want), 0, ones, p, 9)):
+        assert torch.equal(dW, want)
