@@ -569,7 +569,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
                      const float* __restrict__ gamma, const float* __restrict__ mean, const float* __restrict__ rstd,
                      const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                      float* __restrict__ part_g, float* __restrict__ part_b, int rows, int H, int* __restrict__ status) {
-  constexpr int WPR = Cfg::WPR, NW = Cfg::NW, RPB = Cfg::kRows;
+  constexpr int WPR = Cfg::WPR, kLnWarps = Cfg::NW, RPB = Cfg::kRows;
   constexpr int VPL = 2;       // vectors per lane
   extern __shared__ __align__(128) uint8_t ring_smem[];
   __shared__ float2 xch[2][RPB][WPR];
@@ -584,7 +584,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kLnStages; ++i) {
       mbar_init(&bars[i], 1);
-      mbar_init(&bars[kLnStages + i], NW);
+      mbar_init(&bars[kLnStages + i], kLnWarps);
     }
     aborted = 0;
     fence_mbar_init();
@@ -593,7 +593,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   const LnRing ring{bars, bars + kLnStages, &aborted};
   float ag[VPL][8], ab[VPL][8];
   const int rslot = warp / WPR, part = warp % WPR;
-  if (warp == NW) {
+  if (warp == kLnWarps) {
     int c = 0;
     for (int ch = blockIdx.x; ch < chunks; ch += gridDim.x, ++c) {
       if (!ring.wait_empty(c)) break;
@@ -727,7 +727,7 @@ ln_bwd_stream_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* 
   // Every copy has landed and been read: the ring takes the sums of the row slots, [2][RPB][H], which are then added in the order
   // 0, 1, ...  (One slot after the other into one row of sums took eight rounds at one warp per row: 16 x 512 9.5 us instead of 5.5.)
   float* slots = reinterpret_cast<float*>(ring_smem);
-  if (warp < NW) {
+  if (warp < kLnWarps) {
 #pragma unroll
     for (int i = 0; i < VPL; ++i) {
       const int v = (part * VPL + i) * 32 + lane;
