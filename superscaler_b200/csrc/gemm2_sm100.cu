@@ -47,7 +47,9 @@ constexpr int BK2 = 64;
 constexpr int kStagesPlain = 5;
 constexpr int kStagesGather = 4;                 // one stage (32 KB) becomes the pusher's staging area
 constexpr int kStagesWide = 4;                   // of 48 KB
-constexpr int kSwitchGroup = 2;                  // wide tile: K blocks at both ends of a tile that are taken half by half
+// wide tile: K blocks at both ends of a tile that are taken half by half; with one, sustained, 8192 x 2048 over 8192 226.1 -> 227.3 us, fp32
+// over 16384 456 -> 460
+constexpr int kSwitchGroup = 2;
 constexpr int kPushChunk2 = 16384;
 constexpr int kEpiWarps = 16;
 constexpr int kThreads2 = 64 + kEpiWarps * 32;
@@ -715,10 +717,11 @@ int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap
 }
 
 // The tile of 256 x 512 takes a product with a long reduction, where its end (the next tile waits for the epilogue) weighs little,
-// and where counting in whole rounds of 256 columns costs nothing.  us alone / sustained under the power cap, 256 -> 512 columns:
-// 8192 x 2048 bf16 over 4096: 109 -> 117 / 116 -> 119; 6144: 155 -> 160 / 175 -> 172; 8192: 204 -> 204 / 234 -> 225; 12288: 301 -> 291 /
-// 349 -> 330; 4096 x 2048 over 51200: 594 -> 568 / 708 -> 652.  fp32, added to: over 8192 210 -> 224 / 251 -> 246; 16384: 403 -> 416 /
-// 481 -> 455; 32768: 804 -> 751 / 944 -> 875.
+// and where counting in whole rounds of 256 columns costs nothing.  us of a single call / sustained under the power cap, 256 -> 512
+// columns, 8192 x 2048 in bf16: over 4096 109 -> 117 / 116 -> 119; 6144 155 -> 160 / 175 -> 172; 8192 207 -> 210 / 235 -> 226; 10240 252 -> 253;
+// 12288 303 -> 292 / 349 -> 330.  Over 8192, the first length taken, a single call is slower (4096 x 2048 113 -> 116, 2048 x 8192 203 -> 209)
+// and a loop faster (119 -> 114, 231 -> 228); training is loops.  4096 x 2048 over 51200 594 -> 568 / 708 -> 652.  fp32, added to: over 8192
+// 210 -> 224 / 251 -> 246; 16384 406 -> 401 / 485 -> 457, 4096 x 2048 208 -> 210 / 243 -> 226; 32768 818 -> 755 / 956 -> 883.
 constexpr int kWideK = 8192, kWideKFp32 = 16384;
 bool wide_tile(int M, int N, int K, bool out_fp32, int num_sms) {
   const long long m = (M + 255LL) / 256, narrow = m * ((N + 255LL) / 256), wide = m * ((N + 511LL) / 512);
