@@ -739,18 +739,21 @@ bool wide_tile(int M, int N, int K, bool out_fp32, int num_sms) {
 //   not taken  8192 x 2560 over 2048 72.7 -> 76.8 / 75.8 -> 79.8 (160: seven rounds for five), 16384 x 1536 MN-major over 4096 216 -> 194 /
 //              174 -> 178 (192: seven for six), 2048 x 8192 MN-major fp32 over 4096 136 -> 116 / 130 -> 134 (224: more tiles, no padding)
 //   short      reductions end before a tile's epilogue does: 4096 x 5120 over 512 28.6 -> 29.1 sustained, 2048 x 10240 28.7 -> 29.3
-//   off lines  rows off 128 bytes cost the narrower tile of an MN-major B more than it saves: 3064 x 1984 over 4096 57.4 -> 65.3 (192),
-//              with 3072 rows 54.3 -> 53.1
-// 16 x 28 x 28 of 640 channels, 3 x 3, 256 -> 224: forward 67.6 -> 62.0, input gradient 68.5 -> 64.4.
-int tile_columns(int M, int N, int K, bool b_mn, bool whole_lines, int num_sms) {
-  if (b_mn && !whole_lines) return BN2;
+// `more_tiles`: whether there may be more tiles than of 256 columns.  Rows off 128 bytes and an MN-major B: more tiles cost more than
+// they save (3064 x 1984 over 4096 57.4 -> 65.3 with 192 columns, 3072 rows 54.3 -> 53.1); of a product as many do, too (12536 x 640 fp32
+// over 4096 73.5 -> 77.9), of an input gradient they do not (3 x 3, 16 x 56 x 56 of 272 channels 120 -> 112 / 113 -> 97.5 with 160, 8 x 56 x
+// 56 of 560 165 -> 144 / 144 -> 130, 64 x 28 x 28 of 264 133 -> 144 / 142 -> 133), and more do not inside one round (4 x 28 x 28 of 784
+// 56.3 -> 48.1 / 47.1 -> 42.9; two rounds: 4 x 56 x 56 of 392 67.6 -> 70.6 / 61.4 -> 65.6).
+// Convolutions 3 x 3: 16 x 28 x 28 of 640 channels, 224 columns, forward 67.6 -> 62.0, input gradient 68.5 -> 64.4; forward of 16 x 56 x 56
+// of 320, 160 columns, 124 -> 85 / 104 -> 82, of 64 x 28 x 28 of 392, 224 columns, 200 -> 194 / 190 -> 183 (160: 218 / 205).
+int tile_columns(int M, int N, int K, bool b_mn, bool more_tiles, int num_sms) {
   const long long pairs = num_sms / 2, m = (M + 255LL) / 256;
   auto n = [&](int bn) { return (N + bn - 1LL) / bn; };
   auto rounds = [&](int bn) { return (m * n(bn) + pairs - 1) / pairs; };
   auto cost = [&](int bn) { return rounds(bn) * (bn + (b_mn ? 2 * BN2 : BN2)); };
   int best = BN2;
   for (int bn = BN2 - 32; bn >= 160; bn -= 32)
-    if (cost(bn) < cost(best)) best = bn;
+    if (cost(bn) < cost(best) && (more_tiles || n(bn) == n(BN2))) best = bn;
   const bool less_padding = 10 * n(best) * best <= 9 * n(BN2) * BN2;
   const int percent = K < 1024 && rounds(BN2) > 2 ? 90 : !b_mn ? 95 : less_padding ? 96 : 93;
   return 100 * cost(best) <= percent * cost(BN2) ? best : BN2;
@@ -772,7 +775,7 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
   }
   if (rc != 0) return rc;
   const bool wide = !GATHER && wide_tile(p.M, p.N, p.K, p.out_fp32, num_sms);
-  const int bn = GATHER || wide ? BN2 : tile_columns(p.M, p.N, p.K, B_MN, whole_lines(lda, ldb), num_sms);
+  const int bn = GATHER || wide || (B_MN && !whole_lines(lda, ldb)) ? BN2 : tile_columns(p.M, p.N, p.K, B_MN, true, num_sms);
   rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, bn / 2, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
   if (rc != 0) return rc;
   if constexpr (!GATHER)
@@ -784,7 +787,8 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
 
 // Columns of the output tile for a product that this kernel takes.
 int gemm2_tile_columns(int M, int N, int K, bool b_mn, bool whole_lines, bool out_fp32, int num_sms) {
-  return wide_tile(M, N, K, out_fp32, num_sms) ? 2 * BN2 : tile_columns(M, N, K, b_mn, whole_lines, num_sms);
+  if (wide_tile(M, N, K, out_fp32, num_sms)) return 2 * BN2;
+  return b_mn && !whole_lines ? BN2 : tile_columns(M, N, K, b_mn, true, num_sms);
 }
 
 // Same contract as gemm_bf16_launch; callers pick this variant for outputs of at least 256 x 256.
@@ -837,7 +841,8 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
   if ((rc = make_tma_im2col_bf16(&ta, dy, N, Ho, Wo, Kout, lh, lw, -pad, -pad, 1, BM2))) return rc;
   if ((rc = make_tma_2d_bf16(&tb, w, Kout, static_cast<uint64_t>(KH) * KW * C, ldw, BK2, 64))) return rc;
   ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
-  const int bn = tile_columns(p.M, p.N, p.K, true, whole_lines(Kout, ldw), num_sms);
+  const bool one_round = (p.M + 255LL) / 256 * ((p.N + 255LL) / 256) <= num_sms / 2;
+  const int bn = tile_columns(p.M, p.N, p.K, true, whole_lines(Kout, ldw) || one_round, num_sms);
   return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
 }
 

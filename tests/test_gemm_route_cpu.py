@@ -73,7 +73,7 @@ def test_the_faster_kernel_takes_the_call(M, N, K, call, one_cta, cluster):
     # a reduction that ends before the epilogue does, over several rounds
     (4096, 5120, 512, False, True, 256), (2048, 10240, 512, False, True, 256),
     # operands whose rows start off 128 bytes
-    (2560, 4096, 4096, True, False, 256), (2560, 2048, 4096, False, False, 160),
+    (2560, 4096, 4096, True, False, 256), (2560, 2048, 4096, False, False, 160), (12536, 640, 4096, True, False, 256),
 ])
 def test_columns_of_a_tile_on_pairs(M, N, K, b_mn, lines, columns):
     """Narrower tiles only where they are the faster ones, also under the power cap (times in csrc/gemm2_sm100.cu)."""
