@@ -182,10 +182,14 @@ __device__ __forceinline__ TileCoord2 tile_coord2(int tile, int num_m, int num_n
 //           input gradient (A = output gradient, taps flipped, B = filter read MN-major).  A channel block that reaches past C
 //           is zero-filled, so what the filter's block holds there (the next tap) does not matter.
 //   kConvB: filter gradient; the reduction runs over the pixels, B's columns are (tap, channel), C a multiple of 64.
-template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
+// NARROW: a tile of `columns`, else of 256 (9472 x 512 over 64 8.1 -> 7.9 us with the width known to the compiler).
+// FP32: the staged epilogue of fp32 outputs, else that of bf16 outputs; what does not fit either goes by chunks.  With both in one kernel
+// bf16 outputs took longer, the same products 7.9 instead of 7.6 us.
+template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH, bool NARROW, bool FP32>
 __global__ void __launch_bounds__(GATHER ? kThreadsGather : kThreads2, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_a2,
-                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv, const int bn) {
+                  const __grid_constant__ CUtensorMap tma_b, const GemmParams p, const GemmAgComm cm, const ConvLoad cv, const int columns) {
+  const int bn = NARROW ? columns : BN2;            // of an accumulator
   constexpr int kStages2 = NH == 2 ? kStagesWide : GATHER ? kStagesGather : kStagesPlain;
   const int BNT = NH == 2 ? 2 * BN2 : bn;           // columns of a tile
   constexpr int kStageAll = kABytes2 + NH * kBBytes2;
@@ -455,7 +459,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         // Row operands enter and results leave through a swizzled staging tile, so every global access of the warp is four
         // full 128-byte row segments (wide tile: eight of 64 bytes) instead of 32 scattered 32-byte pieces.
         const bool has_operand = p.residual != nullptr || p.act == kActDGelu || p.act == kActDRelu;
-        const bool staged = !p.out_fp32 && !p.accumulate && col0 + 64 <= col_end &&
+        const bool staged = !FP32 && !p.out_fp32 && !p.accumulate && col0 + 64 <= col_end &&
                             !(p.residual != nullptr && (p.act == kActDGelu || p.act == kActDRelu)) &&
                             !(p.preact_out != nullptr && has_operand);
         if (staged) {
@@ -536,7 +540,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         // in turn; with a reduction of 4096 that took longer than the main loop of the next tile.  Alone / sustained under the
         // power cap: weight gradients 51200 x 2048 over 4096 rows 649 -> 600 / 805 -> 754 us, 8192 x 2048 over 8192 216 -> 209 /
         // 255 -> 248.
-        if (p.out_fp32 && col0 + 64 <= col_end && !has_operand && p.preact_out == nullptr) {
+        if (FP32 && p.out_fp32 && col0 + 64 <= col_end && !has_operand && p.preact_out == nullptr) {
           const int srow = lane >> 2, spiece = lane & 3;
           float* out = reinterpret_cast<float*>(p.D) + static_cast<size_t>(row0 + srow) * p.ldd + col0 + spiece * 4;
           auto cell = [&](int rr, int piece) { return stg + rr * 64 + ((piece ^ ((rr >> 1) & 3)) << 4); };
@@ -672,10 +676,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   }
 }
 
-template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH>
+template <bool A_MN, bool B_MN, bool GATHER, int CONV, int NH, bool NARROW, bool FP32>
 int launch_maps(const CUtensorMap& ta, const CUtensorMap& ta2, const CUtensorMap& tb, const GemmParams& p,
                 const GemmAgComm& cm, const ConvLoad& cv, int bn, int num_sms, cudaStream_t stream) {
-  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV, NH>;
+  auto kernel = gemm2_bf16_kernel<A_MN, B_MN, GATHER, CONV, NH, NARROW, FP32>;
   constexpr int threads = GATHER ? kThreadsGather : kThreads2;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -778,9 +782,18 @@ int launch_pair(const void* A, int lda, const void* B, int ldb, const GemmParams
   const int bn = GATHER || wide || (B_MN && !whole_lines(lda, ldb)) ? BN2 : tile_columns(p.M, p.N, p.K, B_MN, true, num_sms);
   rc = !B_MN ? make_tma_2d_bf16(&tb, B, p.N, p.K, ldb, bn / 2, BK2) : make_tma_2d_bf16(&tb, B, p.K, p.N, ldb, BK2, 64);
   if (rc != 0) return rc;
-  if constexpr (!GATHER)
-    if (wide) return launch_maps<A_MN, B_MN, false, kConvNone, 2>(ta, ta2, tb, p, cm, ConvLoad{}, bn, num_sms, stream);
-  return launch_maps<A_MN, B_MN, GATHER, kConvNone, 1>(ta, ta2, tb, p, cm, ConvLoad{}, bn, num_sms, stream);
+  auto launch = [&](auto kernel_for) { return kernel_for(ta, ta2, tb, p, cm, ConvLoad{}, bn, num_sms, stream); };
+  if constexpr (GATHER) {
+    return launch(launch_maps<A_MN, B_MN, true, kConvNone, 1, false, false>);
+  } else if (p.out_fp32) {
+    if (wide) return launch(launch_maps<A_MN, B_MN, false, kConvNone, 2, false, true>);
+    if (bn != BN2) return launch(launch_maps<A_MN, B_MN, false, kConvNone, 1, true, true>);
+    return launch(launch_maps<A_MN, B_MN, false, kConvNone, 1, false, true>);
+  } else {
+    if (wide) return launch(launch_maps<A_MN, B_MN, false, kConvNone, 2, false, false>);
+    if (bn != BN2) return launch(launch_maps<A_MN, B_MN, false, kConvNone, 1, true, false>);
+    return launch(launch_maps<A_MN, B_MN, false, kConvNone, 1, false, false>);
+  }
 }
 
 }  // namespace
@@ -828,7 +841,8 @@ int conv_fprop_launch(const void* x, int N, int H, int W, int C, const void* w, 
   const int bn = tile_columns(p.M, p.N, p.K, false, true, num_sms);
   if ((rc = make_tma_2d_bf16(&tb, w, p.N, p.K, ldw, bn / 2, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<false, false, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
+  auto launch = bn == BN2 ? launch_maps<false, false, false, kConvA, 1, false, false> : launch_maps<false, false, false, kConvA, 1, true, false>;
+  return launch(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
 }
 
 // dx[N, H, W, C] of a stride-1 convolution from dy[N, Ho, Wo, K]; p describes the GEMM [N H W, C] with K = KH * KW * K.
@@ -843,7 +857,8 @@ int conv_dgrad_launch(const void* dy, int N, int H, int W, int Kout, const void*
   ConvLoad cv{Kout, KH, KW, 1, lh, lw, H, W, 1, C};
   const bool one_round = (p.M + 255LL) / 256 * ((p.N + 255LL) / 256) <= num_sms / 2;
   const int bn = tile_columns(p.M, p.N, p.K, true, whole_lines(Kout, ldw) || one_round, num_sms);
-  return launch_maps<false, true, false, kConvA, 1>(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
+  auto launch = bn == BN2 ? launch_maps<false, true, false, kConvA, 1, false, false> : launch_maps<false, true, false, kConvA, 1, true, false>;
+  return launch(ta, ta, tb, p, GemmAgComm{}, cv, bn, num_sms, stream);
 }
 
 // dw[K, KH * KW * C] from dy[N Ho Wo, K] and x; p describes the GEMM [K, KH * KW * C] with K = N Ho Wo.
@@ -854,7 +869,7 @@ int conv_wgrad_launch(const void* dy, int lddy, const void* x, int N, int H, int
   if ((rc = make_tma_2d_bf16(&ta, dy, p.K, p.M, lddy, BK2, 64))) return rc;
   if ((rc = make_tma_im2col_bf16(&tb, x, N, H, W, C, -pad, -pad, pad - (KH - 1), pad - (KW - 1), stride, BK2))) return rc;
   ConvLoad cv{C, KH, KW, stride, -pad, -pad, (H + 2 * pad - KH) / stride + 1, (W + 2 * pad - KW) / stride + 1, 0, C};
-  return launch_maps<true, true, false, kConvB, 1>(ta, ta, tb, p, GemmAgComm{}, cv, BN2, num_sms, stream);
+  return launch_maps<true, true, false, kConvB, 1, false, true>(ta, ta, tb, p, GemmAgComm{}, cv, BN2, num_sms, stream);
 }
 
 }  // namespace ssb
