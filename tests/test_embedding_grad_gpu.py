@@ -58,7 +58,7 @@ def test_no_row_of_the_table_occurs():
         native.ext().embedding_bwd_grouped(ids[:0], None, g[:0], dW, None, 0, 0.0, 0)
 
 
-@pytest.mark.parametrize("H", [8, 264, 2040, 2048, 2056, 2560, 4104])          # one pass of 32 .. 256 threads, two, three
+@pytest.mark.parametrize("H", [8, 16, 64, 120, 200, 264, 2040, 2048, 2056, 2560, 4104])   # 1 to 256 threads a token, two, three passes
 @pytest.mark.parametrize("tokens", [1, 887, 889, 2500])                         # around a token for every block; further rounds
 @pytest.mark.parametrize("places", [False, True])
 def test_lookup(H, tokens, places):
@@ -90,7 +90,7 @@ def test_tables_of_no_columns(places):
     assert native.check_status() == 0
 
 
-@pytest.mark.parametrize("H", [8, 264, 2048, 2056, 4104])                       # several tokens a block, one pass, two, three
+@pytest.mark.parametrize("H", [8, 64, 264, 2048, 2056, 4104])                   # several tokens a block, one pass, two, three
 @pytest.mark.parametrize("tokens", [1, 889, 2500])
 @pytest.mark.parametrize("p", [0.1, 0.996])
 def test_lookup_dropout(H, tokens, p):
