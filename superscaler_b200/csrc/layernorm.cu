@@ -847,11 +847,13 @@ void fold_partials2(const float* part_g, const float* part_b, float* dgamma, flo
 // partials of all slices, every warp an eighth of them and then the eight sums in order, so the result does not depend on which
 // block that is.  The counters are shared by all calls on a device: calls must be ordered on one stream.
 //
-// As many slices as give every SM kColsumBlocks blocks, of 64 rows at least: with a slice per 256 rows and a thread that added the
-// partials of a column one after the other, before -> now: 8192 x 8192 31.8 -> 23.9 us, 32768 x 6144 75.0 -> 61.3 (6.6 TB/s), 32768 x 2048
-// 35.7 -> 26.3, 512 x 512 6.6 -> 4.1.  Short ones wait for loads, the partials and the ticket, one after the other.
-constexpr int kColsumBlocks = 6, kColsumMaxSlices = 128, kColsumMinRows = 64;
-__global__ void __launch_bounds__(256, kColsumBlocks)
+// As many slices as give every SM kColsumBlocks blocks, but no more than colsum_slices: with a slice per 256 rows and a thread that added
+// the partials of a column one after the other, before -> now: 8192 x 8192 31.8 -> 23.9 us, 32768 x 6144 75.0 -> 61.3 (6.6 TB/s), 32768 x
+// 2048 35.7 -> 25.6, 512 x 512 6.6 -> 4.1.  Short ones wait for loads, the partials and the ticket, one after the other; with the matrix
+// still in the L2: 8192 x 2048 8.8 -> 8.1 in 64 slices (9.6 in 111), 4096 x 4096 8.0 -> 7.4 with four blocks an SM (8.4 with six),
+// 8192 x 3072 9.2 -> 8.8 (9.7); from memory 32768 x 768 19.4 -> 15.6 in 128 slices (17.6 in 64).
+constexpr int kColsumBlocks = 4, kColsumMaxSlices = 128;
+__global__ void __launch_bounds__(256, 6)
 colsum_onepass_kernel(const __nv_bfloat16* __restrict__ a, int lda, float* __restrict__ part, float* __restrict__ out,
                       int* __restrict__ tickets, int rows, int N, int rows_per_slice, int accumulate) {
   __shared__ __align__(16) float red[8][256];
@@ -1094,10 +1096,16 @@ int layernorm_bwd_launch(const void* dy, const void* x, const float* gamma, cons
   return static_cast<int>(cudaGetLastError());
 }
 
+// Slices that the one-pass column sum takes at most: of 64 rows at least up to 64 of them, of 256 beyond.
+static int colsum_slices(int rows) {
+  const int few = (rows + 63) / 64, many = rows / 256;
+  const int slices = few < 64 ? few : many > 64 ? many : 64;
+  return slices < kColsumMaxSlices ? slices : kColsumMaxSlices;
+}
+
 // Rows of N partial sums that a call of colsum_launch needs as scratch, whichever of its kernels takes it.
 int colsum_part_rows(int rows) {
-  const int most = (rows + kColsumMinRows - 1) / kColsumMinRows, two_pass = ln_bwd_slices(rows);
-  const int one_pass = most < kColsumMaxSlices ? most : kColsumMaxSlices;
+  const int one_pass = colsum_slices(rows), two_pass = ln_bwd_slices(rows);
   return one_pass > two_pass ? one_pass : two_pass;
 }
 
@@ -1112,8 +1120,7 @@ int colsum_launch(const void* a, int lda, float* out, float* part, int* tickets,
   if (N % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15) == 0 && colblocks <= kColsumTickets &&
       tickets != nullptr) {
     int sl = num_sms * kColsumBlocks / colblocks;
-    const int most = (rows + kColsumMinRows - 1) / kColsumMinRows;
-    sl = sl > kColsumMaxSlices ? kColsumMaxSlices : sl;
+    const int most = colsum_slices(rows);
     sl = sl > most ? most : sl;
     sl = sl < 1 ? 1 : sl;
     const int rows_per = rows > sl ? (rows + sl - 1) / sl : 1;
