@@ -263,10 +263,10 @@ __device__ __forceinline__ float2 exp_pair(uint32_t two, float off) {
 // range are 6 us of it.
 constexpr int kCeMaxCols = 56 * 1024;  // 112 KB of shared memory: two rows per SM
 
-// AHEAD: the next four loads of a thread are under way while it works on the last four, in rows of which it has several rounds:
-// 4096 rows x 51200 193 -> 177 us, x 40000 150 -> 134, x 32000 116 -> 106 (eight loads at a time instead: 201, 152, 109; one round
-// is slower for it, x 2048 12.3 -> 13.1).  Few rows, 512 threads (one round up to 16384 columns): 8 x 16000 3.99 -> 4.16, 64 x 16384 4.10 ->
-// 4.19, but 148 x 16000 5.54 -> 5.43, 296 x 16384 8.09 -> 7.78; 8 x 18432 4.41 -> 4.51, 148 x 18432 6.65 -> 6.03, 64 x 32000 6.66 -> 6.13.
+// AHEAD: the next four loads of a thread are under way while it works on the last four.  4096 rows x 51200 191 -> 176 us, x 40000 148 -> 133,
+// x 32000 115 -> 106, x 20480 71 -> 66 (eight loads at a time instead: x 51200 201).  With one round of loads or two it is slower (4096 x 2048
+// 12.3 -> 13.1, x 15000 52.2 -> 53.1), and where the logits are still in the L2: 2048 x 20480 30.6 -> 31.4, 1024 x 20480 16.2 -> 16.9, 400 x
+// 32000 11.9 -> 12.3, 200 x 51200 12.3 -> 12.8; 700 x 32000 18.8 -> 18.5, 1500 x 32000 42.3 -> 38.9.
 template <int T, bool AHEAD>
 __global__ void __launch_bounds__(T, 1024 / T)
 ce_fused_kernel(__nv_bfloat16* __restrict__ logits, int ld, const long long* __restrict__ targets,
@@ -370,9 +370,12 @@ int ce_fused_launch(void* logits, int ld, const long long* targets, const float*
   // threads 9.5).  Rows that all fit on the chip at once are a matter of latency: 16 rows of 8192 take 4.6 us with 128 threads
   // and 3.8 with 512.
   const bool few = rows <= 2LL * num_sms;
-  if (V > 36 * 1024 || (few && (V > 16 * 1024 || (V > 14 * 1024 && rows >= num_sms)))) return launch(ce_fused_kernel<512, true>, 512);
-  if (few) return launch(ce_fused_kernel<512, false>, 512);
-  return V > 14 * 1024 ? launch(ce_fused_kernel<256, true>, 256) : launch(ce_fused_kernel<128, false>, 128);
+  // Loads ahead: where a thread has at least two rounds of them and the logits have left the L2 since the product that made them.
+  const long long bytes = rows * V * 2;
+  const bool ahead = V > 16 * 1024 && bytes > (V > 24 * 1024 ? 40LL << 20 : 96LL << 20);
+  if (few || V > 36 * 1024) return ahead ? launch(ce_fused_kernel<512, true>, 512) : launch(ce_fused_kernel<512, false>, 512);
+  if (V > 14 * 1024) return ahead ? launch(ce_fused_kernel<256, true>, 256) : launch(ce_fused_kernel<256, false>, 256);
+  return launch(ce_fused_kernel<128, false>, 128);
 }
 
 int embedding_fwd_launch(const long long* ids, const long long* pos, const void* W, const void* P, void* out,
