@@ -15,14 +15,15 @@
 namespace ssb {
 namespace {
 
-constexpr int kEmbedBlocks = 6;  // of 256 threads, per SM; more of shorter ones
+constexpr int kEmbedBlocks = 6;  // of 256 threads, per SM; more of the shorter ones that take one token at a time
 
 // A row of threads per token (`tpr`: 1 to 16 in powers of two, or a multiple of 32), the next token's id and position on their way while
 // this one's rows are.  Bounded by the latency of id -> row and by the hashes of the dropout mask.  A thread per eight columns of
 // the whole output, which divided by the row length and read the id as it went, before -> now: 16384 tokens x 2048 of 51200 rows 29.2
-// -> 25.8 us (with dropout 34.0 -> 32.5), of 2048 rows 25.4 -> 19.5, x 2560 33.9 -> 31.4 (36.6 with six blocks of 160 threads), x 64 3.05 -> 2.56
-// (4.2 with 32 threads a token), 512 x 1024 2.6 -> 2.1.  Eight blocks an SM spill (20.3 of 2048 rows); four tokens at a time leave too few
-// threads (53 instead of 37 us, a cold pass with dropout).
+// -> 25.8 us (with dropout 34.0 -> 32.2), of 2048 rows 25.4 -> 19.5, x 64 3.05 -> 2.55 (4.2 with 32 threads a token), x 2560 33.9 -> 31.5 (36.6
+// with six blocks of 160 threads), 512 x 1024 2.6 -> 2.1.  Blocks of 192 threads for two tokens of 768 columns: 8192 tokens 7.7 -> 5.2 with six,
+// 5.3 with eight.  Eight blocks of 256 spill (20.3 of 2048 rows); four tokens at a time leave too few threads (53 instead of 37 us, a
+// cold pass with dropout).
 __global__ void __launch_bounds__(256, kEmbedBlocks)
 embedding_fwd_kernel(const long long* __restrict__ ids, const long long* __restrict__ pos,
                      const __nv_bfloat16* __restrict__ W, const __nv_bfloat16* __restrict__ P,
@@ -386,7 +387,7 @@ int embedding_fwd_launch(const long long* ids, const long long* pos, const void*
   const int nvec = H / 8, passes = (nvec + 255) / 256;
   int tpr = ((nvec + passes - 1) / passes + 31) / 32 * 32;
   while (tpr <= 32 && tpr / 2 >= nvec) tpr /= 2;
-  const int slots = 256 / tpr, per_sm = kEmbedBlocks * 256 / (slots * tpr);
+  const int slots = 256 / tpr, per_sm = slots > 1 ? kEmbedBlocks : kEmbedBlocks * 256 / tpr;
   const long long want = (tokens + slots - 1) / slots, most = static_cast<long long>(num_sms) * per_sm;
   const int blocks = static_cast<int>(want < 1 ? 1 : (want > most ? most : want));
   embedding_fwd_kernel<<<blocks, slots * tpr, 0, stream>>>(ids, pos, reinterpret_cast<const __nv_bfloat16*>(W),
