@@ -239,8 +239,8 @@ ln_fwd_parts_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict
 // registers; a warp per row read them from the L1 for every row, and its loads, sums and stores came one after the other
 // (warps an SM and loads in flight were what bounded it: DRAM 47 %, issue slots 35 %).  The warps of a row exchange their sums and sums
 // of squares once per R rows.  Three rows: with four the unpacked values spill (32768 x 2048 57 us), two have less in flight (50.4).
-// Bounded by issue slots: what is done once per row is done by a lane per row, not by every lane for all of them (47.6 -> 45.2, x 1800
-// 46.0 -> 43.3, x 512 12.3 -> 12.0).  Measured, a warp per row -> this: 32768 x 2048 55.7 -> 45.2 us, x 1536 49.1 -> 36.5, 4096 x 2048
+// What is done once per row is done by a lane per row, not by every lane for all of them (issue slots 74 -> 64 % busy, DRAM 50 -> 61 %;
+// 47.6 -> 45.2 us, x 1800 46.0 -> 43.3, x 512 12.3 -> 12.0).  Measured, a warp per row -> this: 32768 x 2048 55.7 -> 45.2 us, x 1536 49.1 -> 36.5, 4096 x 2048
 // 11.6 -> 8.7; a copy takes 42.0, 32.4, 7.3.  32768 x 1024 28.4 -> 24.6, x 896 27.6 -> 23.5, x 1280 36.8 -> 33.6, 8192 x 1024 10.2 -> 9.2.
 // Rows of 513 to 768 columns stay with a warp each (x 640 20.0 -> 20.7, x 768 22.3 -> 22.0: the second warp is idle in part), and so do 4096 x
 // 1024 (6.3 -> 6.6: the last groups have none).
